@@ -325,7 +325,8 @@ extern "C" int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, co
                           int32_t* status, int smem_kb, cudaStream_t stream);
 extern "C" int qs_linear_simt(void* C, int c_dtype, const void* A, int a_dtype, const void* W, int w_dtype,
                               const void* bias, int bias_dtype, int act, const void* res1, const void* res2,
-                              int M, int N, int K, long long lda, long long ldc, long long ldr, cudaStream_t stream);
+                              int M, int N, int K, long long lda, long long ldc, long long ldr, float* ws, long long ws_floats,
+                              cudaStream_t stream);
 
 // One product per expert over its rows, all launched by this one call: C[rows of e] = A[rows of e] W[e]^T with
 // W [E][N][K] and the experts' row ranges `offsets` (E + 1 entries, on the HOST).  `use_tc`: the tensor-core product
@@ -383,7 +384,7 @@ QS_API int qs_expert_products(void* C, int c_dtype, long long ldc, const void* A
                                  ws + (size_t)lane * ws_share, ws_share, counters + (size_t)lane * counter_share, counter_share,
                                  status, 0, st)
                     : qs_linear_simt(c, c_dtype, a, a_dtype, w, w_dtype, nullptr, 0, QS_ACT_NONE, nullptr, nullptr, M, N, K, lda,
-                                     ldc, N, st);
+                                     ldc, N, nullptr, 0, st);
     }
     if (pool)                                           // also after a failed launch: `stream` must not run ahead of the others
         for (int i = 0; i < lanes; ++i) {
@@ -422,7 +423,7 @@ QS_API int qs_head_products(void* C, int c_dtype, long long ldc, long long head_
                                  ws + (size_t)lane * ws_share, ws_share, counters + (size_t)lane * counter_share, counter_share,
                                  status, 0, st)
                     : qs_linear_simt(c, c_dtype, a, a_dtype, w, w_dtype, nullptr, 0, QS_ACT_NONE, nullptr, nullptr, M, N, K, lda,
-                                     ldc, N, st);
+                                     ldc, N, nullptr, 0, st);
     }
     if (pool)
         for (int i = 0; i < lanes; ++i) {

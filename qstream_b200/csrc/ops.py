@@ -8,6 +8,7 @@ loaded, or a tensor is not on a CUDA device, the call raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_double, c_float, c_int, c_longlong, c_uint, c_ulonglong, c_void_p
 
 import torch
@@ -31,7 +32,8 @@ _SIGNATURES = {
     "qs_add": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_void_p], c_int),
     "qs_scale": ([c_void_p, c_longlong, c_float, c_void_p], c_int),
     "qs_linear_simt": ([c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
-                        c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p], c_int),
+                        c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_longlong, c_void_p], c_int),
+    "qs_linear_simt_scratch": ([c_int, c_int, c_int], c_longlong),
     "qs_rope_store": ([c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_longlong,
                        c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                        c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_float, c_int, c_void_p], c_int),
@@ -43,7 +45,7 @@ _SIGNATURES = {
                             c_void_p], c_int),
     "qs_attention": ([c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_int,
                       c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p,
-                      c_int, c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p], c_int),
+                      c_int, c_float, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p], c_int),
     "qs_pair_diff_norm": ([c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_float, c_float,
                            c_float, c_void_p], c_int),
     "qs_delta_prepare": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int,
@@ -277,6 +279,12 @@ def scale(x: torch.Tensor, factor: float) -> torch.Tensor:
     return x
 
 
+@functools.lru_cache(maxsize=4096)
+def _linear_simt_scratch(M: int, N: int, K: int) -> int:
+    """Floats of workspace the product takes for the runs' sums where K is cut over several blocks (0: none)."""
+    return int(library().qs_linear_simt_scratch(M, N, K))
+
+
 def linear_simt(x, weight, bias=None, activation=None, residuals=(), out_dtype=None, out=None) -> torch.Tensor:
     """act(x W^T + bias) + residuals, accumulated in true 32-bit on the CUDA cores."""
     M, K, lda = _rows(x)
@@ -296,10 +304,12 @@ def linear_simt(x, weight, bias=None, activation=None, residuals=(), out_dtype=N
             ldr = r.stride(0)
     if len(residuals) > 2 or (len(residuals) == 2 and res[0].stride(0) != res[1].stride(0)):
         raise QStreamError(QsError.INVALID_INPUT, "linear: at most two residuals of one layout")
+    floats = _linear_simt_scratch(M, N, K)
+    ws = torch.empty((floats,), dtype=torch.float32, device=x.device) if floats else None
     check(library().qs_linear_simt(ptr(out), dtype_code(out), ptr(x), dtype_code(x), ptr(weight),
                                    dtype_code(weight), ptr(bias), dtype_code(bias) if bias is not None else 0,
                                    ACTIVATIONS[activation], ptr(res[0]), ptr(res[1]), M, N, K, lda, out.stride(0), ldr,
-                                   stream()))
+                                   ptr(ws), floats, stream()))
     return out
 
 
@@ -363,15 +373,16 @@ def rope_unit_store(q, k, v, eps, n_heads, n_kv_heads, head_dim, rotary_dim, cos
 
 def attention(q, n_heads, n_kv_heads, head_dim, scale, window, tok_slot, tok_pos, page_table,
               page_tokens, k_cache, v_cache, status, out=None, v_head_dim=None, softcap=0.0, chunk=0, keep_first=0,
-              sink=None, maps=1, out_dtype=None) -> torch.Tensor:
-    """Causal attention of every token over its sequence's cache (generic kernel).  `v_head_dim`: the values'
+              sink=None, maps=1, out_dtype=None, n_seq=0) -> torch.Tensor:
+    """Causal attention of every token over its sequence's cache (generic kernels).  `v_head_dim`: the values'
     head size where it differs from the keys'; `softcap` c > 0: scores become c tanh(s / c) before the softmax.
     A query at position p sees the last `window` keys (window > 0), or the keys of its own chunk of `chunk`
     positions counted from 0 (chunk > 0), else all up to p; with `keep_first` also the sequence's first keep_first
     keys.  `sink` (float32 [n_heads]): exp(sink_h) joins each softmax's denominator without key or value.
     `maps` m > 1: a cached key row holds m keys of head_dim side by side and `n_heads` counts m query heads per
     head, query head j reading key j % m of its key head; all of them read the same values.  `out_dtype`
-    torch.float32: the result in 32-bit whatever the queries' type."""
+    torch.float32: the result in 32-bit whatever the queries' type.  `n_seq`: how many sequences the rows belong to
+    (0: not known); it picks the kernel, not the result."""
     T = q.shape[0]
     if sink is not None and (sink.dtype != torch.float32 or sink.numel() != n_heads or not sink.is_contiguous()):
         raise QStreamError(QsError.INVALID_INPUT, "attention: the sinks must be float32, one per query head")
@@ -383,7 +394,7 @@ def attention(q, n_heads, n_kv_heads, head_dim, scale, window, tok_slot, tok_pos
         _int32(page_table, "page_table"), page_table.shape[1], page_tokens, _int32(tok_slot, "tok_slot"),
         _int32(tok_pos, "tok_pos"), T, n_heads, n_kv_heads, head_dim, float(scale), int(window),
         ptr(status), dv, float(softcap or 0.0), int(chunk), int(keep_first), ptr(sink), int(maps),
-        dtype_code(out), stream()))
+        dtype_code(out), int(n_seq), stream()))
     return out
 
 
