@@ -27,7 +27,7 @@
 // sequence and walks the sequence's tokens of this step in order.  A thread owns RK key rows of two neighbouring
 // columns; the KS threads of a pair of columns are neighbours in a warp and add their parts of o by shuffles, in a
 // fixed order, so a token's result does not depend on the batch or on how the prompt was cut.
-#include "common.cuh"
+#include "scan.cuh"
 
 namespace {
 
@@ -37,18 +37,11 @@ constexpr int TILE = 16;            // tokens staged in shared memory at a time
 
 // Which rows a thread owns: groups of four consecutive rows, dealt to the KS threads of a column in turn, so that
 // the threads' 16-byte accesses to a column of the state and to a token's q and k lie side by side.
-__device__ __forceinline__ float log_sigmoid_f32(float z) { return z >= 0.f ? -log1pf(expf(-z)) : z - log1pf(expf(z)); }
-
 __device__ __forceinline__ int row_of(int ks, int ks_log2, int r) { return 4 * (ks + ((r >> 2) << ks_log2)) + (r & 3); }
 
-// PHASE 0: a sequence's tokens in order from the state its slot holds, which is written back at the end.
-// A long prompt is cut into chunks that run side by side, in three steps whose sums are 32-bit throughout:
-// PHASE 1: every chunk by itself from a zero state (its own part of every o, and the state it adds); then
-//          `chunk_prefix_kernel` walks each sequence's chunks, replacing each chunk's added state by the state
-//          the chunk starts from and leaving the sequence's last state in its slot;
-// PHASE 3: every chunk adds to its tokens' o what the state it started from contributes, decayed up to each token.
-// For phases 1 and 3 a "sequence" of the kernel is a chunk and its "slot" the chunk's place in the scratch.
-template <typename TI, int MODE, int PHASE>
+// A sequence's tokens in order from the state its slot holds, which is written back at the end.  A long prompt is cut into
+// chunks that run side by side as matrix products (scan_chunks.cu).
+template <typename TI, int MODE>
 __global__ void __launch_bounds__(256, 2)
 state_scan_kernel(float* __restrict__ o, size_t ldo,
                   const TI* __restrict__ q, size_t ldq, const TI* __restrict__ k, size_t ldk,
@@ -66,8 +59,7 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
     float* sk = sq + TILE * dkp;                        // [TILE][dkp]
     float* sw = sk + TILE * dkp;                        // [TILE][dkp]   (WKV only)
     float* sv = sw + (WKV || DELTA || GLA ? TILE * dkp : 0);   // [TILE][cols]
-    float* carry = sv + TILE * cols;                    // [dkp]         (PHASE 3: the decay from the chunk's start on)
-    float* sa = carry + dkp;                            // [TILE]        (GATED: the tokens' decays)
+    float* sa = sv + TILE * cols;                       // [TILE]        (GATED: the tokens' decays)
     const int dvv = ONES ? dv - 1 : dv;                 // columns that v holds per head: the gated form adds one of ones
     grid_dep_launch();
     grid_dep_wait();
@@ -76,14 +68,14 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
     const int n_cols = min(cols, dv - col0);
     const int tid = threadIdx.x;
     // rows of the packed batch beyond the last sequence belong to nobody: give them a defined value
-    if (PHASE != 3 && s == 0 && (!DELTA || o)) {
+    if (s == 0 && (!DELTA || o)) {
         for (int t = seq_start[n_seq]; t < T_rows; ++t)
             for (int c = tid; c < n_cols; c += blockDim.x) o[(size_t)t * ldo + h * dv + col0 + c] = 0.f;
     }
     const int slot = seq_slot[s];
     const int t0 = seq_start[s], t1 = seq_start[s + 1];
     if (slot < 0) {
-        if (PHASE != 3 && (!DELTA || o))
+        if (!DELTA || o)
             for (int t = t0; t < t1; ++t)
                 for (int c = tid; c < n_cols; c += blockDim.x) o[(size_t)t * ldo + h * dv + col0 + c] = 0.f;
         return;
@@ -99,86 +91,69 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
     for (int r4 = 0; r4 < RK / 4; ++r4) {
         const int i = row_of(ks, ks_log2, 4 * r4);
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-        if (PHASE != 1) {
-            if (vec) {
-                if (own0 && i < dk) x = *reinterpret_cast<const float4*>(scol0 + i);
-                if (own1 && i < dk) y = *reinterpret_cast<const float4*>(scol1 + i);
-            } else {
-                if (own0) { if (i < dk) x.x = scol0[i]; if (i + 1 < dk) x.y = scol0[i + 1]; if (i + 2 < dk) x.z = scol0[i + 2]; if (i + 3 < dk) x.w = scol0[i + 3]; }
-                if (own1) { if (i < dk) y.x = scol1[i]; if (i + 1 < dk) y.y = scol1[i + 1]; if (i + 2 < dk) y.z = scol1[i + 2]; if (i + 3 < dk) y.w = scol1[i + 3]; }
-            }
+        if (vec) {
+            if (own0 && i < dk) x = *reinterpret_cast<const float4*>(scol0 + i);
+            if (own1 && i < dk) y = *reinterpret_cast<const float4*>(scol1 + i);
+        } else {
+            if (own0) { if (i < dk) x.x = scol0[i]; if (i + 1 < dk) x.y = scol0[i + 1]; if (i + 2 < dk) x.z = scol0[i + 2]; if (i + 3 < dk) x.w = scol0[i + 3]; }
+            if (own1) { if (i < dk) y.x = scol1[i]; if (i + 1 < dk) y.y = scol1[i + 1]; if (i + 2 < dk) y.z = scol1[i + 2]; if (i + 3 < dk) y.w = scol1[i + 3]; }
         }
         S0[4 * r4] = x.x; S0[4 * r4 + 1] = x.y; S0[4 * r4 + 2] = x.z; S0[4 * r4 + 3] = x.w;
         S1[4 * r4] = y.x; S1[4 * r4 + 1] = y.y; S1[4 * r4 + 2] = y.z; S1[4 * r4 + 3] = y.w;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            u[4 * r4 + j] = (WKV && PHASE != 3 && i + j < dk) ? load_as_f32(bonus, bonus_dtype, (size_t)h * dk + i + j) : 0.f;
+            u[4 * r4 + j] = (WKV && i + j < dk) ? load_as_f32(bonus, bonus_dtype, (size_t)h * dk + i + j) : 0.f;
     }
     const float decay = (WKV || GATED || GLA) ? 0.f : head_decay[h];
-    if (PHASE == 3)
-        for (int i = tid; i < dkp; i += blockDim.x) carry[i] = 1.0f;
 
     for (int base = t0; base < t1; base += TILE) {
         const int nt = min(TILE, t1 - base);
         __syncthreads();
-        // a thread stages one key row of the tile's tokens, in order: in PHASE 3 the row's decay since the chunk's
-        // start runs along and q arrives multiplied by it
+        // a thread stages one key row of the tile's tokens, in order
         for (int i = tid; i < dkp; i += blockDim.x) {
             // all of the tile's loads first, so that they are in flight together
             TI qraw[TILE], kraw[TILE];
-            float draw[TILE];                           // GATED: b_t (phases 0, 1) or a_t (phase 3)
+            float draw[TILE];                           // GATED: b_t
 #pragma unroll
             for (int tt = 0; tt < TILE; ++tt) {
                 if (tt < nt && i < dk) {
                     const size_t row = (size_t)(base + tt);
                     qraw[tt] = q[row * ldq + hq * dk + i];
-                    if (PHASE != 3) kraw[tt] = k[row * ldk + hq * dk + i];
+                    kraw[tt] = k[row * ldk + hq * dk + i];
                     if (WKV || DELTA || GLA) draw[tt] = dlog[row * ldd + h * dk + i];
-                    if (GATED) draw[tt] = (PHASE == 3 ? ga : gb)[row * ldg + h];
+                    if (GATED) draw[tt] = gb[row * ldg + h];
                 }
             }
-            float run = PHASE == 3 ? carry[i] : 1.0f;
 #pragma unroll
             for (int tt = 0; tt < TILE; ++tt) {
                 if (tt < nt) {
                     float qv = 0.f, kv = 0.f, wv = 0.f;
                     if (i < dk) {
                         qv = apply_activation(to_f32(qraw[tt]), in_act);
-                        if (PHASE != 3) kv = apply_activation(to_f32(kraw[tt]), in_act);
+                        kv = apply_activation(to_f32(kraw[tt]), in_act);
                         if (WKV) wv = expf(-expf(draw[tt]));
                         if (DELTA) wv = draw[tt];
                         if (GLA) wv = expf(log_sigmoid_f32(draw[tt]) * decay_scale);
                         if (!WKV && !DELTA) qv *= q_scale;      // a constant factor on q (or, the sums being bilinear, on k)
-                        if (GATED && PHASE != 3) kv *= draw[tt];
+                        if (GATED) kv *= draw[tt];
                     }
-                    if (PHASE == 3) {
-                        if (WKV) { qv *= run; run *= wv; }
-                        else if (GLA) { run *= wv; qv *= run; }
-                        else if (SSD) { run = fmaf(run, i < dk ? draw[tt] : 0.f, run); qv *= run; }
-                        else if (GATED) { run *= (i < dk ? draw[tt] : 0.f); qv *= run; }
-                        else { run *= decay; qv *= run; }
-                    } else {
-                        sk[tt * dkp + i] = kv;
-                        if (WKV || DELTA || GLA) sw[tt * dkp + i] = wv;
-                    }
+                    sk[tt * dkp + i] = kv;
+                    if (WKV || DELTA || GLA) sw[tt * dkp + i] = wv;
                     sq[tt * dkp + i] = qv;
                 }
             }
-            if (PHASE == 3) carry[i] = run;
         }
-        if (PHASE != 3) {
-            for (int e = tid; e < nt * cols; e += blockDim.x) {
-                const int tt = e / cols, c = e - tt * cols;
-                sv[e] = (c >= n_cols || (DELTA && !v)) ? 0.f : (ONES && col0 + c == dvv) ? 1.0f
-                        : apply_activation(to_f32(v[(size_t)(base + tt) * ldv + h * dvv + col0 + c]), in_act);
-            }
-            if (GATED && tid < nt) sa[tid] = ga[(size_t)(base + tid) * ldg + h];
-            if (DELTA && tid < nt) sa[tid] = gb[(size_t)(base + tid) * ldg + h];
+        for (int e = tid; e < nt * cols; e += blockDim.x) {
+            const int tt = e / cols, c = e - tt * cols;
+            sv[e] = (c >= n_cols || (DELTA && !v)) ? 0.f : (ONES && col0 + c == dvv) ? 1.0f
+                    : apply_activation(to_f32(v[(size_t)(base + tt) * ldv + h * dvv + col0 + c]), in_act);
         }
+        if (GATED && tid < nt) sa[tid] = ga[(size_t)(base + tid) * ldg + h];
+        if (DELTA && tid < nt) sa[tid] = gb[(size_t)(base + tid) * ldg + h];
         __syncthreads();
         for (int tt = 0; tt < nt; ++tt) {
-            const float v0 = (PHASE == 3 || !own0) ? 0.f : sv[tt * cols + CPT * pair];
-            const float v1 = (PHASE == 3 || !own1) ? 0.f : sv[tt * cols + CPT * pair + 1];
+            const float v0 = !own0 ? 0.f : sv[tt * cols + CPT * pair];
+            const float v1 = !own1 ? 0.f : sv[tt * cols + CPT * pair + 1];
             const float4* q4 = reinterpret_cast<const float4*>(sq + tt * dkp) + ks;
             const float4* k4 = reinterpret_cast<const float4*>(sk + tt * dkp) + ks;
             const float4* w4 = reinterpret_cast<const float4*>(sw + tt * dkp) + ks;
@@ -226,38 +201,30 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
             for (int r4 = 0; r4 < RK / 4; ++r4) {
                 const float4 qq = q4[r4 << ks_log2];
                 const float qa[4] = {qq.x, qq.y, qq.z, qq.w};
-                if (PHASE == 3) {
+                const float4 kk = k4[r4 << ks_log2];
+                const float ka[4] = {kk.x, kk.y, kk.z, kk.w};
+                float wa[4] = {0.f, 0.f, 0.f, 0.f};
+                if (WKV || GLA) { const float4 ww = w4[r4 << ks_log2]; wa[0] = ww.x; wa[1] = ww.y; wa[2] = ww.z; wa[3] = ww.w; }
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc0 = fmaf(qa[j], S0[r4 * 4 + j], acc0);
-                        acc1 = fmaf(qa[j], S1[r4 * 4 + j], acc1);
-                    }
-                } else {
-                    const float4 kk = k4[r4 << ks_log2];
-                    const float ka[4] = {kk.x, kk.y, kk.z, kk.w};
-                    float wa[4] = {0.f, 0.f, 0.f, 0.f};
-                    if (WKV || GLA) { const float4 ww = w4[r4 << ks_log2]; wa[0] = ww.x; wa[1] = ww.y; wa[2] = ww.z; wa[3] = ww.w; }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int r = r4 * 4 + j;
-                        const float kv0 = ka[j] * v0, kv1 = ka[j] * v1;
-                        if (WKV) {
-                            acc0 = fmaf(qa[j], fmaf(u[r], kv0, S0[r]), acc0);
-                            acc1 = fmaf(qa[j], fmaf(u[r], kv1, S1[r]), acc1);
-                            S0[r] = fmaf(wa[j], S0[r], kv0);
-                            S1[r] = fmaf(wa[j], S1[r], kv1);
-                        } else if (GLA) {
-                            S0[r] = fmaf(wa[j], S0[r], kv0);
-                            S1[r] = fmaf(wa[j], S1[r], kv1);
-                            acc0 = fmaf(qa[j], S0[r], acc0);
-                            acc1 = fmaf(qa[j], S1[r], acc1);
-                        } else {
-                            const float dec = GATED ? sa[tt] : decay;
-                            S0[r] = fmaf(dec, S0[r], SSD ? fmaf(ka[j], v0, S0[r]) : kv0);
-                            S1[r] = fmaf(dec, S1[r], SSD ? fmaf(ka[j], v1, S1[r]) : kv1);
-                            acc0 = fmaf(qa[j], S0[r], acc0);
-                            acc1 = fmaf(qa[j], S1[r], acc1);
-                        }
+                for (int j = 0; j < 4; ++j) {
+                    const int r = r4 * 4 + j;
+                    const float kv0 = ka[j] * v0, kv1 = ka[j] * v1;
+                    if (WKV) {
+                        acc0 = fmaf(qa[j], fmaf(u[r], kv0, S0[r]), acc0);
+                        acc1 = fmaf(qa[j], fmaf(u[r], kv1, S1[r]), acc1);
+                        S0[r] = fmaf(wa[j], S0[r], kv0);
+                        S1[r] = fmaf(wa[j], S1[r], kv1);
+                    } else if (GLA) {
+                        S0[r] = fmaf(wa[j], S0[r], kv0);
+                        S1[r] = fmaf(wa[j], S1[r], kv1);
+                        acc0 = fmaf(qa[j], S0[r], acc0);
+                        acc1 = fmaf(qa[j], S1[r], acc1);
+                    } else {
+                        const float dec = GATED ? sa[tt] : decay;
+                        S0[r] = fmaf(dec, S0[r], SSD ? fmaf(ka[j], v0, S0[r]) : kv0);
+                        S1[r] = fmaf(dec, S1[r], SSD ? fmaf(ka[j], v1, S1[r]) : kv1);
+                        acc0 = fmaf(qa[j], S0[r], acc0);
+                        acc1 = fmaf(qa[j], S1[r], acc1);
                     }
                 }
             }
@@ -267,63 +234,29 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
             }
             }
             if (ks == 0 && (!DELTA || o)) {
-                // PHASE 3 adds to what PHASE 1 wrote: this thread is the element's only writer in this kernel, and a
-                // reduction that returns nothing does not make the loop wait for the old value
                 float* dst = o + (size_t)(base + tt) * ldo + h * dv + col0 + CPT * pair;
-                if (own0) { if (PHASE == 3) atomicAdd(dst, acc0); else dst[0] = acc0; }
-                if (own1) { if (PHASE == 3) atomicAdd(dst + 1, acc1); else dst[1] = acc1; }
+                if (own0) dst[0] = acc0;
+                if (own1) dst[1] = acc1;
             }
         }
     }
-    if (PHASE != 3) {
 #pragma unroll
-        for (int r4 = 0; r4 < RK / 4; ++r4) {
-            const int i = row_of(ks, ks_log2, 4 * r4);
-            if (vec) {
-                if (own0 && i < dk) *reinterpret_cast<float4*>(scol0 + i) = make_float4(S0[4 * r4], S0[4 * r4 + 1], S0[4 * r4 + 2], S0[4 * r4 + 3]);
-                if (own1 && i < dk) *reinterpret_cast<float4*>(scol1 + i) = make_float4(S1[4 * r4], S1[4 * r4 + 1], S1[4 * r4 + 2], S1[4 * r4 + 3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (own0 && i + j < dk) scol0[i + j] = S0[4 * r4 + j];
-                    if (own1 && i + j < dk) scol1[i + j] = S1[4 * r4 + j];
-                }
-            }
-        }
-    }
-}
-
-// The decay of every key channel over a whole chunk: exp(-sum_t exp(dlog[t])) (the product of the tokens' decays),
-// the product of sigmoid(dlog[t])^sigmoid_power where that power is given,
-// or decay_h ^ tokens for a fixed decay per head.  chunk_decay [chunks][H * dk].
-__global__ void chunk_decay_kernel(float* __restrict__ chunk_decay, const float* __restrict__ dlog, size_t ldd,
-                                   const float* __restrict__ head_decay, const int32_t* __restrict__ chunk_start,
-                                   int n, int dk, const float* __restrict__ ga, size_t ldg, float sigmoid_power,
-                                   int less_one) {
-    const int c = blockIdx.x;
-    const int t0 = chunk_start[c], t1 = chunk_start[c + 1];
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x) {
-        float a;
-        if (dlog && sigmoid_power > 0.f) {              // w = sigmoid(z)^power per token: the product, token by token
-            a = 1.0f;
-            for (int t = t0; t < t1; ++t) a *= expf(log_sigmoid_f32(dlog[(size_t)t * ldd + i]) * sigmoid_power);
-        } else if (dlog) {
-            float sum = 0.f;
-            for (int t = t0; t < t1; ++t) sum += expf(dlog[(size_t)t * ldd + i]);
-            a = expf(-sum);
-        } else if (ga) {                                // a decay per token and head: their product in order
-            a = 1.0f;
-            for (int t = t0; t < t1; ++t) a = less_one ? fmaf(a, ga[(size_t)t * ldg + i / dk], a) : a * ga[(size_t)t * ldg + i / dk];
+    for (int r4 = 0; r4 < RK / 4; ++r4) {
+        const int i = row_of(ks, ks_log2, 4 * r4);
+        if (vec) {
+            if (own0 && i < dk) *reinterpret_cast<float4*>(scol0 + i) = make_float4(S0[4 * r4], S0[4 * r4 + 1], S0[4 * r4 + 2], S0[4 * r4 + 3]);
+            if (own1 && i < dk) *reinterpret_cast<float4*>(scol1 + i) = make_float4(S1[4 * r4], S1[4 * r4 + 1], S1[4 * r4 + 2], S1[4 * r4 + 3]);
         } else {
-            a = 1.0f;
-            const float d = head_decay[i / dk];
-            for (int t = t0; t < t1; ++t) a *= d;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (own0 && i + j < dk) scol0[i + j] = S0[4 * r4 + j];
+                if (own1 && i + j < dk) scol1[i + j] = S1[4 * r4 + j];
+            }
         }
-        chunk_decay[(size_t)c * n + i] = a;
     }
 }
 
-// Walk each sequence's chunks in order: chunk_state[c] (what chunk c adds, from PHASE 1) becomes the state that
+// Walk each sequence's chunks in order: chunk_state[c] (what chunk c adds) becomes the state that
 // chunk c starts from; the state after the last chunk goes to the sequence's slot.  One thread per state element
 // [h][j][i]; the decay belongs to (h, i).
 __global__ void chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
@@ -453,7 +386,7 @@ delta_chunk_prefix_kernel(const float* __restrict__ P, const float* __restrict__
 }
 
 template <typename TI>
-int launch_scan(int mode, int phase, float* o, long long ldo, const void* q, long long ldq, const void* k, long long ldk,
+int launch_scan(int mode, float* o, long long ldo, const void* q, long long ldq, const void* k, long long ldk,
                 const void* v, long long ldv, const float* dlog, long long ldd, const float* head_decay, const void* bonus,
                 int bonus_dtype, float* state, long long slot_stride, const int32_t* seq_start, const int32_t* seq_slot,
                 int n_seq, int T_rows, int H, int dk, int dv, int in_act, const float* ga, const float* gb, long long ldg,
@@ -472,22 +405,22 @@ int launch_scan(int mode, int phase, float* o, long long ldo, const void* q, lon
         cols = (cols / 2 + CPT - 1) / CPT * CPT;       // whole pairs of columns, also for an odd count
     const int threads = ((cols / CPT * KS + 31) / 32) * 32;
     const int dkp = KS * RK;
-    const size_t smem = ((size_t)TILE * ((wkv ? 3 : 2) * dkp + cols) + dkp + TILE) * sizeof(float);
+    const size_t smem = ((size_t)TILE * ((wkv ? 3 : 2) * dkp + cols) + TILE) * sizeof(float);
     const int vec = dk % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state % 16) == 0;
     dim3 grid(n_seq, H, (dv + cols - 1) / cols);
     cudaError_t e;
-#define GO(MODE, PHASE) do { e = smem > 48 * 1024 ? cudaFuncSetAttribute(state_scan_kernel<TI, MODE, PHASE>, \
+#define GO(MODE) do { e = smem > 48 * 1024 ? cudaFuncSetAttribute(state_scan_kernel<TI, MODE>, \
             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess; \
-    if (e == cudaSuccess) e = qs_launch_dependent(state_scan_kernel<TI, MODE, PHASE>, grid, dim3(threads), smem, stream, o, (size_t)ldo, \
+    if (e == cudaSuccess) e = qs_launch_dependent(state_scan_kernel<TI, MODE>, grid, dim3(threads), smem, stream, o, (size_t)ldo, \
         (const TI*)q, (size_t)ldq, (const TI*)k, (size_t)ldk, (const TI*)v, (size_t)ldv, dlog, (size_t)ldd, head_decay, bonus, \
         bonus_dtype, state, (size_t)slot_stride, seq_start, seq_slot, n_seq, T_rows, H, dk, dv, ks_log2, cols, in_act, vec, \
         ga, gb, (size_t)ldg, q_scale, qk_group, decay_scale); } while (0)
-    if (mode == 3) GO(3, 0);
-    else if (mode == 5) { if (phase == 0) GO(5, 0); else if (phase == 1) GO(5, 1); else GO(5, 3); }
-    else if (mode == 4) { if (phase == 0) GO(4, 0); else if (phase == 1) GO(4, 1); else GO(4, 3); }
-    else if (mode == 1) { if (phase == 0) GO(1, 0); else if (phase == 1) GO(1, 1); else GO(1, 3); }
-    else if (mode == 2) { if (phase == 0) GO(2, 0); else if (phase == 1) GO(2, 1); else GO(2, 3); }
-    else { if (phase == 0) GO(0, 0); else if (phase == 1) GO(0, 1); else GO(0, 3); }
+    if (mode == 3) GO(3);
+    else if (mode == 5) GO(5);
+    else if (mode == 4) GO(4);
+    else if (mode == 1) GO(1);
+    else if (mode == 2) GO(2);
+    else GO(0);
 #undef GO
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "state_scan: %s", cudaGetErrorString(e));
     return qs_check_launch("state_scan");
@@ -748,31 +681,26 @@ QS_API int qs_state_scan(int mode, float* o, long long ldo, const void* q, long 
     if (qk_group < 1) qk_group = 1;
     QS_REQUIRE(mode == 3 || mode == 5 ? H % qk_group == 0 : qk_group == 1, "state_scan: %d heads in groups of %d", H, qk_group);
     QS_REQUIRE(dtype == QS_F32 || dtype == QS_BF16, "state_scan: unknown dtype %d", dtype);
-    const bool wkv = mode == 1 || mode == 4;
-    (void)wkv;
-#define SCAN(PHASE, STATE, STRIDE, STARTS, SLOTS, N) (dtype == QS_F32 \
-        ? launch_scan<float>(mode, PHASE, o, ldo, q, ldq, k, ldk, v, ldv, dlog, ldd, head_decay, bonus, bonus_dtype, STATE, STRIDE, \
-                             STARTS, SLOTS, N, T_rows, H, dk, dv, in_act, ga, gb, ldg, q_scale, qk_group, decay_scale, stream) \
-        : launch_scan<__nv_bfloat16>(mode, PHASE, o, ldo, q, ldq, k, ldk, v, ldv, dlog, ldd, head_decay, bonus, bonus_dtype, STATE, \
-                                     STRIDE, STARTS, SLOTS, N, T_rows, H, dk, dv, in_act, ga, gb, ldg, q_scale, qk_group, decay_scale, stream))
-    if (!chunk_start) return SCAN(0, state, slot_stride, seq_start, seq_slot, n_seq);
+    if (!chunk_start)
+        return dtype == QS_F32
+            ? launch_scan<float>(mode, o, ldo, q, ldq, k, ldk, v, ldv, dlog, ldd, head_decay, bonus, bonus_dtype, state, slot_stride,
+                                 seq_start, seq_slot, n_seq, T_rows, H, dk, dv, in_act, ga, gb, ldg, q_scale, qk_group, decay_scale, stream)
+            : launch_scan<__nv_bfloat16>(mode, o, ldo, q, ldq, k, ldk, v, ldv, dlog, ldd, head_decay, bonus, bonus_dtype, state, slot_stride,
+                                         seq_start, seq_slot, n_seq, T_rows, H, dk, dv, in_act, ga, gb, ldg, q_scale, qk_group, decay_scale, stream);
     QS_REQUIRE(n_chunks > 0 && chunk_ids && seq_chunk && chunk_state && chunk_decay, "state_scan: chunks without their scratch");
-    const long long per_chunk = (long long)H * dv * dk;
-    int rc = SCAN(1, chunk_state, per_chunk, chunk_start, chunk_ids, n_chunks);
+    auto chunks = [&](int outputs) {
+        return qs_scan_chunks(mode, outputs, o, ldo, q, ldq, k, ldk, v, ldv, dtype, dlog, ldd, head_decay, bonus, bonus_dtype, H, dk, dv, in_act,
+                              chunk_start, n_chunks, T_rows, chunk_state, chunk_decay, ga, gb, ldg, q_scale, qk_group, decay_scale, stream);
+    };
+    int rc = chunks(0);
     if (rc != QS_OK) return rc;
-    const int n = H * dk;
-    chunk_decay_kernel<<<dim3(n_chunks, (n + 127) / 128), 128, 0, stream>>>(chunk_decay, wkv ? dlog : nullptr, (size_t)ldd,
-                                                                            head_decay, chunk_start, n, dk,
-                                                                            mode == 2 || mode == 5 ? ga : nullptr, (size_t)ldg,
-                                                                            mode == 4 ? decay_scale : 0.f, mode == 5);
-    if ((rc = qs_check_launch("state_scan chunk decay")) != QS_OK) return rc;
+    const long long per_chunk = (long long)H * dv * dk;
     int by = (int)((per_chunk + 255) / 256);
     if (by > 1024) by = 1024;
     chunk_prefix_kernel<<<dim3(n_seq, by), 256, 0, stream>>>(chunk_state, chunk_decay, state, (size_t)slot_stride, seq_chunk,
                                                               seq_slot, H, dk, dv);
     if ((rc = qs_check_launch("state_scan chunk prefix")) != QS_OK) return rc;
-    return SCAN(3, chunk_state, per_chunk, chunk_start, chunk_ids, n_chunks);
-#undef SCAN
+    return chunks(1);
 }
 
 // See delta_chunk_prefix_kernel.  seq_chunk (n_seq + 1) names each sequence's chunks; a sequence's slot must be a row

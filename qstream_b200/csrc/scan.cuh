@@ -1,0 +1,11 @@
+// Shared by the walk in order (recurrent.cu) and the chunks of long prompts (scan_chunks.cu).
+#pragma once
+
+#include "common.cuh"
+
+__device__ __forceinline__ float log_sigmoid_f32(float z) { return z >= 0.f ? -log1pf(expf(-z)) : z - log1pf(expf(z)); }
+
+int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
+                   int dtype, const float* dlog, long long ldd, const float* head_decay, const void* bonus, int bonus_dtype, int H, int dk, int dv,
+                   int in_act, const int32_t* chunk_start, int n_chunks, int T_rows, float* chunk_state, float* chunk_decay, const float* ga, const float* gb,
+                   long long ldg, float q_scale, int qk_group, float decay_scale, cudaStream_t stream);
