@@ -18,7 +18,7 @@
 // every chunk from an empty state and leaves the state it ends with and the sum of the logarithms of its decays; a
 // prefix kernel walks each sequence's chunks and gives each the state it starts from (the slot the last one); PHASE 2
 // walks every chunk from that state for the outputs.  PHASE 0: a sequence in order, from and to its slot.
-#include "common.cuh"
+#include "group_norm.cuh"
 
 namespace {
 
@@ -660,7 +660,15 @@ QS_API int qs_ssd_output(void* out, long long ldo, const float* o, long long ldi
     QS_REQUIRE(smem <= 200 * 1024, "ssd_output: %d channels above the shared memory of a block", n);
     const int threads = n >= 2048 ? 512 : 128;
     cudaError_t e = cudaSuccess;
-#define GO(T) do { if (smem > 48 * 1024) e = cudaFuncSetAttribute(ssd_output_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    const bool pieces = row_group_norm_takes(n, n / parts, 1) && dv % 8 == 0 && in_pieces((const char*)out, ldo) && in_pieces(o, ldi) &&
+                        in_pieces((const char*)x, ldx) && in_pieces((const char*)z, ldz) && in_pieces((const char*)w, 0);
+#define GO(T) do { \
+    if (pieces) { \
+        e = launch_row_group_norm<float, T, T, true>((T*)out, (size_t)ldo, o, (size_t)ldi, w, w_dtype, (const T*)z, (size_t)ldz, QS_ACT_SILU, rows, n, \
+                                                     n / parts, eps, 1, (const T*)x, (size_t)ldx, D, dv, stream); \
+        break; \
+    } \
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(ssd_output_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     if (e == cudaSuccess) e = qs_launch_dependent(ssd_output_kernel<T>, dim3(rows), dim3(threads), smem, stream, (T*)out, (size_t)ldo, o, (size_t)ldi, \
         (const T*)x, (size_t)ldx, (const T*)z, (size_t)ldz, D, w, w_dtype, n, dv, n / parts, eps); } while (0)
     if (dtype == QS_F32) GO(float);

@@ -18,7 +18,7 @@
 //   keep_last_rows     state[slot] = the last row each sequence brought in this step
 //
 // Every sum is taken in 32-bit in a fixed order (block_sum / warp_sum), whatever the storage types.
-#include "common.cuh"
+#include "group_norm.cuh"
 
 namespace {
 
@@ -380,6 +380,13 @@ __global__ void gated_group_norm_kernel(TO* __restrict__ out, size_t ldo, const 
 template <typename TI, typename TG, typename TO>
 int launch_gated(void* out, long long ldo, const void* o, long long ldi, const void* w, int w_dtype, const void* gate,
                  long long ldg, int gate_act, int rows, int n, int group, float eps, int gate_span, cudaStream_t stream) {
+    if (row_group_norm_takes(n, group, gate_span) && in_pieces(out, ldo) && in_pieces(o, ldi) && (!gate || gate_span > 1 || in_pieces(gate, ldg)) &&
+        in_pieces(w, 0)) {
+        const cudaError_t err = launch_row_group_norm<TI, TG, TO, false>((TO*)out, (size_t)ldo, (const TI*)o, (size_t)ldi, w, w_dtype, (const TG*)gate, (size_t)ldg,
+                                                                         gate_act, rows, n, group, eps, gate_span, nullptr, 0, nullptr, 8, stream);
+        if (err != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "gated_group_norm: %s", cudaGetErrorString(err));
+        return qs_check_launch("gated_group_norm");
+    }
     const int n_groups = group > 0 ? n / group : 1;
     const int threads = n >= 2048 ? 256 : 128;
     cudaError_t e = qs_launch_dependent(gated_group_norm_kernel<TI, TG, TO>, dim3(rows), dim3(threads),
