@@ -103,6 +103,7 @@ _SIGNATURES = {
                             c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p], c_int),
     "qs_head_linear": ([c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int,
                         c_int, c_int, c_void_p], c_int),
+    "qs_scan_activate": ([c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p], c_int),
     "qs_moe_route": ([c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                       c_int, c_float, c_int, c_int, c_int, c_float, c_void_p], c_int),
     "qs_moe_expert_up": ([c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
@@ -596,9 +597,15 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: only the delta rule walks without values")
     chunk_start = chunk_ids = seq_chunk = chunk_state = chunk_decay = None
     n_chunks = 0
+    if chunks is not None and ACTIVATIONS[in_activation] != ACT_NONE:      # once per element: the chunks' kernels read q, k and v several times
+        nk, nv = q.shape[1], v.shape[1]
+        ready = torch.empty((T, 2 * nk + nv), dtype=torch.float32, device=q.device)
+        check(library().qs_scan_activate(ptr(ready), ptr(q), q.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), dtype_code(q), T, nk, nv,
+                                         ACTIVATIONS[in_activation], stream()))
+        q, k, v, in_activation = ready[:, :nk], ready[:, nk:2 * nk], ready[:, 2 * nk:], None
     if chunks is not None:
         chunk_start, chunk_ids, seq_chunk, n_chunks = chunks
-        chunk_state = torch.empty((n_chunks, n_heads * value_dim * key_dim), dtype=torch.float32, device=q.device)
+        chunk_state = torch.empty((n_chunks, n_heads * key_dim * (-(-value_dim // 4) * 4)), dtype=torch.float32, device=q.device)
         chunk_decay = torch.empty((n_chunks, n_heads * key_dim), dtype=torch.float32, device=q.device)
     per_token = token_decay if token_decay is not None else token_weight
     if mode == "gla" and (decay_logits is None or decay_logits.dtype != torch.float32 or not decay_power > 0):

@@ -257,37 +257,54 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
 }
 
 // Walk each sequence's chunks in order: chunk_state[c] (what chunk c adds) becomes the state that
-// chunk c starts from; the state after the last chunk goes to the sequence's slot.  One thread per state element
-// [h][j][i]; the decay belongs to (h, i).
-__global__ void chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
-                                    float* __restrict__ state, size_t slot_stride, const int32_t* __restrict__ seq_chunk,
-                                    const int32_t* __restrict__ seq_slot, int H, int dk, int dv) {
+// chunk c starts from; the state after the last chunk goes to the sequence's slot.  One thread per four value columns of a key
+// channel in the chunks' layout [h][i][dvp]; the decay belongs to (h, i).
+__global__ void __launch_bounds__(256)
+chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
+                    float* __restrict__ state, size_t slot_stride, const int32_t* __restrict__ seq_chunk,
+                    const int32_t* __restrict__ seq_slot, int H, int dk, int dv) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int s = blockIdx.x;
     const int slot = seq_slot[s];
     const int c0 = seq_chunk[s], c1 = seq_chunk[s + 1];
     if (slot < 0 || c1 <= c0) return;
-    const size_t n = (size_t)H * dv * dk;
+    const int fours = (dv + 3) / 4;
+    const size_t n = (size_t)H * dk * fours;            // float4s of a chunk's states
+    float4* const chunks = reinterpret_cast<float4*>(chunk_state);
     constexpr int AHEAD = 8;                            // chunks whose loads are in flight together
     for (size_t e = (size_t)blockIdx.y * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.y * blockDim.x) {
-        const int i = (int)(e % dk), h = (int)(e / ((size_t)dv * dk));
-        const float* dec = chunk_decay + (size_t)h * dk + i;
-        float S = state[(size_t)slot * slot_stride + e];
+        const size_t hi = e / fours;                    // h * dk + i
+        const int j = (int)(e - hi * fours) * 4, i = (int)(hi % dk), h = (int)(hi / dk);
+        float* own = state + (size_t)slot * slot_stride + ((size_t)h * dv + j) * dk + i;
+        float4 S;
+        S.x = own[0];
+        S.y = j + 1 < dv ? own[dk] : 0.f;
+        S.z = j + 2 < dv ? own[2 * (size_t)dk] : 0.f;
+        S.w = j + 3 < dv ? own[3 * (size_t)dk] : 0.f;
         for (int c = c0; c < c1; c += AHEAD) {
-            float added[AHEAD], a[AHEAD];
+            float4 added[AHEAD];
+            float a[AHEAD];
 #pragma unroll
             for (int g = 0; g < AHEAD; ++g) {
-                added[g] = c + g < c1 ? chunk_state[(size_t)(c + g) * n + e] : 0.f;
-                a[g] = c + g < c1 ? dec[(size_t)(c + g) * H * dk] : 1.f;
+                added[g] = c + g < c1 ? chunks[(size_t)(c + g) * n + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+                a[g] = c + g < c1 ? chunk_decay[(size_t)(c + g) * H * dk + hi] : 1.f;
             }
 #pragma unroll
             for (int g = 0; g < AHEAD; ++g) {
                 if (c + g < c1) {
-                    chunk_state[(size_t)(c + g) * n + e] = S;
-                    S = fmaf(a[g], S, added[g]);
+                    chunks[(size_t)(c + g) * n + e] = S;
+                    S.x = fmaf(a[g], S.x, added[g].x);
+                    S.y = fmaf(a[g], S.y, added[g].y);
+                    S.z = fmaf(a[g], S.z, added[g].z);
+                    S.w = fmaf(a[g], S.w, added[g].w);
                 }
             }
         }
-        state[(size_t)slot * slot_stride + e] = S;
+        own[0] = S.x;
+        if (j + 1 < dv) own[dk] = S.y;
+        if (j + 2 < dv) own[2 * (size_t)dk] = S.z;
+        if (j + 3 < dv) own[3 * (size_t)dk] = S.w;
     }
 }
 
@@ -688,17 +705,18 @@ QS_API int qs_state_scan(int mode, float* o, long long ldo, const void* q, long 
             : launch_scan<__nv_bfloat16>(mode, o, ldo, q, ldq, k, ldk, v, ldv, dlog, ldd, head_decay, bonus, bonus_dtype, state, slot_stride,
                                          seq_start, seq_slot, n_seq, T_rows, H, dk, dv, in_act, ga, gb, ldg, q_scale, qk_group, decay_scale, stream);
     QS_REQUIRE(n_chunks > 0 && chunk_ids && seq_chunk && chunk_state && chunk_decay, "state_scan: chunks without their scratch");
+    QS_REQUIRE(((uintptr_t)chunk_state % 16) == 0 && in_act == QS_ACT_NONE, "state_scan: chunks take activated operands and aligned scratch");
     auto chunks = [&](int outputs) {
-        return qs_scan_chunks(mode, outputs, o, ldo, q, ldq, k, ldk, v, ldv, dtype, dlog, ldd, head_decay, bonus, bonus_dtype, H, dk, dv, in_act,
+        return qs_scan_chunks(mode, outputs, o, ldo, q, ldq, k, ldk, v, ldv, dtype, dlog, ldd, head_decay, bonus, bonus_dtype, H, dk, dv,
                               chunk_start, n_chunks, T_rows, chunk_state, chunk_decay, ga, gb, ldg, q_scale, qk_group, decay_scale, stream);
     };
     int rc = chunks(0);
     if (rc != QS_OK) return rc;
-    const long long per_chunk = (long long)H * dv * dk;
-    int by = (int)((per_chunk + 255) / 256);
-    if (by > 1024) by = 1024;
-    chunk_prefix_kernel<<<dim3(n_seq, by), 256, 0, stream>>>(chunk_state, chunk_decay, state, (size_t)slot_stride, seq_chunk,
-                                                              seq_slot, H, dk, dv);
+    const long long work = (long long)H * dk * ((dv + 3) / 4);
+    const int by = (int)((work + 255) / 256 < 1024 ? (work + 255) / 256 : 1024);
+    const cudaError_t e = qs_launch_dependent(chunk_prefix_kernel, dim3(n_seq, by), dim3(256), 0, stream, chunk_state, chunk_decay, state, (size_t)slot_stride,
+                                              seq_chunk, seq_slot, H, dk, dv);
+    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "state_scan chunk prefix: %s", cudaGetErrorString(e));
     if ((rc = qs_check_launch("state_scan chunk prefix")) != QS_OK) return rc;
     return chunks(1);
 }

@@ -13,9 +13,13 @@
 // channel in blocks of 16 tokens, a block's own pairs walked in order, pairs of blocks through the products up to the
 // blocks' common edge.
 //
-// Bound by multiply-add issue with 16-byte shared-memory reads beside it.  The walk with a state column pair per thread that
-// stood here before spent three operands from shared memory and a shuffle round per token and column pair:
-// MEASURED_LINES
+// Bound by instruction issue at 12 to 16 warps per SM: multiply-adds (two per instruction) with 16-byte shared-memory reads beside
+// them.  What mattered after the walk was replaced: fetches of a whole slice under way at once (the next slice's while the present one is
+// multiplied), and an activation once per element instead of once per kernel.  On the tensor cores as split 11-bit products the sums,
+// which the unit truncates, were two times further from 64 bits than the walk, at the same speed: not taken.
+// Microseconds of the whole mixer (walk | chunks, serial fetches | now): decay per head, 4,096 tokens, 16 heads of 128 x 128: 949 |
+// 600 | 422; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 329; state-space form, 2,048 tokens, 64 heads of
+// 128 x 64: 822 | 458 | 388 (its output kernel 154, what the chunks add 67).
 #include "scan.cuh"
 
 namespace {
@@ -26,8 +30,6 @@ constexpr int THREADS = 128;
 // Where channel c's column of a staged [channels][64 tokens] tile lies: tokens in groups of four, permuted by the channel's
 // group of four, so that a warp that writes 8 x 4 channels of four tokens meets every bank once.
 __device__ __forceinline__ int at_ct(int c, int t) { return c * CT + (t ^ (((c >> 2) & 7) << 2)); }
-// The same for [channels][columns] tiles written by four lanes per column (16 channels) and eight columns per warp.
-__device__ __forceinline__ int at_kc(int k, int col, int cols) { return k * cols + (col ^ (((k >> 2) & 3) << 3)); }
 
 struct Scan {
     const void *q, *k, *v;
@@ -37,43 +39,61 @@ struct Scan {
     const float *ga, *gb; size_t ldg;                   // per token and head: decays (less one in mode 5), input weights
     const void* bonus; int bonus_dtype;
     const int32_t* chunk_start;
-    float *chunk_state, *chunk_decay;                   // [chunks][H][dv][dk], [chunks][H][dk]
+    float *chunk_state, *chunk_decay;                   // [chunks][H][dk][dvp], [chunks][H][dk]
     float* o; size_t ldo;
-    int H, dk, dv, in_act, qk_group, n_chunks, T_rows;
+    int H, dk, dv, dvp, qk_group, n_chunks, T_rows;       // dvp: dv rounded up to a multiple of four
     float q_scale, decay_scale;
-    int vec_q, vec_k, vec_v, vec_s, vec_o;              // whether rows may be read (written) in pieces of four
+    int vec_q, vec_k, vec_v, vec_o;                    // whether rows may be read (written) in pieces of four
 };
+
+template <int MODE>
+__device__ __forceinline__ float channel_decay(float z, float scale) { return MODE == 1 ? expf(-expf(z)) : expf(log_sigmoid_f32(z) * scale); }
 
 // The decay of channel i of head h at row t, as a factor (mode 5: less one).
 template <int MODE>
 __device__ __forceinline__ float decay_at(const Scan& p, size_t t, int h, int i) {
     if (MODE == 0) return p.head_decay[h];
     if (MODE == 2 || MODE == 5) return p.ga[t * p.ldg + h];
-    const float z = p.dlog[t * p.ldd + (size_t)h * p.dk + i];
-    return MODE == 1 ? expf(-expf(z)) : expf(log_sigmoid_f32(z) * p.decay_scale);
+    return channel_decay<MODE>(p.dlog[t * p.ldd + (size_t)h * p.dk + i], p.decay_scale);
 }
 template <int MODE>
 __device__ __forceinline__ float times_decay(float x, float a) { return MODE == 5 ? fmaf(x, a, x) : x * a; }
 
-// Four channels of a row from channel i on, zeros behind the last.
-template <typename TI>
-__device__ __forceinline__ void load_four(const TI* __restrict__ row, int i, int n, int vec, float (&f)[4]) {
-    f[0] = f[1] = f[2] = f[3] = 0.f;
-    if (i >= n) return;
-    if (vec) {
-        if constexpr (sizeof(TI) == 4) {
-            const float4 x = *reinterpret_cast<const float4*>(row + i);
-            f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w;
-        } else {
-            const uint2 u = *reinterpret_cast<const uint2*>(row + i);
-            f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
-            f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
-        }
-        return;
+// Four neighbouring elements of a row, zeros behind its end: fetched in one step and turned into 32-bit numbers in another, so that
+// many fetches are under way before the first is waited for.
+template <typename TI> struct Raw4;
+template <> struct Raw4<float> {
+    float4 x;
+    __device__ __forceinline__ void get(const float* p) { x = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void zero() { x = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ float4 value() const { return x; }
+};
+template <> struct Raw4<__nv_bfloat16> {
+    uint2 x;
+    __device__ __forceinline__ void get(const __nv_bfloat16* p) { x = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void zero() { x = make_uint2(0u, 0u); }
+    __device__ __forceinline__ float4 value() const {
+        return make_float4(__uint_as_float(x.x << 16), __uint_as_float(x.x & 0xffff0000u), __uint_as_float(x.y << 16), __uint_as_float(x.y & 0xffff0000u));
     }
+};
+template <typename TI>
+__device__ __forceinline__ void get_four(Raw4<TI>& r, const TI* __restrict__ row, int i, int n, bool have, int vec) {
+    if (!have || i >= n) { r.zero(); return; }
+    if (vec) { r.get(row + i); return; }
+    TI f[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) if (i + j < n) f[j] = to_f32(row[i + j]);
+    for (int j = 0; j < 4; ++j) f[j] = i + j < n ? row[i + j] : from_f32<TI>(0.f);
+    if constexpr (sizeof(TI) == 4) r.x = make_float4(f[0], f[1], f[2], f[3]);
+    else {
+        const __nv_bfloat162 a = __halves2bfloat162(f[0], f[1]), b = __halves2bfloat162(f[2], f[3]);
+        r.x = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
 }
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool have) {       // asynchronous; zeros where there is nothing
+    if (have) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+    else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // A chunk of more than 64 tokens (the callers cut none): this block's columns of the state walked in order in global memory.
 template <typename TI, int MODE>
@@ -81,38 +101,38 @@ __device__ void walk_in_order(const Scan& p, float* __restrict__ S, int c, int h
     constexpr bool ONES = MODE == 2, WKV = MODE == 1;
     const int t0 = p.chunk_start[c], t1 = p.chunk_start[c + 1], hq = h / p.qk_group, dvv = ONES ? p.dv - 1 : p.dv;
     for (int col = col0 + (int)threadIdx.x; col < col0 + cols; col += THREADS) {
-        float* s = S + (size_t)col * p.dk;
         for (int t = t0; t < t1; ++t) {
             const TI* qr = (const TI*)p.q + (size_t)t * p.ldq + hq * p.dk;
             const TI* kr = (const TI*)p.k + (size_t)t * p.ldk + hq * p.dk;
-            const float v = ONES && col == dvv ? 1.f : apply_activation(to_f32(((const TI*)p.v)[(size_t)t * p.ldv + (size_t)h * dvv + col]), p.in_act);
+            const float v = ONES && col == dvv ? 1.f : to_f32(((const TI*)p.v)[(size_t)t * p.ldv + (size_t)h * dvv + col]);
             const float b = MODE == 2 || MODE == 5 ? p.gb[(size_t)t * p.ldg + h] : 1.f;
             float o = 0.f;
             for (int i = 0; i < p.dk; ++i) {
-                const float q = apply_activation(to_f32(qr[i]), p.in_act) * (WKV ? 1.f : p.q_scale);
-                const float kv = apply_activation(to_f32(kr[i]), p.in_act) * b * v, a = decay_at<MODE>(p, t, h, i);
-                const float before = s[i], after = times_decay<MODE>(before, a) + kv;
+                const float q = to_f32(qr[i]) * (WKV ? 1.f : p.q_scale);
+                const float kv = to_f32(kr[i]) * b * v, a = decay_at<MODE>(p, t, h, i);
+                float* s = S + (size_t)i * p.dvp + col;
+                const float before = *s, after = times_decay<MODE>(before, a) + kv;
                 o = fmaf(q, WKV ? fmaf(load_as_f32(p.bonus, p.bonus_dtype, (size_t)h * p.dk + i), kv, before) : after, o);
-                s[i] = after;
+                *s = after;
             }
             if (output) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col] = o;
         }
     }
 }
 
-// acc[8][4 NC] += A[k][8 rows] B[k][4 NC columns] over k < n: A a swizzled [k][64] tile (rows 4 ty .. and 32 + 4 ty ..), B rows of
-// `cols` columns (4 tx .. of every 64).  `skew_b`: B is swizzled as by at_kc.
-template <int NC, bool SKEW_B>
+// acc[8][4 NC] += A[k][8 rows] B[k][4 NC columns] over k < n: A a [k][64] tile (rows 4 ty .. and 32 + 4 ty ..; SKEW: swizzled as by
+// at_ct), B rows of 64 NC columns (4 tx .. of every 64).
+template <int NC, bool SKEW>
 __device__ __forceinline__ void tile_product(f32x2 (&acc)[8][2 * NC], const float* __restrict__ A, const float* __restrict__ B, int n, int ty, int tx) {
 #pragma unroll 4
     for (int k = 0; k < n; ++k) {
-        const float4 x = *reinterpret_cast<const float4*>(A + at_ct(k, ty * 4)), y = *reinterpret_cast<const float4*>(A + at_ct(k, 32 + ty * 4));
+        const float4 x = *reinterpret_cast<const float4*>(A + (SKEW ? at_ct(k, ty * 4) : k * CT + ty * 4));
+        const float4 y = *reinterpret_cast<const float4*>(A + (SKEW ? at_ct(k, 32 + ty * 4) : k * CT + 32 + ty * 4));
         const float a[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
         f32x2 b[2 * NC];
 #pragma unroll
         for (int g = 0; g < NC; ++g) {
-            const int col = g * 64 + tx * 4;
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(B + (SKEW_B ? at_kc(k, col, 64 * NC) : k * 64 * NC + col));
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(B + k * 64 * NC + g * 64 + tx * 4);
             b[2 * g] = w.x;
             b[2 * g + 1] = w.y;
         }
@@ -127,29 +147,29 @@ __device__ __forceinline__ void tile_product(f32x2 (&acc)[8][2 * NC], const floa
 
 // ----------------------------------------------------------------------------- what a chunk adds
 
-// A block takes 64 value columns x up to 128 key channels of one head's state: added[col][i] = sum_j v_j[col] kw_j[i], tokens on
-// the sum's side.  kw_j = k_j times the decays behind token j (per channel), or v_j carries them (per head).
+// A block takes 64 key channels x 64 NC value columns of one head's state: added[i][col] = sum_j kw_j[i] v_j[col], the tokens on
+// the sum's side, kw_j = b_j k_j times the decays behind token j.
 template <typename TI, int MODE, int NC>
 __global__ void __launch_bounds__(THREADS)
 added_state_kernel(Scan p) {
     constexpr bool PER_CHANNEL = MODE == 1 || MODE == 4, ONES = MODE == 2;
+    constexpr int COLS = 64 * NC, NK = CT * 16 / THREADS, NV = NK * NC;
     extern __shared__ __align__(16) float smem[];
-    float* sv = smem;                                   // [tokens][64], swizzled as at_ct(token, column)
-    float* sk = sv + CT * CT;                           // [tokens][64 NC]
-    float* part = sk + CT * 64 * NC;                    // PER_CHANNEL: [parts][64 NC]
-    __shared__ float s_a[CT], s_w[CT];
+    float* sk = smem;                                   // [tokens][64]
+    float* sv = sk + CT * 64;                           // [tokens][COLS]
+    __shared__ float s_a[CT], s_w[CT], part[2 * 64], s_whole;
     grid_dep_launch();
     grid_dep_wait();
     const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int dk_tiles = (p.dk + 64 * NC - 1) / (64 * NC), col0 = blockIdx.z / dk_tiles * CT, i0 = blockIdx.z % dk_tiles * 64 * NC;
+    const int dk_tiles = (p.dk + 63) / 64, i0 = blockIdx.z % dk_tiles * 64, col0 = blockIdx.z / dk_tiles * COLS;
     const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, hq = h / p.qk_group;
-    const int dvv = ONES ? p.dv - 1 : p.dv, nk = min(64 * NC, p.dk - i0), nv = min(CT, dvv - col0);
-    float* added = p.chunk_state + ((size_t)c * p.H + h) * p.dv * p.dk;
+    const int dvv = ONES ? p.dv - 1 : p.dv, nk = min(64, p.dk - i0), nv = min(COLS, dvv - col0);
+    float* added = p.chunk_state + ((size_t)c * p.H + h) * p.dk * p.dvp;
     float* decays = p.chunk_decay + ((size_t)c * p.H + h) * p.dk;
     if (n > CT) {
         if (i0 == 0) {
             const int cols = col0 == 0 && ONES ? nv + 1 : nv;
-            for (int e = tid; e < cols * p.dk; e += THREADS) added[((size_t)(e / p.dk < nv ? col0 + e / p.dk : dvv)) * p.dk + e % p.dk] = 0.f;
+            for (int e = tid; e < cols * p.dk; e += THREADS) added[(size_t)(e % p.dk) * p.dvp + (e / p.dk < nv ? col0 + e / p.dk : dvv)] = 0.f;
             __syncthreads();
             walk_in_order<TI, MODE>(p, added, c, h, col0, nv, false);
             if (ONES && col0 == 0) walk_in_order<TI, MODE>(p, added, c, h, dvv, 1, false);
@@ -162,75 +182,63 @@ added_state_kernel(Scan p) {
         }
         return;
     }
+    Raw4<TI> rk[NK], rv[NV];
+#pragma unroll
+    for (int x = 0; x < NK; ++x) {
+        const int e = tid + x * THREADS, j = e >> 4;
+        get_four(rk[x], (const TI*)p.k + (size_t)(t0 + j) * p.ldk + hq * p.dk + i0, (e & 15) * 4, nk, j < n, p.vec_k);
+    }
+#pragma unroll
+    for (int x = 0; x < NV; ++x) {
+        const int e = tid + x * THREADS, j = e / (16 * NC);
+        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)h * dvv + col0, (e % (16 * NC)) * 4, nv, j < n, p.vec_v);
+    }
     if (!PER_CHANNEL) {
-        if (tid < CT) s_a[tid] = tid < n ? decay_at<MODE>(p, t0 + tid, h, 0) : (MODE == 5 ? 0.f : 1.f);
+        if (tid < CT) {
+            s_a[tid] = tid < n ? decay_at<MODE>(p, t0 + tid, h, 0) : (MODE == 5 ? 0.f : 1.f);
+            s_w[tid] = (MODE == 2 || MODE == 5) && tid < n ? p.gb[(size_t)(t0 + tid) * p.ldg + h] : 1.f;
+        }
         __syncthreads();
         if (tid < CT) {                                 // the decays behind token tid, and its weight
             float w = 1.f;
-            for (int t = CT - 1; t > tid; --t) w = times_decay<MODE>(w, s_a[t]);
-            const float whole = times_decay<MODE>(w, s_a[tid]);
-            if (MODE == 2 || MODE == 5) w *= tid < n ? p.gb[(size_t)(t0 + tid) * p.ldg + h] : 0.f;
-            s_w[tid] = w;
-            if (tid == 0) part[0] = whole;
+#pragma unroll 8
+            for (int t = CT - 1; t > 0; --t) if (t > tid) w = times_decay<MODE>(w, s_a[t]);
+            if (tid == 0) s_whole = times_decay<MODE>(w, s_a[0]);
+            s_w[tid] *= w;
         }
         __syncthreads();
         if (col0 == 0)
-            for (int i = tid; i < nk; i += THREADS) decays[i0 + i] = part[0];
+            for (int i = tid; i < nk; i += THREADS) decays[i0 + i] = s_whole;
     }
-    // values: token rows in pieces of four columns
-    for (int e = tid; e < CT * 16; e += THREADS) {
-        const int j = e >> 4, col = (e & 15) * 4;
-        float f[4] = {0.f, 0.f, 0.f, 0.f};
-        if (j < n) {
-            load_four((const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)h * dvv + col0, col, nv, p.vec_v, f);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                if (p.in_act) f[x] = apply_activation(f[x], p.in_act);
-                if (!PER_CHANNEL) f[x] *= s_w[j];
-                if (col + x >= nv) f[x] = 0.f;
-            }
-        }
-        *reinterpret_cast<float4*>(sv + at_ct(j, col)) = make_float4(f[0], f[1], f[2], f[3]);
+    for (int x = 0; x < NK; ++x) {
+        const int e = tid + x * THREADS, j = e >> 4;
+        float4 f = rk[x].value();
+        if (!PER_CHANNEL) { const float w = s_w[j]; f.x *= w; f.y *= w; f.z *= w; f.w *= w; }
+        *reinterpret_cast<float4*>(sk + j * 64 + (e & 15) * 4) = f;
     }
-    for (int e = tid; e < CT * 16 * NC; e += THREADS) {
-        const int j = e / (16 * NC), i = (e - j * 16 * NC) * 4;
-        float f[4] = {0.f, 0.f, 0.f, 0.f};
-        if (j < n) {
-            load_four((const TI*)p.k + (size_t)(t0 + j) * p.ldk + hq * p.dk + i0, i, nk, p.vec_k, f);
-            if (p.in_act) {
 #pragma unroll
-                for (int x = 0; x < 4; ++x) f[x] = i + x < nk ? apply_activation(f[x], p.in_act) : 0.f;
-            }
-        }
-        *reinterpret_cast<float4*>(sk + j * 64 * NC + i) = make_float4(f[0], f[1], f[2], f[3]);
-    }
-    if (PER_CHANNEL) {                                  // a thread takes a channel and a part of the tokens, from the last back
-        constexpr int PARTS = NC == 1 ? 2 : 1, LEN = CT / PARTS;
+    for (int x = 0; x < NV; ++x) *reinterpret_cast<float4*>(sv + (tid + x * THREADS) * 4) = rv[x].value();
+    if (PER_CHANNEL) {                                  // a thread takes a channel and half of the tokens, from the last back
+        constexpr int LEN = CT / 2;
         __syncthreads();
-        const int i = tid % (64 * NC), g = tid / (64 * NC);
-        float run = 1.f;
-        for (int base = LEN - 16; base >= 0; base -= 16) {
-            float a[16];
+        const int i = tid & 63, g = tid >> 6;
+        float a[LEN], run = 1.f;
 #pragma unroll
-            for (int x = 0; x < 16; ++x) {
-                const int t = g * LEN + base + x;
-                a[x] = t < n && i < nk ? decay_at<MODE>(p, t0 + t, h, i0 + i) : 1.f;
-            }
+        for (int x = 0; x < LEN; ++x) a[x] = g * LEN + x < n && i < nk ? p.dlog[(size_t)(t0 + g * LEN + x) * p.ldd + (size_t)h * p.dk + i0 + i] : 0.f;
 #pragma unroll
-            for (int x = 15; x >= 0; --x) {
-                sk[(g * LEN + base + x) * 64 * NC + i] *= run;
-                run *= a[x];
-            }
+        for (int x = LEN - 1; x >= 0; --x) {
+            sk[(g * LEN + x) * 64 + i] *= run;
+            run *= g * LEN + x < n && i < nk ? channel_decay<MODE>(a[x], p.decay_scale) : 1.f;
         }
-        part[g * 64 * NC + i] = run;
+        part[g * 64 + i] = run;
         __syncthreads();
-        if (PARTS == 2 && g == 0) {
-            const float later = part[64 * NC + i];
+        if (g == 0) {
+            const float later = part[64 + i];
 #pragma unroll 8
-            for (int t = 0; t < LEN; ++t) sk[t * 64 * NC + i] *= later;
-            run *= later;
+            for (int t = 0; t < LEN; ++t) sk[t * 64 + i] *= later;
+            if (i < nk && col0 == 0) decays[i0 + i] = run * later;
         }
-        if (g == 0 && i < nk && col0 == 0) decays[i0 + i] = run;
     }
     __syncthreads();
     f32x2 acc[8][2 * NC];
@@ -238,52 +246,56 @@ added_state_kernel(Scan p) {
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 2 * NC; ++j) acc[i][j] = 0ull;
-    tile_product<NC, false>(acc, sv, sk, n, ty, tx);
+    tile_product<NC, false>(acc, sk, sv, n, ty, tx);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int col = (i >> 2) * 32 + ty * 4 + (i & 3);
-        if (col >= nv) continue;
-        float* row = added + (size_t)(col0 + col) * p.dk + i0;
+        const int r = (i >> 2) * 32 + ty * 4 + (i & 3);
+        if (r >= nk) continue;
+        float* row = added + (size_t)(i0 + r) * p.dvp + col0;
 #pragma unroll
         for (int g = 0; g < NC; ++g) {
             const int at = g * 64 + tx * 4;
             const float2 a = unpack2(acc[i][2 * g]), b = unpack2(acc[i][2 * g + 1]);
-            if (p.vec_s && at < nk) *reinterpret_cast<float4*>(row + at) = make_float4(a.x, a.y, b.x, b.y);
+            if (at + 3 < nv) *reinterpret_cast<float4*>(row + at) = make_float4(a.x, a.y, b.x, b.y);
             else {
-                if (at < nk) row[at] = a.x;
-                if (at + 1 < nk) row[at + 1] = a.y;
-                if (at + 2 < nk) row[at + 2] = b.x;
-                if (at + 3 < nk) row[at + 3] = b.y;
+                if (at < nv) row[at] = a.x;
+                if (at + 1 < nv) row[at + 1] = a.y;
+                if (at + 2 < nv) row[at + 2] = b.x;
             }
         }
     }
-    if (ONES && col0 == 0)                              // the column whose values are ones
-        for (int i = tid; i < nk; i += THREADS) {
-            float sum = 0.f;
-            for (int j = 0; j < n; ++j) sum = fmaf(s_w[j], sk[j * 64 * NC + i], sum);
-            added[(size_t)dvv * p.dk + i0 + i] = sum;
-        }
+    if (ONES && col0 == 0 && tid < nk) {                // the column whose values are ones
+        float sum = 0.f;
+        for (int j = 0; j < n; ++j) sum += sk[j * 64 + tid];
+        added[(size_t)(i0 + tid) * p.dvp + dvv] = sum;
+    }
 }
 
 // ----------------------------------------------------------------------------- a chunk's outputs
 
 // A block takes the 64 tokens of a chunk and 64 NC value columns: of one head, or (NH = 2) 64 of each of two neighbouring heads
 // that share q and k, whose products q k^T are then taken once.  The key channels pass in slices through shared memory.
+template <int MODE, int NC>
+constexpr int output_body() {                           // floats of shared memory before the weights
+    const int sl = MODE == 1 || MODE == 4 ? 64 : 32, stage = sl == 64 ? (3 * sl * CT > sl * CT + sl * 64 * NC ? 3 * sl * CT : sl * CT + sl * 64 * NC)
+                                                                      : 2 * sl * CT + 2 * sl * 64 * NC;
+    return stage > CT * 64 * NC ? stage : CT * 64 * NC;
+}
+
 template <typename TI, int MODE, int NC, int NH>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 3)
 chunk_output_kernel(Scan p) {
     constexpr bool PER_CHANNEL = MODE == 1 || MODE == 4, ONES = MODE == 2, WKV = MODE == 1;
     constexpr int SL = PER_CHANNEL ? 64 : 32;           // channels of a slice
     constexpr int PP = CT + 4;                          // pitch of the weights P[j][t]
+    constexpr int COLS = 64 * NC, NQ = CT * SL / 4 / THREADS, NV = CT * 16 * NC / THREADS;
     extern __shared__ __align__(16) float smem[];
     float* sq = smem;                                   // [SL][64 tokens]
     float* sk = sq + SL * CT;                           // [SL][64 tokens]
     float* sw = sk + SL * CT;                           // PER_CHANNEL: the decays [SL][64 tokens]; then the state lies over sk, sw
-    float* ss = PER_CHANNEL ? sk : sw;                  // [SL][64 NC]: a slice of the states the chunk starts from
-    float* svv = smem;                                  // [64 tokens][64 NC]: the values, after the last slice
-    constexpr int STAGE = PER_CHANNEL ? (3 * SL * CT > SL * CT + SL * 64 * NC ? 3 * SL * CT : SL * CT + SL * 64 * NC) : 2 * SL * CT + SL * 64 * NC;
-    constexpr int VALUES = CT * 64 * NC;
-    float* sp = smem + (STAGE > VALUES ? STAGE : VALUES);       // [NH][64 j][PP]
+    float* ss = PER_CHANNEL ? sk : sw;                  // [SL][COLS]: a slice of the states the chunk starts from; two of them in turn per head
+    float* svv = smem;                                  // [64 tokens][COLS]: the values, after the last slice
+    float* sp = smem + output_body<MODE, NC>();         // [NH][64 j][PP]
     float* edge = sp + NH * CT * PP;                    // PER_CHANNEL: [4][SL] the decays of a block of 16 tokens
     __shared__ float s_a[NH][CT], s_cum[NH][CT], s_b[NH][CT];
     grid_dep_launch();
@@ -299,7 +311,7 @@ chunk_output_kernel(Scan p) {
     if (n <= 0) return;
     if (n > CT) {
         for (int x = 0; x < NH; ++x) {
-            float* S = p.chunk_state + ((size_t)c * p.H + h + x) * p.dv * p.dk;
+            float* S = p.chunk_state + ((size_t)c * p.H + h + x) * p.dk * p.dvp;
             walk_in_order<TI, MODE>(p, S, c, h + x, col0, nv, true);
             if (ONES && col0 == 0) walk_in_order<TI, MODE>(p, S, c, h + x, dvv, 1, true);
         }
@@ -323,45 +335,71 @@ chunk_output_kernel(Scan p) {
     if (PER_CHANNEL)
         for (int e = tid; e < CT * PP; e += THREADS) sp[e] = 0.f;
 
+    // q and k of a slice on their way to registers; the states' slice on its way to shared memory
+    Raw4<TI> rq[NQ], rk[NQ];
+    constexpr int LANES = SL / 4;                       // lanes that share a token's slice; a warp writes every bank of the staged tile once
+    auto token_of = [&](int e) { return PER_CHANNEL ? e / LANES : (e >> 5) * 4 + ((e & 31) >> 3); };
+    auto channel_of = [&](int e) { return PER_CHANNEL ? (e % LANES) * 4 : (e & 7) * 4; };
+    auto fetch = [&](int i0) {
+        const int nk = min(SL, p.dk - i0);
+#pragma unroll
+        for (int x = 0; x < NQ; ++x) {
+            const int e = tid + x * THREADS, t = token_of(e), i = channel_of(e);
+            get_four(rq[x], (const TI*)p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk + i0, i, nk, t < n, p.vec_q);
+            get_four(rk[x], (const TI*)p.k + (size_t)(t0 + t) * p.ldk + hq * p.dk + i0, i, nk, t < n, p.vec_k);
+        }
+    };
+    auto fetch_state = [&](int i0, float* dst) {
+        const int nk = min(SL, p.dk - i0);
+#pragma unroll 4
+        for (int e = tid; e < SL * 16 * NC; e += THREADS) {
+            const int i = e / (16 * NC), col = (e % (16 * NC)) * 4, x = NH == 2 ? col >> 6 : 0, own = NH == 2 ? col & 63 : col0 + col;
+            copy16(dst + e * 4, p.chunk_state + (((size_t)c * p.H + h + x) * p.dk + i0 + i) * p.dvp + own, i < nk && own < dvv);
+        }
+    };
+    fetch(0);
+    if (!PER_CHANNEL) {
+        fetch_state(0, ss);
+        __syncthreads();
+        for (int e = tid; e < NH * CT; e += THREADS) {  // the decays between two tokens, with the earlier one's weight; those since the start
+            const int x = e / CT, j = e % CT;
+            float w = s_b[x][j], cum = 1.f;
+#pragma unroll 8
+            for (int t = 0; t < CT; ++t) {
+                const float a = s_a[x][t];
+                if (t > j) w = times_decay<MODE>(w, a);
+                if (t <= j) cum = times_decay<MODE>(cum, a);
+                sp[(x * CT + j) * PP + t] = t >= j ? w : 0.f;
+            }
+            s_cum[x][j] = cum;
+        }
+    }
     for (int i0 = 0; i0 < p.dk; i0 += SL) {
         const int nk = min(SL, p.dk - i0);
+        float* const s_now = PER_CHANNEL ? ss : ss + (i0 / SL & 1) * SL * COLS;
         __syncthreads();
-        // q and k: eight (sixteen) lanes share a token's slice, a warp writes every bank once
-        constexpr int LANES = SL / 4;
-        for (int e = tid; e < CT * LANES; e += THREADS) {
-            const int t = PER_CHANNEL ? e / LANES : (e >> 5) * 4 + ((e & 31) >> 3), i = PER_CHANNEL ? (e % LANES) * 4 : (e & 7) * 4;
-            float fq[4] = {0.f, 0.f, 0.f, 0.f}, fk[4] = {0.f, 0.f, 0.f, 0.f};
-            if (t < n) {
-                load_four((const TI*)p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk + i0, i, nk, p.vec_q, fq);
-                load_four((const TI*)p.k + (size_t)(t0 + t) * p.ldk + hq * p.dk + i0, i, nk, p.vec_k, fk);
-            }
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                if (p.in_act) { fq[x] = apply_activation(fq[x], p.in_act); fk[x] = apply_activation(fk[x], p.in_act); }
-                if (!WKV) fq[x] *= p.q_scale;
-                if (i + x >= nk) fq[x] = fk[x] = 0.f;
-                sq[at_ct(i + x, t)] = fq[x];
-                sk[at_ct(i + x, t)] = fk[x];
+        for (int x = 0; x < NQ; ++x) {
+            const int e = tid + x * THREADS, t = token_of(e), i = channel_of(e);
+            const float4 q4 = rq[x].value(), k4 = rk[x].value();
+            const float fq[4] = {q4.x, q4.y, q4.z, q4.w}, fk[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                sq[at_ct(i + y, t)] = WKV ? fq[y] : fq[y] * p.q_scale;
+                sk[at_ct(i + y, t)] = fk[y];
             }
             if (PER_CHANNEL) {
 #pragma unroll
-                for (int x = 0; x < 4; ++x) sw[at_ct(i + x, t)] = t < n && i + x < nk ? decay_at<MODE>(p, t0 + t, h, i0 + i + x) : 1.f;
+                for (int y = 0; y < 4; ++y) sw[at_ct(i + y, t)] = t < n && i + y < nk ? decay_at<MODE>(p, t0 + t, h, i0 + i + y) : 1.f;
             }
         }
-        auto stage_state = [&]() {
-            for (int e = tid; e < 64 * NC * LANES; e += THREADS) {          // four lanes take 16 channels of a column
-                const int col = (e / 4) % (64 * NC), i = (e / (4 * 64 * NC)) * 16 + (e & 3) * 4;
-                const int x = NH == 2 ? col >> 6 : 0, own = NH == 2 ? col & 63 : col0 + col;
-                float f[4] = {0.f, 0.f, 0.f, 0.f};
-                if (own < dvv)
-                    load_four(p.chunk_state + (((size_t)c * p.H + h + x) * p.dv + own) * p.dk + i0, i, nk, p.vec_s, f);
-#pragma unroll
-                for (int y = 0; y < 4; ++y) ss[at_kc(i + y, col, 64 * NC)] = f[y];
-            }
-        };
         if (!PER_CHANNEL) {
-            stage_state();
+            copies_done();
             __syncthreads();
+            if (i0 + SL < p.dk) {
+                fetch_state(i0 + SL, ss + ((i0 / SL + 1) & 1) * SL * COLS);
+                fetch(i0 + SL);
+            }
             // q k^T and q S0 of this slice
 #pragma unroll 4
             for (int k = 0; k < SL; ++k) {
@@ -371,7 +409,7 @@ chunk_output_kernel(Scan p) {
                 f32x2 b[2 * NC];
 #pragma unroll
                 for (int g = 0; g < NC; ++g) {
-                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ss + at_kc(k, g * 64 + tx * 4, 64 * NC));
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(s_now + k * COLS + g * 64 + tx * 4);
                     b[2 * g] = w.x;
                     b[2 * g + 1] = w.y;
                 }
@@ -385,8 +423,8 @@ chunk_output_kernel(Scan p) {
                 }
             }
             if (ONES && blockIdx.z == 0 && tid < CT) {
-                const float* last = p.chunk_state + (((size_t)c * p.H + h) * p.dv + dvv) * p.dk + i0;
-                for (int i = 0; i < nk; ++i) ones_part = fmaf(sq[at_ct(i, tid)], last[i], ones_part);
+                const float* last = p.chunk_state + (((size_t)c * p.H + h) * p.dk + i0) * p.dvp + dvv;
+                for (int i = 0; i < nk; ++i) ones_part = fmaf(sq[at_ct(i, tid)], last[(size_t)i * p.dvp], ones_part);
             }
         } else {
             __syncthreads();
@@ -458,32 +496,28 @@ chunk_output_kernel(Scan p) {
             }
             __syncthreads();
             // q times the decays since the chunk's start; the state over k and the decays
+            fetch_state(i0, ss);
+            if (i0 + SL < p.dk) fetch(i0 + SL);
             for (int e = tid; e < SL * 48; e += THREADS) {
                 const int i = e % SL, t = 16 + e / SL;
                 float x = 1.f;
                 for (int m = 0; m < t / 16; ++m) x *= edge[m * SL + i];
                 sq[at_ct(i, t)] *= x;
             }
-            stage_state();
+            copies_done();
             __syncthreads();
             tile_product<NC, true>(acc, sq, ss, SL, ty, tx);
         }
     }
+    Raw4<TI> rv[NV];
+#pragma unroll
+    for (int x = 0; x < NV; ++x) {
+        const int e = tid + x * THREADS, j = e / (16 * NC), col = (e % (16 * NC)) * 4, head = NH == 2 ? col >> 6 : 0, own = NH == 2 ? col & 63 : col;
+        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)(h + head) * dvv + (NH == 2 ? 0 : col0), own, nv, j < n, p.vec_v);
+    }
     __syncthreads();
     // the weights P[j][t], and acc times the decays since the chunk's start
     if (!PER_CHANNEL) {
-        for (int e = tid; e < NH * CT; e += THREADS) {
-            const int x = e / CT, j = e % CT;
-            float w = s_b[x][j];
-            for (int t = 0; t < CT; ++t) {
-                if (t > j) w = times_decay<MODE>(w, s_a[x][t]);
-                sp[(x * CT + j) * PP + t] = t >= j ? w : 0.f;
-            }
-            float cum = 1.f;
-            for (int t = 0; t <= j; ++t) cum = times_decay<MODE>(cum, s_a[x][t]);
-            s_cum[x][j] = cum;
-        }
-        __syncthreads();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int t = (i >> 2) * 32 + ty * 4 + (i & 3);
@@ -503,19 +537,11 @@ chunk_output_kernel(Scan p) {
         }
     }
     bool odd = false;                                   // a value that is not finite must not meet the weights of zero of earlier tokens
-    for (int e = tid; e < CT * 16 * NC; e += THREADS) {
-        const int j = e / (16 * NC), col = (e - j * 16 * NC) * 4;
-        const int x = NH == 2 ? col >> 6 : 0, own = NH == 2 ? col & 63 : col;
-        float f[4] = {0.f, 0.f, 0.f, 0.f};
-        if (j < n) {
-            load_four((const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)(h + x) * dvv + (NH == 2 ? 0 : col0), own, nv, p.vec_v, f);
 #pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                if (p.in_act) f[y] = own + y < nv ? apply_activation(f[y], p.in_act) : 0.f;
-                odd |= !(fabsf(f[y]) <= 3.402823466e38f);
-            }
-        }
-        *reinterpret_cast<float4*>(svv + j * 64 * NC + col) = make_float4(f[0], f[1], f[2], f[3]);
+    for (int x = 0; x < NV; ++x) {
+        const float4 f = rv[x].value();
+        odd |= !(fabsf(f.x) <= 3.402823466e38f && fabsf(f.y) <= 3.402823466e38f && fabsf(f.z) <= 3.402823466e38f && fabsf(f.w) <= 3.402823466e38f);
+        *reinterpret_cast<float4*>(svv + (tid + x * THREADS) * 4) = f;
     }
     odd = __syncthreads_or(odd);
     // tokens j: the first 32 meet every t, the others only the last 32
@@ -578,9 +604,9 @@ chunk_output_kernel(Scan p) {
 template <typename TI, int MODE, int NC>
 int launch_added(const Scan& p, int n_chunks, cudaStream_t stream) {
     const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
-    const size_t smem = (size_t)(CT * CT + CT * 64 * NC + 2 * 64 * NC) * sizeof(float);
-    cudaError_t e = smem > 48 * 1024 ? cudaFuncSetAttribute(added_state_kernel<TI, MODE, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
-    const int tiles = ((dvv + CT - 1) / CT) * ((p.dk + 64 * NC - 1) / (64 * NC));
+    const size_t smem = (size_t)(CT * 64 + CT * 64 * NC) * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(added_state_kernel<TI, MODE, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int tiles = ((dvv + 64 * NC - 1) / (64 * NC)) * ((p.dk + 63) / 64);
     if (e == cudaSuccess) e = qs_launch_dependent(added_state_kernel<TI, MODE, NC>, dim3(n_chunks, p.H, tiles), dim3(THREADS), smem, stream, p);
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "state_scan, added states: %s", cudaGetErrorString(e));
     return qs_check_launch("state_scan, added states");
@@ -588,12 +614,8 @@ int launch_added(const Scan& p, int n_chunks, cudaStream_t stream) {
 
 template <typename TI, int MODE, int NC, int NH>
 int launch_output(const Scan& p, int n_chunks, cudaStream_t stream) {
-    constexpr bool PER_CHANNEL = MODE == 1 || MODE == 4;
-    constexpr int SL = PER_CHANNEL ? 64 : 32;
-    constexpr int STAGE = PER_CHANNEL ? (3 * SL * CT > SL * CT + SL * 64 * NC ? 3 * SL * CT : SL * CT + SL * 64 * NC) : 2 * SL * CT + SL * 64 * NC;
-    constexpr int VALUES = CT * 64 * NC;
     const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
-    const size_t smem = (size_t)((STAGE > VALUES ? STAGE : VALUES) + NH * CT * (CT + 4) + (PER_CHANNEL ? 4 * SL : 0)) * sizeof(float);
+    const size_t smem = (size_t)(output_body<MODE, NC>() + NH * CT * (CT + 4) + (MODE == 1 || MODE == 4 ? 4 * 64 : 0)) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(chunk_output_kernel<TI, MODE, NC, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int tiles = NH == 2 ? 1 : (dvv + 64 * NC - 1) / (64 * NC);
     if (e == cudaSuccess)
@@ -605,7 +627,7 @@ int launch_output(const Scan& p, int n_chunks, cudaStream_t stream) {
 template <typename TI, int MODE>
 int run(const Scan& p, int n_chunks, bool outputs, cudaStream_t stream) {
     const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
-    if (!outputs) return p.dk > 64 ? launch_added<TI, MODE, 2>(p, n_chunks, stream) : launch_added<TI, MODE, 1>(p, n_chunks, stream);
+    if (!outputs) return dvv > 64 ? launch_added<TI, MODE, 2>(p, n_chunks, stream) : launch_added<TI, MODE, 1>(p, n_chunks, stream);
     if constexpr (MODE == 5)                            // two heads that share q and k: their products once
         if (dvv <= 64 && dvv > 32 && p.qk_group % 2 == 0) return launch_output<TI, MODE, 2, 2>(p, n_chunks, stream);
     return dvv > 64 ? launch_output<TI, MODE, 2, 1>(p, n_chunks, stream) : launch_output<TI, MODE, 1, 1>(p, n_chunks, stream);
@@ -623,13 +645,64 @@ int pick(int mode, const Scan& p, int n_chunks, bool outputs, cudaStream_t strea
     return qs_fail(QS_ERR_INVALID_INPUT, "state_scan: mode %d has no chunks", mode);
 }
 
+// The activation of q, k and v, once per element, for chunks whose kernels read them several times.
+template <typename TI>
+__global__ void __launch_bounds__(256)
+activate_rows_kernel(float* __restrict__ out, const TI* __restrict__ q, size_t ldq, const TI* __restrict__ k, size_t ldk, const TI* __restrict__ v, size_t ldv,
+                     int nk, int nv, int act) {
+    grid_dep_launch();
+    grid_dep_wait();
+    const size_t t = blockIdx.x;
+    const int n = 2 * nk + nv;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const TI* src = i < nk ? q + t * ldq + i : i < 2 * nk ? k + t * ldk + i - nk : v + t * ldv + i - 2 * nk;
+        out[t * n + i] = apply_activation(to_f32(*src), act);
+    }
+}
+template <typename TI>
+__global__ void __launch_bounds__(256)
+activate_fours_kernel(float4* __restrict__ out, const TI* __restrict__ q, size_t ldq, const TI* __restrict__ k, size_t ldk, const TI* __restrict__ v, size_t ldv,
+                      int nk4, int nv4, int act) {
+    grid_dep_launch();
+    grid_dep_wait();
+    const size_t t = blockIdx.x;
+    const int n = 2 * nk4 + nv4;
+    for (int i = threadIdx.x + blockIdx.y * blockDim.x; i < n; i += blockDim.x * gridDim.y) {
+        const TI* src = i < nk4 ? q + t * ldq + 4 * i : i < 2 * nk4 ? k + t * ldk + 4 * (i - nk4) : v + t * ldv + 4 * (i - 2 * nk4);
+        Raw4<TI> r;
+        r.get(src);
+        float4 f = r.value();
+        f.x = apply_activation(f.x, act); f.y = apply_activation(f.y, act); f.z = apply_activation(f.z, act); f.w = apply_activation(f.w, act);
+        out[t * n + i] = f;
+    }
+}
+
 }  // namespace
+
+// out [rows][2 nk + nv] = act(q), act(k), act(v) side by side, in 32-bit.
+QS_API int qs_scan_activate(float* out, const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv, int dtype, int rows, int nk, int nv,
+                            int act, cudaStream_t stream) {
+    if (rows == 0) return QS_OK;
+    QS_REQUIRE(rows > 0 && nk > 0 && nv > 0 && (dtype == QS_F32 || dtype == QS_BF16), "scan_activate: bad sizes");
+    const size_t item = dtype == QS_F32 ? 4 : 2;
+    auto fits = [&](const void* ptr, long long ld) { return ld % 4 == 0 && ((uintptr_t)ptr % (4 * item)) == 0; };
+    const bool fours = nk % 4 == 0 && nv % 4 == 0 && fits(q, ldq) && fits(k, ldk) && fits(v, ldv);
+    cudaError_t e;
+#define GO(T) do { if (fours) e = qs_launch_dependent(activate_fours_kernel<T>, dim3(rows, 2), dim3(256), 0, stream, (float4*)out, (const T*)q, (size_t)ldq, \
+        (const T*)k, (size_t)ldk, (const T*)v, (size_t)ldv, nk / 4, nv / 4, act); \
+    else e = qs_launch_dependent(activate_rows_kernel<T>, dim3(rows), dim3(256), 0, stream, out, (const T*)q, (size_t)ldq, (const T*)k, (size_t)ldk, (const T*)v, \
+        (size_t)ldv, nk, nv, act); } while (0)
+    if (dtype == QS_F32) GO(float); else GO(__nv_bfloat16);
+#undef GO
+    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "scan_activate: %s", cudaGetErrorString(e));
+    return qs_check_launch("scan_activate");
+}
 
 // The first (outputs == 0: chunk_state becomes what every chunk adds, chunk_decay its decays) and the last kernel (chunk_state
 // holds the states the chunks start from) of a scan in chunks; operands as for `qs_state_scan`.
 int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                    int dtype, const float* dlog, long long ldd, const float* head_decay, const void* bonus, int bonus_dtype, int H, int dk, int dv,
-                   int in_act, const int32_t* chunk_start, int n_chunks, int T_rows, float* chunk_state, float* chunk_decay, const float* ga, const float* gb,
+                   const int32_t* chunk_start, int n_chunks, int T_rows, float* chunk_state, float* chunk_decay, const float* ga, const float* gb,
                    long long ldg, float q_scale, int qk_group, float decay_scale, cudaStream_t stream) {
     const size_t item = dtype == QS_F32 ? 4 : 2;
     auto fours = [&](const void* ptr, long long ld, int per_head) { return (int)(per_head % 4 == 0 && ld % 4 == 0 && ((uintptr_t)ptr % (4 * item)) == 0); };
@@ -637,11 +710,10 @@ int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q
     p.q = q; p.k = k; p.v = v; p.ldq = (size_t)ldq; p.ldk = (size_t)ldk; p.ldv = (size_t)ldv;
     p.dlog = dlog; p.ldd = (size_t)ldd; p.head_decay = head_decay; p.ga = ga; p.gb = gb; p.ldg = (size_t)ldg;
     p.bonus = bonus; p.bonus_dtype = bonus_dtype; p.chunk_start = chunk_start; p.chunk_state = chunk_state; p.chunk_decay = chunk_decay;
-    p.o = o; p.ldo = (size_t)ldo; p.H = H; p.dk = dk; p.dv = dv; p.in_act = in_act; p.qk_group = qk_group;
+    p.o = o; p.ldo = (size_t)ldo; p.H = H; p.dk = dk; p.dv = dv; p.dvp = (dv + 3) / 4 * 4; p.qk_group = qk_group;
     p.q_scale = q_scale; p.decay_scale = decay_scale;
     p.vec_q = fours(q, ldq, dk); p.vec_k = fours(k, ldk, dk); p.vec_v = fours(v, ldv, mode == 2 ? dv - 1 : dv);
     p.vec_o = mode != 2 && dv % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)o % 16) == 0;
     p.n_chunks = n_chunks; p.T_rows = T_rows;
-    p.vec_s = dk % 4 == 0 && ((uintptr_t)chunk_state % 16) == 0;
     return dtype == QS_F32 ? pick<float>(mode, p, n_chunks, outputs != 0, stream) : pick<__nv_bfloat16>(mode, p, n_chunks, outputs != 0, stream);
 }
