@@ -230,10 +230,23 @@ __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x,
     for (int i = threadIdx.x; i < D; i += blockDim.x) dst[i] = src[i];
 }
 
+// The same in 16-byte pieces (rows of `pieces` of them, `pitch` apart in x).
+__global__ void gather_pieces_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, const int32_t* __restrict__ rows, int pieces, size_t pitch) {
+    const uint4* src = x + (size_t)rows[blockIdx.x] * pitch;
+    uint4* dst = out + (size_t)blockIdx.x * pieces;
+#pragma unroll 2
+    for (int i = threadIdx.x; i < pieces; i += blockDim.x) dst[i] = src[i];
+}
+
 QS_API int qs_gather_rows(void* out, const void* x, int dtype, const int32_t* rows, int n, int D,
                           long long ldx, cudaStream_t stream) {
     if (n == 0) return QS_OK;
     QS_REQUIRE(n > 0 && D > 0, "gather_rows: bad sizes n=%d D=%d", n, D);
+    const long long row_bytes = (long long)D * (dtype == QS_F32 ? 4 : 2), pitch = ldx * (dtype == QS_F32 ? 4 : 2);
+    if ((dtype == QS_F32 || dtype == QS_BF16) && row_bytes % 16 == 0 && pitch % 16 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0) {
+        gather_pieces_kernel<<<n, row_bytes >= 4096 ? 256 : 128, 0, stream>>>((uint4*)out, (const uint4*)x, rows, (int)(row_bytes / 16), (size_t)(pitch / 16));
+        return qs_check_launch("gather_rows");
+    }
     if (dtype == QS_F32) gather_rows_kernel<float><<<n, 256, 0, stream>>>((float*)out, (const float*)x, rows, D, (size_t)ldx);
     else if (dtype == QS_BF16) gather_rows_kernel<__nv_bfloat16><<<n, 256, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)x, rows, D, (size_t)ldx);
     else return qs_fail(QS_ERR_INVALID_INPUT, "gather_rows: unknown dtype %d", dtype);

@@ -70,11 +70,17 @@ template <int BN> constexpr int p_smem_bytes() { return p_stages<BN>() * stage_b
 // run together share rows of W and all of A stays in L2).  Two accumulators in TMEM: while the four
 // epilogue warps drain tile i, the MMA warp already accumulates tile i + 1 into the other one, and the
 // TMA producer runs ahead across tile borders through the same ring of stages.
-template <int BN>
+//
+// GROUPED: several products in one launch, rows offsets[e] .. offsets[e + 1] of A and C against matrix e of W (matrices of
+// ep.N rows one below the other).  The offsets are read on the device, so the host need not know them.  Tiles run through
+// a group's rows first, then its columns, then the groups; a tile's rows beyond its group are computed from the next group's and not
+// stored.
+constexpr int MAX_GROUPS = 1024;
+template <int BN, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                           const Epilogue ep, const int K, const int m_tiles, const int n_tiles,
-                          int32_t* __restrict__ status) {
+                          int32_t* __restrict__ status, const int32_t* __restrict__ offsets, const int n_groups) {
     constexpr int STAGES = p_stages<BN>();
     constexpr int STAGE = stage_bytes<BN>();
     constexpr uint32_t TMEM_COLS = 2 * BN;
@@ -90,7 +96,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = (K + BK - 1) / BK;
-    const int total_tiles = m_tiles * n_tiles;
+    __shared__ int first_row[GROUPED ? MAX_GROUPS + 1 : 1], first_tile[GROUPED ? MAX_GROUPS + 1 : 1];
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -101,23 +107,51 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         prefetch_tensormap(&map_w);
     }
     if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    if (GROUPED) {
+        for (int e = threadIdx.x; e <= n_groups; e += THREADS) first_row[e] = offsets[e];
+        __syncthreads();
+        if (warp == 2) {                                // the groups' first tiles: a running sum, 32 groups at a time
+            int run = 0;
+            for (int base = 0; base < n_groups; base += 32) {
+                const int e = base + lane;
+                const int mine = e < n_groups ? (first_row[e + 1] - first_row[e] + BM - 1) / BM * n_tiles : 0;
+                int sum = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+                if (e < n_groups) first_tile[e] = run + sum - mine;
+                run += __shfl_sync(0xffffffffu, sum, 31);
+            }
+            if (lane == 0) first_tile[n_groups] = run;
+        }
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    const int total_tiles = GROUPED ? first_tile[n_groups] : m_tiles * n_tiles;
+    // a tile's first row of A, the end of its rows, its first column of C and its first row of W; `group` only moves on
+    struct Place { int m0, m_end, n0, w0; };
+    auto place = [&](int t, int& group) {
+        if (!GROUPED) { const int n0 = (t / m_tiles) * BN; return Place{(t % m_tiles) * BM, ep.M, n0, n0}; }
+        while (t >= first_tile[group + 1]) ++group;
+        const int lo = first_row[group], hi = first_row[group + 1], tiles = (hi - lo + BM - 1) / BM, mine = t - first_tile[group];
+        const int n0 = (mine / tiles) * BN;
+        return Place{lo + (mine % tiles) * BM, hi, n0, group * ep.N + n0};
+    };
 
     if (warp == 0) {
         if (elect_one()) {
             uint32_t it = 0;
+            int group = 0;
             for (int t = blockIdx.x; t < total_tiles && !*aborted; t += gridDim.x) {
-                const int m0 = (t % m_tiles) * BM, n0 = (t / m_tiles) * BN;
+                const Place at = place(t, group);
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!wait_or_abort(&empty[s], ((it / STAGES) & 1) ^ 1, aborted)) { atomicExch(status, 121); *aborted = 1; break; }
                     uint8_t* tile = smem + s * STAGE;
                     mbar_expect_tx(&full[s], STAGE);
-                    tma_load_2d(tile, &map_a, &full[s], kb * BK, m0);
-                    tma_load_2d(tile + BM * BK * 2, &map_w, &full[s], kb * BK, n0);
+                    tma_load_2d(tile, &map_a, &full[s], kb * BK, at.m0);
+                    tma_load_2d(tile + BM * BK * 2, &map_w, &full[s], kb * BK, at.w0);
                 }
             }
         }
@@ -153,10 +187,11 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                             (!ep.res1 || ((ep.ldr % 8) == 0 && ((uintptr_t)ep.res1 % 16) == 0)) &&
                             (!ep.res2 || ((uintptr_t)ep.res2 % 16) == 0);
         const bool bias_vec = ep.bias && ((uintptr_t)ep.bias % 32) == 0;
-        int i = 0;
+        int i = 0, group = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++i) {
             const int buf = i & 1;
-            const int m = (t % m_tiles) * BM + r, n0 = (t / m_tiles) * BN;
+            const Place at = place(t, group);
+            const int m = at.m0 + r, n0 = at.n0;
             if (!wait_or_abort(&acc_full[buf], (i >> 1) & 1, aborted)) { atomicExch(status, 124); *aborted = 1; break; }
             tc_fence_after_sync();
 #pragma unroll 1
@@ -165,7 +200,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 tmem_load_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN + c * 32), raw);
                 tmem_load_wait();
                 const int nc = n0 + c * 32;
-                if (m >= ep.M || nc >= ep.N) continue;
+                if (m >= at.m_end || nc >= ep.N) continue;
                 if (vec_ok && nc + 32 <= ep.N) {
                     // 32 consecutive outputs of one row: bias and activation on the accumulator, residuals
                     // added in 32-bit, one rounding, four 16-byte stores
@@ -1015,13 +1050,14 @@ int launch_pair(const CUtensorMap& ma, const void* W, long long ldw, const Epilo
     return qs_check_launch("gemm_tc pair");
 }
 
-template <int BN>
+// offsets null: one product of M rows.  Else `n_groups` products whose rows the device finds in `offsets` (M: all rows together).
+template <int BN, bool GROUPED>
 int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilogue& ep, int M, int N, int K,
-                      int32_t* status, cudaStream_t stream) {
+                      int32_t* status, const int32_t* offsets, int n_groups, cudaStream_t stream) {
     static bool configured = false;
     static int sm_count = 0;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              p_smem_bytes<BN>());
         int dev = 0;
         if (e == cudaSuccess) e = cudaGetDevice(&dev);
@@ -1031,9 +1067,9 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilog
         configured = true;
     }
     const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
-    const long long total = (long long)m_tiles * n_tiles;
+    const long long total = (long long)(m_tiles + (GROUPED ? n_groups : 0)) * n_tiles;     // groups: at most a tile row more each
     const int grid = (int)(total < sm_count ? total : sm_count);
-    gemm_tc_persistent_kernel<BN><<<grid, THREADS, p_smem_bytes<BN>(), stream>>>(ma, mw, ep, K, m_tiles, n_tiles, status);
+    gemm_tc_persistent_kernel<BN, GROUPED><<<grid, THREADS, p_smem_bytes<BN>(), stream>>>(ma, mw, ep, K, m_tiles, n_tiles, status, offsets, n_groups);
     return qs_check_launch("gemm_tc persistent");
 }
 
@@ -1086,8 +1122,8 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
         }
         const int bn = N > 128 ? 256 : 128;
         if ((rc = tensor_map(&mw, W, N, K, ldw, bn)) != QS_OK) return rc;
-        if (bn == 256) return launch_persistent<256>(ma, mw, ep, M, N, K, status, stream);
-        return launch_persistent<128>(ma, mw, ep, M, N, K, status, stream);
+        if (bn == 256) return launch_persistent<256, false>(ma, mw, ep, M, N, K, status, nullptr, 0, stream);
+        return launch_persistent<128, false>(ma, mw, ep, M, N, K, status, nullptr, 0, stream);
     }
     const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
     if ((rc = tensor_map(&ma, A, M, K, lda, bn)) != QS_OK) return rc;
@@ -1095,4 +1131,27 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
     if (bn == 32) return launch_stream<32>(W, ldw, ma, ep, N, K, ws, ws_floats, counters, n_counters, status, smem_kb, stream);
     if (bn == 64) return launch_stream<64>(W, ldw, ma, ep, N, K, ws, ws_floats, counters, n_counters, status, smem_kb, stream);
     return launch_stream<128>(W, ldw, ma, ep, N, K, ws, ws_floats, counters, n_counters, status, smem_kb, stream);
+}
+
+// C[rows of e] = A[rows of e] W[e]^T for the groups e of rows offsets[e] .. offsets[e + 1] (E + 1 ascending entries on the DEVICE, from 0
+// to at most M), W [E][N][K] contiguous; A [M, K] bfloat16 with row stride lda, C [M, N] bfloat16 or float32.  One launch; rows
+// of no group are left alone.
+QS_API int qs_gemm_tc_grouped(void* C, int c_dtype, long long ldc, const void* A, long long lda, const void* W, const int32_t* offsets, int E, int M, int N,
+                              int K, int32_t* status, cudaStream_t stream) {
+    if (M == 0) return QS_OK;
+    QS_REQUIRE(M > 0 && N > 0 && K > 0 && E > 0 && E <= MAX_GROUPS && offsets, "gemm_tc_grouped: bad sizes M=%d N=%d K=%d E=%d", M, N, K, E);
+    QS_REQUIRE(K % 8 == 0 && lda % 8 == 0 && lda >= K && ldc >= N, "gemm_tc_grouped: K=%d and the row stride %lld must be multiples of 8", K, lda);
+    QS_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0, "gemm_tc_grouped: operands must be 16-byte aligned");
+    QS_REQUIRE(c_dtype == QS_F32 || c_dtype == QS_BF16, "gemm_tc_grouped: unknown output type %d", c_dtype);
+    QS_REQUIRE((long long)E * N <= 0x7fffffffll, "gemm_tc_grouped: %d matrices of %d rows", E, N);
+    const Epilogue ep{C, c_dtype, ldc, nullptr, 0, QS_ACT_NONE, nullptr, nullptr, N, M, N};
+    // tiles half as wide where whole ones would leave SMs without any (few rows: every group still has its tile row)
+    const long long rows = (M + BM - 1) / BM + (E < M ? E : M) / 2, wide = rows * ((N + 255) / 256);
+    const int bn = N > 128 && wide >= 148 ? 256 : 128;
+    CUtensorMap ma, mw;
+    int rc;
+    if ((rc = tensor_map(&ma, A, M, K, lda, BM)) != QS_OK) return rc;
+    if ((rc = tensor_map(&mw, W, (long long)E * N, K, K, bn)) != QS_OK) return rc;
+    return bn == 256 ? launch_persistent<256, true>(ma, mw, ep, M, N, K, status, offsets, E, stream)
+                     : launch_persistent<128, true>(ma, mw, ep, M, N, K, status, offsets, E, stream);
 }

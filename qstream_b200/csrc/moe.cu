@@ -179,6 +179,240 @@ __global__ void moe_expert_down_kernel(float* __restrict__ out, size_t ldo, cons
     }
 }
 
+// ----------------------------------------------------------------------------- few tokens, bfloat16, each expert's matrices read once
+//
+// The pairs of a step of few tokens grouped by expert inside the kernels: rows of an expert's matrix are the 16-row side of
+// mma.sync products (bfloat16, 32-bit sums), its tokens the side of eight columns, both straight from memory to registers.  The k's
+// of a product are permuted so that a lane's 16 bytes of a row are two products' worth: lane t of a row's four takes the k's
+// 8 t .. 8 t + 7 of 32, on both sides.  A column does not meet the others and K is cut in four wherever the token stands, so a
+// token's result does not depend on the batch.
+//
+// Bound by the matrices' way from memory.  8 tokens, 16 experts of 4,096 x 1,024 x 3, 4 per token: the feed-forward with its
+// router 218 -> 92 us (every pair read its expert by itself before); 3,000 tokens of width 2,048, all products of all experts in two launches
+// (gemm_tc.cu) instead of one each behind a wait for the host: 428 -> 197 us.
+constexpr int CHUNK_TOKENS = 32;                        // tokens of a block: at most this many columns of an expert
+
+__device__ __forceinline__ void mma_bf16_16x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint4 piece(const __nv_bfloat16* row, int k, int K) {        // eight elements, zeros behind the end
+    return row && k < K ? *reinterpret_cast<const uint4*>(row + k) : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// acc[m][n] += rows of matrix m (`lo`: this lane's row of the first eight, `hi`: of the last eight) times columns of tile n, k from
+// k0 to k1 (multiples of 32); U steps of 32 fetched together.
+template <int MATS, int NT, int U>
+__device__ __forceinline__ void stream_rows(float (&acc)[MATS][NT][4], const __nv_bfloat16* const (&lo)[MATS], const __nv_bfloat16* const (&hi)[MATS],
+                                            const __nv_bfloat16* const (&col)[NT], int k0, int k1, int K) {
+    const int t8 = (threadIdx.x & 3) * 8;
+    for (int k = k0; k < k1; k += 32 * U) {
+        uint4 a[U][MATS], b[U][MATS], x[U][NT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int at = k + u * 32 + t8, end = min(k1, K);
+#pragma unroll
+            for (int m = 0; m < MATS; ++m) { a[u][m] = piece(lo[m], at, end); b[u][m] = piece(hi[m], at, end); }
+#pragma unroll
+            for (int n = 0; n < NT; ++n) x[u][n] = piece(col[n], at, end);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int m = 0; m < MATS; ++m)
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    mma_bf16_16x8(acc[m][n], a[u][m].x, b[u][m].x, a[u][m].y, b[u][m].y, x[u][n].x, x[u][n].y);
+                    mma_bf16_16x8(acc[m][n], a[u][m].z, b[u][m].z, a[u][m].w, b[u][m].w, x[u][n].z, x[u][n].w);
+                }
+    }
+}
+
+// hidden[pair, f] of 16 hidden units f of one expert, for the chunk's pairs that chose it; four warps share K.
+template <int MATS, int NT>
+__device__ void up_columns(__nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ x, size_t ldx, const __nv_bfloat16* __restrict__ w,
+                           const int* list, int n, int top, int D, int F, int f0, int act, float* red) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const __nv_bfloat16 *lo[MATS], *hi[MATS], *col[NT];
+#pragma unroll
+    for (int m = 0; m < MATS; ++m) {
+        lo[m] = f0 + g < F ? w + ((size_t)m * F + f0 + g) * D : nullptr;
+        hi[m] = f0 + g + 8 < F ? w + ((size_t)m * F + f0 + g + 8) * D : nullptr;
+    }
+#pragma unroll
+    for (int c = 0; c < NT; ++c) col[c] = c * 8 + g < n ? x + (size_t)(list[c * 8 + g] / top) * ldx : nullptr;
+    float acc[MATS][NT][4];
+#pragma unroll
+    for (int m = 0; m < MATS; ++m)
+#pragma unroll
+        for (int c = 0; c < NT; ++c) acc[m][c][0] = acc[m][c][1] = acc[m][c][2] = acc[m][c][3] = 0.f;
+    const int per = ((D + 31) / 32 + 3) / 4 * 32;
+    stream_rows<MATS, NT, NT == 1 ? 4 : 2>(acc, lo, hi, col, warp * per, min((warp + 1) * per, (D + 31) / 32 * 32), D);
+    constexpr int PITCH = NT * 8 + 1;                   // red [4 warps][MATS][16 rows][PITCH]
+#pragma unroll
+    for (int m = 0; m < MATS; ++m)
+#pragma unroll
+        for (int c = 0; c < NT; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) red[((warp * MATS + m) * 16 + g + 8 * (e >> 1)) * PITCH + c * 8 + 2 * t + (e & 1)] = acc[m][c][e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < 16 * n; e += blockDim.x) {
+        const int r = e & 15, c = e >> 4;
+        float v[MATS];
+#pragma unroll
+        for (int m = 0; m < MATS; ++m) {
+            v[m] = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[m] += red[((q * MATS + m) * 16 + r) * PITCH + c];
+        }
+        const float y = apply_activation_wide(v[0], act);
+        if (f0 + r < F) hidden[(size_t)list[c] * ldh + f0 + r] = __float2bfloat16_rn(MATS == 2 ? y * v[MATS - 1] : y);
+    }
+    __syncthreads();
+}
+
+template <bool GATED>
+__global__ void __launch_bounds__(128)
+moe_up_grouped_kernel(__nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ x, size_t ldx, const __nv_bfloat16* __restrict__ w_up,
+                      const int32_t* __restrict__ idx, const int32_t* __restrict__ tok_slot, int T, int top, int D, int F, int act, int n_experts) {
+    constexpr int MATS = GATED ? 2 : 1;
+    extern __shared__ int list[];                       // the chunk's pairs that chose this expert, in order
+    __shared__ float red[4 * MATS * 16 * 33];
+    __shared__ int count[4];
+    grid_dep_launch();
+    grid_dep_wait();
+    const int e = blockIdx.y, f0 = blockIdx.x * 16, first = blockIdx.z * CHUNK_TOKENS * top, n_pairs = min(T - blockIdx.z * CHUNK_TOKENS, CHUNK_TOKENS) * top;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int n = 0;
+    for (int base = 0; base < n_pairs; base += 128) {
+        const int p = base + threadIdx.x;
+        const int mine = p < n_pairs ? idx[first + p] : -1;
+        const bool live = p < n_pairs && tok_slot[(first + p) / top] >= 0;
+        if (e == 0 && p < n_pairs && (!live || mine >= n_experts))     // nobody's row, or an expert that returns its input: nothing hidden
+            for (int f = f0; f < min(F, f0 + 16); ++f) hidden[(size_t)(first + p) * ldh + f] = __float2bfloat16_rn(0.f);
+        const unsigned hit = __ballot_sync(0xffffffffu, live && mine == e);
+        if (lane == 0) count[warp] = __popc(hit);
+        __syncthreads();
+        int at = n;
+        for (int q = 0; q < warp; ++q) at += count[q];
+        if (hit >> lane & 1) list[at + __popc(hit & ((1u << lane) - 1))] = first + p;
+        n += count[0] + count[1] + count[2] + count[3];
+        __syncthreads();
+    }
+    const __nv_bfloat16* w = w_up + (size_t)e * MATS * F * D;
+    for (int c = 0; c < n; c += 32) {
+        const int m = min(32, n - c);
+        if (m <= 8) up_columns<MATS, 1>(hidden, ldh, x, ldx, w, list + c, m, top, D, F, f0, act, red);
+        else if (m <= 16) up_columns<MATS, 2>(hidden, ldh, x, ldx, w, list + c, m, top, D, F, f0, act, red);
+        else up_columns<MATS, 4>(hidden, ldh, x, ldx, w, list + c, m, top, D, F, f0, act, red);
+    }
+}
+
+// Sixteen output elements d of a chunk's tokens: warp w takes quarter w mod 4 of K of every second expert in use; the quarters' sums
+// rest in shared memory until the tokens' choices are added up in order.
+template <int NT>
+__device__ void down_columns(float* __restrict__ part, const __nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ w, const int* list,
+                             int n, int first, int D, int F, int d0, int quarter) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const __nv_bfloat16* const lo[1] = {d0 + g < D ? w + (size_t)(d0 + g) * F : nullptr};
+    const __nv_bfloat16* const hi[1] = {d0 + g + 8 < D ? w + (size_t)(d0 + g + 8) * F : nullptr};
+    const __nv_bfloat16* col[NT];
+#pragma unroll
+    for (int c = 0; c < NT; ++c) col[c] = c * 8 + g < n ? hidden + (size_t)(first + list[c * 8 + g]) * ldh : nullptr;
+    float acc[1][NT][4];
+#pragma unroll
+    for (int c = 0; c < NT; ++c) acc[0][c][0] = acc[0][c][1] = acc[0][c][2] = acc[0][c][3] = 0.f;
+    const int per = ((F + 31) / 32 + 3) / 4 * 32;
+    stream_rows<1, NT, NT == 1 ? 8 : 4>(acc, lo, hi, col, quarter * per, min((quarter + 1) * per, (F + 31) / 32 * 32), F);
+#pragma unroll
+    for (int c = 0; c < NT; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int at = c * 8 + 2 * t + (e & 1);
+            if (at < n) part[list[at] * 16 + g + 8 * (e >> 1)] = acc[0][c][e];
+        }
+}
+
+__global__ void __launch_bounds__(256)
+moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ w_down,
+                        const int32_t* __restrict__ idx, const float* __restrict__ wts, const int32_t* __restrict__ tok_slot, const void* __restrict__ add,
+                        int add_dtype, size_t ldadd, const float* __restrict__ add_scale, int T, int top, int D, int F, const __nv_bfloat16* __restrict__ x,
+                        size_t ldx, int n_experts) {
+    extern __shared__ float smem[];
+    const int tokens = min(T - (int)blockIdx.z * CHUNK_TOKENS, CHUNK_TOKENS), n_pairs = tokens * top, most = CHUNK_TOKENS * top;
+    const int t0 = blockIdx.z * CHUNK_TOKENS, first = t0 * top, d0 = blockIdx.x * 16;
+    float* part = smem;                                 // [4][pairs][16]
+    int* of = reinterpret_cast<int*>(part + 4 * most * 16);    // a pair's expert (behind all others: no matrices to read)
+    int* order = of + most;                             // the pairs ordered by expert
+    int* start = order + most;                          // where an expert's pairs begin
+    __shared__ int n_live, n_used;
+    grid_dep_launch();
+    grid_dep_wait();
+    if (threadIdx.x == 0) n_live = n_used = 0;
+    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+        const int e = idx[first + p];
+        of[p] = e < n_experts && tok_slot[t0 + p / top] >= 0 ? e : 0x7fffffff;
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+        const int e = of[p];
+        int rank = 0, before = 0;
+        bool opens = e != 0x7fffffff;
+        for (int q = 0; q < n_pairs; ++q) {
+            const int o = of[q];
+            rank += o < e || (o == e && q < p);
+            if (o == e && q < p) opens = false;
+        }
+        order[rank] = p;
+        if (e != 0x7fffffff) atomicAdd(&n_live, 1);
+        if (opens) {                                    // experts in use below this one
+            for (int q = 0; q < n_pairs; ++q) {
+                if (of[q] >= e) continue;
+                bool once = true;
+                for (int r = 0; r < q; ++r) once &= of[r] != of[q];
+                before += once;
+            }
+            start[before] = rank;
+            atomicAdd(&n_used, 1);
+        }
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, quarter = warp & 3;
+    for (int u = warp >> 2; u < n_used; u += 2) {
+        const int lo = start[u], hi = u + 1 < n_used ? start[u + 1] : n_live;
+        const __nv_bfloat16* w = w_down + (size_t)of[order[lo]] * D * F;
+        for (int c = lo; c < hi; c += 32) {
+            const int m = min(32, hi - c);
+            float* mine = part + quarter * most * 16;
+            if (m <= 8) down_columns<1>(mine, hidden, ldh, w, order + c, m, first, D, F, d0, quarter);
+            else if (m <= 16) down_columns<2>(mine, hidden, ldh, w, order + c, m, first, D, F, d0, quarter);
+            else down_columns<4>(mine, hidden, ldh, w, order + c, m, first, D, F, d0, quarter);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < tokens * 16; e += blockDim.x) {
+        const int t = e >> 4, r = e & 15, d = d0 + r;
+        if (d >= D) continue;
+        const size_t row = t0 + t;
+        float total = 0.f;
+        if (tok_slot[row] >= 0) {
+            for (int j = 0; j < top; ++j) {
+                const int p = t * top + j;
+                float y;
+                if (of[p] == 0x7fffffff) y = __bfloat162float(x[row * ldx + d]);
+                else {
+                    y = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) y += part[(q * most + p) * 16 + r];
+                }
+                total = fmaf(wts[row * top + j], y, total);
+            }
+            if (add) total = fmaf(load_as_f32(add, add_dtype, row * ldadd + d), add_scale ? add_scale[row] : 1.0f, total);
+        }
+        out[row * ldo + d] = total;
+    }
+}
+
 // The (token, choice) pairs ordered by expert, by one block: offsets[e] .. offsets[e + 1] are expert e's places,
 // place_token[p] the token whose row goes there, pair_place[pair] the place of a pair.  Pairs of padding rows
 // (slot < 0) are counted for the expert they name: their rows are zeros and nobody reads their results.
@@ -205,17 +439,43 @@ __global__ void moe_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restri
 }
 
 // out[t, :] = sum_j wts[t, j] * y[pair_place[t * top + j], :]  (+ add[t, :] * add_scale[t]), in 32-bit; a place from n_rows on
-// stands for the token's own input x[t, :].
-template <typename TY>
+// (`rows_dev`: the number read on the device) stands for the token's own input x[t, :].  VEC: four elements at a time.
+template <typename TY, bool VEC>
 __global__ void moe_combine_kernel(float* __restrict__ out, size_t ldo, const TY* __restrict__ y, size_t ldy,
                                    const int32_t* __restrict__ pair_place, const float* __restrict__ wts,
                                    const int32_t* __restrict__ tok_slot, const void* __restrict__ add, int add_dtype,
                                    size_t ldadd, const float* __restrict__ add_scale, int top, int D, const void* __restrict__ x,
-                                   int x_dtype, size_t ldx, int n_rows) {
+                                   int x_dtype, size_t ldx, int n_rows, const int32_t* __restrict__ rows_dev) {
     grid_dep_launch();
     grid_dep_wait();
     const size_t t = blockIdx.x;
     const bool live = tok_slot[t] >= 0;
+    if (rows_dev) n_rows = *rows_dev;
+    if (VEC) {
+        for (int d = threadIdx.x * 4; d < D; d += blockDim.x * 4) {
+            float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live) {
+#pragma unroll 4
+                for (int j = 0; j < top; ++j) {
+                    const int place = pair_place[t * top + j];
+                    const float w = wts[t * top + j];
+                    float4 v;
+                    if (place < n_rows) v = *reinterpret_cast<const float4*>(y + (size_t)place * ldy + d);
+                    else v = make_float4(load_as_f32(x, x_dtype, t * ldx + d), load_as_f32(x, x_dtype, t * ldx + d + 1),
+                                         load_as_f32(x, x_dtype, t * ldx + d + 2), load_as_f32(x, x_dtype, t * ldx + d + 3));
+                    total.x = fmaf(w, v.x, total.x); total.y = fmaf(w, v.y, total.y); total.z = fmaf(w, v.z, total.z); total.w = fmaf(w, v.w, total.w);
+                }
+                if (add) {
+                    const float w = add_scale ? add_scale[t] : 1.0f;
+                    const size_t at = t * ldadd + d;
+                    total.x = fmaf(load_as_f32(add, add_dtype, at), w, total.x); total.y = fmaf(load_as_f32(add, add_dtype, at + 1), w, total.y);
+                    total.z = fmaf(load_as_f32(add, add_dtype, at + 2), w, total.z); total.w = fmaf(load_as_f32(add, add_dtype, at + 3), w, total.w);
+                }
+            }
+            *reinterpret_cast<float4*>(out + t * ldo + d) = total;
+        }
+        return;
+    }
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
         float total = 0.f;
         if (live) {
@@ -253,6 +513,18 @@ QS_API int qs_moe_expert_up(void* hidden, long long ldh, const void* x, long lon
     if (T == 0) return QS_OK;
     QS_REQUIRE(T > 0 && top > 0 && D > 0 && F > 0, "moe_expert_up: bad sizes");
     QS_REQUIRE((size_t)D * sizeof(float) <= 200 * 1024, "moe_expert_up: width %d does not fit shared memory", D);
+    if (dtype == QS_BF16 && D % 8 == 0 && ldx % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w_up % 16) == 0 &&
+        ((uintptr_t)hidden % 16) == 0 && n_experts <= 65535 && top <= 64) {
+        typedef __nv_bfloat16 bf16;
+        const dim3 blocks((F + 15) / 16, n_experts, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS);
+        const cudaError_t err = gated
+            ? qs_launch_dependent(moe_up_grouped_kernel<true>, blocks, dim3(128), CHUNK_TOKENS * top * sizeof(int), stream, (bf16*)hidden, (size_t)ldh,
+                                  (const bf16*)x, (size_t)ldx, (const bf16*)w_up, idx, tok_slot, T, top, D, F, act, n_experts)
+            : qs_launch_dependent(moe_up_grouped_kernel<false>, blocks, dim3(128), CHUNK_TOKENS * top * sizeof(int), stream, (bf16*)hidden, (size_t)ldh,
+                                  (const bf16*)x, (size_t)ldx, (const bf16*)w_up, idx, tok_slot, T, top, D, F, act, n_experts);
+        if (err != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "moe_expert_up: %s", cudaGetErrorString(err));
+        return qs_check_launch("moe_expert_up");
+    }
     const int rows_per_block = 32;
     const size_t smem = (size_t)D * sizeof(float);
     const int vec = D % 8 == 0 && ((uintptr_t)w_up % 16) == 0;
@@ -277,6 +549,17 @@ QS_API int qs_moe_expert_down(float* out, long long ldo, const void* hidden, lon
     QS_REQUIRE(T > 0 && top > 0 && D > 0 && F > 0, "moe_expert_down: bad sizes");
     const size_t smem = (size_t)top * F * sizeof(float);
     QS_REQUIRE(smem <= 200 * 1024, "moe_expert_down: %d x %d hidden values do not fit shared memory", top, F);
+    const size_t grouped = (size_t)CHUNK_TOKENS * top * (4 * 16 + 3) * sizeof(float);
+    if (dtype == QS_BF16 && F % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)hidden % 16) == 0 && ((uintptr_t)w_down % 16) == 0 && top <= 16) {
+        cudaError_t err = cudaSuccess;
+        if (grouped > 48 * 1024) err = cudaFuncSetAttribute(moe_down_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grouped);
+        if (err == cudaSuccess)
+            err = qs_launch_dependent(moe_down_grouped_kernel, dim3((D + 15) / 16, 1, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS), dim3(256), grouped, stream, out, (size_t)ldo,
+                                      (const __nv_bfloat16*)hidden, (size_t)ldh, (const __nv_bfloat16*)w_down, idx, wts, tok_slot, add, add_dtype, (size_t)ldadd, add_scale,
+                                      T, top, D, F, (const __nv_bfloat16*)x, (size_t)ldx, n_experts);
+        if (err != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "moe_expert_down: %s", cudaGetErrorString(err));
+        return qs_check_launch("moe_expert_down");
+    }
     const int rows_per_block = 32;
     const int vec = F % 8 == 0 && ((uintptr_t)w_down % 16) == 0;
     dim3 grid(T, (D + rows_per_block - 1) / rows_per_block);
@@ -303,15 +586,16 @@ QS_API int qs_moe_sort(int32_t* offsets, int32_t* place_token, int32_t* pair_pla
 QS_API int qs_moe_combine(float* out, long long ldo, const void* y, int y_dtype, long long ldy, const int32_t* pair_place,
                           const float* wts, const int32_t* tok_slot, const void* add, int add_dtype, long long ldadd,
                           const float* add_scale, int T, int top, int D, const void* x, int x_dtype, long long ldx, int n_rows,
-                          cudaStream_t stream) {
+                          const int32_t* rows_dev, cudaStream_t stream) {
     if (T == 0) return QS_OK;
     QS_REQUIRE(T > 0 && top > 0 && D > 0, "moe_combine: bad sizes");
     const int threads = D >= 1024 ? 256 : 128;
     cudaError_t e;
-#define GO(TY) e = qs_launch_dependent(moe_combine_kernel<TY>, dim3(T), dim3(threads), 0, stream, out, (size_t)ldo, (const TY*)y, \
-        (size_t)ldy, pair_place, wts, tok_slot, add, add_dtype, (size_t)ldadd, add_scale, top, D, x, x_dtype, (size_t)ldx, n_rows)
-    if (y_dtype == QS_F32) GO(float);
-    else if (y_dtype == QS_BF16) GO(__nv_bfloat16);
+#define GO(TY, VEC) e = qs_launch_dependent(moe_combine_kernel<TY, VEC>, dim3(T), dim3(threads), 0, stream, out, (size_t)ldo, (const TY*)y, \
+        (size_t)ldy, pair_place, wts, tok_slot, add, add_dtype, (size_t)ldadd, add_scale, top, D, x, x_dtype, (size_t)ldx, n_rows, rows_dev)
+    if (y_dtype == QS_F32 && D % 4 == 0 && ldy % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)y % 16) == 0 && ((uintptr_t)out % 16) == 0) GO(float, true);
+    else if (y_dtype == QS_F32) GO(float, false);
+    else if (y_dtype == QS_BF16) GO(__nv_bfloat16, false);
     else return qs_fail(QS_ERR_INVALID_INPUT, "moe_combine: unknown dtype %d", y_dtype);
 #undef GO
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "moe_combine: %s", cudaGetErrorString(e));

@@ -103,6 +103,7 @@ _SIGNATURES = {
                             c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p], c_int),
     "qs_head_linear": ([c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int,
                         c_int, c_int, c_void_p], c_int),
+    "qs_gemm_tc_grouped": ([c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     "qs_scan_activate": ([c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p], c_int),
     "qs_moe_route": ([c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                       c_int, c_float, c_int, c_int, c_int, c_float, c_void_p], c_int),
@@ -112,7 +113,7 @@ _SIGNATURES = {
                             c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p], c_int),
     "qs_moe_sort": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p], c_int),
     "qs_moe_combine": ([c_void_p, c_longlong, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                        c_longlong, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p], c_int),
+                        c_longlong, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p], c_int),
     "qs_token_shift": ([c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_longlong,
                         c_void_p, c_void_p, c_int, c_int, c_int, c_void_p], c_int),
     "qs_argmax": ([c_void_p, c_void_p, c_int, c_int, c_longlong, c_void_p], c_int),
@@ -1035,10 +1036,23 @@ def expert_products(out, x, w_all, offsets) -> None:
     check(rc)
 
 
-def moe_combine(y, pair_place, wts, tok_slot, add=None, add_scale=None, x=None) -> torch.Tensor:
+def grouped_products(out, x, w_all, offsets) -> None:
+    """`expert_products` with the rows' bounds on the device (int32 [>= experts + 1], the first experts + 1 count): one launch, for
+    bfloat16 operands that the tensor-core product takes.  Rows of no expert are left alone."""
+    from . import gemm_tc
+    E, N, K = w_all.shape
+    rows, K2, lda = _rows(x)
+    if K2 != K or out.shape != (rows, N) or out.stride(1) != 1 or not w_all.is_contiguous() or offsets.numel() < E + 1:
+        raise QStreamError(QsError.INVALID_INPUT, "grouped_products: operands do not fit")
+    check(library().qs_gemm_tc_grouped(ptr(out), dtype_code(out), out.stride(0), ptr(x), lda, ptr(w_all), _int32(offsets, "offsets"), E, rows, N, K,
+                                       ptr(gemm_tc.status_word(x.device)), stream()))
+
+
+def moe_combine(y, pair_place, wts, tok_slot, add=None, add_scale=None, x=None, n_rows=None) -> torch.Tensor:
     """out[t] = sum_j wts[t, j] y[pair_place[t, j]] (+ add[t] * add_scale[t]) in float32.  With `x` [T, D] a place behind y's last
-    row stands for x[t] (an expert that returns its input)."""
-    n_rows, D, ldy = _rows(y)
+    row stands for x[t] (an expert that returns its input); `n_rows` (one int32 on the device): how many rows of y count,
+    where the host does not know."""
+    all_rows, D, ldy = _rows(y)
     if x is not None and (x.shape != (wts.shape[0], D) or x.stride(1) != 1):
         raise QStreamError(QsError.INVALID_INPUT, "moe_combine: the tokens' inputs do not fit")
     T, top = wts.shape
@@ -1046,7 +1060,7 @@ def moe_combine(y, pair_place, wts, tok_slot, add=None, add_scale=None, x=None) 
     check(library().qs_moe_combine(ptr(out), D, ptr(y), dtype_code(y), ldy, ptr(pair_place), ptr(wts),
                                    _int32(tok_slot, "tok_slot"), ptr(add), _code(add), add.stride(0) if add is not None else 0,
                                    ptr(add_scale), T, top, D, ptr(x), _code(x), x.stride(0) if x is not None else 0,
-                                   n_rows if x is not None else 2**31 - 1, stream()))
+                                   all_rows if x is not None else 2**31 - 1, ptr(n_rows) if x is not None else None, stream()))
     return out
 
 

@@ -99,7 +99,7 @@ class RoutedExperts(FeedForward):
     (an expert's gate rows stacked above its up rows in one matrix; the clamped gated unit is a kernel of its own
     between the two products), and `identity` more router outputs whose expert returns its input (the kernels that add a
     token's results up read the input itself there)."""
-    captures_any_step = False           # a step with many tokens reads the experts' row counts on the host
+    captures_any_step = False           # a step with many tokens may read the experts' row counts on the host (float32)
 
     @classmethod
     def declare(cls, spec):
@@ -155,6 +155,7 @@ class RoutedExperts(FeedForward):
 
     def forward(self, h, step, residuals=(), out_dtype=None):
         import torch
+        from ..csrc import gemm_tc
         s, b = self.spec, step.batch
         z = linear(h, self.w_router, out_dtype=torch.float32)
         idx, wts, gate = ops.moe_route(z, self.correction, self.outputs, s.top, s.groups, s.keep, s.route_scale,
@@ -171,19 +172,26 @@ class RoutedExperts(FeedForward):
         else:
             offsets, place_token, pair_place = ops.moe_sort(idx, self.outputs)
             rows = ops.gather_rows(h, place_token)
-            bounds = offsets.tolist()[:s.n_experts + 1]     # waits for the device: how many rows each expert got
-            rows = rows[:bounds[-1]]                        # behind them lie the pairs whose expert returns its input
+            # on the tensor cores all experts' products are one launch that finds their rows on the device; else the host reads how
+            # many rows each expert got and launches a product per expert
+            grouped = gemm_tc.takes(rows, self.w_up[0]) and self.w_down.shape[2] % 8 == 0 and self.w_down.data_ptr() % 16 == 0
+            if not grouped:
+                bounds = offsets.tolist()[:s.n_experts + 1]
+                rows = rows[:bounds[-1]]                    # behind them lie the pairs whose expert returns its input
+            products = ops.grouped_products if grouped else ops.expert_products
+            bounds = offsets if grouped else bounds
             hidden = torch.empty((rows.shape[0], self.w_up.shape[1]), dtype=h.dtype, device=h.device)
             y = torch.empty((rows.shape[0], s.width), dtype=torch.float32, device=h.device)
-            ops.expert_products(hidden, rows, self.w_up, bounds)        # a product per expert, launched by one call
+            products(hidden, rows, self.w_up, bounds)
             if self.gated == "act":
                 hidden = ops.gated_act(hidden, s.activation)            # one launch for all experts' rows
             elif self.gated:
                 hidden = ops.clamped_glu(hidden, *self.glu)
             else:
                 ops.activate(hidden, s.activation)
-            ops.expert_products(y, hidden, self.w_down, bounds)
-            out = ops.moe_combine(y, pair_place, wts, b.tok_slot, shared, gate, x=h if self.outputs > s.n_experts else None)
+            products(y, hidden, self.w_down, bounds)
+            out = ops.moe_combine(y, pair_place, wts, b.tok_slot, shared, gate, x=h if self.outputs > s.n_experts else None,
+                                  n_rows=offsets[s.n_experts:s.n_experts + 1] if grouped else None)
         if residuals:
             raise QStreamError(QsError.INVALID_INPUT, "routed experts: residuals are added by the arrangement")
         return out if out_dtype in (None, torch.float32) else ops.convert(out, out_dtype)
