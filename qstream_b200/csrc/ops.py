@@ -72,8 +72,9 @@ _SIGNATURES = {
                        c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
                        c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                        c_void_p, c_void_p, c_longlong, c_float, c_int, c_float, c_void_p], c_int),
-    "qs_delta_chunk_prefix": ([c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                               c_void_p], c_int),
+    "qs_delta_chunks_scratch": ([c_int, c_int, c_int, c_int], c_longlong),
+    "qs_delta_chunks": ([c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
+                         c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p], c_int),
     "qs_mlstm_gates": ([c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_float, c_void_p, c_longlong,
                         c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     "qs_mlstm_output": ([c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int,
@@ -577,9 +578,8 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     a column of ones, whose state is the normaliser n <- a_t n + b_t k and whose output n.q is each head's last element.
     mode "delta": S' = diag(g_t) S, u = beta_t (v - S'^T k), S <- S' + k u^T, o = S^T q, with g = `key_decay` (float32
     [T, heads * key_dim]) and beta = `token_weight` (float32 [T, heads]); q and k hold heads / `qk_group` heads, head h
-    reading number h // qk_group.  With `chunks` the delta rule runs the same walk three times over the chunks side by
-    side (what a chunk does to an identity, what it writes from an empty state, and, once a prefix over the chunks has
-    given each its starting state, the chunk's outputs).  In mode "decay" `q_scale` multiplies q as well.
+    reading number h // qk_group.  With `chunks` the delta rule solves each chunk's writes as a triangular system, side by
+    side, and walks the chunks in order (csrc/delta_chunks.cu; float32 operands).  In mode "decay" `q_scale` multiplies q as well.
     mode "gla": S <- diag(w_t) S + k v^T, o = S^T (q q_scale), w_t = sigmoid(decay_logits)^`decay_power` per token and key
     channel (float32 [T, heads * key_dim]), taken in 32-bit inside the walk.
     mode "ssd": S <- a_t S + b_t k v^T, o = S^T (q q_scale) with a - 1 = `token_decay`, b = `token_weight` (float32
@@ -630,21 +630,21 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
 
 
 def _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_dim, key_decay, token_weight, qk_group, chunks):
-    """The delta rule of a long prompt, its chunks side by side.  A chunk acts on the state it starts from as
-    S <- P S + Q: P is what the chunk's walk (values of zero) makes of an identity, Q what it writes from an empty state;
-    `qs_delta_chunk_prefix` then gives every chunk its starting state and the slot its last one, and the walk runs once
-    more for the outputs.  The same arithmetic as the walk in order, regrouped; nothing is divided by a decay."""
+    """The delta rule of a long prompt, its chunks as matrix products (csrc/delta_chunks.cu): what each chunk's tokens ask of the
+    state it starts from and what they write, side by side; the chunks' states in order; the outputs, side by side."""
     chunk_start, chunk_ids, seq_chunk, n_chunks = chunks
-    dev = q.device
-    P = torch.eye(key_dim, dtype=torch.float32, device=dev).repeat(n_chunks, n_heads, 1, 1)
-    Q = torch.zeros((n_chunks, n_heads, value_dim, key_dim), dtype=torch.float32, device=dev)
-    walk = dict(key_decay=key_decay, token_weight=token_weight, qk_group=qk_group)
-    state_scan("delta", q, k, None, P, chunk_start, chunk_ids, n_chunks, n_heads, key_dim, key_dim, want_output=False, **walk)
-    state_scan("delta", q, k, v, Q, chunk_start, chunk_ids, n_chunks, n_heads, key_dim, value_dim, want_output=False, **walk)
-    start = torch.empty_like(Q)
-    check(library().qs_delta_chunk_prefix(ptr(P), ptr(Q), ptr(start), ptr(state), state.stride(0), _int32(seq_chunk, "seq_chunk"),
-                                          _int32(seq_slot, "seq_slot"), int(n_seq), n_heads, key_dim, value_dim, stream()))
-    return state_scan("delta", q, k, v, start, chunk_start, chunk_ids, n_chunks, n_heads, key_dim, value_dim, **walk)
+    T = q.shape[0]
+    if any(t.dtype != torch.float32 or t.stride(1) != 1 for t in (q, k, v, key_decay, token_weight)):
+        raise QStreamError(QsError.INVALID_INPUT, "state_scan: the delta rule in chunks takes float32 operands")
+    lib = library()
+    o = torch.empty((T, n_heads * value_dim), dtype=torch.float32, device=q.device)
+    scratch = torch.empty((lib.qs_delta_chunks_scratch(int(n_chunks), n_heads, key_dim, value_dim),), dtype=torch.float32, device=q.device)
+    check(lib.qs_delta_chunks(ptr(o), o.stride(0), ptr(q), q.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), ptr(key_decay), key_decay.stride(0),
+                              ptr(token_weight), token_weight.stride(0), ptr(state), state.stride(0), _int32(seq_slot, "seq_slot"), int(n_seq), T,
+                              n_heads, int(qk_group), key_dim, value_dim, _int32(chunk_start, "chunk_start"), int(n_chunks),
+                              _int32(seq_chunk, "seq_chunk"), ptr(scratch), stream()))
+    count_launches(2)
+    return o
 
 
 def delta_prepare(q, k, v, conv_q, conv_k, conv_v, conv_state, a, b, a_log, tok_slot, tok_pos, n_qk_heads, n_heads,

@@ -12,7 +12,7 @@
 //       S' = diag(g_t) S_{t-1},   u_t = beta_t (v_t - S'^T k_t),   S_t = S' + k_t u_t^T,   o_t = S_t^T q_t
 //       (q, k, v arrive ready: activated, normed, scaled; several heads may share one head of q and k).  A column of S
 //       does not meet the others, so the threads of a column pair take S'^T k, S'^T q and k.q in one round of
-//       shuffles, and o_t = S'^T q + u_t (k.q).  In order only (PHASE 0).
+//       shuffles, and o_t = S'^T q + u_t (k.q).  Long prompts: delta_chunks.cu.
 //   gated linear attention with a decay per token and key channel ("gla"):
 //       S_t = diag(w_t) S_{t-1} + k_t v_t^T,   o_t = S_t^T (q_t * q_scale),   w_t = sigmoid(z_t)^decay_scale
 //       (the decay acts before the token's own output, where "wkv" applies it after)
@@ -329,76 +329,6 @@ __global__ void token_shift_kernel(T* __restrict__ out, size_t ldo, size_t mix_s
         const float diff = (before ? to_f32(before[i]) : 0.f) - cur;
         for (int m = 0; m < n_mix; ++m)
             out[(size_t)m * mix_stride + (size_t)t * ldo + i] = from_f32<T>(fmaf(diff, mu[(size_t)m * D + i], cur));
-    }
-}
-
-// The delta rule over chunks that ran side by side.  A chunk's tokens act on the state as S <- P S + Q, with
-// P = A_n .. A_1 (A_t = (I - beta_t k_t k_t^T) diag(g_t), the same for every value column) and Q what the chunk
-// writes from an empty state; both come from the scan itself (P: the scan of an identity with values of zero).  This
-// kernel walks a sequence's chunks in order: it leaves in `start` the state each chunk starts from and in the slot the
-// state after the last.  Layouts as the state's: P [chunks][H][dk (column j)][dk (row i)], Q and start
-// [chunks][H][dv][dk].  A block owns DCB value columns of one head; nothing is divided by a decay, so small decays
-// cost no precision.
-constexpr int DCB = 16;
-__global__ void __launch_bounds__(128)
-delta_chunk_prefix_kernel(const float* __restrict__ P, const float* __restrict__ Q, float* __restrict__ start,
-                          float* __restrict__ state, size_t slot_stride, const int32_t* __restrict__ seq_chunk,
-                          const int32_t* __restrict__ seq_slot, int H, int dk, int dv) {
-    extern __shared__ float s_cur[];                    // [dk][DCB]: the state's rows of this block's columns
-    grid_dep_launch();
-    grid_dep_wait();
-    const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * DCB;
-    const int slot = seq_slot[s];
-    if (slot < 0) return;
-    const int n_cols = min(DCB, dv - col0);
-    float* mine = state + (size_t)slot * slot_stride + ((size_t)h * dv + col0) * dk;
-    for (int e = threadIdx.x; e < DCB * dk; e += blockDim.x) {
-        const int c = e / dk, i = e - c * dk;
-        s_cur[i * DCB + c] = c < n_cols ? mine[(size_t)c * dk + i] : 0.f;
-    }
-    for (int ch = seq_chunk[s]; ch < seq_chunk[s + 1]; ++ch) {
-        __syncthreads();
-        float* st = start + (((size_t)ch * H + h) * dv + col0) * dk;
-        for (int e = threadIdx.x; e < n_cols * dk; e += blockDim.x) {
-            const int c = e / dk, i = e - c * dk;
-            st[(size_t)c * dk + i] = s_cur[i * DCB + c];
-        }
-        const float* Pc = P + ((size_t)ch * H + h) * dk * dk;
-        const float* Qc = Q + (((size_t)ch * H + h) * dv + col0) * dk;
-        float acc[2][DCB];                              // rows threadIdx.x and threadIdx.x + 128 (dk is at most 256)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int i = threadIdx.x + r * 128;
-#pragma unroll
-            for (int c = 0; c < DCB; ++c) acc[r][c] = (i < dk && c < n_cols) ? Qc[(size_t)c * dk + i] : 0.f;
-        }
-        for (int j = 0; j < dk; ++j) {
-            const float p0 = threadIdx.x < dk ? Pc[(size_t)j * dk + threadIdx.x] : 0.f;
-            const float p1 = threadIdx.x + 128 < dk ? Pc[(size_t)j * dk + threadIdx.x + 128] : 0.f;
-            const float4* row = reinterpret_cast<const float4*>(s_cur + j * DCB);
-#pragma unroll
-            for (int c4 = 0; c4 < DCB / 4; ++c4) {
-                const float4 x = row[c4];
-                acc[0][4 * c4] = fmaf(p0, x.x, acc[0][4 * c4]);         acc[1][4 * c4] = fmaf(p1, x.x, acc[1][4 * c4]);
-                acc[0][4 * c4 + 1] = fmaf(p0, x.y, acc[0][4 * c4 + 1]); acc[1][4 * c4 + 1] = fmaf(p1, x.y, acc[1][4 * c4 + 1]);
-                acc[0][4 * c4 + 2] = fmaf(p0, x.z, acc[0][4 * c4 + 2]); acc[1][4 * c4 + 2] = fmaf(p1, x.z, acc[1][4 * c4 + 2]);
-                acc[0][4 * c4 + 3] = fmaf(p0, x.w, acc[0][4 * c4 + 3]); acc[1][4 * c4 + 3] = fmaf(p1, x.w, acc[1][4 * c4 + 3]);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int i = threadIdx.x + r * 128;
-            if (i < dk) {
-#pragma unroll
-                for (int c = 0; c < DCB; ++c) s_cur[i * DCB + c] = acc[r][c];
-            }
-        }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n_cols * dk; e += blockDim.x) {
-        const int c = e / dk, i = e - c * dk;
-        mine[(size_t)c * dk + i] = s_cur[i * DCB + c];
     }
 }
 
@@ -723,18 +653,6 @@ QS_API int qs_state_scan(int mode, float* o, long long ldo, const void* q, long 
 
 // See delta_chunk_prefix_kernel.  seq_chunk (n_seq + 1) names each sequence's chunks; a sequence's slot must be a row
 // of `state` (or negative: skipped).
-QS_API int qs_delta_chunk_prefix(const float* P, const float* Q, float* start, float* state, long long slot_stride,
-                                 const int32_t* seq_chunk, const int32_t* seq_slot, int n_seq, int H, int dk, int dv,
-                                 cudaStream_t stream) {
-    if (n_seq == 0) return QS_OK;
-    QS_REQUIRE(n_seq > 0 && H > 0 && dk > 0 && dk <= 256 && dv > 0 && H <= 65535, "delta_chunk_prefix: bad sizes");
-    const size_t smem = (size_t)dk * DCB * sizeof(float);
-    cudaError_t e = qs_launch_dependent(delta_chunk_prefix_kernel, dim3(n_seq, H, (dv + DCB - 1) / DCB), dim3(128), smem, stream,
-                                        P, Q, start, state, (size_t)slot_stride, seq_chunk, seq_slot, H, dk, dv);
-    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "delta_chunk_prefix: %s", cudaGetErrorString(e));
-    return qs_check_launch("delta_chunk_prefix");
-}
-
 QS_API int qs_token_shift(void* out, long long ldo, long long mix_stride, const void* h, long long ldh, int dtype,
                           const float* mu, const void* last_row, long long ld_last, const int32_t* tok_slot,
                           const int32_t* tok_pos, int T, int D, int n_mix, cudaStream_t stream) {

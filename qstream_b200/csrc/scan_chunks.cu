@@ -21,15 +21,9 @@
 // 600 | 422; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 329; state-space form, 2,048 tokens, 64 heads of
 // 128 x 64: 822 | 458 | 388 (its output kernel 154, what the chunks add 67).
 #include "scan.cuh"
+#include "scan_tiles.cuh"
 
 namespace {
-
-constexpr int CT = 64;                                  // tokens of a chunk
-constexpr int THREADS = 128;
-
-// Where channel c's column of a staged [channels][64 tokens] tile lies: tokens in groups of four, permuted by the channel's
-// group of four, so that a warp that writes 8 x 4 channels of four tokens meets every bank once.
-__device__ __forceinline__ int at_ct(int c, int t) { return c * CT + (t ^ (((c >> 2) & 7) << 2)); }
 
 struct Scan {
     const void *q, *k, *v;
@@ -59,42 +53,6 @@ __device__ __forceinline__ float decay_at(const Scan& p, size_t t, int h, int i)
 template <int MODE>
 __device__ __forceinline__ float times_decay(float x, float a) { return MODE == 5 ? fmaf(x, a, x) : x * a; }
 
-// Four neighbouring elements of a row, zeros behind its end: fetched in one step and turned into 32-bit numbers in another, so that
-// many fetches are under way before the first is waited for.
-template <typename TI> struct Raw4;
-template <> struct Raw4<float> {
-    float4 x;
-    __device__ __forceinline__ void get(const float* p) { x = *reinterpret_cast<const float4*>(p); }
-    __device__ __forceinline__ void zero() { x = make_float4(0.f, 0.f, 0.f, 0.f); }
-    __device__ __forceinline__ float4 value() const { return x; }
-};
-template <> struct Raw4<__nv_bfloat16> {
-    uint2 x;
-    __device__ __forceinline__ void get(const __nv_bfloat16* p) { x = *reinterpret_cast<const uint2*>(p); }
-    __device__ __forceinline__ void zero() { x = make_uint2(0u, 0u); }
-    __device__ __forceinline__ float4 value() const {
-        return make_float4(__uint_as_float(x.x << 16), __uint_as_float(x.x & 0xffff0000u), __uint_as_float(x.y << 16), __uint_as_float(x.y & 0xffff0000u));
-    }
-};
-template <typename TI>
-__device__ __forceinline__ void get_four(Raw4<TI>& r, const TI* __restrict__ row, int i, int n, bool have, int vec) {
-    if (!have || i >= n) { r.zero(); return; }
-    if (vec) { r.get(row + i); return; }
-    TI f[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) f[j] = i + j < n ? row[i + j] : from_f32<TI>(0.f);
-    if constexpr (sizeof(TI) == 4) r.x = make_float4(f[0], f[1], f[2], f[3]);
-    else {
-        const __nv_bfloat162 a = __halves2bfloat162(f[0], f[1]), b = __halves2bfloat162(f[2], f[3]);
-        r.x = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-    }
-}
-__device__ __forceinline__ void copy16(float* dst, const float* src, bool have) {       // asynchronous; zeros where there is nothing
-    if (have) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-    else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // A chunk of more than 64 tokens (the callers cut none): this block's columns of the state walked in order in global memory.
 template <typename TI, int MODE>
 __device__ void walk_in_order(const Scan& p, float* __restrict__ S, int c, int h, int col0, int cols, bool output) {
@@ -116,31 +74,6 @@ __device__ void walk_in_order(const Scan& p, float* __restrict__ S, int c, int h
                 *s = after;
             }
             if (output) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col] = o;
-        }
-    }
-}
-
-// acc[8][4 NC] += A[k][8 rows] B[k][4 NC columns] over k < n: A a [k][64] tile (rows 4 ty .. and 32 + 4 ty ..; SKEW: swizzled as by
-// at_ct), B rows of 64 NC columns (4 tx .. of every 64).
-template <int NC, bool SKEW>
-__device__ __forceinline__ void tile_product(f32x2 (&acc)[8][2 * NC], const float* __restrict__ A, const float* __restrict__ B, int n, int ty, int tx) {
-#pragma unroll 4
-    for (int k = 0; k < n; ++k) {
-        const float4 x = *reinterpret_cast<const float4*>(A + (SKEW ? at_ct(k, ty * 4) : k * CT + ty * 4));
-        const float4 y = *reinterpret_cast<const float4*>(A + (SKEW ? at_ct(k, 32 + ty * 4) : k * CT + 32 + ty * 4));
-        const float a[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-        f32x2 b[2 * NC];
-#pragma unroll
-        for (int g = 0; g < NC; ++g) {
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(B + k * 64 * NC + g * 64 + tx * 4);
-            b[2 * g] = w.x;
-            b[2 * g + 1] = w.y;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const f32x2 aa = pack2(a[i], a[i]);
-#pragma unroll
-            for (int j = 0; j < 2 * NC; ++j) acc[i][j] = fma2(aa, b[j], acc[i][j]);
         }
     }
 }
@@ -287,7 +220,6 @@ __global__ void __launch_bounds__(THREADS, 3)
 chunk_output_kernel(Scan p) {
     constexpr bool PER_CHANNEL = MODE == 1 || MODE == 4, ONES = MODE == 2, WKV = MODE == 1;
     constexpr int SL = PER_CHANNEL ? 64 : 32;           // channels of a slice
-    constexpr int PP = CT + 4;                          // pitch of the weights P[j][t]
     constexpr int COLS = 64 * NC, NQ = CT * SL / 4 / THREADS, NV = CT * 16 * NC / THREADS;
     extern __shared__ __align__(16) float smem[];
     float* sq = smem;                                   // [SL][64 tokens]
@@ -544,38 +476,8 @@ chunk_output_kernel(Scan p) {
         *reinterpret_cast<float4*>(svv + (tid + x * THREADS) * 4) = f;
     }
     odd = __syncthreads_or(odd);
-    // tokens j: the first 32 meet every t, the others only the last 32
-    auto add_values = [&](bool later_only) {
-#pragma unroll 2
-        for (int j = 0; j < n; ++j) {
-            f32x2 b[2 * NC];
-#pragma unroll
-            for (int g = 0; g < NC; ++g) {
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(svv + j * 64 * NC + g * 64 + tx * 4);
-                b[2 * g] = w.x;
-                b[2 * g + 1] = w.y;
-            }
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                if (g == 0 && j >= 32) continue;
-#pragma unroll
-                for (int x = 0; x < NH; ++x) {
-                    const float4 w = *reinterpret_cast<const float4*>(sp + (x * CT + j) * PP + g * 32 + ty * 4);
-                    const float a[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        if (later_only && g * 32 + ty * 4 + i < j) continue;
-                        const f32x2 aa = pack2(a[i], a[i]);
-#pragma unroll
-                        for (int y = 0; y < 2 * NC; ++y)
-                            if (NH == 1 || (y >> 1) == x) acc[g * 4 + i][y] = fma2(aa, b[y], acc[g * 4 + i][y]);
-                    }
-                }
-            }
-        }
-    };
-    if (odd) add_values(true);
-    else add_values(false);
+    if (odd) add_values<NC, NH, true>(acc, sp, svv, n, ty, tx);
+    else add_values<NC, NH, false>(acc, sp, svv, n, ty, tx);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int t = (i >> 2) * 32 + ty * 4 + (i & 3);
