@@ -264,8 +264,7 @@ __global__ void rope_store_vec_kernel(__nv_bfloat16* __restrict__ q, const __nv_
 // ----------------------------------------------------------------------------- attention
 
 // One warp per (token, query head).  Keys are visited 32 at a time in position order (groups of 32 positions counted
-// from the sequence's first token): lane l scores key base+l (s = q.k / sqrt(dh), QStream src/engine.c:888-906; the
-// even and the odd dims in a sum each), the
+// from the sequence's first token): lane l scores key base+l (s = q.k / sqrt(dh), QStream src/engine.c:888-906), the
 // running maximum and sum are updated (softmax with max subtraction,
 // src/kernels_scalar.c:188-213, in its streaming form) and the 32 weighted values are
 // added in key order (src/engine.c:913-922).  Scores, maximum, exponentials, sum and
@@ -331,14 +330,9 @@ attention_kernel(TO* __restrict__ out, const T* __restrict__ q, size_t ldo, size
                 const size_t off = ((size_t)page * n_kv_heads + kvh) * page_tokens + (key & (page_tokens - 1));
                 const T* krow = k_cache + off * krow_width + k_off;
                 vrow = v_cache + off * dv;
-                float even = 0.f, odd = 0.f;
-                int d = 0;
-                for (; d + 1 < dh; d += 2) {
-                    even = fmaf(qs[d], to_f32(krow[d]), even);
-                    odd = fmaf(qs[d + 1], to_f32(krow[d + 1]), odd);
-                }
-                if (d < dh) even = fmaf(qs[d], to_f32(krow[d]), even);
-                s = (even + odd) * scale;
+                float dot = 0.f;
+                for (int d = 0; d < dh; ++d) dot = fmaf(qs[d], to_f32(krow[d]), dot);
+                s = dot * scale;
                 if (softcap > 0.f) s = softcap * tanhf(s / softcap);
             }
         }
@@ -379,7 +373,7 @@ attention_kernel(TO* __restrict__ out, const T* __restrict__ q, size_t ldo, size
 
 // The same for steps that bring many tokens per sequence, in the float32 engine: a block takes 64 consecutive rows of the
 // packed batch and one query head, and walks the sequence's keys 64 at a time with q, keys and values in shared memory.
-// Every sum has the order of `attention_kernel` (groups of 32 keys, even and odd dims, the same tree over a group's
+// Every sum has the order of `attention_kernel` (groups of 32 keys, ascending dims, the same tree over a group's
 // weights), so a row's result is the same bits whichever of the two kernels computes it.  Rows of several sequences in
 // a block: one walk per sequence, the other rows masked.
 //
@@ -409,8 +403,8 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
     __shared__ int s_slot[TQ], s_pos[TQ], s_first[TQ], s_kept[TQ], s_ok[TK], s_end;
     __shared__ float s_alpha[2][TQ];
     const int pitch = dh + 4, vp = NG * 64;
-    float* sq = tile_smem;                              // [TQ][pitch]
-    float* sk = sq + TQ * pitch;                        // [TK][pitch]; after the scores the weights [TK][TQ + 4] lie here
+    float* sq = tile_smem;                              // [dh][TQ + 4]: transposed, so that neighbouring rows form pairs
+    float* sk = sq + dh * (TQ + 4);                      // [TK][pitch]; after the scores the weights [TK][TQ + 4] lie here
     float* sp = sk;
     float* sv = sk + TK * (pitch > TQ + 4 ? pitch : TQ + 4);      // [TK][vp]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -427,9 +421,10 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
         s_kept[tid] = min(keep_first, first);
     }
     for (int e = tid; e < TQ * (dh / 4); e += 128) {
-        const int r = e / (dh / 4), d = (e - r * (dh / 4)) * 4;
-        *reinterpret_cast<float4*>(sq + r * pitch + d) =
-            r < n_rows ? *reinterpret_cast<const float4*>(q + (size_t)(row0 + r) * ldq + (size_t)head * dh + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int r = e % TQ, d = e / TQ * 4;           // neighbouring lanes on neighbouring rows: their stores meet different banks
+        const float4 x = r < n_rows ? *reinterpret_cast<const float4*>(q + (size_t)(row0 + r) * ldq + (size_t)head * dh + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float* dst = sq + d * (TQ + 4) + r;
+        dst[0] = x.x; dst[TQ + 4] = x.y; dst[2 * (TQ + 4)] = x.z; dst[3 * (TQ + 4)] = x.w;
     }
     if (vp > dv)                                        // columns of no value: zeros, once
         for (int e = tid; e < TK * (vp - dv); e += 128) sv[(e / (vp - dv)) * vp + dv + e % (vp - dv)] = 0.f;
@@ -498,20 +493,28 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
             }
             cp_async_wait();
             __syncthreads();
-            f32x2 s2[8][4];
+            f32x2 s2[4][4];                             // rows 2 i, 2 i + 1 of this thread's eight against its four keys
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
             for (int d = 0; d < dh; d += 4) {
-                ulonglong2 kk[4];
+                float4 kk[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const ulonglong2*>(sk + (half * 32 + j * 8 + sub) * pitch + d);
+                for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const float4*>(sk + (half * 32 + j * 8 + sub) * pitch + d);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(sq + row_of(i) * pitch + d);
+                for (int y = 0; y < 4; ++y) {
+                    const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(sq + (d + y) * (TQ + 4) + ty * 4);
+                    const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(sq + (d + y) * (TQ + 4) + 32 + ty * 4);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) s2[i][j] = fma2(qq.y, kk[j].y, fma2(qq.x, kk[j].x, s2[i][j]));
+                    for (int j = 0; j < 4; ++j) {
+                        const float kv = y == 0 ? kk[j].x : y == 1 ? kk[j].y : y == 2 ? kk[j].z : kk[j].w;
+                        const f32x2 k2 = pack2(kv, kv);
+                        s2[0][j] = fma2(qa.x, k2, s2[0][j]);
+                        s2[1][j] = fma2(qa.y, k2, s2[1][j]);
+                        s2[2][j] = fma2(qb.x, k2, s2[2][j]);
+                        s2[3][j] = fma2(qb.y, k2, s2[3][j]);
+                    }
                 }
             }
             __syncthreads();                            // the keys have been read: the weights go where they were
@@ -525,8 +528,8 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
                 for (int j = 0; j < 4; ++j) {
                     const int at = half * 32 + j * 8 + sub, key = base + at;
                     live[j] = mine && key <= pos && (key >= first || key < row_kept) && s_ok[at] >= 0;
-                    const float2 two = unpack2(s2[i][j]);
-                    s[j] = (two.x + two.y) * scale;
+                    const float2 two = unpack2(s2[i >> 1][j]);
+                    s[j] = (i & 1 ? two.y : two.x) * scale;
                     if (softcap > 0.f) s[j] = softcap * tanhf(s[j] / softcap);
                     if (!live[j]) s[j] = -INFINITY;
                 }
@@ -626,7 +629,7 @@ int launch_attention(void* out, const void* q, long long ldo, long long ldq, con
         dh % 4 == 0 && dv % 4 == 0 && dh <= 256 && dv <= 256 && ldq % 4 == 0 && ((uintptr_t)q % 16) == 0 &&
         ((uintptr_t)k_cache % 16) == 0 && ((uintptr_t)v_cache % 16) == 0) {
         const int ng = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4), pitch = dh + 4;
-        const size_t bytes = (size_t)(TQ * pitch + TK * (pitch > TQ + 4 ? pitch : TQ + 4) + TK * ng * 64) * sizeof(float);
+        const size_t bytes = (size_t)(dh * (TQ + 4) + TK * (pitch > TQ + 4 ? pitch : TQ + 4) + TK * ng * 64) * sizeof(float);
         cudaError_t e = cudaSuccess;
 #define GOT(NG_) do { if (bytes > 40 * 1024) e = cudaFuncSetAttribute(attention_tile_kernel<NG_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
         if (e == cudaSuccess) attention_tile_kernel<NG_><<<dim3((T_tokens + TQ - 1) / TQ, n_heads), 128, bytes, stream>>>( \
