@@ -9,13 +9,13 @@
 //   S_end = diag(G_n) S0 + sum_j (g_{j+1} .. g_n k_j) u_j^T,      o_t = (G_t q_t)^T S0 + sum_{j <= t} B[t][j] u_j.
 //
 //   delta_terms_kernel    per chunk and head, side by side: A and B (as for a decay per channel in scan_chunks.cu), the solution by
-//                         substitution with a column pair per thread in registers, the decayed q and k
+//                         substitution with a column per thread in registers, the decayed q and k
 //   delta_walk_kernel     per sequence, head and 16 value columns, the chunks in order: u and the next state, two small products each
 //   delta_output_kernel   per chunk and head, side by side: the outputs
 //
 // All 32-bit; decays only as products of factors up to one.  Three walks of every chunk token by token (what it does to an
 // identity, what it writes from nothing, its outputs) and a product of dk x dk matrices in the prefix stood here before: 2,000 tokens, 16
-// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 532 (the terms 214, the walk 134, the outputs 59).
+// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 422 (the terms 108, the walk 133, the outputs 56).
 #include "scan.cuh"
 #include "scan_tiles.cuh"
 
@@ -39,183 +39,281 @@ struct Delta {
     int vec_q, vec_k, vec_g;
 };
 
-// X[t] <- beta_t R[t] - sum_{j < t} (beta_t A[t][j]) X[j] for two columns per thread, the 64 tokens' values in registers.  minus [64][PP]
-// holds -beta A; rows of R from `rows` on count as zero.
-__device__ __noinline__ void substitute(float* __restrict__ X, int ldx, const float* R, size_t ldr, int cols, int rows, const float* __restrict__ minus,
-                                        const float* __restrict__ beta) {
-    for (int c = 2 * threadIdx.x; c < cols; c += 2 * THREADS) {
-        f32x2 x[CT];
-        const bool two = c + 1 < cols;
+// The terms.  256 threads in four groups of two warps; a group has 32 of the pass's 128 channels and takes them through all steps by
+// itself: inside blocks of 16 tokens the pairs' decays as running products, across blocks as products of q (and k) times the decays
+// since their block's start with k times the decays up to that block.  Then the groups' sums are added, and a thread solves for a
+// column of W or U, its 64 values in registers.
+//
+// Bound by instruction issue and shared memory's pipe (a third and four fifths of their rates).  What it took before, 214 us for 2,000 tokens and 16 heads of 128 x 128, was 36,000 instructions per
+// warp: a condition and two decays per pair of tokens across blocks, a wait of the whole block between steps, two columns and 2,016
+// steps unrolled per thread (more code than the instruction cache holds); now
+// 108 us.
+constexpr int TERMS = 256, GROUPS = 4, GCH = 32, PASS = GROUPS * GCH;
+// a group's sums: pairs of tokens across blocks, [16 t][16 I j] of block I with rows of 16 I + 1 (read along t), and a block's own, [16][17]
+constexpr int CROSS = 16 * (17 + 33 + 49), OWN = 16 * 17;
+constexpr int TERMS_SMEM = (3 * PASS * CT + 4 * PASS) * sizeof(float);
+static_assert(GROUPS * (2 * CROSS + 4 * OWN) + CT * CT <= 3 * PASS * CT, "the groups' sums and A lie over the staged channels");
+// [channel][64 tokens], pieces of four tokens swapped so that neighbouring channels, and every fourth one, meet different banks
+__device__ __forceinline__ int at_pass(int c, int t) { return c * CT + (t ^ (((c ^ (c >> 2)) & 7) << 2)); }
+__device__ __forceinline__ void group_wait(int group) { asm volatile("bar.sync %0, 64;" :: "r"(1 + group) : "memory"); }
+
+// acc[x][pair of t] += sum over the group's channels of X[i][t] k[i][j]: block I's tokens t = 4 (lane / 8) .. + 3 against the earlier
+// blocks' tokens j = 16 m + 2 (lane % 8) + {0, 1}, x = 2 m + {0, 1}
+template <int I>
+__device__ __forceinline__ void cross_product(f32x2 (&acc)[2 * I][2], const float* __restrict__ X, const float* __restrict__ sk, int c0, int lane) {
+#pragma unroll 4
+    for (int i = c0; i < c0 + GCH; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(X + at_pass(i, I * 16 + (lane >> 3) * 4));
 #pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            const float a = t < rows ? R[(size_t)t * ldr + c] : 0.f, b = t < rows && two ? R[(size_t)t * ldr + c + 1] : 0.f;
-            x[t] = pack2(a, b);
-        }
-#pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            const float b = beta[t];
-            f32x2 sum = mul2(pack2(b, b), x[t]);
-#pragma unroll
-            for (int j = 0; j < t; j += 4) {
-                const float4 m = *reinterpret_cast<const float4*>(minus + t * PP + j);
-                sum = fma2(pack2(m.x, m.x), x[j], sum);
-                if (j + 1 < t) sum = fma2(pack2(m.y, m.y), x[j + 1], sum);
-                if (j + 2 < t) sum = fma2(pack2(m.z, m.z), x[j + 2], sum);
-                if (j + 3 < t) sum = fma2(pack2(m.w, m.w), x[j + 3], sum);
-            }
-            x[t] = sum;
-            const float2 v = unpack2(sum);
-            X[(size_t)t * ldx + c] = v.x;
-            if (two) X[(size_t)t * ldx + c + 1] = v.y;
+        for (int m = 0; m < I; ++m) {
+            const float2 b = *reinterpret_cast<const float2*>(sk + at_pass(i, m * 16 + (lane & 7) * 2));
+            const f32x2 b0 = pack2(b.x, b.x), b1 = pack2(b.y, b.y);
+            acc[2 * m][0] = fma2(a.x, b0, acc[2 * m][0]);
+            acc[2 * m][1] = fma2(a.y, b0, acc[2 * m][1]);
+            acc[2 * m + 1][0] = fma2(a.x, b1, acc[2 * m + 1][0]);
+            acc[2 * m + 1][1] = fma2(a.y, b1, acc[2 * m + 1][1]);
         }
     }
 }
+__device__ __forceinline__ int cross_at(int I) { return 16 * (8 * I * (I - 1) + I - 1); }      // where block I's sums begin
+template <int I>
+__device__ __forceinline__ void cross_store(float* __restrict__ dst, const f32x2 (&acc)[2 * I][2], int lane) {
+    dst += cross_at(I);
+#pragma unroll
+    for (int x = 0; x < 2 * I; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            const float2 v = unpack2(acc[x][y]);
+            float* at = dst + ((lane >> 3) * 4 + 2 * y) * (16 * I + 1) + (x >> 1) * 16 + (lane & 7) * 2 + (x & 1);
+            at[0] = v.x;
+            at[16 * I + 1] = v.y;
+        }
+}
+// four tokens of a channel times a decay
+__device__ __forceinline__ void scale_four(float* at, float d) {
+    float4 v = *reinterpret_cast<float4*>(at);
+    v.x *= d; v.y *= d; v.z *= d; v.w *= d;
+    *reinterpret_cast<float4*>(at) = v;
+}
 
-constexpr int SL = 64;                                  // key channels of a slice
-constexpr int TERMS_SMEM = (3 * SL * CT + 2 * CT * PP + 4 * SL) * sizeof(float);
-
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(TERMS, 2)
 delta_terms_kernel(Delta p) {
     extern __shared__ __align__(16) float smem[];
-    float* sq = smem;                                   // [SL][64 tokens]
-    float* sk = sq + SL * CT;
-    float* sw = sk + SL * CT;                           // the decays; then k times the decays since its block's start
-    float* sA = sw + SL * CT;                           // [64 t][PP]
-    float* sB = sA + CT * PP;                           // [64 j][PP]
-    float* edge = sB + CT * PP;                         // [4][SL] the decays of a block of 16 tokens
+    float* sq = smem;                                   // [PASS][64 tokens]: q, then q times the decays since its block's start
+    float* sk = sq + PASS * CT;                         // k, then k times the decays up to its block's end, the next blocks' starts
+    float* sw = sk + PASS * CT;                         // the decays, then k times the decays since its block's start
+    float* edge = sw + PASS * CT;                       // [4][PASS] the decays of a block of 16 tokens
+    float* sums = smem;                                 // after the passes: [GROUPS][B, A][CROSS], [GROUPS][4 blocks][OWN]
+    float* minus = sums + GROUPS * (2 * CROSS + 4 * OWN);       // [64 j][64 t]
     __shared__ float s_beta[CT];
     grid_dep_launch();
     grid_dep_wait();
-    const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, group = tid >> 6, second = tid >> 5 & 1;
     const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, hq = h / p.group;
     if (n <= 0 || n > CT) return;                       // longer chunks are walked token by token
     const size_t unit = (size_t)c * p.H + h;
     if (tid < CT) s_beta[tid] = tid < n ? p.beta[(size_t)(t0 + tid) * p.ldb + h] : 0.f;
-    for (int e = tid; e < 2 * CT * PP; e += THREADS) sA[e] = 0.f;
-    constexpr int FOURS = SL / 4, NQ = CT * FOURS / THREADS;
-    for (int i0 = 0; i0 < p.dkp; i0 += SL) {
-        const int nk = min(SL, p.dk - i0);
-        Raw4<float> rq[NQ], rk[NQ], rg[NQ];
+    const int c0 = group * GCH;                         // the group's channels of a pass
+    const int jj = lane & 15, block = second * 2 + (lane >> 4);         // this lane's token within a block
+    float da[16], db[16];
+    f32x2 x1[2][2], x2[4][2], x3[6][2];
 #pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            const int e = tid + x * THREADS, t = e / FOURS, i = (e % FOURS) * 4;
-            get_four(rq[x], p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk + i0, i, nk, t < n, p.vec_q);
-            get_four(rk[x], p.k + (size_t)(t0 + t) * p.ldk + hq * p.dk + i0, i, nk, t < n, p.vec_k);
-            get_four(rg[x], p.g + (size_t)(t0 + t) * p.ldg + h * p.dk + i0, i, nk, t < n, p.vec_g);
-        }
-        __syncthreads();
+    for (int x = 0; x < 16; ++x) da[x] = db[x] = 0.f;
 #pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            const int e = tid + x * THREADS, t = e / FOURS, i = (e % FOURS) * 4;
-            const float4 a = rq[x].value(), b = rk[x].value(), d = rg[x].value();
-            const float fq[4] = {a.x, a.y, a.z, a.w}, fk[4] = {b.x, b.y, b.z, b.w}, fg[4] = {d.x, d.y, d.z, d.w};
+    for (int x = 0; x < 6; ++x) {
+        if (x < 2) x1[x][0] = x1[x][1] = 0ull;
+        if (x < 4) x2[x][0] = x2[x][1] = 0ull;
+        x3[x][0] = x3[x][1] = 0ull;
+    }
+    for (int i0 = 0; i0 < p.dkp; i0 += PASS) {
+        const int nk = min(PASS, p.dk - i0), i = c0 + (lane & 7) * 4;
+        // eight pieces of four channels by four tokens per step: whole 128-byte lines, and no two lanes of a store on one bank
 #pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                sq[at_ct(i + y, t)] = fq[y];
-                sk[at_ct(i + y, t)] = fk[y];
-                sw[at_ct(i + y, t)] = t < n && i + y < nk ? fg[y] : 1.f;
-            }
-        }
-        __syncthreads();
-        // pairs of tokens within a block of 16, a warp per block: lane = token j and half of the channels
-        {
-            const int jj = lane & 15, b0 = warp * 16;
-            float da[16], db[16];
+        for (int s = 0; s < 8; s += 4) {
+            Raw4<float> rq[4], rk[4], rg[4];
 #pragma unroll
-            for (int x = 0; x < 16; ++x) da[x] = db[x] = 0.f;
-            for (int i = (lane >> 4) * (SL / 2); i < (lane >> 4) * (SL / 2) + SL / 2; ++i) {
-                float run = sk[at_ct(i, b0 + jj)];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(sq + at_ct(i, b0 + 4 * b)), k4 = *reinterpret_cast<const float4*>(sk + at_ct(i, b0 + 4 * b));
-                    const float4 w4 = *reinterpret_cast<const float4*>(sw + at_ct(i, b0 + 4 * b));
-                    const float fq[4] = {q4.x, q4.y, q4.z, q4.w}, fk[4] = {k4.x, k4.y, k4.z, k4.w}, fw[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                    for (int y = 0; y < 4; ++y) {
-                        const int x = 4 * b + y;
-                        if (x > jj) {
-                            run *= fw[y];
-                            da[x] = fmaf(fk[y], run, da[x]);
-                        }
-                        if (x >= jj) db[x] = fmaf(fq[y], run, db[x]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-                const float a = da[x] + __shfl_xor_sync(0xffffffffu, da[x], 16), b = db[x] + __shfl_xor_sync(0xffffffffu, db[x], 16);
-                if (lane < 16 && x >= jj) {
-                    sB[(b0 + jj) * PP + b0 + x] += b;
-                    if (x > jj) sA[(b0 + x) * PP + b0 + jj] += a;
-                }
-            }
-        }
-        __syncthreads();
-        // q and k times the decays since the start of their block of 16, k times those up to the block's end, the block's whole decay
-        for (int e = tid; e < SL * 4; e += THREADS) {
-            const int i = e % SL, b = e / SL;
-            float a[16], run = 1.f;
-#pragma unroll
-            for (int x = 0; x < 16; ++x) a[x] = sw[at_ct(i, b * 16 + x)];
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-                run *= a[x];
-                sq[at_ct(i, b * 16 + x)] *= run;
-                sw[at_ct(i, b * 16 + x)] = sk[at_ct(i, b * 16 + x)] * run;
-            }
-            edge[b * SL + i] = run;
-            run = 1.f;
-#pragma unroll
-            for (int x = 15; x >= 0; --x) {
-                sk[at_ct(i, b * 16 + x)] *= run;
-                run *= a[x];
-            }
-        }
-        __syncthreads();
-        // pairs of blocks: (1,0) (2,0) (2,1) (3,0) (3,1) (3,2); a warp takes eight tokens t against the 16 j of a pair of blocks at a time
-        for (int e = warp; e < 12; e += 4) {
-            const int pair = e >> 1, I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
-            const int t = I * 16 + (e & 1) * 8 + (lane >> 2), j = J * 16 + (lane & 3) * 4;
-            float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-            for (int i = 0; i < SL; ++i) {
-                float d = 1.f;
-                for (int m = J + 1; m < I; ++m) d *= edge[m * SL + i];
-                const float x = sq[at_ct(i, t)] * d, y = sw[at_ct(i, t)] * d;
-                const float4 kk = *reinterpret_cast<const float4*>(sk + at_ct(i, j));
-                sb[0] = fmaf(x, kk.x, sb[0]); sb[1] = fmaf(x, kk.y, sb[1]); sb[2] = fmaf(x, kk.z, sb[2]); sb[3] = fmaf(x, kk.w, sb[3]);
-                sa[0] = fmaf(y, kk.x, sa[0]); sa[1] = fmaf(y, kk.y, sa[1]); sa[2] = fmaf(y, kk.z, sa[2]); sa[3] = fmaf(y, kk.w, sa[3]);
+            for (int x = 0; x < 4; ++x) {
+                const int t = second * 32 + (s + x) * 4 + (lane >> 3);
+                get_four(rq[x], p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk + i0, i, nk, t < n, p.vec_q);
+                get_four(rk[x], p.k + (size_t)(t0 + t) * p.ldk + hq * p.dk + i0, i, nk, t < n, p.vec_k);
+                get_four(rg[x], p.g + (size_t)(t0 + t) * p.ldg + h * p.dk + i0, i, nk, t < n, p.vec_g);
             }
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                sB[(j + x) * PP + t] += sb[x];
-                sA[t * PP + j + x] += sa[x];
+                const int t = second * 32 + (s + x) * 4 + (lane >> 3);
+                const float4 a = rq[x].value(), b = rk[x].value(), d = rg[x].value();
+                const float fq[4] = {a.x, a.y, a.z, a.w}, fk[4] = {b.x, b.y, b.z, b.w}, fg[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const int at = at_pass(i + y, t);
+                    sq[at] = fq[y];
+                    sk[at] = fk[y];
+                    sw[at] = t < n && i + y < nk ? fg[y] : 1.f;
+                }
             }
         }
-        // the same relative to the chunk's ends, for the products with the states
-        const int nw = min(SL, p.dkp - i0);
-        for (int e = tid; e < CT * SL; e += THREADS) {
-            const int i = e % SL, t = e / SL, b = t >> 4;
-            if (i >= nw) continue;
-            float before = 1.f, after = 1.f;
-            for (int m = 0; m < b; ++m) before *= edge[m * SL + i];
-            for (int m = b + 1; m < 4; ++m) after *= edge[m * SL + i];
-            const size_t at = (unit * CT + t) * p.dkp + i0 + i;
-            p.Q[at] = sq[at_ct(i, t)] * before;
-            p.W[at] = sw[at_ct(i, t)] * before;
-            p.K[at] = sk[at_ct(i, t)] * after;
-            if (t == 0) p.decay[unit * p.dkp + i0 + i] = edge[i] * after;
+        group_wait(group);
+        // pairs of tokens within a block of 16: lane = token j; where x < j the sums mean nothing
+#pragma unroll 1
+        for (int e = c0; e < c0 + GCH; ++e) {
+            float run = sk[at_pass(e, block * 16 + jj)];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int at = at_pass(e, block * 16 + 4 * b);
+                const float4 q4 = *reinterpret_cast<const float4*>(sq + at), k4 = *reinterpret_cast<const float4*>(sk + at);
+                const float4 w4 = *reinterpret_cast<const float4*>(sw + at);
+                const float fq[4] = {q4.x, q4.y, q4.z, q4.w}, fk[4] = {k4.x, k4.y, k4.z, k4.w}, fw[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const int x = 4 * b + y;
+                    if (x > jj) run *= fw[y];
+                    da[x] = fmaf(fk[y], run, da[x]);
+                    db[x] = fmaf(fq[y], run, db[x]);
+                }
+            }
         }
-        __syncthreads();
-    }
-    for (int e = tid; e < CT * CT; e += THREADS) {
-        const int r = e >> 6, j = e & 63;
-        sA[r * PP + j] *= -s_beta[r];
-        p.B[unit * CT * CT + e] = sB[r * PP + j];
+        group_wait(group);
+        // a lane per channel and half of the tokens: what the decays of a block of 16 do to its tokens
+        {
+            const int ch = c0 + second * 16 + (lane & 15);
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const int b = (lane >> 4) * 2 + y;
+                float4 w[4];
+                float run = 1.f;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) w[x] = *reinterpret_cast<const float4*>(sw + at_pass(ch, b * 16 + 4 * x));
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int at = at_pass(ch, b * 16 + 4 * x);
+                    float4 q4 = *reinterpret_cast<const float4*>(sq + at), k4 = *reinterpret_cast<const float4*>(sk + at);
+                    run *= w[x].x; q4.x *= run; k4.x *= run;
+                    run *= w[x].y; q4.y *= run; k4.y *= run;
+                    run *= w[x].z; q4.z *= run; k4.z *= run;
+                    run *= w[x].w; q4.w *= run; k4.w *= run;
+                    *reinterpret_cast<float4*>(sq + at) = q4;
+                    *reinterpret_cast<float4*>(sw + at) = k4;
+                }
+                edge[b * PASS + ch] = run;
+                run = 1.f;
+#pragma unroll
+                for (int x = 3; x >= 0; --x) {
+                    const int at = at_pass(ch, b * 16 + 4 * x);
+                    float4 k4 = *reinterpret_cast<const float4*>(sk + at);
+                    k4.w *= run; run *= w[x].w;
+                    k4.z *= run; run *= w[x].z;
+                    k4.y *= run; run *= w[x].y;
+                    k4.x *= run; run *= w[x].x;
+                    *reinterpret_cast<float4*>(sk + at) = k4;
+                }
+            }
+        }
+        // a block's tokens against all earlier ones, whose k are taken on to this block's start: one warp for B, the other for A
+        const float* X = second ? sw : sq;
+        const int ch = c0 + second * 16 + (lane & 15), eighth = (lane >> 4) * 8;
+        group_wait(group);
+        cross_product<1>(x1, X, sk, c0, lane);
+        group_wait(group);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) scale_four(sk + at_pass(ch, eighth + 4 * x), edge[PASS + ch]);
+        group_wait(group);
+        cross_product<2>(x2, X, sk, c0, lane);
+        group_wait(group);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) scale_four(sk + at_pass(ch, 2 * eighth + 4 * x), edge[2 * PASS + ch]);
+        group_wait(group);
+        cross_product<3>(x3, X, sk, c0, lane);
+        // relative to the chunk's ends, for the products with the states
+        if (i0 + i < p.dkp) {
+            float e0[4], e1[4], e2[4], e3[4];
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                e0[y] = edge[i + y];
+                e1[y] = e0[y] * edge[PASS + i + y];
+                e2[y] = e1[y] * edge[2 * PASS + i + y];
+                e3[y] = edge[3 * PASS + i + y];
+            }
+            if (second && lane < 8)
+                *reinterpret_cast<float4*>(p.decay + unit * p.dkp + i0 + i) = make_float4(e2[0] * e3[0], e2[1] * e3[1], e2[2] * e3[2], e2[3] * e3[3]);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                const int b = second * 2 + (s >> 2), t = second * 32 + s * 4 + (lane >> 3);
+                const size_t at = (unit * CT + t) * p.dkp + i0 + i;
+                float q[4], w[4], k[4];
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const float before = b == 0 ? 1.f : b == 1 ? e0[y] : b == 2 ? e1[y] : e2[y];
+                    const int from = at_pass(i + y, t);
+                    q[y] = sq[from] * before;
+                    w[y] = sw[from] * before;
+                    k[y] = sk[from] * (b == 3 ? 1.f : e3[y]);
+                }
+                *reinterpret_cast<float4*>(p.Q + at) = make_float4(q[0], q[1], q[2], q[3]);
+                *reinterpret_cast<float4*>(p.W + at) = make_float4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<float4*>(p.K + at) = make_float4(k[0], k[1], k[2], k[3]);
+            }
+        }
+        group_wait(group);
     }
     __syncthreads();
-    substitute(p.W + unit * CT * p.dkp, p.dkp, p.W + unit * CT * p.dkp, p.dkp, p.dk, CT, sA, s_beta);
-    substitute(p.U + unit * CT * p.dvp, p.dvp, p.v + (size_t)t0 * p.ldv + (size_t)h * p.dv, p.ldv, p.dv, n, sA, s_beta);
+    {
+        float* mine = sums + (group * 2 + second) * CROSS;
+        cross_store<1>(mine, x1, lane);
+        cross_store<2>(mine, x2, lane);
+        cross_store<3>(mine, x3, lane);
+        float* own = sums + GROUPS * 2 * CROSS + (group * 4 + block) * OWN;     // A at (j, x), x > j; B at (x, j), x >= j
+#pragma unroll
+        for (int x = 0; x < 16; ++x) {
+            if (x > jj) own[jj * 17 + x] = da[x];
+            if (x >= jj) own[x * 17 + jj] = db[x];
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < CT * CT; e += TERMS) {
+        const int j = e >> 6, t = e & 63, I = t >> 4;
+        float a = 0.f, b = 0.f;
+        if (I > j >> 4) {
+            const float* at = sums + cross_at(I) + (t & 15) * (16 * I + 1) + j;
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) { b += at[g * 2 * CROSS]; a += at[(g * 2 + 1) * CROSS]; }
+        } else if (t >= j) {
+            const float* at = sums + GROUPS * 2 * CROSS + I * OWN;
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) {
+                if (t > j) a += at[g * 4 * OWN + (j & 15) * 17 + (t & 15)];
+                b += at[g * 4 * OWN + (t & 15) * 17 + (j & 15)];
+            }
+        }
+        minus[e] = -s_beta[t] * a;
+        p.B[unit * CT * CT + e] = b;
+    }
+    __syncthreads();
+    // X[t] = beta_t R[t] - sum_{j < t} beta_t A[t][j] X[j], a column of W (R in place) or U (R: the values) per thread.  A token that is
+    // done takes no harm from being "updated" by itself: minus is zero there and nobody reads it any more.
+    for (int col = tid; col < p.dk + p.dv; col += TERMS) {
+        const bool of_w = col < p.dk;
+        const float* from = of_w ? p.W + unit * CT * p.dkp + col : p.v + (size_t)t0 * p.ldv + (size_t)h * p.dv + (col - p.dk);
+        const size_t step = of_w ? p.dkp : p.ldv;
+        float* to = of_w ? p.W + unit * CT * p.dkp + col : p.U + unit * CT * p.dvp + (col - p.dk);
+        const int width = of_w ? p.dkp : p.dvp;
+        f32x2 x[CT / 2];
+#pragma unroll
+        for (int t = 0; t < CT; t += 2)
+            x[t / 2] = mul2(pack2(s_beta[t], s_beta[t + 1]), pack2(t < n ? from[t * step] : 0.f, t + 1 < n ? from[(t + 1) * step] : 0.f));
+#pragma unroll
+        for (int j = 0; j < CT; ++j) {
+            const float2 two = unpack2(x[j / 2]);
+            const float own = j & 1 ? two.y : two.x;
+            to[j * width] = own;
+            const f32x2 o = pack2(own, own);
+#pragma unroll
+            for (int t = (j + 1) / 4 * 4; t < CT; t += 4) {
+                const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(minus + j * CT + t);
+                x[t / 2] = fma2(m.x, o, x[t / 2]);
+                x[t / 2 + 1] = fma2(m.y, o, x[t / 2 + 1]);
+            }
+        }
+    }
 }
 
 __host__ __device__ inline int walk_stage(int dkp) { return CT * (dkp + 4) + CT * dkp; }       // W and K of a chunk
@@ -515,7 +613,7 @@ QS_API int qs_delta_chunks(float* o, long long ldo, const float* q, long long ld
     p.decay = p.B + units * CT * CT;
     p.start = p.decay + units * p.dkp;
     cudaError_t e = cudaFuncSetAttribute(delta_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TERMS_SMEM);
-    if (e == cudaSuccess) e = qs_launch_dependent(delta_terms_kernel, dim3(n_chunks, H), dim3(THREADS), TERMS_SMEM, stream, p);
+    if (e == cudaSuccess) e = qs_launch_dependent(delta_terms_kernel, dim3(n_chunks, H), dim3(TERMS), TERMS_SMEM, stream, p);
     const size_t walk = walk_smem(p.dkp);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
     if (e == cudaSuccess) e = qs_launch_dependent(delta_walk_kernel, dim3(n_seq, H, (dv + WC - 1) / WC), dim3(WALK), walk, stream, p, walk_stages(p.dkp));
