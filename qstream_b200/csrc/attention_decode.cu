@@ -212,6 +212,253 @@ decode_split_kernel(float* __restrict__ partial, const __nv_bfloat16* __restrict
     }
 }
 
+// Query heads that share a key head, up to four to a CTA, on mma.sync: a warp scores its page's 64 keys (rows of the product, straight
+// from the page to registers; lane t of a row's four takes the dims 8 t .. 8 t + 7 of 32, of the queries as well) against the heads
+// (columns), takes the softmax in 32-bit as the kernels above, and adds the values.  A weight p stays 32-bit: it enters as the
+// sum of three bfloat16 numbers, hi + mid + lo, which are rows of their own (hi of head h in row h, mid in row h + 4, lo in row
+// h + 8 of the product's 16), so the exact weights cost no product more.  The values' columns are permuted instead of transposed: tile j
+// of a block of 64 dims holds the dims 8 g + j, so that a lane's 16 bytes of two keys interleave into eight tiles' operands.
+//
+// Bound by the pages' way from memory: every key and value is read once per four heads and costs one load and three instructions per
+// 16 bytes.  32 sequences of 2,048 keys, 16 query and 4 key heads of 128, capped scores: 46 us, two heads per CTA on the CUDA
+// cores 65 us (with the merge kernel 54 and 81); 32 of 2,048, 64 and 8 of 64: 77 us with the merge, 138 us.  Its distance from
+// float64 is that of the kernels above (1.76e-7 and 1.75e-7 of the result's norm at the first size; 1.50e-7 and 1.54e-7 at the second).
+// d = a b.  The unit cuts off where it adds up, so a product of 16 starts from zero, and products are added rounded, in pairs first.
+__device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Term 0, 1 or 2 (hi, mid, lo) of two numbers.
+__device__ __forceinline__ void three_terms(float2 p, uint32_t (&term)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        term[i] = pack_bf16(p.x, p.y);
+        p.x -= __uint_as_float(term[i] << 16);
+        p.y -= __uint_as_float(term[i] & 0xffff0000u);
+    }
+}
+
+// 16 bytes that nobody on this SM reads again, loaded where the program says so.
+__device__ __forceinline__ uint4 load_once(const __nv_bfloat16* p) {
+    uint4 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+
+constexpr int HEADS = 4;                            // query heads of a CTA
+// ND: blocks of 64 dims that keys and values span at most.
+template <int ND>
+__global__ void __launch_bounds__(WARPS * 32)
+decode_split_heads_kernel(float* __restrict__ partial, const __nv_bfloat16* __restrict__ q, size_t ldq,
+                          const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
+                          const int32_t* __restrict__ page_table, int max_pages,
+                          const int32_t* __restrict__ tok_slot, const int32_t* __restrict__ tok_pos,
+                          int n_heads, int n_kv_heads, int dh, float scale, int window, int max_splits,
+                          int32_t* __restrict__ status, int dv, float softcap, int chunk) {
+    __shared__ __align__(16) float s_p[WARPS][HEADS][PAGE];
+    __shared__ float s_m[WARPS][HEADS], s_l[WARPS][HEADS];
+    extern __shared__ float s_acc[];                 // [WARPS][HEADS][dv]
+
+    const int per_group = n_heads / n_kv_heads, tiles = (per_group + HEADS - 1) / HEADS;
+    const int split = blockIdx.x, kvh = blockIdx.y / tiles, tile = blockIdx.y % tiles, t_row = blockIdx.z;
+    const int head0 = kvh * per_group + tile * HEADS, nh = min(HEADS, per_group - tile * HEADS);
+    const int slot = tok_slot[t_row];
+    if (slot < 0) return;
+    const int pos = tok_pos[t_row];
+    if (pos < 0 || pos >= max_splits * SPLIT) {
+        if (threadIdx.x == 0 && split == 0 && blockIdx.y == 0) atomicExch(status, 1);
+        return;
+    }
+    const int first = window > 0 ? max(0, pos - window + 1) : (chunk > 0 ? pos - pos % chunk : 0);
+    if (split * SPLIT > pos || (split + 1) * SPLIT <= first) return;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int key0 = split * SPLIT + warp * PAGE;
+    float m[HEADS], l[HEADS];
+#pragma unroll
+    for (int h = 0; h < HEADS; ++h) { m[h] = -INFINITY; l[h] = 0.f; }
+    float acc[ND * 8][4];
+#pragma unroll
+    for (int j = 0; j < ND * 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    if (key0 <= pos && key0 + PAGE > first) {
+        const int page = page_table[(size_t)slot * max_pages + (key0 >> 6)];
+        if (page < 0) {
+            if (lane == 0) atomicExch(status, 3);
+        } else {
+            const size_t base = ((size_t)page * n_kv_heads + kvh) * PAGE;
+            const __nv_bfloat16* kp = k_cache + base * dh;
+            const __nv_bfloat16* vp = v_cache + base * dv;
+            const int n_keys = min(PAGE, pos - key0 + 1);
+            const uint4 none = make_uint4(0, 0, 0, 0);
+            uint4 qf[2 * ND];
+            const __nv_bfloat16* qrow = q + (size_t)t_row * ldq + (size_t)(head0 + g) * dh;
+#pragma unroll
+            for (int s = 0; s < 2 * ND; ++s) qf[s] = g < nh && s * 32 + t * 8 < dh ? *reinterpret_cast<const uint4*>(qrow + s * 32 + t * 8) : none;
+            // All loads are issued as early as registers hold them: the second half of the keys before the first is scored, a half of
+            // the values as soon as a half of the keys has been.
+            constexpr int MB = ND == 1 ? 4 : ND == 2 ? 2 : 1, KB = ND <= 2 ? 2 : 1;      // 16-key tiles loaded together: keys, values
+            constexpr bool AHEAD = ND <= 2;
+            struct Keys { uint4 lo[MB][2 * ND], hi[MB][2 * ND]; };
+            struct Values { uint4 x[KB][ND][4]; };   // keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of a tile, dims 8 g .. of a block
+            auto load_keys = [&](Keys& r, int mt0) {
+#pragma unroll
+                for (int i = 0; i < MB; ++i)
+#pragma unroll
+                    for (int s = 0; s < 2 * ND; ++s) {
+                        const int k = (mt0 + i) * 16 + g, d = s * 32 + t * 8;
+                        r.lo[i][s] = k < n_keys && d < dh ? load_once(kp + (size_t)k * dh + d) : none;
+                        r.hi[i][s] = k + 8 < n_keys && d < dh ? load_once(kp + (size_t)(k + 8) * dh + d) : none;
+                    }
+            };
+            auto load_values = [&](Values& r, int ks0) {
+#pragma unroll
+                for (int i = 0; i < KB; ++i)
+#pragma unroll
+                    for (int b = 0; b < ND; ++b)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int k = (ks0 + i) * 16 + 2 * t + (e & 1) + 8 * (e >> 1), d = b * 64 + g * 8;
+                            r.x[i][b][e] = k < n_keys && d < dv ? load_once(vp + (size_t)k * dv + d) : none;
+                        }
+            };
+            auto score = [&](const Keys& r, int mt0) {
+#pragma unroll
+                for (int i = 0; i < MB; ++i) {
+                    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int s = 0; s < 2 * ND; ++s) {
+                        float d0[4], d1[4];
+                        mma_bf16_16x8x16(d0, r.lo[i][s].x, r.hi[i][s].x, r.lo[i][s].y, r.hi[i][s].y, qf[s].x, qf[s].y);
+                        mma_bf16_16x8x16(d1, r.lo[i][s].z, r.hi[i][s].z, r.lo[i][s].w, r.hi[i][s].w, qf[s].z, qf[s].w);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) c[e] += d0[e] + d1[e];
+                    }
+                    if (t < 2) {                     // columns 2 t, 2 t + 1: the heads
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int k = (mt0 + i) * 16 + g + 8 * (e >> 1);
+                            float sc = c[e] * scale;
+                            if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+                            s_p[warp][2 * t + (e & 1)][k] = k < n_keys && key0 + k >= first ? sc : -INFINITY;
+                        }
+                    }
+                }
+            };
+            auto add_values = [&](const Values& r, int ks0) {
+                uint32_t w[KB][4];                   // rows 0-3 hi, 4-7 mid; rows 8-11 lo, 12-15 nothing
+#pragma unroll
+                for (int i = 0; i < KB; ++i) {
+                    const float* p = &s_p[warp][g & 3][(ks0 + i) * 16 + 2 * t];
+                    uint32_t near[3], far[3];
+                    three_terms(*reinterpret_cast<const float2*>(p), near);
+                    three_terms(*reinterpret_cast<const float2*>(p + 8), far);
+                    const bool low = g < 4;
+                    w[i][0] = low ? near[0] : near[1]; w[i][1] = low ? near[2] : 0u; w[i][2] = low ? far[0] : far[1]; w[i][3] = low ? far[2] : 0u;
+                }
+#pragma unroll
+                for (int b = 0; b < ND; ++b)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float d[KB][4];
+#pragma unroll
+                        for (int i = 0; i < KB; ++i) {
+                            uint32_t x[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) x[e] = j < 2 ? r.x[i][b][e].x : j < 4 ? r.x[i][b][e].y : j < 6 ? r.x[i][b][e].z : r.x[i][b][e].w;
+                            const int half = j & 1 ? 0x7632 : 0x5410;
+                            mma_bf16_16x8x16(d[i], w[i][0], w[i][1], w[i][2], w[i][3], __byte_perm(x[0], x[1], half), __byte_perm(x[2], x[3], half));
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[b * 8 + j][e] += KB == 2 ? d[0][e] + d[KB - 1][e] : d[0][e];
+                    }
+            };
+            Values v0, v1;
+            if constexpr (AHEAD) {
+                Keys k0, k1;
+                load_keys(k0, 0);
+                if (MB == 2) load_keys(k1, 2);
+                score(k0, 0);
+                load_values(v0, 0);
+                if (MB == 2 && n_keys > 32) score(k1, 2);
+                load_values(v1, 2);
+            } else {
+#pragma unroll
+                for (int mt0 = 0; mt0 < 4; mt0 += MB) {
+                    if (mt0 * 16 >= n_keys) break;
+                    Keys k0;
+                    load_keys(k0, mt0);
+                    score(k0, mt0);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < HEADS; ++h) {
+                const float s0 = h < nh && lane < n_keys ? s_p[warp][h][lane] : -INFINITY;
+                const float s1 = h < nh && lane + 32 < n_keys ? s_p[warp][h][lane + 32] : -INFINITY;
+                m[h] = warp_max(fmaxf(s0, s1));
+                const float p0 = m[h] == -INFINITY ? 0.f : expf(s0 - m[h]);
+                const float p1 = m[h] == -INFINITY ? 0.f : expf(s1 - m[h]);
+                l[h] = warp_sum(p0 + p1);
+                __syncwarp();
+                s_p[warp][h][lane] = p0;
+                s_p[warp][h][lane + 32] = p1;
+            }
+            __syncwarp();
+            if constexpr (AHEAD) {
+                add_values(v0, 0);
+                if (n_keys > 32) add_values(v1, 2);
+            } else {
+#pragma unroll
+                for (int ks0 = 0; ks0 < 4; ks0 += KB) {
+                    if (ks0 * 16 >= n_keys) break;
+                    load_values(v0, ks0);
+                    add_values(v0, ks0);
+                }
+            }
+        }
+    }
+    // hi + (mid + lo) of head g, mid from the lane four rows on; where an infinite or undefined value makes hi one, the terms' zeros times it say nothing
+#pragma unroll
+    for (int j = 0; j < ND * 8; ++j) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float mid = __shfl_xor_sync(0xffffffffu, acc[j][e], 16);
+            const int d = (j >> 3) * 64 + 8 * (2 * t + e) + (j & 7);
+            if (g < nh && d < dv) s_acc[((size_t)warp * HEADS + g) * dv + d] = isfinite(acc[j][e]) ? acc[j][e] + (mid + acc[j][e + 2]) : acc[j][e];
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int h = 0; h < HEADS; ++h) { s_m[warp][h] = m[h]; s_l[warp][h] = l[h]; }
+    }
+    __syncthreads();
+    for (int h = 0; h < nh; ++h) {
+        float M = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, s_m[w][h]);
+        float* out = partial + (((size_t)t_row * n_heads + head0 + h) * max_splits + split) * (dv + 2);
+        for (int d = threadIdx.x; d < dv; d += blockDim.x) {
+            float o = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w)
+                if (s_m[w][h] != -INFINITY) o += s_acc[((size_t)w * HEADS + h) * dv + d] * expf(s_m[w][h] - M);
+            out[d] = o;
+        }
+        if (threadIdx.x == 0) {
+            float L = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w)
+                if (s_m[w][h] != -INFINITY) L += s_l[w][h] * expf(s_m[w][h] - M);
+            out[dv] = M;
+            out[dv + 1] = L;
+        }
+    }
+}
+
 // The same for HG query heads that share a key head: one pass over the page's keys and values serves them all
 // (a CTA per query head reads the pages once per head, all but once from L2).  blockIdx.y = the group of HG
 // query heads; the partial results are laid out per query head as above, so the merge kernel is the same.
@@ -551,17 +798,25 @@ QS_API int qs_attention_decode_masked(void* out, long long ldo, const void* q, l
         scratch, (const __nv_bfloat16*)q, (size_t)ldq, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, \
         page_table, max_pages, tok_slot, tok_pos, n_heads, n_kv_heads, dh, gs_log2, scale, window, max_splits, status, \
         dv, softcap, chunk, keep_first, maps)
-    // Query heads that share a key head go through the pages together, two to a CTA (chunk slots of one or two per
-    // lane only).  Four to a CTA were measured slower (32 x 2,048 keys, 16 query and 4 key heads of 128: 108 us
-    // against 81 us with two and 96 us with one): four heads' accumulators leave room for three CTAs per SM and
-    // two loads in flight per lane.
     const int per_group = n_heads / n_kv_heads;
+    const int widest = dh > dv ? dh : dv;
+    // Query heads that share a key head go through the pages together, four to a CTA on the tensor cores.  Heads wider than 128 take
+    // the registers of two warps and work for 256 dims however many they have: with four heads to share that it is still faster (32 x
+    // 1,024 keys of 256: 52 us against 83 us), with two it is at 160 and 192 (42 against 52 us, 28 against 32) and not beyond (256: 54 and
+    // 54, 58 with capped scores against 60).  Those, and heads wider than 256 in pairs, go two to a CTA on the CUDA cores; the masks that
+    // keep first tokens or have several maps, a query head per CTA.
+    const bool by_heads = per_group > 1 && (per_group > 2 || widest <= 192) && widest <= 256 && keep_first == 0 && maps == 1;
+#define HEADS_GO(ND) decode_split_heads_kernel<ND><<<dim3(max_splits, n_kv_heads * ((per_group + HEADS - 1) / HEADS), T_tokens), WARPS * 32, \
+        smem * HEADS, stream>>>(scratch, (const __nv_bfloat16*)q, (size_t)ldq, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, \
+        page_table, max_pages, tok_slot, tok_pos, n_heads, n_kv_heads, dh, scale, window, max_splits, status, dv, softcap, chunk)
     const int hg = (nch <= 2 && per_group % 2 == 0 && !masked) ? 2 : 1;      // the masked forms: a query head per CTA
 #define GROUP(NCH, UNROLL, HG) decode_split_group_kernel<NCH, UNROLL, HG><<<dim3(max_splits, n_heads / HG, T_tokens), WARPS * 32, \
         smem * HG, stream>>>(scratch, (const __nv_bfloat16*)q, (size_t)ldq, (const __nv_bfloat16*)k_cache, \
         (const __nv_bfloat16*)v_cache, page_table, max_pages, tok_slot, tok_pos, n_heads, n_kv_heads, dh, gs_log2, scale, window, \
         max_splits, status, dv, softcap)
-    if (hg == 2 && nch == 1) GROUP(1, 8, 2);
+    if (by_heads && widest <= 64) HEADS_GO(1);
+    else if (by_heads && widest <= 128) HEADS_GO(2);
+    else if (by_heads) HEADS_GO(4);
     else if (hg == 2) GROUP(2, 4, 2);
     else if (nch == 1) GO(1, 8);
     else if (nch == 3) GO(3, 4);
@@ -569,6 +824,7 @@ QS_API int qs_attention_decode_masked(void* out, long long ldo, const void* q, l
     else if (few_ctas) GO(2, 8);
     else GO(2, 4);
 #undef GROUP
+#undef HEADS_GO
 #undef GO
 #undef GO1
     int rc = qs_check_launch("attention_decode");
