@@ -49,52 +49,12 @@ struct Delta {
 // steps unrolled per thread (more code than the instruction cache holds); now
 // 108 us.
 constexpr int TERMS = 256, GROUPS = 4, GCH = 32, PASS = GROUPS * GCH;
-// a group's sums: pairs of tokens across blocks, [16 t][16 I j] of block I with rows of 16 I + 1 (read along t), and a block's own, [16][17]
-constexpr int CROSS = 16 * (17 + 33 + 49), OWN = 16 * 17;
+constexpr int OWN = 16 * 17;                            // a block's own pairs, [16][17]
 constexpr int TERMS_SMEM = (3 * PASS * CT + 4 * PASS) * sizeof(float);
 static_assert(GROUPS * (2 * CROSS + 4 * OWN) + CT * CT <= 3 * PASS * CT, "the groups' sums and A lie over the staged channels");
 // [channel][64 tokens], pieces of four tokens swapped so that neighbouring channels, and every fourth one, meet different banks
 __device__ __forceinline__ int at_pass(int c, int t) { return c * CT + (t ^ (((c ^ (c >> 2)) & 7) << 2)); }
 __device__ __forceinline__ void group_wait(int group) { asm volatile("bar.sync %0, 64;" :: "r"(1 + group) : "memory"); }
-
-// acc[x][pair of t] += sum over the group's channels of X[i][t] k[i][j]: block I's tokens t = 4 (lane / 8) .. + 3 against the earlier
-// blocks' tokens j = 16 m + 2 (lane % 8) + {0, 1}, x = 2 m + {0, 1}
-template <int I>
-__device__ __forceinline__ void cross_product(f32x2 (&acc)[2 * I][2], const float* __restrict__ X, const float* __restrict__ sk, int c0, int lane) {
-#pragma unroll 4
-    for (int i = c0; i < c0 + GCH; ++i) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(X + at_pass(i, I * 16 + (lane >> 3) * 4));
-#pragma unroll
-        for (int m = 0; m < I; ++m) {
-            const float2 b = *reinterpret_cast<const float2*>(sk + at_pass(i, m * 16 + (lane & 7) * 2));
-            const f32x2 b0 = pack2(b.x, b.x), b1 = pack2(b.y, b.y);
-            acc[2 * m][0] = fma2(a.x, b0, acc[2 * m][0]);
-            acc[2 * m][1] = fma2(a.y, b0, acc[2 * m][1]);
-            acc[2 * m + 1][0] = fma2(a.x, b1, acc[2 * m + 1][0]);
-            acc[2 * m + 1][1] = fma2(a.y, b1, acc[2 * m + 1][1]);
-        }
-    }
-}
-__device__ __forceinline__ int cross_at(int I) { return 16 * (8 * I * (I - 1) + I - 1); }      // where block I's sums begin
-template <int I>
-__device__ __forceinline__ void cross_store(float* __restrict__ dst, const f32x2 (&acc)[2 * I][2], int lane) {
-    dst += cross_at(I);
-#pragma unroll
-    for (int x = 0; x < 2 * I; ++x)
-#pragma unroll
-        for (int y = 0; y < 2; ++y) {
-            const float2 v = unpack2(acc[x][y]);
-            float* at = dst + ((lane >> 3) * 4 + 2 * y) * (16 * I + 1) + (x >> 1) * 16 + (lane & 7) * 2 + (x & 1);
-            at[0] = v.x;
-            at[16 * I + 1] = v.y;
-        }
-}
-// four tokens of a channel times a decay
-__device__ __forceinline__ void scale_four(float* at, float d) {
-    float4 v = *reinterpret_cast<float4*>(at);
-    v.x *= d; v.y *= d; v.z *= d; v.w *= d;
-    *reinterpret_cast<float4*>(at) = v;
-}
 
 __global__ void __launch_bounds__(TERMS, 2)
 delta_terms_kernel(Delta p) {
@@ -212,17 +172,17 @@ delta_terms_kernel(Delta p) {
         const float* X = second ? sw : sq;
         const int ch = c0 + second * 16 + (lane & 15), eighth = (lane >> 4) * 8;
         group_wait(group);
-        cross_product<1>(x1, X, sk, c0, lane);
+        cross_product<1, GCH, at_pass>(x1, X, sk, c0, lane);
         group_wait(group);
 #pragma unroll
         for (int x = 0; x < 2; ++x) scale_four(sk + at_pass(ch, eighth + 4 * x), edge[PASS + ch]);
         group_wait(group);
-        cross_product<2>(x2, X, sk, c0, lane);
+        cross_product<2, GCH, at_pass>(x2, X, sk, c0, lane);
         group_wait(group);
 #pragma unroll
         for (int x = 0; x < 4; ++x) scale_four(sk + at_pass(ch, 2 * eighth + 4 * x), edge[2 * PASS + ch]);
         group_wait(group);
-        cross_product<3>(x3, X, sk, c0, lane);
+        cross_product<3, GCH, at_pass>(x3, X, sk, c0, lane);
         // relative to the chunk's ends, for the products with the states
         if (i0 + i < p.dkp) {
             float e0[4], e1[4], e2[4], e3[4];

@@ -18,8 +18,9 @@
 // multiplied), and an activation once per element instead of once per kernel.  On the tensor cores as split 11-bit products the sums,
 // which the unit truncates, were two times further from 64 bits than the walk, at the same speed: not taken.
 // Microseconds of the whole mixer (walk | chunks, serial fetches | now): decay per head, 4,096 tokens, 16 heads of 128 x 128: 949 |
-// 600 | 422; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 329; state-space form, 2,048 tokens, 64 heads of
-// 128 x 64: 822 | 458 | 388 (its output kernel 154, what the chunks add 67).
+// 600 | 416; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 285; state-space form, 2,048 tokens, 64 heads of
+// 128 x 64: 822 | 458 | 377 (its output kernel 143, what the chunks add 71).  Pairs of blocks of 16 with the later block's decays
+// applied to every pair, a token's q against one block's k at a time, took the per-channel output kernel from 114 to 163 us.
 #include "scan.cuh"
 #include "scan_tiles.cuh"
 
@@ -380,7 +381,7 @@ chunk_output_kernel(Scan p) {
 #pragma unroll
                     for (int x = 0; x < 16; ++x) {
                         if (x > jj && !WKV) run *= fw[x];
-                        if (x >= jj) d[x] = fmaf(fq[x], WKV && x == jj ? u * kj : run, d[x]);
+                        d[x] = fmaf(fq[x], WKV && x == jj ? u * kj : run, d[x]);         // means nothing where x < jj
                         if (x > jj && WKV) run *= fw[x];
                     }
                 }
@@ -392,50 +393,81 @@ chunk_output_kernel(Scan p) {
             }
             __syncthreads();
             // q times the decays since the start of its block of 16, k times those up to the block's end, the block's whole decay
-            for (int e = tid; e < SL * 4; e += THREADS) {
-                const int i = e % SL, g = e / SL;
+            for (int e = tid; e < SL * 4; e += THREADS) {        // neighbouring lanes four channels apart: other banks
+                const int i = (e & 15) * 4 + (e >> 4 & 3), g = e >> 6;
+                float4 w[4];
                 float run = 1.f;
 #pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    float* x = sq + at_ct(i, g * 16 + t);
-                    const float a = sw[at_ct(i, g * 16 + t)];
-                    if (!WKV) run *= a;
-                    *x *= run;
-                    if (WKV) run *= a;
+                for (int x = 0; x < 4; ++x) {
+                    w[x] = *reinterpret_cast<const float4*>(sw + at_ct(i, g * 16 + 4 * x));
+                    float4* at = reinterpret_cast<float4*>(sq + at_ct(i, g * 16 + 4 * x));
+                    float4 f = *at;
+                    if (!WKV) run *= w[x].x;
+                    f.x *= run; run *= WKV ? w[x].x : w[x].y;
+                    f.y *= run; run *= WKV ? w[x].y : w[x].z;
+                    f.z *= run; run *= WKV ? w[x].z : w[x].w;
+                    f.w *= run;
+                    if (WKV) run *= w[x].w;
+                    *at = f;
                 }
                 edge[g * SL + i] = run;
                 run = 1.f;
 #pragma unroll
-                for (int t = 15; t >= 0; --t) {
-                    sk[at_ct(i, g * 16 + t)] *= run;
-                    run *= sw[at_ct(i, g * 16 + t)];
+                for (int x = 3; x >= 0; --x) {
+                    float4* at = reinterpret_cast<float4*>(sk + at_ct(i, g * 16 + 4 * x));
+                    float4 f = *at;
+                    f.w *= run; run *= w[x].w;
+                    f.z *= run; run *= w[x].z;
+                    f.y *= run; run *= w[x].y;
+                    f.x *= run; run *= w[x].x;
+                    *at = f;
                 }
             }
             __syncthreads();
-            // pairs of blocks: (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), 256 pairs of tokens each; a warp takes eight tokens t against the 16 j
-            // of a pair of blocks at a time, a thread one t and four j
-            for (int e = blk; e < 12; e += 4) {
-                const int pair = e >> 1, I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
-                const int t = I * 16 + (e & 1) * 8 + (lane >> 2) , j = J * 16 + (lane & 3) * 4;
-                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-                for (int i = 0; i < SL; ++i) {
-                    float x = sq[at_ct(i, t)];
-                    for (int m = J + 1; m < I; ++m) x *= edge[m * SL + i];
-                    const float4 kk = *reinterpret_cast<const float4*>(sk + at_ct(i, j));
-                    s0 = fmaf(x, kk.x, s0); s1 = fmaf(x, kk.y, s1); s2 = fmaf(x, kk.z, s2); s3 = fmaf(x, kk.w, s3);
-                }
-                sp[j * PP + t] += s0; sp[(j + 1) * PP + t] += s1; sp[(j + 2) * PP + t] += s2; sp[(j + 3) * PP + t] += s3;
+            // a block's tokens against all earlier ones, whose k are taken on to this block's start; a warp has 16 of the channels
+            f32x2 x1[2][2], x2[4][2], x3[6][2];
+#pragma unroll
+            for (int x = 0; x < 6; ++x) {
+                if (x < 2) x1[x][0] = x1[x][1] = 0ull;
+                if (x < 4) x2[x][0] = x2[x][1] = 0ull;
+                x3[x][0] = x3[x][1] = 0ull;
             }
+            const int ch = blk * 16 + (jj & 3) * 4 + (jj >> 2), eighth = (lane >> 4) * 8;
+            cross_product<1, 16, at_ct>(x1, sq, sk, blk * 16, lane);
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < 2; ++x) scale_four(sk + at_ct(ch, eighth + 4 * x), edge[SL + ch]);
+            __syncwarp();
+            cross_product<2, 16, at_ct>(x2, sq, sk, blk * 16, lane);
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < 4; ++x) scale_four(sk + at_ct(ch, 2 * eighth + 4 * x), edge[2 * SL + ch]);
+            __syncwarp();
+            cross_product<3, 16, at_ct>(x3, sq, sk, blk * 16, lane);
             __syncthreads();
-            // q times the decays since the chunk's start; the state over k and the decays
-            fetch_state(i0, ss);
-            if (i0 + SL < p.dk) fetch(i0 + SL);
-            for (int e = tid; e < SL * 48; e += THREADS) {
-                const int i = e % SL, t = 16 + e / SL;
+            // the warps' sums over k and the decays, then added up; q times the decays since the chunk's start
+            cross_store<1>(sk + blk * CROSS, x1, lane);
+            cross_store<2>(sk + blk * CROSS, x2, lane);
+            cross_store<3>(sk + blk * CROSS, x3, lane);
+            for (int e = tid; e < SL * 12; e += THREADS) {
+                const int i = (e & 15) * 4 + (e >> 4 & 3), t = 16 + (e >> 6) * 4;
                 float x = 1.f;
                 for (int m = 0; m < t / 16; ++m) x *= edge[m * SL + i];
-                sq[at_ct(i, t)] *= x;
+                scale_four(sq + at_ct(i, t), x);
             }
+            __syncthreads();
+#pragma unroll
+            for (int pair = 0; pair < 6; ++pair) {      // blocks (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+                const int I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
+                for (int e = tid; e < 256; e += THREADS) {
+                    const int t = e & 15, j = J * 16 + (e >> 4);
+                    const float* at = sk + cross_at(I) + t * (16 * I + 1) + j;
+                    sp[j * PP + I * 16 + t] += (at[0] + at[CROSS]) + (at[2 * CROSS] + at[3 * CROSS]);
+                }
+            }
+            __syncthreads();
+            fetch_state(i0, ss);                        // over k and the decays
+            if (i0 + SL < p.dk) fetch(i0 + SL);
             copies_done();
             __syncthreads();
             tile_product<NC, true>(acc, sq, ss, SL, ty, tx);

@@ -49,6 +49,47 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool have) 
 }
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Sums over pairs of tokens in different blocks of 16: [16 t][16 I j] of block I with rows of 16 I + 1 (they are read along t)
+constexpr int CROSS = 16 * (17 + 33 + 49);
+// acc[x][pair of t] += sum over N channels from c0 on of X[i][t] k[i][j]: block I's tokens t = 4 (lane / 8) .. + 3 against the earlier
+// blocks' tokens j = 16 m + 2 (lane % 8) + {0, 1}, x = 2 m + {0, 1}
+template <int I, int N, int (*AT)(int, int)>
+__device__ __forceinline__ void cross_product(f32x2 (&acc)[2 * I][2], const float* __restrict__ X, const float* __restrict__ sk, int c0, int lane) {
+#pragma unroll 4
+    for (int i = c0; i < c0 + N; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(X + AT(i, I * 16 + (lane >> 3) * 4));
+#pragma unroll
+        for (int m = 0; m < I; ++m) {
+            const float2 b = *reinterpret_cast<const float2*>(sk + AT(i, m * 16 + (lane & 7) * 2));
+            const f32x2 b0 = pack2(b.x, b.x), b1 = pack2(b.y, b.y);
+            acc[2 * m][0] = fma2(a.x, b0, acc[2 * m][0]);
+            acc[2 * m][1] = fma2(a.y, b0, acc[2 * m][1]);
+            acc[2 * m + 1][0] = fma2(a.x, b1, acc[2 * m + 1][0]);
+            acc[2 * m + 1][1] = fma2(a.y, b1, acc[2 * m + 1][1]);
+        }
+    }
+}
+__device__ __forceinline__ int cross_at(int I) { return 16 * (8 * I * (I - 1) + I - 1); }      // where block I's sums begin
+template <int I>
+__device__ __forceinline__ void cross_store(float* __restrict__ dst, const f32x2 (&acc)[2 * I][2], int lane) {
+    dst += cross_at(I);
+#pragma unroll
+    for (int x = 0; x < 2 * I; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            const float2 v = unpack2(acc[x][y]);
+            float* at = dst + ((lane >> 3) * 4 + 2 * y) * (16 * I + 1) + (x >> 1) * 16 + (lane & 7) * 2 + (x & 1);
+            at[0] = v.x;
+            at[16 * I + 1] = v.y;
+        }
+}
+// four tokens of a channel times a decay
+__device__ __forceinline__ void scale_four(float* at, float d) {
+    float4 v = *reinterpret_cast<float4*>(at);
+    v.x *= d; v.y *= d; v.z *= d; v.w *= d;
+    *reinterpret_cast<float4*>(at) = v;
+}
+
 // acc[8][4 NC] += A[k][8 rows] B[k][4 NC columns] over k < n: A a [k][64] tile (rows 4 ty .. and 32 + 4 ty ..; SKEW: swizzled as by
 // at_ct), B rows of 64 NC columns (4 tx .. of every 64).
 template <int NC, bool SKEW>
