@@ -258,7 +258,8 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
 
 // Walk each sequence's chunks in order: chunk_state[c] (what chunk c adds) becomes the state that
 // chunk c starts from; the state after the last chunk goes to the sequence's slot.  One thread per four value columns of a key
-// channel in the chunks' layout [h][i][dvp]; the decay belongs to (h, i).
+// channel in the chunks' layout [h][i][dvp]; the decay belongs to (h, i).  Bound by memory: 64 chunks of 16 heads of 128 x 128 (134 MB)
+// 21 us, 6.5 TB/s; 56 us when eight chunks were read only after the eight before had been written, 22 us with four at a time.
 __global__ void __launch_bounds__(256)
 chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
                     float* __restrict__ state, size_t slot_stride, const int32_t* __restrict__ seq_chunk,
@@ -272,7 +273,7 @@ chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ c
     const int fours = (dv + 3) / 4;
     const size_t n = (size_t)H * dk * fours;            // float4s of a chunk's states
     float4* const chunks = reinterpret_cast<float4*>(chunk_state);
-    constexpr int AHEAD = 8;                            // chunks whose loads are in flight together
+    constexpr int AHEAD = 8;                            // chunks whose loads are in flight together, while the eight before are written
     for (size_t e = (size_t)blockIdx.y * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.y * blockDim.x) {
         const size_t hi = e / fours;                    // h * dk + i
         const int j = (int)(e - hi * fours) * 4, i = (int)(hi % dk), h = (int)(hi / dk);
@@ -282,14 +283,22 @@ chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ c
         S.y = j + 1 < dv ? own[dk] : 0.f;
         S.z = j + 2 < dv ? own[2 * (size_t)dk] : 0.f;
         S.w = j + 3 < dv ? own[3 * (size_t)dk] : 0.f;
+        float4 next[AHEAD];
+        float next_a[AHEAD];
+        auto fetch = [&](int c) {
+#pragma unroll
+            for (int g = 0; g < AHEAD; ++g) {
+                next[g] = c + g < c1 ? chunks[(size_t)(c + g) * n + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+                next_a[g] = c + g < c1 ? chunk_decay[(size_t)(c + g) * H * dk + hi] : 1.f;
+            }
+        };
+        fetch(c0);
         for (int c = c0; c < c1; c += AHEAD) {
             float4 added[AHEAD];
             float a[AHEAD];
 #pragma unroll
-            for (int g = 0; g < AHEAD; ++g) {
-                added[g] = c + g < c1 ? chunks[(size_t)(c + g) * n + e] : make_float4(0.f, 0.f, 0.f, 0.f);
-                a[g] = c + g < c1 ? chunk_decay[(size_t)(c + g) * H * dk + hi] : 1.f;
-            }
+            for (int g = 0; g < AHEAD; ++g) { added[g] = next[g]; a[g] = next_a[g]; }
+            if (c + AHEAD < c1) fetch(c + AHEAD);
 #pragma unroll
             for (int g = 0; g < AHEAD; ++g) {
                 if (c + g < c1) {
