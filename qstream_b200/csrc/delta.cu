@@ -215,6 +215,8 @@ QS_API int qs_delta_prepare(float* qo, float* ko, float* vo, float* go, float* b
     QS_REQUIRE(smem <= 200 * 1024, "delta_prepare: %d channels above the shared memory of a block", 2 * G * dk + H * dv);
     const int threads = 256;
     cudaError_t e;
+    // Pieces of eight channels where every row and weight begins on a piece, a head is a power of two of one warp's lanes, and the taps
+    // are as many as are unrolled; from 512 tokens on a block per token fills the GPU, below that a token's pieces go to several blocks.
     const int lanes = dk / 8;
     auto fits = [&](const void* ptr) { return ((uintptr_t)ptr % 32) == 0 || (dtype == QS_BF16 && ((uintptr_t)ptr % 16) == 0); };
     if (dtype == w_dtype && taps >= 2 && taps <= 4 && dk % 8 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && dv % 8 == 0 && ldp % 8 == 0 && lda % 8 == 0 &&
