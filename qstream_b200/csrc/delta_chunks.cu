@@ -15,7 +15,7 @@
 //
 // All 32-bit; decays only as products of factors up to one.  Three walks of every chunk token by token (what it does to an
 // identity, what it writes from nothing, its outputs) and a product of dk x dk matrices in the prefix stood here before: 2,000 tokens, 16
-// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 422 (the terms 108, the walk 133, the outputs 56).
+// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 426 (the terms 108, the walk 133, the outputs 56).
 #include "scan.cuh"
 #include "scan_tiles.cuh"
 

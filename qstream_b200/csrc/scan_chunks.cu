@@ -18,8 +18,8 @@
 // multiplied), and an activation once per element instead of once per kernel.  On the tensor cores as split 11-bit products the sums,
 // which the unit truncates, were two times further from 64 bits than the walk, at the same speed: not taken.
 // Microseconds of the whole mixer (walk | chunks, serial fetches | now): decay per head, 4,096 tokens, 16 heads of 128 x 128: 949 |
-// 600 | 416; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 285; state-space form, 2,048 tokens, 64 heads of
-// 128 x 64: 822 | 458 | 377 (its output kernel 143, what the chunks add 71).  Pairs of blocks of 16 with the later block's decays
+// 600 | 407; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 286; state-space form, 2,048 tokens, 64 heads of
+// 128 x 64: 822 | 458 | 379 (its output kernel 143, what the chunks add 71).  Pairs of blocks of 16 with the later block's decays
 // applied to every pair, a token's q against one block's k at a time, took the per-channel output kernel from 114 to 163 us.
 #include "scan.cuh"
 #include "scan_tiles.cuh"
