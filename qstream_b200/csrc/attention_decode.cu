@@ -223,11 +223,7 @@ decode_split_kernel(float* __restrict__ partial, const __nv_bfloat16* __restrict
 // 16 bytes.  32 sequences of 2,048 keys, 16 query and 4 key heads of 128, capped scores: 46 us, two heads per CTA on the CUDA
 // cores 65 us (with the merge kernel 54 and 81); 32 of 2,048, 64 and 8 of 64: 77 us with the merge, 138 us.  Its distance from
 // float64 is that of the kernels above (1.76e-7 and 1.75e-7 of the result's norm at the first size; 1.50e-7 and 1.54e-7 at the second).
-// d = a b.  The unit cuts off where it adds up, so a product of 16 starts from zero, and products are added rounded, in pairs first.
-__device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
+// The products are added rounded, in pairs first.
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&r);

@@ -182,7 +182,8 @@ __global__ void moe_expert_down_kernel(float* __restrict__ out, size_t ldo, cons
 // ----------------------------------------------------------------------------- few tokens, bfloat16, each expert's matrices read once
 //
 // The pairs of a step of few tokens grouped by expert inside the kernels: rows of an expert's matrix are the 16-row side of
-// mma.sync products (bfloat16, 32-bit sums), its tokens the side of eight columns, both straight from memory to registers.  The k's
+// mma.sync products of bfloat16 numbers, its tokens the side of eight columns, both straight from memory to registers.  Every product of
+// 16 starts from zero and is added with a rounded 32-bit addition, as in the decode attention.  The k's
 // of a product are permuted so that a lane's 16 bytes of a row are two products' worth: lane t of a row's four takes the k's
 // 8 t .. 8 t + 7 of 32, on both sides.  A column does not meet the others and K is cut in four wherever the token stands, so a
 // token's result does not depend on the batch.
@@ -192,17 +193,14 @@ __global__ void moe_expert_down_kernel(float* __restrict__ out, size_t ldo, cons
 // (gemm_tc.cu) instead of one each behind a wait for the host: 428 -> 197 us.
 constexpr int CHUNK_TOKENS = 32;                        // tokens of a block: at most this many columns of an expert
 
-__device__ __forceinline__ void mma_bf16_16x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint4 piece(const __nv_bfloat16* row, int k, int K) {        // eight elements, zeros behind the end
     return row && k < K ? *reinterpret_cast<const uint4*>(row + k) : make_uint4(0u, 0u, 0u, 0u);
 }
 
 // acc[m][n] += rows of matrix m (`lo`: this lane's row of the first eight, `hi`: of the last eight) times columns of tile n, k from
-// k0 to k1 (multiples of 32); U steps of 32 fetched together.
-template <int MATS, int NT, int U>
+// k0 to k1 (multiples of 32); U steps of 32 fetched together.  FINE, where the result is not rounded to 16 bits: products of eight and
+// sums over four steps in pairs, so that the sum is as near to float64 as one of 32-bit multiply-adds.
+template <int MATS, int NT, int U, bool FINE>
 __device__ __forceinline__ void stream_rows(float (&acc)[MATS][NT][4], const __nv_bfloat16* const (&lo)[MATS], const __nv_bfloat16* const (&hi)[MATS],
                                             const __nv_bfloat16* const (&col)[NT], int k0, int k1, int K) {
     const int t8 = (threadIdx.x & 3) * 8;
@@ -216,14 +214,34 @@ __device__ __forceinline__ void stream_rows(float (&acc)[MATS][NT][4], const __n
 #pragma unroll
             for (int n = 0; n < NT; ++n) x[u][n] = piece(col[n], at, end);
         }
+        float run[FINE ? 2 : 1][MATS][NT][4];
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int m = 0; m < MATS; ++m)
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    mma_bf16_16x8(acc[m][n], a[u][m].x, b[u][m].x, a[u][m].y, b[u][m].y, x[u][n].x, x[u][n].y);
-                    mma_bf16_16x8(acc[m][n], a[u][m].z, b[u][m].z, a[u][m].w, b[u][m].w, x[u][n].z, x[u][n].w);
+                    float d0[4], d1[4], d2[4], d3[4];
+                    if constexpr (FINE) {
+                        mma_bf16_16x8x8(d0, a[u][m].x, b[u][m].x, x[u][n].x);
+                        mma_bf16_16x8x8(d1, a[u][m].y, b[u][m].y, x[u][n].y);
+                        mma_bf16_16x8x8(d2, a[u][m].z, b[u][m].z, x[u][n].z);
+                        mma_bf16_16x8x8(d3, a[u][m].w, b[u][m].w, x[u][n].w);
+                    } else {
+                        mma_bf16_16x8x16(d0, a[u][m].x, b[u][m].x, a[u][m].y, b[u][m].y, x[u][n].x, x[u][n].y);
+                        mma_bf16_16x8x16(d1, a[u][m].z, b[u][m].z, a[u][m].w, b[u][m].w, x[u][n].z, x[u][n].w);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if constexpr (FINE) {
+                            float &r0 = run[0][m][n][e], &r1 = run[1][m][n][e];
+                            const float step = (d0[e] + d1[e]) + (d2[e] + d3[e]);
+                            if (u % 4 == 0) r0 = step;
+                            else if (u % 4 == 1) r0 += step;
+                            else if (u % 4 == 2) r1 = step;
+                            else acc[m][n][e] += r0 + (r1 + step);
+                        } else acc[m][n][e] += d0[e] + d1[e];
+                    }
                 }
     }
 }
@@ -247,7 +265,7 @@ __device__ void up_columns(__nv_bfloat16* __restrict__ hidden, size_t ldh, const
 #pragma unroll
         for (int c = 0; c < NT; ++c) acc[m][c][0] = acc[m][c][1] = acc[m][c][2] = acc[m][c][3] = 0.f;
     const int per = ((D + 31) / 32 + 3) / 4 * 32;
-    stream_rows<MATS, NT, NT == 1 ? 4 : 2>(acc, lo, hi, col, warp * per, min((warp + 1) * per, (D + 31) / 32 * 32), D);
+    stream_rows<MATS, NT, NT == 1 ? 4 : 2, false>(acc, lo, hi, col, warp * per, min((warp + 1) * per, (D + 31) / 32 * 32), D);
     constexpr int PITCH = NT * 8 + 1;                   // red [4 warps][MATS][16 rows][PITCH]
 #pragma unroll
     for (int m = 0; m < MATS; ++m)
@@ -261,9 +279,8 @@ __device__ void up_columns(__nv_bfloat16* __restrict__ hidden, size_t ldh, const
         float v[MATS];
 #pragma unroll
         for (int m = 0; m < MATS; ++m) {
-            v[m] = 0.f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[m] += red[((q * MATS + m) * 16 + r) * PITCH + c];
+            const float* at = red + (m * 16 + r) * PITCH + c;
+            v[m] = (at[0] + at[MATS * 16 * PITCH]) + (at[2 * MATS * 16 * PITCH] + at[3 * MATS * 16 * PITCH]);
         }
         const float y = apply_activation_wide(v[0], act);
         if (f0 + r < F) hidden[(size_t)list[c] * ldh + f0 + r] = __float2bfloat16_rn(MATS == 2 ? y * v[MATS - 1] : y);
@@ -323,7 +340,7 @@ __device__ void down_columns(float* __restrict__ part, const __nv_bfloat16* __re
 #pragma unroll
     for (int c = 0; c < NT; ++c) acc[0][c][0] = acc[0][c][1] = acc[0][c][2] = acc[0][c][3] = 0.f;
     const int per = ((F + 31) / 32 + 3) / 4 * 32;
-    stream_rows<1, NT, NT == 1 ? 8 : 4>(acc, lo, hi, col, quarter * per, min((quarter + 1) * per, (F + 31) / 32 * 32), F);
+    stream_rows<1, NT, NT == 1 ? 8 : 4, true>(acc, lo, hi, col, quarter * per, min((quarter + 1) * per, (F + 31) / 32 * 32), F);
 #pragma unroll
     for (int c = 0; c < NT; ++c)
 #pragma unroll
@@ -333,7 +350,7 @@ __device__ void down_columns(float* __restrict__ part, const __nv_bfloat16* __re
         }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ w_down,
                         const int32_t* __restrict__ idx, const float* __restrict__ wts, const int32_t* __restrict__ tok_slot, const void* __restrict__ add,
                         int add_dtype, size_t ldadd, const float* __restrict__ add_scale, int T, int top, int D, int F, const __nv_bfloat16* __restrict__ x,
@@ -401,9 +418,8 @@ moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16
                 float y;
                 if (of[p] == 0x7fffffff) y = __bfloat162float(x[row * ldx + d]);
                 else {
-                    y = 0.f;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) y += part[(q * most + p) * 16 + r];
+                    const float* at = part + p * 16 + r;
+                    y = (at[0] + at[most * 16]) + (at[2 * most * 16] + at[3 * most * 16]);
                 }
                 total = fmaf(wts[row * top + j], y, total);
             }

@@ -60,6 +60,25 @@ def test_few_tokens(T, top, E, D, F, gated):
         assert torch.equal(one[0], got[t])
 
 
+@pytest.mark.parametrize("F", [512, 1024, 4096, 8200])
+def test_long_sums_are_rounded_and_not_cut_off(F):
+    """The second product alone, on hidden values as they are: positive terms, whose sum loses to a unit that cuts off at every step."""
+    T, D = 8, 512
+    g = torch.Generator(device="cuda").manual_seed(F)
+    hidden, w = ((torch.rand(s, generator=g, device="cuda") + 0.5).to(BF) for s in ((T, F), (1, D, F)))
+    x, out = torch.zeros(T, D, dtype=BF, device="cuda"), torch.empty(T, D, device="cuda")
+    p, slots = ops.ptr, i32(range(T))
+    idx, wts = i32([[0]] * T), torch.ones(T, 1, device="cuda")
+    ops.check(ops.library().qs_moe_expert_down(p(out), D, p(hidden), F, p(w), ops.dtype_code(hidden), p(idx), p(wts), p(slots), None, 0, 0, None, T, 1, D, F, p(x), D, 1,
+                                               ops.stream()))
+    ref = hidden.double() @ w[0].double().T
+    off = (out.double() - ref) / ref
+    # rounded additions (F / 128 in a row in a quarter of the sum, four behind them) err either way: at most 2^-24 each, nothing on average over
+    # the 4,096 results; a product of 16 terms of one size, cut off inside the unit, loses at most 2^-23 and as much again for the terms' sizes
+    assert off.abs().max() <= (F / 128 + 4) * 2.0 ** -24 + 2.0 ** -22
+    assert off.mean().abs() <= 2.0 ** -22
+
+
 @pytest.mark.parametrize("counts", [[5], [0, 0, 129, 1, 0, 128, 127], [300, 0, 7], [1] * 70, [40] * 16, [0, 0], [1000, 513]])
 @pytest.mark.parametrize("N,K", [(64, 72), (512, 128), (300, 2048), (1024, 512)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, BF])
