@@ -365,33 +365,34 @@ moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16
     __shared__ int n_live, n_used;
     grid_dep_launch();
     grid_dep_wait();
-    if (threadIdx.x == 0) n_live = n_used = 0;
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-        const int e = idx[first + p];
-        of[p] = e < n_experts && tok_slot[t0 + p / top] >= 0 ? e : 0x7fffffff;
+    constexpr int NONE = 0x7fffffff;
+    for (int p = threadIdx.x; p < (n_pairs + 3) / 4 * 4; p += blockDim.x) {
+        const int e = p < n_pairs ? idx[first + p] : NONE;
+        of[p] = e < n_experts && tok_slot[t0 + p / top] >= 0 ? e : NONE;
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {   // a pair's place: behind the lower experts' pairs and the earlier ones of its own
         const int e = of[p];
-        int rank = 0, before = 0;
-        bool opens = e != 0x7fffffff;
-        for (int q = 0; q < n_pairs; ++q) {
-            const int o = of[q];
-            rank += o < e || (o == e && q < p);
-            if (o == e && q < p) opens = false;
+        int rank = 0;
+        for (int q = 0; q < n_pairs; q += 4) {
+            const int4 o = *reinterpret_cast<const int4*>(of + q);
+            rank += (o.x < e || (o.x == e && q < p)) + (o.y < e || (o.y == e && q + 1 < p)) + (o.z < e || (o.z == e && q + 2 < p)) +
+                    (o.w < e || (o.w == e && q + 3 < p));
         }
         order[rank] = p;
-        if (e != 0x7fffffff) atomicAdd(&n_live, 1);
-        if (opens) {                                    // experts in use below this one
-            for (int q = 0; q < n_pairs; ++q) {
-                if (of[q] >= e) continue;
-                bool once = true;
-                for (int r = 0; r < q; ++r) once &= of[r] != of[q];
-                before += once;
-            }
-            start[before] = rank;
-            atomicAdd(&n_used, 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {                             // the experts in use: where one begins along `order`
+        int used = 0, live = 0;
+        for (int base = 0; base < n_pairs; base += 32) {
+            const int r = base + threadIdx.x, e = r < n_pairs ? of[order[r]] : NONE;
+            const bool opens = e != NONE && (r == 0 || of[order[r - 1]] != e);
+            const unsigned open = __ballot_sync(0xffffffffu, opens);
+            if (opens) start[used + __popc(open & ((1u << threadIdx.x) - 1))] = r;
+            used += __popc(open);
+            live += __popc(__ballot_sync(0xffffffffu, e != NONE));
         }
+        if (threadIdx.x == 0) { n_used = used; n_live = live; }
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, quarter = warp & 3;
@@ -416,7 +417,7 @@ moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16
             for (int j = 0; j < top; ++j) {
                 const int p = t * top + j;
                 float y;
-                if (of[p] == 0x7fffffff) y = __bfloat162float(x[row * ldx + d]);
+                if (of[p] == NONE) y = __bfloat162float(x[row * ldx + d]);
                 else {
                     const float* at = part + p * 16 + r;
                     y = (at[0] + at[most * 16]) + (at[2 * most * 16] + at[3 * most * 16]);

@@ -79,6 +79,34 @@ def test_long_sums_are_rounded_and_not_cut_off(F):
     assert off.mean().abs() <= 2.0 ** -22
 
 
+def took(T, top, E, D, F):
+    """Milliseconds of a step of T tokens that choose `top` of E experts each, best of a few, ten steps in a row without the host between them."""
+    x, w_up, w_down = torch.randn(T, D, device="cuda").to(BF), torch.zeros(E, 2 * F, D, dtype=BF, device="cuda"), torch.zeros(E, D, F, dtype=BF, device="cuda")
+    g = torch.Generator().manual_seed(T)
+    idx, wts = i32(torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)])), torch.ones(T, top, device="cuda")
+    slots, graph, best = i32(range(T)), torch.cuda.CUDAGraph(), []
+    step = lambda: ops.moe_experts_indirect(x, w_up, w_down, idx, wts, slots, "silu", gated=True)         # noqa: E731
+    step()
+    with torch.cuda.graph(graph):
+        for _ in range(10):
+            step()
+    for _ in range(5):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        graph.replay()
+        b.record()
+        torch.cuda.synchronize()
+        best.append(a.elapsed_time(b) / 10)
+    return min(best)
+
+
+def test_many_pairs_cost_no_more_than_their_matrices():
+    """The same 64 experts' matrices for four times the pairs, as many as a block takes: putting the pairs in order must not show (it took
+    six sevenths of the step when it grew with the square of their number; now the step is a quarter longer)."""
+    few, many = took(32, 4, 64, 2048, 512), took(32, 16, 64, 2048, 512)
+    assert many <= 2.5 * few, (few, many)
+
+
 @pytest.mark.parametrize("counts", [[5], [0, 0, 129, 1, 0, 128, 127], [300, 0, 7], [1] * 70, [40] * 16, [0, 0], [1000, 513]])
 @pytest.mark.parametrize("N,K", [(64, 72), (512, 128), (300, 2048), (1024, 512)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, BF])
