@@ -188,9 +188,12 @@ __global__ void moe_expert_down_kernel(float* __restrict__ out, size_t ldo, cons
 // 8 t .. 8 t + 7 of 32, on both sides.  A column does not meet the others and K is cut in four wherever the token stands, so a
 // token's result does not depend on the batch.
 //
-// Bound by the matrices' way from memory.  8 tokens, 16 experts of 4,096 x 1,024 x 3, 4 per token: the feed-forward with its
-// router 218 -> 92 us (every pair read its expert by itself before); 3,000 tokens of width 2,048, all products of all experts in two launches
-// (gemm_tc.cu) instead of one each behind a wait for the host: 428 -> 197 us.
+// Bound by the matrices' way from memory.  Microseconds of the two kernels (every pair reading its expert by itself, as before | now), gated
+// experts of D x F, `top` per token:
+//   16 of 4,096 x 1,024, 4: 1 token 87 | 38, 8: 196 | 93, 16: 323 | 97, 32: 538 | 110;  16 of 2,048 x 512, 4: 128 tokens 558 | 97
+//   64 of 2,048 x 512: 32 tokens of 8: 319 | 108, of 16: 667 | 132;  256 of 2,048 x 512, 8: 1 token 65 | 27, 4: 80 | 64, 8: 122 | 99, 32: 323 | 226
+// 3,000 tokens of width 2,048 with the router: all products of all experts in two launches (gemm_tc.cu) instead of one each behind a wait for
+// the host: 428 -> 197 us.
 constexpr int CHUNK_TOKENS = 32;                        // tokens of a block: at most this many columns of an expert
 
 __device__ __forceinline__ uint4 piece(const __nv_bfloat16* row, int k, int K) {        // eight elements, zeros behind the end
@@ -298,14 +301,22 @@ moe_up_grouped_kernel(__nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv
     __shared__ int count[4];
     grid_dep_launch();
     grid_dep_wait();
-    const int e = blockIdx.y, f0 = blockIdx.x * 16, first = blockIdx.z * CHUNK_TOKENS * top, n_pairs = min(T - blockIdx.z * CHUNK_TOKENS, CHUNK_TOKENS) * top;
+    const int f0 = blockIdx.x * 16, first = blockIdx.z * CHUNK_TOKENS * top, n_pairs = min(T - (int)blockIdx.z * CHUNK_TOKENS, CHUNK_TOKENS) * top;
+    // a block per expert, or, where the chunk has fewer pairs than there are experts, per pair: the first one that chose an expert serves it
+    const bool by_pair = (int)gridDim.y < n_experts;
+    int e = blockIdx.y;
+    if (by_pair) {
+        e = e < n_pairs && tok_slot[(first + e) / top] >= 0 ? idx[first + e] : -1;
+        if (e >= n_experts) e = -1;
+        if (e < 0 && blockIdx.y > 0) return;
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int n = 0;
     for (int base = 0; base < n_pairs; base += 128) {
         const int p = base + threadIdx.x;
         const int mine = p < n_pairs ? idx[first + p] : -1;
         const bool live = p < n_pairs && tok_slot[(first + p) / top] >= 0;
-        if (e == 0 && p < n_pairs && (!live || mine >= n_experts))     // nobody's row, or an expert that returns its input: nothing hidden
+        if (blockIdx.y == 0 && p < n_pairs && (!live || mine >= n_experts))     // nobody's row, or an expert that returns its input: nothing hidden
             for (int f = f0; f < min(F, f0 + 16); ++f) hidden[(size_t)(first + p) * ldh + f] = __float2bfloat16_rn(0.f);
         const unsigned hit = __ballot_sync(0xffffffffu, live && mine == e);
         if (lane == 0) count[warp] = __popc(hit);
@@ -316,6 +327,7 @@ moe_up_grouped_kernel(__nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv
         n += count[0] + count[1] + count[2] + count[3];
         __syncthreads();
     }
+    if (by_pair && (n == 0 || list[0] != first + (int)blockIdx.y)) return;
     const __nv_bfloat16* w = w_up + (size_t)e * MATS * F * D;
     for (int c = 0; c < n; c += 32) {
         const int m = min(32, n - c);
@@ -325,7 +337,7 @@ moe_up_grouped_kernel(__nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv
     }
 }
 
-// Sixteen output elements d of a chunk's tokens: warp w takes quarter w mod 4 of K of every second expert in use; the quarters' sums
+// Sixteen output elements d of a chunk's tokens: warp w takes quarter w mod 4 of K of every second (fourth) expert in use; the quarters' sums
 // rest in shared memory until the tokens' choices are added up in order.
 template <int NT>
 __device__ void down_columns(float* __restrict__ part, const __nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ w, const int* list,
@@ -350,7 +362,7 @@ __device__ void down_columns(float* __restrict__ part, const __nv_bfloat16* __re
         }
 }
 
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(512)
 moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ w_down,
                         const int32_t* __restrict__ idx, const float* __restrict__ wts, const int32_t* __restrict__ tok_slot, const void* __restrict__ add,
                         int add_dtype, size_t ldadd, const float* __restrict__ add_scale, int T, int top, int D, int F, const __nv_bfloat16* __restrict__ x,
@@ -396,7 +408,7 @@ moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, quarter = warp & 3;
-    for (int u = warp >> 2; u < n_used; u += 2) {
+    for (int u = warp >> 2; u < n_used; u += blockDim.x >> 7) {
         const int lo = start[u], hi = u + 1 < n_used ? start[u + 1] : n_live;
         const __nv_bfloat16* w = w_down + (size_t)of[order[lo]] * D * F;
         for (int c = lo; c < hi; c += 32) {
@@ -531,9 +543,10 @@ QS_API int qs_moe_expert_up(void* hidden, long long ldh, const void* x, long lon
     QS_REQUIRE(T > 0 && top > 0 && D > 0 && F > 0, "moe_expert_up: bad sizes");
     QS_REQUIRE((size_t)D * sizeof(float) <= 200 * 1024, "moe_expert_up: width %d does not fit shared memory", D);
     if (dtype == QS_BF16 && D % 8 == 0 && ldx % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w_up % 16) == 0 &&
-        ((uintptr_t)hidden % 16) == 0 && n_experts <= 65535 && top <= 64) {
+        ((uintptr_t)hidden % 16) == 0 && top <= 64) {
         typedef __nv_bfloat16 bf16;
-        const dim3 blocks((F + 15) / 16, n_experts, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS);
+        const int pairs = (T < CHUNK_TOKENS ? T : CHUNK_TOKENS) * top;
+        const dim3 blocks((F + 15) / 16, n_experts < pairs ? n_experts : pairs, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS);
         const cudaError_t err = gated
             ? qs_launch_dependent(moe_up_grouped_kernel<true>, blocks, dim3(128), CHUNK_TOKENS * top * sizeof(int), stream, (bf16*)hidden, (size_t)ldh,
                                   (const bf16*)x, (size_t)ldx, (const bf16*)w_up, idx, tok_slot, T, top, D, F, act, n_experts)
@@ -568,10 +581,12 @@ QS_API int qs_moe_expert_down(float* out, long long ldo, const void* hidden, lon
     QS_REQUIRE(smem <= 200 * 1024, "moe_expert_down: %d x %d hidden values do not fit shared memory", top, F);
     const size_t grouped = (size_t)CHUNK_TOKENS * top * (4 * 16 + 3) * sizeof(float);
     if (dtype == QS_BF16 && F % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)hidden % 16) == 0 && ((uintptr_t)w_down % 16) == 0 && top <= 16) {
+        // sixteen warps to a block where the blocks leave SMs to themselves
+        const int threads = (D + 15) / 16 * ((T + CHUNK_TOKENS - 1) / CHUNK_TOKENS) <= 148 ? 512 : 256;
         cudaError_t err = cudaSuccess;
         if (grouped > 48 * 1024) err = cudaFuncSetAttribute(moe_down_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grouped);
         if (err == cudaSuccess)
-            err = qs_launch_dependent(moe_down_grouped_kernel, dim3((D + 15) / 16, 1, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS), dim3(256), grouped, stream, out, (size_t)ldo,
+            err = qs_launch_dependent(moe_down_grouped_kernel, dim3((D + 15) / 16, 1, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS), dim3(threads), grouped, stream, out, (size_t)ldo,
                                       (const __nv_bfloat16*)hidden, (size_t)ldh, (const __nv_bfloat16*)w_down, idx, wts, tok_slot, add, add_dtype, (size_t)ldadd, add_scale,
                                       T, top, D, F, (const __nv_bfloat16*)x, (size_t)ldx, n_experts);
         if (err != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "moe_expert_down: %s", cudaGetErrorString(err));

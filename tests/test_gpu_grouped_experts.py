@@ -107,6 +107,12 @@ def test_many_pairs_cost_no_more_than_their_matrices():
     assert many <= 2.5 * few, (few, many)
 
 
+def test_experts_that_nobody_chose_cost_nothing():
+    """One token with four of 1,024 experts or of eight: only blocks that have work (with a block per expert it took two to three times as long)."""
+    few, many = took(1, 4, 8, 256, 256), took(1, 4, 1024, 256, 256)
+    assert many <= 1.5 * few, (few, many)
+
+
 @pytest.mark.parametrize("counts", [[5], [0, 0, 129, 1, 0, 128, 127], [300, 0, 7], [1] * 70, [40] * 16, [0, 0], [1000, 513]])
 @pytest.mark.parametrize("N,K", [(64, 72), (512, 128), (300, 2048), (1024, 512)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, BF])
