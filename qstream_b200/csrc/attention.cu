@@ -371,11 +371,12 @@ attention_kernel(TO* __restrict__ out, const T* __restrict__ q, size_t ldo, size
     }
 }
 
-// The same for steps that bring many tokens per sequence, in the float32 engine: a block takes 64 consecutive rows of the
+// The same for steps that bring many tokens per sequence, in the float32 engine: a block takes up to 64 consecutive rows of the
 // packed batch and one query head, and walks the sequence's keys 64 at a time with q, keys and values in shared memory.
 // Every sum has the order of `attention_kernel` (groups of 32 keys, ascending dims, the same tree over a group's
-// weights), so a row's result is the same bits whichever of the two kernels computes it.  Rows of several sequences in
-// a block: one walk per sequence, the other rows masked.
+// weights), so a row's result is the same bits whichever of the two kernels computes it.  With `seq_start` a block's rows are
+// those of one sequence (its first 64, its next 64 ..), so that the walks of short sequences run side by side; without, the batch is cut
+// every 64 rows and a block makes one walk per sequence, the other rows masked.
 //
 // 128 threads as 8 row groups x 16: a thread scores 8 rows x 4 keys and then accumulates 8 rows x 4 NG dims.  Within a group of
 // 32 keys lane l of eight holds keys l, l + 8, l + 16, l + 24, so that the sum over the group has the butterfly's order.
@@ -398,7 +399,7 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
                       const int32_t* __restrict__ tok_slot, const int32_t* __restrict__ tok_pos,
                       int T_tokens, int n_heads, int n_kv_heads, int dh, float scale, int window,
                       int32_t* __restrict__ status, int dv, float softcap, int chunk, int keep_first,
-                      const float* __restrict__ sink, int maps) {
+                      const float* __restrict__ sink, int maps, const int32_t* __restrict__ seq_start, int n_seq) {
     extern __shared__ __align__(16) float tile_smem[];
     __shared__ int s_slot[TQ], s_pos[TQ], s_first[TQ], s_kept[TQ], s_ok[TK], s_end;
     __shared__ float s_alpha[2][TQ];
@@ -408,8 +409,33 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
     float* sp = sk;
     float* sv = sk + TK * (pitch > TQ + 4 ? pitch : TQ + 4);      // [TK][vp]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int row0 = (gridDim.x - 1 - blockIdx.x) * TQ, head = blockIdx.y;      // the longest contexts first
-    const int n_rows = min(TQ, T_tokens - row0);
+    const int head = blockIdx.y;
+    int row0 = (gridDim.x - 1 - blockIdx.x) * TQ, n_rows = min(TQ, T_tokens - row0);     // the longest contexts first
+    if (seq_start) {                                    // the block's sequence: tiles counted from the last rows, a lane per sequence
+        __shared__ int s_row0, s_rows;
+        if (tid == 0) s_rows = 0;
+        if (tid < 32) {
+            int run = 0;
+            for (int base = 0; base <= n_seq && run <= (int)blockIdx.x; base += 32) {
+                const int s = n_seq - base - tid;       // number n_seq: the rows behind the last sequence
+                const int lo = s >= 0 ? seq_start[s] : 0, hi = s < 0 ? 0 : s < n_seq ? min(seq_start[s + 1], T_tokens) : T_tokens;
+                const int tiles = hi > lo ? (hi - lo + TQ - 1) / TQ : 0;
+                int sum = tiles;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (tid >= o) sum += v; }
+                const int at = (int)blockIdx.x - (run + sum - tiles);
+                if (at >= 0 && at < tiles) {
+                    s_row0 = lo + (tiles - 1 - at) * TQ;
+                    s_rows = min(TQ, hi - s_row0);
+                }
+                run += __shfl_sync(0xffffffffu, sum, 31);
+            }
+        }
+        __syncthreads();
+        row0 = s_row0;
+        n_rows = s_rows;
+        if (n_rows == 0) return;                        // the grid has a block to spare per sequence
+    }
     const int kvh = (head / maps) / (n_heads / maps / n_kv_heads);
     const int krow_width = dh * maps, k_off = (head % maps) * dh, page_tokens = 1 << page_shift;
     if (tid < TQ) {
@@ -615,26 +641,42 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
     }
 }
 
-// From how many rows per sequence on the tile kernel serves: below, most of a block's 64 rows would be masked.
-constexpr int TILE_ROWS_PER_SEQUENCE = 16;
+// Where the tile kernel serves: from 16 rows per sequence on (the mean: a tile of fewer rows is a block of its own), and with no more keys
+// than one group of 32 from 32 rows on.  Microseconds (tiles | a warp per query), heads of 128, 1 and 16 sequences of so many rows
+// behind so many cached keys:
+//              1 sequence, 16 heads                                         16 sequences, 16 heads
+//   rows       0 keys    48        112       500        2,000               0 keys     48         500          2,000
+//   16         25 | 20   29 | 51   45 | 96   158 | 369  543 | 1,393         31 | 35    37 | 137   221 | 1,071  771 | 4,075
+//   24         25 | 23   41 | 60   59 | 104  158 | 373  547 | 1,393         31 | 68    55 | 258   223 | 2,014  780 | 7,560
+//   32         27 | 28   43 | 63   59 | 109  164 | 375  562 | 1,397         33 | 100   57 | 322   227 | 2,404  786 | 9,232
+// A prompt of 2,000 tokens beside 64 sequences that bring one token behind 2,000 keys: 3.4 ms, 17.2 with a warp per query, 28.9 with
+// tiles cut every 64 rows, whose blocks walk sequence after sequence.
+constexpr int TILE_ROWS = 16, TILE_ROWS_SHORT = 32, TILE_KEYS = 33;
+bool tiles_serve(long long rows, int n_seq, int longest) {
+    return n_seq > 0 && rows >= (longest == 0 || longest >= TILE_KEYS ? TILE_ROWS : TILE_ROWS_SHORT) * (long long)n_seq;
+}
 
 template <typename T, typename TO>
 int launch_attention(void* out, const void* q, long long ldo, long long ldq, const void* k_cache,
                      const void* v_cache, const int32_t* page_table, int max_pages, int page_shift,
                      const int32_t* tok_slot, const int32_t* tok_pos, int T_tokens, int n_heads,
                      int n_kv_heads, int dh, float scale, int window, int32_t* status, int dv, float softcap,
-                     int chunk, int keep_first, const float* sink, int maps, int n_seq, cudaStream_t stream) {
+                     int chunk, int keep_first, const float* sink, int maps, int n_seq, const int32_t* seq_start, int longest,
+                     cudaStream_t stream) {
     // the tile kernel copies 16-byte pieces and holds the tiles of a head in shared memory
-    if (sizeof(T) == 4 && sizeof(TO) == 4 && n_seq > 0 && T_tokens >= TILE_ROWS_PER_SEQUENCE * (long long)n_seq && n_heads <= 65535 &&
+    if (sizeof(T) == 4 && sizeof(TO) == 4 && tiles_serve(T_tokens, n_seq, longest) && n_heads <= 65535 &&
         dh % 4 == 0 && dv % 4 == 0 && dh <= 256 && dv <= 256 && ldq % 4 == 0 && ((uintptr_t)q % 16) == 0 &&
         ((uintptr_t)k_cache % 16) == 0 && ((uintptr_t)v_cache % 16) == 0) {
         const int ng = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4), pitch = dh + 4;
         const size_t bytes = (size_t)(dh * (TQ + 4) + TK * (pitch > TQ + 4 ? pitch : TQ + 4) + TK * ng * 64) * sizeof(float);
+        if (n_seq == 1) seq_start = nullptr;            // cut every 64 rows all the same
+        const int blocks = seq_start ? T_tokens / TQ + n_seq + 1 : (T_tokens + TQ - 1) / TQ;
         cudaError_t e = cudaSuccess;
 #define GOT(NG_) do { if (bytes > 40 * 1024) e = cudaFuncSetAttribute(attention_tile_kernel<NG_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
-        if (e == cudaSuccess) attention_tile_kernel<NG_><<<dim3((T_tokens + TQ - 1) / TQ, n_heads), 128, bytes, stream>>>( \
+        if (e == cudaSuccess) attention_tile_kernel<NG_><<<dim3(blocks, n_heads), 128, bytes, stream>>>( \
             (float*)out, (const float*)q, (size_t)ldo, (size_t)ldq, (const float*)k_cache, (const float*)v_cache, page_table, max_pages, \
-            page_shift, tok_slot, tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window, status, dv, softcap, chunk, keep_first, sink, maps); } while (0)
+            page_shift, tok_slot, tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window, status, dv, softcap, chunk, keep_first, sink, maps, \
+            seq_start, n_seq); } while (0)
         if (ng == 1) GOT(1); else if (ng == 2) GOT(2); else GOT(4);
 #undef GOT
         if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "attention: %s", cudaGetErrorString(e));
@@ -1103,14 +1145,15 @@ QS_API int qs_rope_unit_store(void* q, const void* k, const void* v, int dtype, 
     return qs_check_launch("rope_unit_store");
 }
 
-// n_seq: how many sequences the rows belong to (0: not known); it only picks the kernel.
+// n_seq: how many sequences the rows belong to (0: not known), seq_start [n_seq + 1] (device, or null): where each begins, longest: the
+// most keys a row sees (0: not known); they pick the kernel and its tiles, not the result.
 QS_API int qs_attention(void* out, const void* q, int dtype, long long ldo, long long ldq,
                         const void* k_cache, const void* v_cache,
                         const int32_t* page_table, int max_pages, int page_tokens,
                         const int32_t* tok_slot, const int32_t* tok_pos, int T_tokens,
                         int n_heads, int n_kv_heads, int dh, float scale, int window,
                         int32_t* status, int dv, float softcap, int chunk, int keep_first, const float* sink,
-                        int maps, int out_dtype, int n_seq, cudaStream_t stream) {
+                        int maps, int out_dtype, int n_seq, const int32_t* seq_start, int longest, cudaStream_t stream) {
     if (T_tokens == 0) return QS_OK;
     if (dv <= 0) dv = dh;
     if (maps <= 0) maps = 1;
@@ -1130,15 +1173,15 @@ QS_API int qs_attention(void* out, const void* q, int dtype, long long ldo, long
     if (dtype == QS_F32)
         return launch_attention<float, float>(out, q, ldo, ldq, k_cache, v_cache, page_table, max_pages, shift, tok_slot,
                                        tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window, status, dv, softcap,
-                                       chunk, keep_first, sink, maps, n_seq, stream);
+                                       chunk, keep_first, sink, maps, n_seq, seq_start, longest, stream);
     if (dtype == QS_BF16 && out_dtype == QS_F32)
         return launch_attention<__nv_bfloat16, float>(out, q, ldo, ldq, k_cache, v_cache, page_table, max_pages, shift,
                                                       tok_slot, tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window,
-                                                      status, dv, softcap, chunk, keep_first, sink, maps, n_seq, stream);
+                                                      status, dv, softcap, chunk, keep_first, sink, maps, n_seq, seq_start, longest, stream);
     if (dtype == QS_BF16)
         return launch_attention<__nv_bfloat16, __nv_bfloat16>(out, q, ldo, ldq, k_cache, v_cache, page_table, max_pages, shift,
                                                               tok_slot, tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window,
-                                                              status, dv, softcap, chunk, keep_first, sink, maps, n_seq, stream);
+                                                              status, dv, softcap, chunk, keep_first, sink, maps, n_seq, seq_start, longest, stream);
     return qs_fail(QS_ERR_INVALID_INPUT, "attention: unknown dtype %d", dtype);
 }
 

@@ -45,7 +45,7 @@ _SIGNATURES = {
                             c_void_p], c_int),
     "qs_attention": ([c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_int,
                       c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p,
-                      c_int, c_float, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p], c_int),
+                      c_int, c_float, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p], c_int),
     "qs_pair_diff_norm": ([c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_float, c_float,
                            c_float, c_void_p], c_int),
     "qs_delta_prepare": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int,
@@ -376,7 +376,7 @@ def rope_unit_store(q, k, v, eps, n_heads, n_kv_heads, head_dim, rotary_dim, cos
 
 def attention(q, n_heads, n_kv_heads, head_dim, scale, window, tok_slot, tok_pos, page_table,
               page_tokens, k_cache, v_cache, status, out=None, v_head_dim=None, softcap=0.0, chunk=0, keep_first=0,
-              sink=None, maps=1, out_dtype=None, n_seq=0) -> torch.Tensor:
+              sink=None, maps=1, out_dtype=None, n_seq=0, seq_start=None, longest=0) -> torch.Tensor:
     """Causal attention of every token over its sequence's cache (generic kernels).  `v_head_dim`: the values'
     head size where it differs from the keys'; `softcap` c > 0: scores become c tanh(s / c) before the softmax.
     A query at position p sees the last `window` keys (window > 0), or the keys of its own chunk of `chunk`
@@ -385,7 +385,8 @@ def attention(q, n_heads, n_kv_heads, head_dim, scale, window, tok_slot, tok_pos
     `maps` m > 1: a cached key row holds m keys of head_dim side by side and `n_heads` counts m query heads per
     head, query head j reading key j % m of its key head; all of them read the same values.  `out_dtype`
     torch.float32: the result in 32-bit whatever the queries' type.  `n_seq`: how many sequences the rows belong to
-    (0: not known); it picks the kernel, not the result."""
+    (0: not known), `seq_start` (int32 [n_seq + 1] on the device) where each begins, `longest` the most keys a row sees (0: not
+    known); they pick the kernel and its tiles, not the result."""
     T = q.shape[0]
     if sink is not None and (sink.dtype != torch.float32 or sink.numel() != n_heads or not sink.is_contiguous()):
         raise QStreamError(QsError.INVALID_INPUT, "attention: the sinks must be float32, one per query head")
@@ -397,7 +398,7 @@ def attention(q, n_heads, n_kv_heads, head_dim, scale, window, tok_slot, tok_pos
         _int32(page_table, "page_table"), page_table.shape[1], page_tokens, _int32(tok_slot, "tok_slot"),
         _int32(tok_pos, "tok_pos"), T, n_heads, n_kv_heads, head_dim, float(scale), int(window),
         ptr(status), dv, float(softcap or 0.0), int(chunk), int(keep_first), ptr(sink), int(maps),
-        dtype_code(out), int(n_seq), stream()))
+        dtype_code(out), int(n_seq), _int32(seq_start, "seq_start") if seq_start is not None else None, int(longest), stream()))
     return out
 
 

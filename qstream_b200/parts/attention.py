@@ -233,7 +233,8 @@ class Attention(Mixer):
             o = ops.attention(q, s.n_heads * self.maps, s.n_kv_heads, s.head_dim, s.scale, s.window, b.tok_slot, b.tok_pos,
                               view.page_table, view.page_tokens, view.k, view.v, step.status, out=None if two or gate is not None else out,
                               v_head_dim=s.value_dim, softcap=s.softcap, chunk=self.chunk, keep_first=self.keep_first,
-                              sink=self.sink, maps=self.maps, out_dtype=wide, n_seq=b.n_seq)
+                              sink=self.sink, maps=self.maps, out_dtype=wide, n_seq=b.n_seq, seq_start=b.seq_start,
+                              longest=b.max_total)
         if two:
             o = ops.pair_diff_norm(o, s.n_heads, s.value_dim, self.lam, 1.0 - float(s.diff), float(s.eps), q.dtype)
         if gate is not None:
@@ -257,7 +258,8 @@ def attend(q, spec, step, view, out=None, gate=None, sink=None):
             return done
     o = ops.attention(q, spec.n_heads, spec.n_kv_heads, spec.head_dim, spec.scale, spec.window,
                       b.tok_slot, b.tok_pos, view.page_table, view.page_tokens, view.k, view.v,
-                      step.status, out=out, v_head_dim=spec.value_dim, softcap=spec.softcap, sink=sink, n_seq=b.n_seq)
+                      step.status, out=out, v_head_dim=spec.value_dim, softcap=spec.softcap, sink=sink, n_seq=b.n_seq, seq_start=b.seq_start,
+                      longest=b.max_total)
     if gate is not None:
         o = ops.gated_group_norm(o, 0, None, gate, "sigmoid", 0.0, o.dtype, gate_span=spec.value_dim if spec.gate == "head" else 1)
     return o

@@ -79,6 +79,48 @@ def test_tiles_of_queries_are_the_same_bits(dh, dv, H, G, maps, mask):
             assert bool(torch.isfinite(tiled).all()) and not bool(tiled[20].any()) and not bool(tiled[133].any())
 
 
+def mixed_step(lens, before, H, dh, seed):
+    """A step in which sequence i brings lens[i] tokens behind before[i] cached ones, with three rows of nobody behind."""
+    case = PagedCase("float32", [a + b for a, b in zip(lens, before)], 1, H, dh, seed=seed, n_slots=len(lens), fill=0.0)
+    g = torch.Generator().manual_seed(seed)
+    case.k_cache.copy_(torch.randn(case.k_cache.shape, generator=g))
+    case.v_cache.copy_(torch.randn(case.v_cache.shape, generator=g))
+    slot = torch.tensor([s for s, n in zip(case.slots, lens) for _ in range(n)] + [-1] * 3, dtype=torch.int32).cuda()
+    pos = torch.tensor([b + i for n, b in zip(lens, before) for i in range(n)] + [0] * 3, dtype=torch.int32).cuda()
+    start = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32).cuda()
+    q = torch.randn(sum(lens) + 3, H * dh, generator=g).cuda()
+    assert slot.numel() == pos.numel() == q.shape[0]
+    args = (q, H, H, dh, dh ** -0.5, 0, slot, pos, case.table.cuda(), 64, case.k_cache, case.v_cache, case.status)
+    return case, args, dict(n_seq=len(lens), seq_start=start, longest=max(a + b for a, b in zip(lens, before)))
+
+
+@pytest.mark.parametrize("lens,before", [([130], [0]), ([64, 64], [0, 0]), ([1] * 40 + [900], [77] * 40 + [0]), ([16, 17, 63, 64, 65, 129], [200, 0, 3, 64, 1, 0]),
+                                         ([700, 1, 1], [0, 300, 64]), ([33] * 35, [5 * i for i in range(35)])])
+def test_tiles_within_a_sequence_are_the_same_bits(lens, before):
+    """Tiles that begin where a sequence begins, one to more sequences than a warp looks at together, among them single rows."""
+    case, args, hints = mixed_step(lens, before, 2, 64, len(lens) + lens[0])
+    by_row, tiled = ops.attention(*args), ops.attention(*args, **hints)
+    assert int(case.status.item()) == 0 and torch.equal(by_row, tiled) and not bool(tiled[sum(lens):].any())
+
+
+def test_a_prompt_among_decoding_sequences_takes_no_longer_in_tiles():
+    """A long prompt beside 64 sequences that bring one token each: their walks run side by side (one after the other in the blocks
+    that hold them, the step took 1.7 times as long as with a warp per query; side by side about a quarter)."""
+    _, args, hints = mixed_step([1200] + [1] * 64, [0] + [1500] * 64, 4, 128, 3)
+    took = {}
+    for name, kw in (("tiles", hints), ("rows", {})):
+        times = []
+        for _ in range(4):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            ops.attention(*args, **kw)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took[name] = min(times)
+    assert took["tiles"] <= took["rows"], took
+
+
 def test_tiles_keep_what_is_not_finite_to_the_rows_that_see_it():
     lens = [150]
     case, q, slot, pos = attention_args(64, 64, 2, 2, 1, lens, 5)
