@@ -656,6 +656,11 @@ bool tiles_serve(long long rows, int n_seq, int longest) {
     return n_seq > 0 && rows >= (longest == 0 || longest >= TILE_KEYS ? TILE_ROWS : TILE_ROWS_SHORT) * (long long)n_seq;
 }
 
+size_t tile_smem_bytes(int dh, int ng) {
+    const int pitch = dh + 4 > TQ + 4 ? dh + 4 : TQ + 4;
+    return (size_t)(dh * (TQ + 4) + TK * pitch + TK * ng * 64) * sizeof(float);
+}
+
 template <typename T, typename TO>
 int launch_attention(void* out, const void* q, long long ldo, long long ldq, const void* k_cache,
                      const void* v_cache, const int32_t* page_table, int max_pages, int page_shift,
@@ -667,12 +672,13 @@ int launch_attention(void* out, const void* q, long long ldo, long long ldq, con
     if (sizeof(T) == 4 && sizeof(TO) == 4 && tiles_serve(T_tokens, n_seq, longest) && n_heads <= 65535 &&
         dh % 4 == 0 && dv % 4 == 0 && dh <= 256 && dv <= 256 && ldq % 4 == 0 && ((uintptr_t)q % 16) == 0 &&
         ((uintptr_t)k_cache % 16) == 0 && ((uintptr_t)v_cache % 16) == 0) {
-        const int ng = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4), pitch = dh + 4;
-        const size_t bytes = (size_t)(dh * (TQ + 4) + TK * (pitch > TQ + 4 ? pitch : TQ + 4) + TK * ng * 64) * sizeof(float);
+        const int ng = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4);
+        const size_t bytes = tile_smem_bytes(dh, ng);
         if (n_seq == 1) seq_start = nullptr;            // cut every 64 rows all the same
         const int blocks = seq_start ? T_tokens / TQ + n_seq + 1 : (T_tokens + TQ - 1) / TQ;
         cudaError_t e = cudaSuccess;
-#define GOT(NG_) do { if (bytes > 40 * 1024) e = cudaFuncSetAttribute(attention_tile_kernel<NG_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+        // the limit is set to what the widest heads need, whatever these need: another thread's launch may come between it and this one's
+#define GOT(NG_) do { e = cudaFuncSetAttribute(attention_tile_kernel<NG_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem_bytes(256, NG_)); \
         if (e == cudaSuccess) attention_tile_kernel<NG_><<<dim3(blocks, n_heads), 128, bytes, stream>>>( \
             (float*)out, (const float*)q, (size_t)ldo, (size_t)ldq, (const float*)k_cache, (const float*)v_cache, page_table, max_pages, \
             page_shift, tok_slot, tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window, status, dv, softcap, chunk, keep_first, sink, maps, \

@@ -575,7 +575,9 @@ QS_API int qs_delta_chunks(float* o, long long ldo, const float* q, long long ld
     cudaError_t e = cudaFuncSetAttribute(delta_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TERMS_SMEM);
     if (e == cudaSuccess) e = qs_launch_dependent(delta_terms_kernel, dim3(n_chunks, H), dim3(TERMS), TERMS_SMEM, stream, p);
     const size_t walk = walk_smem(p.dkp);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
+    // the most any head takes (two stages of 128 channels or one of 256), so that threads with models of other sizes set the same
+    const size_t most = walk_smem(256) > walk_smem(128) ? walk_smem(256) : walk_smem(128);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e == cudaSuccess) e = qs_launch_dependent(delta_walk_kernel, dim3(n_seq, H, (dv + WC - 1) / WC), dim3(WALK), walk, stream, p, walk_stages(p.dkp));
 #define GO(NC) do { const size_t smem = output_floats<NC>() * sizeof(float); \
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_output_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \

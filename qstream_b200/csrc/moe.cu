@@ -579,14 +579,15 @@ QS_API int qs_moe_expert_down(float* out, long long ldo, const void* hidden, lon
     QS_REQUIRE(T > 0 && top > 0 && D > 0 && F > 0, "moe_expert_down: bad sizes");
     const size_t smem = (size_t)top * F * sizeof(float);
     QS_REQUIRE(smem <= 200 * 1024, "moe_expert_down: %d x %d hidden values do not fit shared memory", top, F);
-    const size_t grouped = (size_t)CHUNK_TOKENS * top * (4 * 16 + 3) * sizeof(float);
-    if (dtype == QS_BF16 && F % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)hidden % 16) == 0 && ((uintptr_t)w_down % 16) == 0 && top <= 16) {
+    constexpr int MOST_CHOICES = 16;
+    auto grouped = [](int choices) { return (size_t)CHUNK_TOKENS * choices * (4 * 16 + 3) * sizeof(float); };
+    if (dtype == QS_BF16 && F % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)hidden % 16) == 0 && ((uintptr_t)w_down % 16) == 0 && top <= MOST_CHOICES) {
         // sixteen warps to a block where the blocks leave SMs to themselves
         const int threads = (D + 15) / 16 * ((T + CHUNK_TOKENS - 1) / CHUNK_TOKENS) <= 148 ? 512 : 256;
-        cudaError_t err = cudaSuccess;
-        if (grouped > 48 * 1024) err = cudaFuncSetAttribute(moe_down_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grouped);
+        // the limit for the most choices, whatever these are: another thread's launch may come between it and this one's
+        cudaError_t err = cudaFuncSetAttribute(moe_down_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grouped(MOST_CHOICES));
         if (err == cudaSuccess)
-            err = qs_launch_dependent(moe_down_grouped_kernel, dim3((D + 15) / 16, 1, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS), dim3(threads), grouped, stream, out, (size_t)ldo,
+            err = qs_launch_dependent(moe_down_grouped_kernel, dim3((D + 15) / 16, 1, (T + CHUNK_TOKENS - 1) / CHUNK_TOKENS), dim3(threads), grouped(top), stream, out, (size_t)ldo,
                                       (const __nv_bfloat16*)hidden, (size_t)ldh, (const __nv_bfloat16*)w_down, idx, wts, tok_slot, add, add_dtype, (size_t)ldadd, add_scale,
                                       T, top, D, F, (const __nv_bfloat16*)x, (size_t)ldx, n_experts);
         if (err != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "moe_expert_down: %s", cudaGetErrorString(err));
