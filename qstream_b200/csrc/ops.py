@@ -580,7 +580,7 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     mode "delta": S' = diag(g_t) S, u = beta_t (v - S'^T k), S <- S' + k u^T, o = S^T q, with g = `key_decay` (float32
     [T, heads * key_dim]) and beta = `token_weight` (float32 [T, heads]); q and k hold heads / `qk_group` heads, head h
     reading number h // qk_group.  With `chunks` the delta rule solves each chunk's writes as a triangular system, side by
-    side, and walks the chunks in order (csrc/delta_chunks.cu; float32 operands).  In mode "decay" `q_scale` multiplies q as well.
+    side, and walks the chunks in order (csrc/delta_chunks.cu).  In mode "decay" `q_scale` multiplies q as well.
     mode "gla": S <- diag(w_t) S + k v^T, o = S^T (q q_scale), w_t = sigmoid(decay_logits)^`decay_power` per token and key
     channel (float32 [T, heads * key_dim]), taken in 32-bit inside the walk.
     mode "ssd": S <- a_t S + b_t k v^T, o = S^T (q q_scale) with a - 1 = `token_decay`, b = `token_weight` (float32
@@ -599,12 +599,9 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: only the delta rule walks without values")
     chunk_start = chunk_ids = seq_chunk = chunk_state = chunk_decay = None
     n_chunks = 0
-    if chunks is not None and ACTIVATIONS[in_activation] != ACT_NONE:      # once per element: the chunks' kernels read q, k and v several times
-        nk, nv = q.shape[1], v.shape[1]
-        ready = torch.empty((T, 2 * nk + nv), dtype=torch.float32, device=q.device)
-        check(library().qs_scan_activate(ptr(ready), ptr(q), q.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), dtype_code(q), T, nk, nv,
-                                         ACTIVATIONS[in_activation], stream()))
-        q, k, v, in_activation = ready[:, :nk], ready[:, nk:2 * nk], ready[:, 2 * nk:], None
+    if chunks is not None and ACTIVATIONS[in_activation] != ACT_NONE:
+        q, k, v = _activated(q, k, v, in_activation)
+        in_activation = None
     if chunks is not None:
         chunk_start, chunk_ids, seq_chunk, n_chunks = chunks
         chunk_state = torch.empty((n_chunks, n_heads * key_dim * (-(-value_dim // 4) * 4)), dtype=torch.float32, device=q.device)
@@ -630,13 +627,28 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     return o
 
 
+def _activated(q, k, v, activation):
+    """act(q), act(k), act(v) in 32-bit, once per element: the chunks' kernels read them several times."""
+    T, nk, nv = q.shape[0], q.shape[1], v.shape[1]
+    ready = torch.empty((T, 2 * nk + nv), dtype=torch.float32, device=q.device)
+    check(library().qs_scan_activate(ptr(ready), ptr(q), q.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), dtype_code(q), T, nk, nv,
+                                     ACTIVATIONS[activation], stream()))
+    return ready[:, :nk], ready[:, nk:2 * nk], ready[:, 2 * nk:]
+
+
 def _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_dim, key_decay, token_weight, qk_group, chunks):
     """The delta rule of a long prompt, its chunks as matrix products (csrc/delta_chunks.cu): what each chunk's tokens ask of the
     state it starts from and what they write, side by side; the chunks' states in order; the outputs, side by side."""
     chunk_start, chunk_ids, seq_chunk, n_chunks = chunks
     T = q.shape[0]
-    if any(t.dtype != torch.float32 or t.stride(1) != 1 for t in (q, k, v, key_decay, token_weight)):
-        raise QStreamError(QsError.INVALID_INPUT, "state_scan: the delta rule in chunks takes float32 operands")
+    if any(t.dtype != torch.float32 or t.stride(1) != 1 for t in (key_decay, token_weight)):
+        raise QStreamError(QsError.INVALID_INPUT, "state_scan: the delta rule takes float32 decays and step sizes")
+    if v is None:
+        v = torch.zeros((T, n_heads * value_dim), dtype=q.dtype, device=q.device)
+    if any(t.dtype != q.dtype or t.stride(1) != 1 for t in (q, k, v)):
+        raise QStreamError(QsError.INVALID_INPUT, "state_scan: q, k and v must be rows of one type")
+    if q.dtype != torch.float32:
+        q, k, v = _activated(q, k, v, None)
     lib = library()
     o = torch.empty((T, n_heads * value_dim), dtype=torch.float32, device=q.device)
     scratch = torch.empty((lib.qs_delta_chunks_scratch(int(n_chunks), n_heads, key_dim, value_dim),), dtype=torch.float32, device=q.device)

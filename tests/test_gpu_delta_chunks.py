@@ -73,3 +73,26 @@ def test_what_is_not_finite_reaches_no_earlier_token():
     o = run(q, k, v, g, beta, state, [0, T], [0], cut([T])).cpu().numpy().reshape(T, H, dv)
     assert np.isfinite(o[:90]).all() and np.isfinite(o[:100, 0]).all() and np.isfinite(o[90:110, 1, :3]).all()
     assert not np.isfinite(o[90, 1, 3]) and not np.isfinite(o[100, 0]).any() and not np.isfinite(o[110, 1]).any() and np.isfinite(o[111:, 1, :3]).all()
+
+
+def test_operands_in_bfloat16_and_absent_values():
+    """What the walk in order takes, the chunks take: bfloat16 q, k and v (exact in 32-bit: the same bits), and no values at all."""
+    T, H, dk, dv = 200, 2, 40, 24
+    q, k, v, g, beta = make(T, H, 1, dk, dv, 8, False)
+    wide = torch.from_numpy(np.concatenate([x.reshape(T, -1) for x in (q, k, v)], 1)).to(torch.bfloat16).cuda()
+    q, k, v = wide[:, :dk], wide[:, dk:2 * dk], wide[:, 2 * dk:]
+    g, beta = (torch.from_numpy(x.reshape(T, -1)).float().cuda() for x in (g, beta))
+    S0 = torch.randn(1, H, dv, dk, generator=torch.Generator().manual_seed(1)).cuda()
+
+    def scan(q, k, v, chunks):
+        state = S0.clone()
+        o = ops.state_scan("delta", q, k, v, state, i32([0, T]), i32([0]), 1, H, dk, dv, chunks=chunks, key_decay=g, token_weight=beta, qk_group=H)
+        return o, state
+
+    for values in (v, None):
+        low = scan(q, k, values, cut([T]))
+        high = scan(q.float(), k.float(), v.float() if values is not None else torch.zeros(T, H * dv, device="cuda"), cut([T]))
+        walked = scan(q, k, values, None)
+        for a, b, c in zip(low, high, walked):
+            assert torch.equal(a, b)
+            assert (a - c).norm() <= 4 * 2.0 ** -24 * (np.sqrt(64) + np.sqrt(dk)) * np.sqrt(T / 16) * c.norm()
