@@ -88,10 +88,11 @@ row_group_norm_kernel(TO* __restrict__ out, size_t ldo, const TI* __restrict__ o
     }
 }
 
-// Whether the kernel above takes a row of n elements in groups of `group`, spans of `gate_span`.
-inline bool row_group_norm_takes(int n, int group, int gate_span) {
+// Whether the kernel above takes a row of n elements in groups of `group`, spans of `gate_span`; rows of fewer than `fewest` elements are
+// the general kernels'.
+inline bool row_group_norm_takes(int n, int group, int gate_span, int fewest) {
     const bool pow2 = group >= 8 && group <= 256 && (group & (group - 1)) == 0;
-    return n % 8 == 0 && n <= 8 * 256 * 4 && (group == 0 || group == n || pow2) && (gate_span == 1 || gate_span % 8 == 0);
+    return n % 8 == 0 && n >= fewest && n <= 8 * 256 * 4 && (group == 0 || group == n || pow2) && (gate_span == 1 || gate_span % 8 == 0);
 }
 template <typename T>
 inline bool in_pieces(const T* p, long long ld) { return !p || (((uintptr_t)p % 16) == 0 && ld % 8 == 0); }

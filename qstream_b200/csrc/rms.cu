@@ -380,7 +380,11 @@ __global__ void gated_group_norm_kernel(TO* __restrict__ out, size_t ldo, const 
 template <typename TI, typename TG, typename TO>
 int launch_gated(void* out, long long ldo, const void* o, long long ldi, const void* w, int w_dtype, const void* gate,
                  long long ldg, int gate_act, int rows, int n, int group, float eps, int gate_span, cudaStream_t stream) {
-    if (row_group_norm_takes(n, group, gate_span) && in_pieces(out, ldo) && in_pieces(o, ldi) && (!gate || gate_span > 1 || in_pieces(gate, ldg)) &&
+    // Eight elements to a thread are a longer chain than one: short rows are faster in the general kernel until there are enough of them
+    // to keep every SM busy.  Microseconds, general | pieces, bfloat16 with one norm over the row: 64 elements, 1 row 2.0 | 3.0, 4,096 rows
+    // 5.0 | 6.3; 128: 2.0 | 3.0, 6.1 | 6.3; 192: 2.8 | 3.0, 7.1 | 6.4; 256: 2.8 | 3.0, 7.6 | 6.5; 384: 3.5 | 3.0, 9.8 | 7.6.
+    const int fewest = rows >= 4096 ? 192 : 264;
+    if (row_group_norm_takes(n, group, gate_span, fewest) && in_pieces(out, ldo) && in_pieces(o, ldi) && (!gate || gate_span > 1 || in_pieces(gate, ldg)) &&
         in_pieces(w, 0)) {
         const cudaError_t err = launch_row_group_norm<TI, TG, TO, false>((TO*)out, (size_t)ldo, (const TI*)o, (size_t)ldi, w, w_dtype, (const TG*)gate, (size_t)ldg,
                                                                          gate_act, rows, n, group, eps, gate_span, nullptr, 0, nullptr, 8, stream);

@@ -5,6 +5,7 @@ import torch
 from qstream_b200.csrc import ops
 
 pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
 ACT = {"sigmoid": torch.sigmoid, "silu": torch.nn.functional.silu}
 
 
@@ -40,7 +41,18 @@ def test_gated_group_norm(n, group, types):
         close(ops.gated_group_norm(o, group, None, gate, "sigmoid", 1e-5, tout, gate_span=8), ref, group)
 
 
-@pytest.mark.parametrize("H,dv,parts", [(64, 64, 1), (8, 16, 4), (6, 8, 3), (32, 64, 8), (5, 7, 1), (16, 12, 2), (130, 64, 1)])
+@pytest.mark.parametrize("n,group", [(184, 184), (192, 192), (192, 64), (256, 256), (256, 8), (264, 264), (264, 8), (272, 16)])
+@pytest.mark.parametrize("rows", [3, 4095, 4096])
+@pytest.mark.parametrize("dtype", [torch.float32, BF16])
+def test_rows_around_the_shortest_that_are_taken_in_pieces(n, group, rows, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n + group)
+    o, gate, w = torch.randn(rows, n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda").to(dtype), torch.rand(n, generator=g, device="cuda").to(dtype)
+    ref = o.double().view(rows, -1, group)
+    ref = (ref / torch.sqrt(ref.square().mean(-1, keepdim=True) + 1e-5)).view(rows, n)
+    close(ops.gated_group_norm(o, group, w, gate, "silu", 1e-5, dtype), ref * w.double() * ACT["silu"](gate.double()), group)
+
+
+@pytest.mark.parametrize("H,dv,parts", [(64, 64, 1), (8, 16, 4), (6, 8, 3), (32, 64, 8), (5, 7, 1), (16, 12, 2), (130, 64, 1), (23, 8, 1), (24, 8, 1), (3, 64, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_ssd_output(H, dv, parts, dtype):
     g = torch.Generator(device="cuda").manual_seed(H * dv + parts)
