@@ -216,14 +216,15 @@ QS_API int qs_delta_prepare(float* qo, float* ko, float* vo, float* go, float* b
     const int threads = 256;
     cudaError_t e;
     // Pieces of eight channels where every row and weight begins on a piece, a head is a power of two of one warp's lanes, and the taps
-    // are as many as are unrolled; from 512 tokens on a block per token fills the GPU, below that a token's pieces go to several blocks.
+    // are as many as are unrolled; from 512 tokens on a block per token fills the GPU, below that a token's pieces go to several blocks.  No
+    // more threads than pieces: 2,000 float32 tokens of 96 pieces take 11.9 us, 21.4 in blocks of 256 (a channel at a time 15.8).
     const int lanes = dk / 8;
     auto fits = [&](const void* ptr) { return ((uintptr_t)ptr % 32) == 0 || (dtype == QS_BF16 && ((uintptr_t)ptr % 16) == 0); };
     if (dtype == w_dtype && taps >= 2 && taps <= 4 && dk % 8 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && dv % 8 == 0 && ldp % 8 == 0 && lda % 8 == 0 &&
         slot_stride % 8 == 0 && fits(q) && fits(k) && fits(v) && fits(wq) && fits(wk) && fits(wv) && fits(conv_state) && ((uintptr_t)a % 16) == 0 &&
         ((uintptr_t)qo % 16) == 0 && ((uintptr_t)ko % 16) == 0 && ((uintptr_t)vo % 16) == 0 && ((uintptr_t)go % 16) == 0) {
-        const int pieces = (2 * G * dk + H * dv + H * dk) / 8, by = T_rows >= 512 ? 1 : (pieces + 255) / 256;
-#define GOP(TI, TAPS) e = qs_launch_dependent(delta_prepare_pieces_kernel<TI, TAPS>, dim3(T_rows, by), dim3(256), 0, stream, qo, ko, vo, go, bo, (const TI*)q, \
+        const int pieces = (2 * G * dk + H * dv + H * dk) / 8, by = T_rows >= 512 ? 1 : (pieces + 255) / 256, threads = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
+#define GOP(TI, TAPS) e = qs_launch_dependent(delta_prepare_pieces_kernel<TI, TAPS>, dim3(T_rows, by), dim3(threads), 0, stream, qo, ko, vo, go, bo, (const TI*)q, \
         (const TI*)k, (const TI*)v, (size_t)ldp, (const TI*)wq, (const TI*)wk, (const TI*)wv, (const TI*)conv_state, (size_t)slot_stride, a, (size_t)lda, bl, \
         (size_t)ldb, a_log, a_log_dtype, tok_slot, tok_pos, G, H, dk, dv, q_scale, unit_eps)
 #define GOT(TI) do { if (taps == 2) GOP(TI, 2); else if (taps == 3) GOP(TI, 3); else GOP(TI, 4); } while (0)
