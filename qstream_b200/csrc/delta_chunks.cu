@@ -47,7 +47,7 @@ struct Delta {
 // Bound by instruction issue and shared memory's pipe (a third and four fifths of their rates).  What it took before, 214 us for 2,000 tokens and 16 heads of 128 x 128, was 36,000 instructions per
 // warp: a condition and two decays per pair of tokens across blocks, a wait of the whole block between steps, two columns and 2,016
 // steps unrolled per thread (more code than the instruction cache holds); now
-// 108 us.
+// 108 us.  128 registers a thread at two blocks per SM; 164 bytes are spilled.
 constexpr int TERMS = 256, GROUPS = 4, GCH = 32, PASS = GROUPS * GCH;
 constexpr int OWN = 16 * 17;                            // a block's own pairs, [16][17]
 constexpr int TERMS_SMEM = (3 * PASS * CT + 4 * PASS) * sizeof(float);

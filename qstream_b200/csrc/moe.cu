@@ -338,7 +338,8 @@ moe_up_grouped_kernel(__nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv
 }
 
 // Sixteen output elements d of a chunk's tokens: warp w takes quarter w mod 4 of K of every second (fourth) expert in use; the quarters' sums
-// rest in shared memory until the tokens' choices are added up in order.
+// rest in shared memory until the tokens' choices are added up in order.  128 registers a thread (two blocks of eight warps or one of sixteen);
+// the form for up to 32 tokens of one expert spills 36 bytes.
 template <int NT>
 __device__ void down_columns(float* __restrict__ part, const __nv_bfloat16* __restrict__ hidden, size_t ldh, const __nv_bfloat16* __restrict__ w, const int* list,
                              int n, int first, int D, int F, int d0, int quarter) {

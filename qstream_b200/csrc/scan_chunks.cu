@@ -209,6 +209,9 @@ added_state_kernel(Scan p) {
 
 // A block takes the 64 tokens of a chunk and 64 NC value columns: of one head, or (NH = 2) 64 of each of two neighbouring heads
 // that share q and k, whose products q k^T are then taken once.  The key channels pass in slices through shared memory.
+// Three blocks per SM leave a thread 168 registers.  The bfloat16 forms fit (at most 16 bytes spilled); the float32 ones, which a decay per head
+// behind an activation takes too, hold a slice of q and k on its way in twice the room and spill 340 bytes, 700 to 780 per channel and with
+// the column of ones.
 template <int MODE, int NC>
 constexpr int output_body() {                           // floats of shared memory before the weights
     const int sl = MODE == 1 || MODE == 4 ? 64 : 32, stage = sl == 64 ? (3 * sl * CT > sl * CT + sl * 64 * NC ? 3 * sl * CT : sl * CT + sl * 64 * NC)

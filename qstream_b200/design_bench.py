@@ -438,12 +438,11 @@ def kernel_table_fofinex(torch, np, pk, width=2048, T=4096, batch=32, ctx=2048):
         rows_ = ops.gather_rows(h, place_token)
         yy = torch.empty((rows_.shape[0], width), dtype=torch.float32, device=dev)
         hid = torch.empty((rows_.shape[0], F), dtype=bf, device=dev)
-        bounds = offsets.tolist()
-        ops.expert_products(hid, rows_, w_up, bounds)
+        ops.grouped_products(hid, rows_, w_up, offsets)
         ops.activate(hid, "relu2")
-        ops.expert_products(yy, hid, w_down, bounds)
+        ops.grouped_products(yy, hid, w_down, offsets)
         return ops.moe_combine(yy, pair_place, wts, slot_all)
-    add(f"experts ordered by expert, {T} tokens (sort, gather, {2 * E} products, activation, combine)", "feed-forward products",
+    add(f"experts ordered by expert, {T} tokens (sort, gather, two launches of products, activation, combine)", "feed-forward products",
         t.kernel(grouped, repeats=5), flops=4.0 * T * top * F * width, bound="tensor")
     wg = torch.randn(2 * 5632, width, device=dev, dtype=bf) * 0.02
     from .parts.linear import linear as lin
@@ -564,7 +563,7 @@ def kernel_table_sefuvik(torch, np, pk, width=2048, T=4096, batch=32, ctx=2048):
             add(f"state scan delta prompt {T} (in order: what short prompts take)", "", ms, flops=8.0 * T * H * d * d, bound="fp32")
             ms = t.kernel(lambda: ops.state_scan("delta", qo, ko, vo, state, starts, slots, n_seq, H, d, d, key_decay=decay, token_weight=beta,
                                                  qk_group=H // Gq, chunks=chunks), repeats=5)
-            add(f"state scan delta prompt {T} (chunks: three walks and a prefix)", "state scan decay prompt", ms, flops=8.0 * T * H * d * d, bound="fp32")
+            add(f"state scan delta prompt {T} (chunks: triangular systems, their states in order, outputs)", "state scan decay prompt", ms, flops=8.0 * T * H * d * d, bound="fp32")
         else:
             add(f"state scan delta decode {batch}", "state scan decay decode", ms, 2 * state.numel() * 4)
     ql, kl, vl = (torch.randn(T, H * d, device=dev, dtype=bf) for _ in range(3))
@@ -727,12 +726,11 @@ def kernel_table_nutatar(torch, np, pk, width=2048, T=4096, batch=32, ctx=2048):
         rows_ = ops.gather_rows(h, place_token)
         yy = torch.empty((rows_.shape[0], width), dtype=torch.float32, device=dev)
         hid = torch.empty((rows_.shape[0], 2 * F if gated else F), dtype=bf, device=dev)
-        bounds = offsets.tolist()
-        ops.expert_products(hid, rows_, w_gu if gated else w_up, bounds)
+        ops.grouped_products(hid, rows_, w_gu if gated else w_up, offsets)
         hid = ops.clamped_glu(hid, *glu) if gated else ops.activate(hid, "relu2")
-        ops.expert_products(yy, hid, w_down, bounds)
+        ops.grouped_products(yy, hid, w_down, offsets)
         return ops.moe_combine(yy, pair_place, wts, slot_all)
-    add(f"gated experts ordered by expert, {T} tokens (sort, gather, {2 * E} products, gated unit, combine)", "experts ordered by expert",
+    add(f"gated experts ordered by expert, {T} tokens (sort, gather, two launches of products, gated unit, combine)", "experts ordered by expert",
         t.kernel(lambda: grouped(True), repeats=5), flops=6.0 * T * top * F * width, bound="tensor")
     add(f"experts ordered by expert, {T} tokens (Fofinex)", "", t.kernel(lambda: grouped(False), repeats=5), flops=4.0 * T * top * F * width, bound="tensor")
     return rows
@@ -888,10 +886,9 @@ def kernel_table_fotanex(torch, np, pk, width=2048, T=4096, batch=32, ctx=2048):
         rows_ = ops.gather_rows(h, place_token)
         yy = torch.empty((rows_.shape[0], width), dtype=f32, device=dev)
         hid = torch.empty((rows_.shape[0], 2 * F), dtype=bf, device=dev)
-        bounds = offsets.tolist()
-        ops.expert_products(hid, rows_, w_gu, bounds)
+        ops.grouped_products(hid, rows_, w_gu, offsets)
         hid = ops.gated_act(hid, "silu") if plain else ops.clamped_glu(hid, 7.0)
-        ops.expert_products(yy, hid, w_down, bounds)
+        ops.grouped_products(yy, hid, w_down, offsets)
         return ops.moe_combine(yy, pair_place, wts, slot_all)
     for plain, who in ((True, ""), (False, " (Nutatar)")):
         add(f"gated experts ordered by expert, {T} tokens{who}", "" if who else "the clamped gated experts", t.kernel(lambda: grouped(plain), repeats=5),
@@ -1005,13 +1002,11 @@ def kernel_table_vofinex(torch, np, pk, width=2048, T=4096, batch=32, ctx=2048):
         def grouped():
             offsets, place_token, pair_place = ops.moe_sort(idx, n_out)
             rows_ = ops.gather_rows(h, place_token)
-            bounds = offsets.tolist()[:E + 1]
-            rows_ = rows_[:bounds[-1]]
             yy = torch.empty((rows_.shape[0], width), dtype=f32, device=dev)
             hid = torch.empty((rows_.shape[0], 2 * F), dtype=bf, device=dev)
-            ops.expert_products(hid, rows_, w_gu, bounds)
-            ops.expert_products(yy, ops.gated_act(hid, "silu"), w_down, bounds)
-            return ops.moe_combine(yy, pair_place, wts, slot_all, x=None if who else h)
+            ops.grouped_products(hid, rows_, w_gu, offsets)
+            ops.grouped_products(yy, ops.gated_act(hid, "silu"), w_down, offsets)
+            return ops.moe_combine(yy, pair_place, wts, slot_all, x=None if who else h, n_rows=offsets[E:E + 1])
         add(f"gated experts ordered by expert, {T} tokens ({pairs} pairs with matrices){who}", "" if who else "without outputs that return their input",
             t.kernel(grouped, repeats=5), flops=6.0 * pairs * F * width, bound="tensor")
     # the factor on the logits of a decode step

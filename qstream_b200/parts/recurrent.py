@@ -42,7 +42,15 @@ from .linear import linear
 
 
 CHUNK_TOKENS = 64            # a long prompt is cut into chunks of this many tokens that run side by side
-CHUNKED_FROM = 256           # the longest sequence of a step from which that pays
+# The longest sequence of a step from which the chunks serve: all forms gain there, with one sequence as with several.  Shorter prompts would
+# gain in some of them already.  Microseconds of the scan, walk | chunks, one sequence at 64, 128 and 256 tokens, then four sequences:
+#   decay per head, 16 heads of 128 x 128   59 | 44, 111 | 44, 213 | 70      53 | 83,  96 | 85,  182 | 95
+#   per channel (gla), 16 of 64 x 128       78 | 93, 147 | 97, 289 | 101     78 | 99,  147 | 101, 285 | 103
+#   per channel (wkv), 16 of 64 x 64        82 | 46, 156 | 46, 306 | 44      82 | 58,  156 | 56, 305 | 58
+#   state-space form, 64 of 128 x 64        70 | 48, 129 | 60, 254 | 67      74 | 79,  135 | 87, 260 | 142
+#   gated memory, 4 of 256 x 256            63 | 75, 117 | 81, 225 | 81      68 | 153, 127 | 151, 246 | 152
+#   delta rule, 16 of 128 x 128             72 | 79, 137 | 85, 264 | 103     72 | 101, 131 | 122, 254 | 179
+CHUNKED_FROM = 256
 
 
 def scan_chunks(batch, device):
