@@ -588,15 +588,18 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     `chunks` = (chunk_start, chunk_ids, seq_chunk, n_chunks), int32 device tensors: every sequence of the step cut
     into consecutive chunks (rows chunk_start[c] .. chunk_start[c + 1] of the packed batch; sequence s owns chunks
     seq_chunk[s] .. seq_chunk[s + 1]; chunk_ids = 0 .. n_chunks - 1).  The chunks then run side by side and a
-    prefix over each sequence's chunks joins them; the result equals the walk in order up to 32-bit rounding."""
+    prefix over each sequence's chunks joins them; the result equals the walk in order up to 32-bit rounding.
+    Without `v` (mode "delta") the values are zeros; a walk in order without `want_output` returns None."""
     T = q.shape[0]
     if state.dtype != torch.float32 or state.stride(-1) != 1:
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: the state must be float32")
-    if mode == "delta" and chunks is not None:
-        return _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_dim, key_decay, token_weight, qk_group, chunks)
-    o = torch.empty((T, n_heads * value_dim), dtype=torch.float32, device=q.device) if want_output else None
     if v is None and mode != "delta":
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: only the delta rule walks without values")
+    if v is None:                                       # values of zero
+        v = torch.zeros((T, n_heads * value_dim), dtype=q.dtype, device=q.device)
+    if mode == "delta" and chunks is not None:
+        return _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_dim, key_decay, token_weight, qk_group, chunks)
+    o = torch.empty((T, n_heads * value_dim), dtype=torch.float32, device=q.device)
     chunk_start = chunk_ids = seq_chunk = chunk_state = chunk_decay = None
     n_chunks = 0
     if chunks is not None and ACTIVATIONS[in_activation] != ACT_NONE:
@@ -616,15 +619,15 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     if mode in ("gated", "ssd") and (token_decay.dtype != torch.float32 or token_decay.stride() != token_weight.stride()):
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: the tokens' decays and weights must be float32 of one layout")
     check(library().qs_state_scan(
-        {"decay": 0, "wkv": 1, "gated": 2, "delta": 3, "gla": 4, "ssd": 5}[mode], ptr(o), o.stride(0) if o is not None else 0, ptr(q), q.stride(0),
-        ptr(k), k.stride(0), ptr(v), v.stride(0) if v is not None else 0,
+        {"decay": 0, "wkv": 1, "gated": 2, "delta": 3, "gla": 4, "ssd": 5}[mode], ptr(o), o.stride(0), ptr(q), q.stride(0),
+        ptr(k), k.stride(0), ptr(v), v.stride(0),
         dtype_code(q), ptr(decay_logits), decay_logits.stride(0) if decay_logits is not None else 0, ptr(head_decay),
         ptr(bonus), _code(bonus), ptr(state), state.stride(0), _int32(seq_start, "seq_start"),
         _int32(seq_slot, "seq_slot"), int(n_seq), T, n_heads, key_dim, value_dim, ACTIVATIONS[in_activation],
         ptr(chunk_start), ptr(chunk_ids), int(n_chunks), ptr(seq_chunk), ptr(chunk_state), ptr(chunk_decay),
         ptr(token_decay), ptr(token_weight), per_token.stride(0) if per_token is not None else 0, float(q_scale),
         int(qk_group), float(decay_power), stream()))
-    return o
+    return o if want_output else None
 
 
 def _activated(q, k, v, activation):
@@ -643,8 +646,6 @@ def _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_di
     T = q.shape[0]
     if any(t.dtype != torch.float32 or t.stride(1) != 1 for t in (key_decay, token_weight)):
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: the delta rule takes float32 decays and step sizes")
-    if v is None:
-        v = torch.zeros((T, n_heads * value_dim), dtype=q.dtype, device=q.device)
     if any(t.dtype != q.dtype or t.stride(1) != 1 for t in (q, k, v)):
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: q, k and v must be rows of one type")
     if q.dtype != torch.float32:

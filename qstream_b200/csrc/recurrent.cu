@@ -68,16 +68,15 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
     const int n_cols = min(cols, dv - col0);
     const int tid = threadIdx.x;
     // rows of the packed batch beyond the last sequence belong to nobody: give them a defined value
-    if (s == 0 && (!DELTA || o)) {
+    if (s == 0) {
         for (int t = seq_start[n_seq]; t < T_rows; ++t)
             for (int c = tid; c < n_cols; c += blockDim.x) o[(size_t)t * ldo + h * dv + col0 + c] = 0.f;
     }
     const int slot = seq_slot[s];
     const int t0 = seq_start[s], t1 = seq_start[s + 1];
     if (slot < 0) {
-        if (!DELTA || o)
-            for (int t = t0; t < t1; ++t)
-                for (int c = tid; c < n_cols; c += blockDim.x) o[(size_t)t * ldo + h * dv + col0 + c] = 0.f;
+        for (int t = t0; t < t1; ++t)
+            for (int c = tid; c < n_cols; c += blockDim.x) o[(size_t)t * ldo + h * dv + col0 + c] = 0.f;
         return;
     }
     if (t1 <= t0) return;
@@ -145,7 +144,7 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
         }
         for (int e = tid; e < nt * cols; e += blockDim.x) {
             const int tt = e / cols, c = e - tt * cols;
-            sv[e] = (c >= n_cols || (DELTA && !v)) ? 0.f : (ONES && col0 + c == dvv) ? 1.0f
+            sv[e] = c >= n_cols ? 0.f : (ONES && col0 + c == dvv) ? 1.0f
                     : apply_activation(to_f32(v[(size_t)(base + tt) * ldv + h * dvv + col0 + c]), in_act);
         }
         if (GATED && tid < nt) sa[tid] = ga[(size_t)(base + tid) * ldg + h];
@@ -233,7 +232,7 @@ state_scan_kernel(float* __restrict__ o, size_t ldo,
                 acc1 += __shfl_xor_sync(0xffffffffu, acc1, off);
             }
             }
-            if (ks == 0 && (!DELTA || o)) {
+            if (ks == 0) {
                 float* dst = o + (size_t)(base + tt) * ldo + h * dv + col0 + CPT * pair;
                 if (own0) dst[0] = acc0;
                 if (own1) dst[1] = acc1;
@@ -660,8 +659,6 @@ QS_API int qs_state_scan(int mode, float* o, long long ldo, const void* q, long 
     return chunks(1);
 }
 
-// See delta_chunk_prefix_kernel.  seq_chunk (n_seq + 1) names each sequence's chunks; a sequence's slot must be a row
-// of `state` (or negative: skipped).
 QS_API int qs_token_shift(void* out, long long ldo, long long mix_stride, const void* h, long long ldh, int dtype,
                           const float* mu, const void* last_row, long long ld_last, const int32_t* tok_slot,
                           const int32_t* tok_pos, int T, int D, int n_mix, cudaStream_t stream) {

@@ -84,9 +84,9 @@ def test_operands_in_bfloat16_and_absent_values():
     g, beta = (torch.from_numpy(x.reshape(T, -1)).float().cuda() for x in (g, beta))
     S0 = torch.randn(1, H, dv, dk, generator=torch.Generator().manual_seed(1)).cuda()
 
-    def scan(q, k, v, chunks):
+    def scan(q, k, v, chunks, **kw):
         state = S0.clone()
-        o = ops.state_scan("delta", q, k, v, state, i32([0, T]), i32([0]), 1, H, dk, dv, chunks=chunks, key_decay=g, token_weight=beta, qk_group=H)
+        o = ops.state_scan("delta", q, k, v, state, i32([0, T]), i32([0]), 1, H, dk, dv, chunks=chunks, key_decay=g, token_weight=beta, qk_group=H, **kw)
         return o, state
 
     for values in (v, None):
@@ -96,3 +96,5 @@ def test_operands_in_bfloat16_and_absent_values():
         for a, b, c in zip(low, high, walked):
             assert torch.equal(a, b)
             assert (a - c).norm() <= 4 * 2.0 ** -24 * (np.sqrt(64) + np.sqrt(dk)) * np.sqrt(T / 16) * c.norm()
+        alone = scan(q, k, values, None, want_output=False)
+        assert alone[0] is None and torch.equal(alone[1], walked[1])
