@@ -14,7 +14,7 @@
 //
 // The order of the sums is the same in every form below (tile sizes, cut over the runs or not), so the
 // choice of the form by M, N and K never changes a bit of the result.
-#include "common.cuh"
+#include "linear_finish.cuh"
 
 namespace {
 
@@ -32,16 +32,6 @@ __device__ __forceinline__ float4 load4(const T* __restrict__ row, int c, int en
     }
     return make_float4(to_f32(row[c]), c + 1 < end ? to_f32(row[c + 1]) : 0.f, c + 2 < end ? to_f32(row[c + 2]) : 0.f,
                        c + 3 < end ? to_f32(row[c + 3]) : 0.f);
-}
-
-template <typename TA, typename TC>
-__device__ __forceinline__ void finish(TC* __restrict__ C, float v, int gm, int gn, const void* __restrict__ bias, int bias_dtype, int act,
-                                       const TA* __restrict__ res1, const TA* __restrict__ res2, size_t ldc, size_t ldr) {
-    if (bias) v += load_as_f32(bias, bias_dtype, gn);
-    v = apply_activation(v, act);
-    if (res1) v += to_f32(res1[(size_t)gm * ldr + gn]);
-    if (res2) v += to_f32(res2[(size_t)gm * ldr + gn]);
-    C[(size_t)gm * ldc + gn] = from_f32<TC>(v);
 }
 
 // A block computes a tile of BM x BN outputs, a thread TM x TN of them (rows in groups of four, columns in groups of four,
@@ -203,27 +193,6 @@ linear_tile_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __res
             if (totals) v = sT[(i * TN + j) * THREADS + tid] + v;
             finish(C, v, gm, gn, bias, bias_dtype, act, res1, res2, ldc, ldr);
         }
-    }
-}
-
-// C = act(sum of the runs' sums, in order, + bias) + residuals.
-template <typename TA, typename TC>
-__global__ void __launch_bounds__(256)
-linear_join_kernel(TC* __restrict__ C, const float* __restrict__ partial, int runs, const void* __restrict__ bias, int bias_dtype, int act,
-                   const TA* __restrict__ res1, const TA* __restrict__ res2, int M, int N, size_t ldc, size_t ldr) {
-    const size_t mn = (size_t)M * N;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < mn; e += (size_t)gridDim.x * blockDim.x) {
-        float total = 0.f;
-        int r = 0;
-        for (; r + 8 <= runs; r += 8) {                     // eight loads in flight
-            float v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = partial[(r + i) * mn + e];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) total += v[i];
-        }
-        for (; r < runs; ++r) total += partial[r * mn + e];
-        finish(C, total, (int)(e / N), (int)(e % N), bias, bias_dtype, act, res1, res2, ldc, ldr);
     }
 }
 

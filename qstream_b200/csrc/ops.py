@@ -34,6 +34,9 @@ _SIGNATURES = {
     "qs_linear_simt": ([c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                         c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_longlong, c_void_p], c_int),
     "qs_linear_simt_scratch": ([c_int, c_int, c_int], c_longlong),
+    "qs_linear_split": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
+                         c_longlong, c_void_p, c_longlong, c_void_p, c_void_p], c_int),
+    "qs_linear_split_scratch": ([c_int, c_int, c_int], c_longlong),
     "qs_rope_store": ([c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_longlong,
                        c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                        c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_float, c_int, c_void_p], c_int),
@@ -288,12 +291,8 @@ def _linear_simt_scratch(M: int, N: int, K: int) -> int:
     return int(library().qs_linear_simt_scratch(M, N, K))
 
 
-def linear_simt(x, weight, bias=None, activation=None, residuals=(), out_dtype=None, out=None) -> torch.Tensor:
-    """act(x W^T + bias) + residuals, accumulated in true 32-bit on the CUDA cores."""
-    M, K, lda = _rows(x)
-    N, K2 = weight.shape
-    if K2 != K or not weight.is_contiguous():
-        raise QStreamError(QsError.INVALID_INPUT, f"linear: x is [{M}, {K}] but weight is {tuple(weight.shape)}")
+def _product_views(x, M, N, residuals, out_dtype, out):
+    """(output, the two residuals or None, their row stride) of a product of x with N results per row."""
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype or x.dtype, device=x.device)
     elif out.shape != (M, N) or out.stride(1) != 1:
@@ -307,12 +306,51 @@ def linear_simt(x, weight, bias=None, activation=None, residuals=(), out_dtype=N
             ldr = r.stride(0)
     if len(residuals) > 2 or (len(residuals) == 2 and res[0].stride(0) != res[1].stride(0)):
         raise QStreamError(QsError.INVALID_INPUT, "linear: at most two residuals of one layout")
+    return out, res, ldr
+
+
+def linear_simt(x, weight, bias=None, activation=None, residuals=(), out_dtype=None, out=None) -> torch.Tensor:
+    """act(x W^T + bias) + residuals, accumulated in true 32-bit on the CUDA cores."""
+    M, K, lda = _rows(x)
+    N, K2 = weight.shape
+    if K2 != K or not weight.is_contiguous():
+        raise QStreamError(QsError.INVALID_INPUT, f"linear: x is [{M}, {K}] but weight is {tuple(weight.shape)}")
+    out, res, ldr = _product_views(x, M, N, residuals, out_dtype, out)
     floats = _linear_simt_scratch(M, N, K)
     ws = torch.empty((floats,), dtype=torch.float32, device=x.device) if floats else None
     check(library().qs_linear_simt(ptr(out), dtype_code(out), ptr(x), dtype_code(x), ptr(weight),
                                    dtype_code(weight), ptr(bias), dtype_code(bias) if bias is not None else 0,
                                    ACTIVATIONS[activation], ptr(res[0]), ptr(res[1]), M, N, K, lda, out.stride(0), ldr,
                                    ptr(ws), floats, stream()))
+    return out
+
+
+@functools.lru_cache(maxsize=4096)
+def _linear_split_scratch(M: int, N: int, K: int) -> int:
+    return int(library().qs_linear_split_scratch(M, N, K))
+
+
+def split_takes(x, weight, out=None) -> bool:
+    """Whether the float32 product on the tensor cores takes these operands: rows in 16-byte pieces."""
+    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2 and x.shape[1] % 4 == 0
+            and x.stride(1) == 1 and x.stride(0) % 4 == 0 and weight.is_contiguous() and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and (out is None or out.dtype == torch.float32))
+
+
+def linear_split(x, weight, bias=None, activation=None, residuals=(), out=None) -> torch.Tensor:
+    """act(x W^T + bias) + residuals, all float32, on the tensor cores: every number as three bfloat16 terms, sums no further from
+    64 bits than those of `linear_simt`."""
+    from . import gemm_tc
+    M, K, lda = _rows(x)
+    N = weight.shape[0]
+    if not split_takes(x, weight, out) or weight.shape[1] != K:
+        raise QStreamError(QsError.INVALID_INPUT, f"linear: x is [{M}, {K}] and weight {tuple(weight.shape)}, not float32 or not aligned")
+    out, res, ldr = _product_views(x, M, N, residuals, None, out)
+    floats = _linear_split_scratch(M, N, K)
+    ws = torch.empty((floats,), dtype=torch.float32, device=x.device) if floats else None
+    check(library().qs_linear_split(ptr(out), ptr(x), ptr(weight), ptr(bias), dtype_code(bias) if bias is not None else 0, ACTIVATIONS[activation],
+                                    ptr(res[0]), ptr(res[1]), M, N, K, lda, out.stride(0), ldr, ptr(ws), floats,
+                                    ptr(gemm_tc.status_word(x.device)), stream()))
     return out
 
 

@@ -1,9 +1,11 @@
 """The matrix product y = act(x W^T + b) + residuals, and the choice of its kernel.
 
 bfloat16 activations with a bfloat16 matrix run on the tensor cores (tcgen05, fed by
-TMA, 32-bit accumulation); everything else (the float32 engine, a matrix stored in
-32-bit) runs on the CUDA cores in true 32-bit.  Both kernels sum a row's products in
-an order that does not depend on the other rows of the batch.
+TMA, 32-bit accumulation).  float32 activations with a float32 matrix run there too, every
+number as three bfloat16 terms and the sums rounded in 32 bits outside the unit, where more than a
+few rows meet enough products; everything else (few rows, mixed types) runs on the CUDA cores in
+true 32-bit.  Each kernel sums a row's products in an order that does not depend on
+the other rows' contents.
 """
 from __future__ import annotations
 
@@ -12,6 +14,10 @@ import torch
 from ..csrc import ops
 
 TENSOR_CORE_ACTIVATIONS = (None, "none", "gelu_new", "gelu")
+# float32: from how many rows and products per result on the tensor cores serve.  Microseconds, CUDA cores | tensor cores (caches
+# flushed, launches included): 16 rows, 6144 x 2048: 32 | 34; 17 rows, 2048 x 8192: 54 | 40; 32, 2048 x 2048: 28 | 21; 64, 6144 x 2048: 60 | 36; 700,
+# 64 x 1024: 24 | 24; 700, 2048 x 64: 49 | 18, but 64 x 64: 12 | 12; 128, 256 x 256: 20 | 15; 700, 6144 x 2048: 412 | 99; 2048, 16384 x 4096: 5159 | 1138.
+SPLIT_ROWS, SPLIT_PRODUCTS = 17, 256
 OWN_KERNEL_ACTIVATIONS = ("relu2",)         # in no product's epilogue: applied by a kernel of their own behind the product
 
 
@@ -25,6 +31,11 @@ def linear(x, weight, bias=None, activation=None, residuals=(), out_dtype=None, 
                 return gemm_tc.linear(x, weight, bias, activation, residuals, out_dtype, out)
             if not residuals:       # an activation that the tensor-core epilogue does not offer: a kernel of its own behind it
                 return ops.activate(gemm_tc.linear(x, weight, bias, None, (), out_dtype, out), activation)
+    if x.dtype == torch.float32 and out_dtype in (None, torch.float32) and x.dim() == 2 and x.shape[0] >= SPLIT_ROWS \
+            and x.shape[1] >= SPLIT_PRODUCTS and ops.split_takes(x, weight, out):
+        own = activation in OWN_KERNEL_ACTIVATIONS and not residuals
+        y = ops.linear_split(x, weight, bias, None if own else activation, residuals, out)
+        return ops.activate(y, activation) if own else y
     if activation in OWN_KERNEL_ACTIVATIONS and not residuals:
         return ops.activate(ops.linear_simt(x, weight, bias, None, (), out_dtype, out), activation)
     return ops.linear_simt(x, weight, bias, activation, residuals, out_dtype, out)
