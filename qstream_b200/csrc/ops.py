@@ -74,7 +74,7 @@ _SIGNATURES = {
     "qs_state_scan": ([c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int,
                        c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
                        c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_longlong, c_float, c_int, c_float, c_void_p], c_int),
+                       c_void_p, c_void_p, c_longlong, c_float, c_int, c_float, c_void_p, c_void_p], c_int),
     "qs_delta_chunks_scratch": ([c_int, c_int, c_int, c_int], c_longlong),
     "qs_delta_chunks": ([c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
                          c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p], c_int),
@@ -628,6 +628,7 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     seq_chunk[s] .. seq_chunk[s + 1]; chunk_ids = 0 .. n_chunks - 1).  The chunks then run side by side and a
     prefix over each sequence's chunks joins them; the result equals the walk in order up to 32-bit rounding.
     Without `v` (mode "delta") the values are zeros; a walk in order without `want_output` returns None."""
+    from . import gemm_tc
     T = q.shape[0]
     if state.dtype != torch.float32 or state.stride(-1) != 1:
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: the state must be float32")
@@ -664,7 +665,7 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
         _int32(seq_slot, "seq_slot"), int(n_seq), T, n_heads, key_dim, value_dim, ACTIVATIONS[in_activation],
         ptr(chunk_start), ptr(chunk_ids), int(n_chunks), ptr(seq_chunk), ptr(chunk_state), ptr(chunk_decay),
         ptr(token_decay), ptr(token_weight), per_token.stride(0) if per_token is not None else 0, float(q_scale),
-        int(qk_group), float(decay_power), stream()))
+        int(qk_group), float(decay_power), ptr(gemm_tc.status_word(q.device)), stream()))
     return o if want_output else None
 
 

@@ -8,21 +8,26 @@
 //   added_state_kernel      what each chunk adds to the state it starts from, and its decays
 //   chunk_prefix_kernel     (recurrent.cu) the state each chunk starts from, and the sequence's last one
 //   chunk_output_kernel     every token's o, written once
-// All arithmetic is 32-bit on the CUDA cores (paired multiply-adds).  Decays enter as products of at most 64 factors up to
-// one, never as quotients, so small ones cost no precision: per token and head by a recursion down the columns of P; per
-// channel in blocks of 16 tokens, a block's own pairs walked in order, pairs of blocks through the products up to the
-// blocks' common edge.
+// Decays enter as products of at most 64 factors up to one, never as quotients, so small ones cost no precision: per token and head by a
+// recursion from a token back over the earlier ones; per channel in blocks of 16 tokens, a block's own pairs walked in order, pairs of blocks
+// through the products up to the blocks' common edge.
 //
-// Bound by instruction issue at 12 to 16 warps per SM: multiply-adds (two per instruction) with 16-byte shared-memory reads beside
-// them.  What mattered after the walk was replaced: fetches of a whole slice under way at once (the next slice's while the present one is
-// multiplied), and an activation once per element instead of once per kernel.  On the tensor cores as split 11-bit products the sums,
-// which the unit truncates, were two times further from 64 bits than the walk, at the same speed: not taken.
-// Microseconds of the whole mixer (walk | chunks, serial fetches | now): decay per head, 4,096 tokens, 16 heads of 128 x 128: 949 |
-// 600 | 407; per channel, 3,401 tokens, 16 heads of 64 x 128: 578 | 393 | 286; state-space form, 2,048 tokens, 64 heads of
-// 128 x 64: 822 | 458 | 379 (its output kernel 143, what the chunks add 71).  Pairs of blocks of 16 with the later block's decays
-// applied to every pair, a token's q against one block's k at a time, took the per-channel output kernel from 114 to 163 us.
+// The products of 32-bit numbers run on tcgen05 as products of bfloat16 terms (terms.cuh), in runs of 64 whose sums are added outside; against
+// float64 they are nearer than the multiply-adds that stood here before (o, 2-norm: state-space form 1.4e-7 instead of 1.5e-7, gated memory
+// 1.4e-7 instead of 1.9e-7, decay per head 7.9e-7 instead of 8.8e-7).  q, k and v that come as bfloat16 are one term: q k^T is then one product instead
+// of six.  Bound by each block's chain of fetch, split, barrier, MMAs and stores at two blocks per SM (leaving out the MMAs: 63 of 76 us
+// for the outputs, 42 of 47 for what the chunks add, at 4,096 tokens of 16 heads of 128 x 128, float32 operands); the split needs half of
+// the issue slots.  On mma.sync the same products took 138 and 59 us, multiply-adds 139 and 66.
+//
+// Microseconds of the scan alone (multiply-adds | now; caches flushed): decay per head, 4,096 tokens, 16 heads of 128 x 128, float32: 236 | 151; 1,000
+// tokens, bfloat16: 85 | 38; state-space form, 2,048 tokens, 64 heads of 128 x 64: 237 | 142; gated memory, 1,000 tokens, 4 heads of 256 x 256:
+// 136 | 79; per channel (its outputs on the CUDA cores), 3,401 tokens, 16 heads of 64 x 128: 175 | 163.
 #include "scan.cuh"
 #include "scan_tiles.cuh"
+#include "sm100.cuh"
+#include "terms.cuh"
+
+using namespace sm100;
 
 namespace {
 
@@ -39,6 +44,7 @@ struct Scan {
     int H, dk, dv, dvp, qk_group, n_chunks, T_rows;       // dvp: dv rounded up to a multiple of four
     float q_scale, decay_scale;
     int vec_q, vec_k, vec_v, vec_o;                    // whether rows may be read (written) in pieces of four
+    int32_t* status;                                    // receives a code if a bounded wait ran out
 };
 
 template <int MODE>
@@ -59,7 +65,7 @@ template <typename TI, int MODE>
 __device__ void walk_in_order(const Scan& p, float* __restrict__ S, int c, int h, int col0, int cols, bool output) {
     constexpr bool ONES = MODE == 2, WKV = MODE == 1;
     const int t0 = p.chunk_start[c], t1 = p.chunk_start[c + 1], hq = h / p.qk_group, dvv = ONES ? p.dv - 1 : p.dv;
-    for (int col = col0 + (int)threadIdx.x; col < col0 + cols; col += THREADS) {
+    for (int col = col0 + (int)threadIdx.x; col < col0 + cols; col += blockDim.x) {
         for (int t = t0; t < t1; ++t) {
             const TI* qr = (const TI*)p.q + (size_t)t * p.ldq + hq * p.dk;
             const TI* kr = (const TI*)p.k + (size_t)t * p.ldk + hq * p.dk;
@@ -79,53 +85,161 @@ __device__ void walk_in_order(const Scan& p, float* __restrict__ S, int c, int h
     }
 }
 
+__device__ __forceinline__ bool is_number(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+// ---- tiles of terms in shared memory as tcgen05 operands: 64 elements to a row of 128 bytes, swizzled by 128 bytes.  A tile of
+// 64 rows is 8 KB; wider ones are several of them.  The same tile serves with its rows on the sum's side or on the other.
+constexpr int TILE_THREADS = 256;                       // eight warps: a quarter of the TMEM lanes each, two halves of the columns
+constexpr int TILE = CT * 128;                          // bytes
+constexpr uint32_t A_TURNED = 1u << 15, B_TURNED = 1u << 16;       // instruction descriptor: rows on the sum's side
+
+__device__ __forceinline__ uint32_t place_in_tile(int r, int c) { return (uint32_t)(r * 128 + ((((c >> 3) ^ r) & 7) << 4) + (c & 7) * 2); }
+
+// Four neighbouring numbers as terms at dst, dst + term ...  P = 1: they come as bfloat16.
+template <int P>
+__device__ __forceinline__ void put_terms(uint32_t dst, uint32_t term, float4 f) {
+    uint32_t a[3], b[3];
+    terms_of(pack2(f.x, f.y), a[0], a[1], a[2]);
+    terms_of(pack2(f.z, f.w), b[0], b[1], b[2]);
+#pragma unroll
+    for (int i = 0; i < P; ++i) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + i * term), "r"(a[i]), "r"(b[i]) : "memory");
+}
+// Eight neighbouring numbers as terms.
+__device__ __forceinline__ void put_eight(uint32_t dst, uint32_t term, const float (&f)[8]) {
+    uint32_t t[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) terms_of(pack2(f[2 * j], f[2 * j + 1]), t[0][j], t[1][j], t[2][j]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + i * term), "r"(t[i][0]), "r"(t[i][1]), "r"(t[i][2]), "r"(t[i][3]) : "memory");
+}
+
+// D (+)= A B over 64 products, A in PA terms that lie `a_term` apart, B in PB: small products first, from zero.  TURNED operands: rows on the
+// sum's side, 64 elements of the other side per tile; else the sum along the rows.
+template <int PA, int PB, bool A_T, bool B_T>
+__device__ __forceinline__ void multiply_tiles(uint32_t d, uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term, int N) {
+    const uint32_t idesc = idesc_bf16_f32(128, N) | (A_T ? A_TURNED : 0u) | (B_T ? B_TURNED : 0u);
+    bool first = true;
+#pragma unroll
+    for (int order = 2; order >= 0; --order)
+#pragma unroll
+        for (int x = 0; x < PA; ++x) {
+            const int y = order - x;
+            if (y < 0 || y >= PB) continue;
+            const uint32_t at = a + x * a_term, bt = b + y * b_term;
+            const uint64_t da = A_T ? smem_desc_sw128_mn(at, TILE, 1024) : smem_desc_sw128(at), db = B_T ? smem_desc_sw128_mn(bt, TILE, 1024) : smem_desc_sw128(bt);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {               // 16 of the sum's elements: 32 bytes of a row, or two groups of eight rows
+                mma_bf16(d, da + (A_T ? 128 : 2) * k, db + (B_T ? 128 : 2) * k, idesc, !first);
+                first = false;
+            }
+        }
+}
+
+__device__ __forceinline__ bool wait_done(uint64_t* bar, uint32_t parity, int32_t* status) {
+    if (__all_sync(0xffffffffu, mbar_wait(bar, parity))) return true;
+    atomicExch(status, 171);
+    return false;
+}
+// sum[0 .. N) += the thread's lane, columns from `taddr` on
+template <int N>
+__device__ __forceinline__ void take_sums(float (&sum)[N], uint32_t taddr, bool first) {
+#pragma unroll
+    for (int c = 0; c < N; c += 16) {
+        uint32_t raw[16];
+        tmem_load_32x16(taddr + c, raw);
+        tmem_load_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sum[c + j] = first ? __uint_as_float(raw[j]) : sum[c + j] + __uint_as_float(raw[j]);
+    }
+}
+
+
 // ----------------------------------------------------------------------------- what a chunk adds
 
-// A block takes 64 key channels x 64 NC value columns of one head's state: added[i][col] = sum_j kw_j[i] v_j[col], the tokens on
-// the sum's side, kw_j = b_j k_j times the decays behind token j.
-template <typename TI, int MODE, int NC>
-__global__ void __launch_bounds__(THREADS)
-added_state_kernel(Scan p) {
+// A block takes 64 NC value columns of one head's state, up to 128 key channels at a time: added[i][col] = sum_j kw_j[i] v_j[col], the
+// tokens on the sum's side, kw_j = b_j k_j times the decays behind token j.  kw in three terms, v in VT (one where it comes as bfloat16).
+// Columns on the TMEM lanes, so that a warp writes 32 neighbouring ones.
+// The sum of channel i over the chunk's tokens, from the last back, by multiply-adds; `v_at` < 0: of values that are all one.  `s_w`: the tokens' weights and
+// decays behind them, where there is one decay per head.
+template <typename TI, int MODE>
+__device__ __noinline__ float plain_added(const Scan& p, int h, int i, int t0, int n, long long v_at, const float* s_w) {
+    const TI* k = (const TI*)p.k + (size_t)t0 * p.ldk + (size_t)(h / p.qk_group) * p.dk + i;
+    float sum = 0.f, run = 1.f;
+    for (int j = n - 1; j >= 0; --j) {
+        const float v = v_at < 0 ? 1.f : to_f32(((const TI*)p.v)[(size_t)(t0 + j) * p.ldv + v_at]);
+        sum = fmaf(to_f32(k[(size_t)j * p.ldk]) * (MODE == 1 || MODE == 4 ? run : s_w[j]), v, sum);
+        if (MODE == 1 || MODE == 4) run *= decay_at<MODE>(p, t0 + j, h, i);
+    }
+    return sum;
+}
+// The sums of a column that the terms gave no number for.
+template <typename TI, int MODE>
+__device__ __noinline__ void mend_added(const Scan& p, float* to, int rows, int h, int i, int t0, int n, long long v_at, const float* s_w) {
+    for (int x = 0; x < rows; ++x)
+        if (!is_number(to[(size_t)x * p.dvp])) to[(size_t)x * p.dvp] = plain_added<TI, MODE>(p, h, i + x, t0, n, v_at, s_w);
+}
+
+template <typename TI> constexpr int added_smem() { return 1024 + (3 + (sizeof(TI) == 2 ? 1 : 3)) * 2 * TILE; }
+
+template <typename TI, int MODE>
+__global__ void __launch_bounds__(TILE_THREADS, 2)
+added_state_kernel(const __grid_constant__ Scan p) {
     constexpr bool PER_CHANNEL = MODE == 1 || MODE == 4, ONES = MODE == 2;
-    constexpr int COLS = 64 * NC, NK = CT * 16 / THREADS, NV = NK * NC;
-    extern __shared__ __align__(16) float smem[];
-    float* sk = smem;                                   // [tokens][64]
-    float* sv = sk + CT * 64;                           // [tokens][COLS]
-    __shared__ float s_a[CT], s_w[CT], part[2 * 64], s_whole;
+    constexpr int VT = sizeof(TI) == 2 ? 1 : 3, COLS = 128, NK = CT * 16 / TILE_THREADS, NV = 2 * NK;
+    constexpr uint32_t TERM = 2 * TILE, TMEM = 128;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(16) float s_a[CT], s_w[CT], part[4 * 64];
+    __shared__ float s_whole;
+    __shared__ uint64_t done;
+    __shared__ uint32_t tmem_slot;
+    const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) { mbar_init(&done, 1); mbar_fence_init(); }
+    if (warp == 0) { tmem_alloc(&tmem_slot, TMEM); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
     grid_dep_launch();
     grid_dep_wait();
-    const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int dk_tiles = (p.dk + 63) / 64, i0 = blockIdx.z % dk_tiles * 64, col0 = blockIdx.z / dk_tiles * COLS;
+    const uint32_t tmem = tmem_slot, tk = (smem_u32(smem_raw) + 1023) & ~1023u, tv = tk + 3 * TERM;      // [3][2 halves of 128 channels][tokens], [VT][2][tokens]
+    const int col0 = blockIdx.z * COLS;
     const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, hq = h / p.qk_group;
-    const int dvv = ONES ? p.dv - 1 : p.dv, nk = min(64, p.dk - i0), nv = min(COLS, dvv - col0);
+    const int dvv = ONES ? p.dv - 1 : p.dv, nv = min(COLS, dvv - col0);
     float* added = p.chunk_state + ((size_t)c * p.H + h) * p.dk * p.dvp;
     float* decays = p.chunk_decay + ((size_t)c * p.H + h) * p.dk;
+    auto leave = [&]() {
+        tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(tmem, TMEM);
+    };
     if (n > CT) {
-        if (i0 == 0) {
-            const int cols = col0 == 0 && ONES ? nv + 1 : nv;
-            for (int e = tid; e < cols * p.dk; e += THREADS) added[(size_t)(e % p.dk) * p.dvp + (e / p.dk < nv ? col0 + e / p.dk : dvv)] = 0.f;
-            __syncthreads();
-            walk_in_order<TI, MODE>(p, added, c, h, col0, nv, false);
-            if (ONES && col0 == 0) walk_in_order<TI, MODE>(p, added, c, h, dvv, 1, false);
-            if (col0 == 0)
-                for (int i = tid; i < p.dk; i += THREADS) {
-                    float a = 1.f;
-                    for (int t = t0; t < t0 + n; ++t) a = times_decay<MODE>(a, decay_at<MODE>(p, t, h, i));
-                    decays[i] = a;
-                }
-        }
+        const int cols = col0 == 0 && ONES ? nv + 1 : nv;
+        for (int e = tid; e < cols * p.dk; e += TILE_THREADS) added[(size_t)(e % p.dk) * p.dvp + (e / p.dk < nv ? col0 + e / p.dk : dvv)] = 0.f;
+        __syncthreads();
+        walk_in_order<TI, MODE>(p, added, c, h, col0, nv, false);
+        if (ONES && col0 == 0) walk_in_order<TI, MODE>(p, added, c, h, dvv, 1, false);
+        if (col0 == 0)
+            for (int i = tid; i < p.dk; i += TILE_THREADS) {
+                float a = 1.f;
+                for (int t = t0; t < t0 + n; ++t) a = times_decay<MODE>(a, decay_at<MODE>(p, t, h, i));
+                decays[i] = a;
+            }
+        leave();
         return;
     }
     Raw4<TI> rk[NK], rv[NV];
+    auto fetch_k = [&](int i0) {
 #pragma unroll
-    for (int x = 0; x < NK; ++x) {
-        const int e = tid + x * THREADS, j = e >> 4;
-        get_four(rk[x], (const TI*)p.k + (size_t)(t0 + j) * p.ldk + hq * p.dk + i0, (e & 15) * 4, nk, j < n, p.vec_k);
-    }
+        for (int x = 0; x < NK; ++x) {
+            const int e = tid + x * TILE_THREADS, j = e >> 4;
+            get_four(rk[x], (const TI*)p.k + (size_t)(t0 + j) * p.ldk + hq * p.dk + i0, (e & 15) * 4, min(64, p.dk - i0), j < n, p.vec_k);
+        }
+    };
+    fetch_k(0);
 #pragma unroll
     for (int x = 0; x < NV; ++x) {
-        const int e = tid + x * THREADS, j = e / (16 * NC);
-        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)h * dvv + col0, (e % (16 * NC)) * 4, nv, j < n, p.vec_v);
+        const int e = tid + x * TILE_THREADS, j = e >> 5;
+        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)h * dvv + col0, (e & 31) * 4, nv, j < n, p.vec_v);
     }
     if (!PER_CHANNEL) {
         if (tid < CT) {
@@ -142,67 +256,93 @@ added_state_kernel(Scan p) {
         }
         __syncthreads();
         if (col0 == 0)
-            for (int i = tid; i < nk; i += THREADS) decays[i0 + i] = s_whole;
+            for (int i = tid; i < p.dk; i += TILE_THREADS) decays[i] = s_whole;
     }
 #pragma unroll
-    for (int x = 0; x < NK; ++x) {
-        const int e = tid + x * THREADS, j = e >> 4;
-        float4 f = rk[x].value();
-        if (!PER_CHANNEL) { const float w = s_w[j]; f.x *= w; f.y *= w; f.z *= w; f.w *= w; }
-        *reinterpret_cast<float4*>(sk + j * 64 + (e & 15) * 4) = f;
+    for (int x = 0; x < NV; ++x) {
+        const int e = tid + x * TILE_THREADS, col = (e & 31) * 4;
+        put_terms<VT>(tv + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), TERM, rv[x].value());
     }
+    uint32_t round = 0;
+    bool ok = true;
+    for (int base = 0; base < p.dk; base += 128, ++round) {
+        const int halves = p.dk - base > 64 ? 2 : 1;
+        for (int half = 0; half < halves; ++half) {     // 64 channels
+            const int i0 = base + half * 64, nk = min(64, p.dk - i0);
+            const uint32_t to = tk + half * TILE;
+            if (!PER_CHANNEL) {
 #pragma unroll
-    for (int x = 0; x < NV; ++x) *reinterpret_cast<float4*>(sv + (tid + x * THREADS) * 4) = rv[x].value();
-    if (PER_CHANNEL) {                                  // a thread takes a channel and half of the tokens, from the last back
-        constexpr int LEN = CT / 2;
-        __syncthreads();
-        const int i = tid & 63, g = tid >> 6;
-        float a[LEN], run = 1.f;
+                for (int x = 0; x < NK; ++x) {
+                    const int e = tid + x * TILE_THREADS, j = e >> 4;
+                    float4 f = rk[x].value();
+                    const float w = s_w[j];
+                    f.x *= w; f.y *= w; f.z *= w; f.w *= w;
+                    put_terms<3>(to + place_in_tile(j, (e & 15) * 4), TERM, f);
+                }
+            } else {                                    // a thread takes a channel and a quarter of the tokens, from the last back
+                constexpr int LEN = CT / 4;
+                __shared__ __align__(16) float behind[CT * 64];       // the decays behind a token
+                const int i = tid & 63, g = tid >> 6;
+                float a[LEN], run = 1.f;
 #pragma unroll
-        for (int x = 0; x < LEN; ++x) a[x] = g * LEN + x < n && i < nk ? p.dlog[(size_t)(t0 + g * LEN + x) * p.ldd + (size_t)h * p.dk + i0 + i] : 0.f;
+                for (int x = 0; x < LEN; ++x) a[x] = g * LEN + x < n && i < nk ? p.dlog[(size_t)(t0 + g * LEN + x) * p.ldd + (size_t)h * p.dk + i0 + i] : 0.f;
 #pragma unroll
-        for (int x = LEN - 1; x >= 0; --x) {
-            sk[(g * LEN + x) * 64 + i] *= run;
-            run *= g * LEN + x < n && i < nk ? channel_decay<MODE>(a[x], p.decay_scale) : 1.f;
+                for (int x = LEN - 1; x >= 0; --x) {
+                    behind[(g * LEN + x) * 64 + i] = run;
+                    run *= g * LEN + x < n && i < nk ? channel_decay<MODE>(a[x], p.decay_scale) : 1.f;
+                }
+                part[g * 64 + i] = run;
+                __syncthreads();
+#pragma unroll
+                for (int x = 0; x < NK; ++x) {
+                    const int e = tid + x * TILE_THREADS, j = e >> 4, at = (e & 15) * 4, q = j / LEN;
+                    float4 d = *reinterpret_cast<const float4*>(behind + j * 64 + at), f = rk[x].value();
+                    for (int later = q + 1; later < 4; ++later) {
+                        const float4 more = *reinterpret_cast<const float4*>(part + later * 64 + at);
+                        d.x *= more.x; d.y *= more.y; d.z *= more.z; d.w *= more.w;
+                    }
+                    f.x *= d.x; f.y *= d.y; f.z *= d.z; f.w *= d.w;
+                    put_terms<3>(to + place_in_tile(j, at), TERM, f);
+                }
+                if (tid < nk && col0 == 0) decays[i0 + tid] = (part[tid] * part[64 + tid]) * (part[128 + tid] * part[192 + tid]);
+                __syncthreads();
+            }
+            if (i0 + 64 < p.dk) fetch_k(i0 + 64);
         }
-        part[g * 64 + i] = run;
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
         __syncthreads();
-        if (g == 0) {
-            const float later = part[64 + i];
-#pragma unroll 8
-            for (int t = 0; t < LEN; ++t) sk[t * 64 + i] *= later;
-            if (i < nk && col0 == 0) decays[i0 + i] = run * later;
+        const int width = halves * 64;
+        if (warp == 0 && elect_one()) {
+            tc_fence_after_sync();
+            multiply_tiles<VT, 3, true, true>(tmem, tv, TERM, tk, TERM, width);
+            mma_commit(&done);
         }
-    }
-    __syncthreads();
-    f32x2 acc[8][2 * NC];
+        __syncwarp();
+        if (ONES && col0 == 0 && tid < min(width, p.dk - base))         // the column whose values are ones
+            added[(size_t)(base + tid) * p.dvp + dvv] = plain_added<TI, MODE>(p, h, base + tid, t0, n, -1, s_w);
+        if (ok) ok = wait_done(&done, round & 1, p.status);
+        tc_fence_after_sync();
+        const int col = (warp & 3) * 32 + lane;
+#pragma unroll 1
+        for (int at = (warp >> 2) * (width / 2); at < (warp >> 2) * (width / 2) + width / 2; at += 32) {
+            float sum[32];
+            take_sums<32>(sum, tmem + ((uint32_t)((warp & 3) * 32) << 16) + at, true);
+            float* to = added + (size_t)(base + at) * p.dvp + col0 + col;
+            if (col < nv) {
+                const int rows = min(32, p.dk - base - at);
+                bool odd = false;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * NC; ++j) acc[i][j] = 0ull;
-    tile_product<NC, false>(acc, sk, sv, n, ty, tx);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = (i >> 2) * 32 + ty * 4 + (i & 3);
-        if (r >= nk) continue;
-        float* row = added + (size_t)(i0 + r) * p.dvp + col0;
-#pragma unroll
-        for (int g = 0; g < NC; ++g) {
-            const int at = g * 64 + tx * 4;
-            const float2 a = unpack2(acc[i][2 * g]), b = unpack2(acc[i][2 * g + 1]);
-            if (at + 3 < nv) *reinterpret_cast<float4*>(row + at) = make_float4(a.x, a.y, b.x, b.y);
-            else {
-                if (at < nv) row[at] = a.x;
-                if (at + 1 < nv) row[at + 1] = a.y;
-                if (at + 2 < nv) row[at + 2] = b.x;
+                for (int x = 0; x < 32; ++x) {
+                    odd |= !is_number(sum[x]);
+                    if (x < rows) to[(size_t)x * p.dvp] = sum[x];
+                }
+                if (odd) mend_added<TI, MODE>(p, to, rows, h, base + at, t0, n, (long long)h * dvv + col0 + col, s_w);
             }
         }
+        tc_fence_before_sync();
     }
-    if (ONES && col0 == 0 && tid < nk) {                // the column whose values are ones
-        float sum = 0.f;
-        for (int j = 0; j < n; ++j) sum += sk[j * 64 + tid];
-        added[(size_t)(i0 + tid) * p.dvp + dvv] = sum;
-    }
+    leave();
 }
 
 // ----------------------------------------------------------------------------- a chunk's outputs
@@ -538,25 +678,262 @@ chunk_output_kernel(Scan p) {
     }
 }
 
-template <typename TI, int MODE, int NC>
+// ----------------------------------------------------------------------------- a chunk's outputs, one decay per head
+
+// A block takes the 64 tokens of a chunk and 128 value columns of one head, or (NH = 2) 64 of each of two neighbouring heads that share
+// q and k, whose products q k^T are then taken once.  The key channels pass in slices of 64 through shared memory, as terms: q, k and v in QT
+// (one where they come as bfloat16), the states and the weights in three.  A slice is a run in the tensor unit; the runs' sums, from two sets
+// of accumulators, are added in registers.  Columns on the TMEM lanes for the outputs, tokens for q k^T.
+template <typename TI, int NH> constexpr int tile_smem() {
+    const int qt = sizeof(TI) == 2 ? 1 : 3, slices = (2 * qt + 6) * TILE, weights = (3 * NH + 2 * qt) * TILE;
+    return 1024 + (slices > weights ? slices : weights);
+}
+
+// One output by multiply-adds, where the tensor unit gave no number.  The weights are taken from their terms at `tp` where they have some.
+template <typename TI, int MODE>
+__device__ __noinline__ float plain_output(const Scan& p, const float* __restrict__ S, const float* __restrict__ a, const float* __restrict__ b, float cum,
+                                           uint32_t tp, int h, int t0, int t, int col) {
+    constexpr bool ONES = MODE == 2;
+    const int hq = h / p.qk_group, dvv = ONES ? p.dv - 1 : p.dv;
+    const TI* q = (const TI*)p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk;
+    float o = 0.f, d = 1.f;
+    for (int i = 0; i < p.dk; ++i) o = fmaf(to_f32(q[i]) * p.q_scale, S[(size_t)i * p.dvp + col], o);
+    o *= cum;
+    for (int j = t; j >= 0 && o == o; --j) {           // NaN stays NaN
+        float w = 0.f;
+        for (int i = 2; i >= 0; --i) {
+            uint16_t term;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(term) : "r"(tp + i * TILE + place_in_tile(t, j)));
+            w += __uint_as_float((uint32_t)term << 16);
+        }
+        if (!is_number(w)) {
+            const TI* k = (const TI*)p.k + (size_t)(t0 + j) * p.ldk + hq * p.dk;
+            float raw = 0.f;
+            for (int i = 0; i < p.dk; ++i) raw = fmaf(to_f32(q[i]) * p.q_scale, to_f32(k[i]), raw);
+            w = b[j] * d * raw;
+        }
+        o = fmaf(w, ONES && col == dvv ? 1.f : to_f32(((const TI*)p.v)[(size_t)(t0 + j) * p.ldv + (size_t)h * dvv + col]), o);
+        d = times_decay<MODE>(d, a[j]);
+    }
+    return o;
+}
+
+// MANY: more than 128 key channels, more than two runs; without it no sums are held while slices pass.
+template <typename TI, int MODE, int NH, bool MANY>
+__global__ void __launch_bounds__(TILE_THREADS, 2)
+tile_output_kernel(const __grid_constant__ Scan p) {
+    constexpr bool ONES = MODE == 2;
+    constexpr int QT = sizeof(TI) == 2 ? 1 : 3, NQ = CT * 16 / TILE_THREADS, NS = 2 * NQ;
+    constexpr uint32_t TMEM = 256;                      // two runs' sums: the outputs [128 columns][64 tokens], q k^T [64 tokens (128 lanes)][64]
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ float s_a[NH][CT], s_cum[NH][CT], s_b[NH][CT], s_ones[2][CT];
+    __shared__ uint64_t done;
+    __shared__ uint32_t tmem_slot;
+    const int c = blockIdx.x, h = blockIdx.y * NH, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
+    if (tid == 0) { mbar_init(&done, 1); mbar_fence_init(); }
+    if (warp == 0) { tmem_alloc(&tmem_slot, TMEM); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem = tmem_slot, own = tmem + ((uint32_t)(quad * 32) << 16) + half * 32;
+    const uint32_t tq = (smem_u32(smem_raw) + 1023) & ~1023u, tk = tq + QT * TILE, ts = tk + QT * TILE;     // [QT][tokens], [QT][tokens], [3][2 halves of the columns][channels]
+    const uint32_t tp = tq, tv = tp + 3 * NH * TILE;    // after the slices: [NH][3][tokens][earlier tokens], [QT][2][tokens]
+    const int dvv = ONES ? p.dv - 1 : p.dv, col0 = blockIdx.z * 128, nv = NH == 2 ? dvv : min(128, dvv - col0);
+    const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, hq = h / p.qk_group;
+    auto leave = [&]() {
+        tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(tmem, TMEM);
+    };
+    if (c == 0)                                         // rows behind the last sequence belong to nobody: a defined value
+        for (int t = p.chunk_start[p.n_chunks]; t < p.T_rows; ++t) {
+            for (int e = tid; e < NH * nv; e += TILE_THREADS) p.o[(size_t)t * p.ldo + (size_t)(h + e / nv) * p.dv + (NH == 2 ? 0 : col0) + e % nv] = 0.f;
+            if (ONES && col0 == 0 && tid == 0) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + dvv] = 0.f;
+        }
+    if (n <= 0 || n > CT) {
+        if (n > CT)
+            for (int x = 0; x < NH; ++x) {
+                float* S = p.chunk_state + ((size_t)c * p.H + h + x) * p.dk * p.dvp;
+                walk_in_order<TI, MODE>(p, S, c, h + x, col0, nv, true);
+                if (ONES && col0 == 0) walk_in_order<TI, MODE>(p, S, c, h + x, dvv, 1, true);
+            }
+        leave();
+        return;
+    }
+    for (int e = tid; e < NH * CT; e += TILE_THREADS) { // the tokens' decays and weights
+        const int x = e / CT, t = e % CT;
+        s_a[x][t] = t < n ? decay_at<MODE>(p, t0 + t, h + x, 0) : (MODE == 5 ? 0.f : 1.f);
+        s_b[x][t] = t >= n ? 0.f : (MODE == 2 || MODE == 5) ? p.gb[(size_t)(t0 + t) * p.ldg + h + x] : 1.f;
+    }
+    float out[32], raw[32], ones_part = 0.f;            // column quad 32 + lane of tokens half 32 ..; token quad 32 + lane (< 64) against tokens half 32 ..
+    const int slices = (p.dk + 63) / 64;
+    bool ok = true;
+    for (int s = 0; s < slices; ++s) {
+        const int i0 = s * 64, nk = min(64, p.dk - i0);
+        Raw4<float> rs[NS];
+        Raw4<TI> rq[NQ], rk[NQ];
+#pragma unroll
+        for (int x = 0; x < NQ; ++x) {
+            const int e = tid + x * TILE_THREADS, t = e >> 4, i = (e & 15) * 4;
+            get_four(rq[x], (const TI*)p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk + i0, i, nk, t < n, p.vec_q);
+            get_four(rk[x], (const TI*)p.k + (size_t)(t0 + t) * p.ldk + hq * p.dk + i0, i, nk, t < n, p.vec_k);
+        }
+#pragma unroll
+        for (int x = 0; x < NS; ++x) {
+            const int e = tid + x * TILE_THREADS, i = e >> 5, col = (e & 31) * 4, at = NH == 2 ? col & 63 : col0 + col;
+            get_four(rs[x], p.chunk_state + (((size_t)c * p.H + h + (NH == 2 ? col >> 6 : 0)) * p.dk + i0 + i) * p.dvp, at, (dvv + 3) / 4 * 4, i < nk, 1);
+        }
+        if (s && ok) ok = wait_done(&done, (s - 1) & 1, p.status);
+        if (MANY && s >= 2) {                                 // the set of accumulators that comes next is full: onto the thread's sums
+            tc_fence_after_sync();
+            take_sums<32>(out, own + (s & 1) * 128, s == 2);
+            if (quad < 2) take_sums<32>(raw, own + (s & 1) * 128 + 64, s == 2);
+        }
+#pragma unroll
+        for (int x = 0; x < NQ; ++x) {
+            const int e = tid + x * TILE_THREADS;
+            const uint32_t at = place_in_tile(e >> 4, (e & 15) * 4);
+            put_terms<QT>(tq + at, TILE, rq[x].value());
+            put_terms<QT>(tk + at, TILE, rk[x].value());
+        }
+#pragma unroll
+        for (int x = 0; x < NS; ++x) {
+            const int e = tid + x * TILE_THREADS, col = (e & 31) * 4;
+            put_terms<3>(ts + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), 2 * TILE, rs[x].value());
+        }
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 0 && elect_one()) {
+            tc_fence_after_sync();
+            multiply_tiles<3, QT, true, false>(tmem + (s & 1) * 128, ts, 2 * TILE, tq, TILE, CT);           // S0^T q
+            multiply_tiles<QT, QT, false, false>(tmem + (s & 1) * 128 + 64, tq, TILE, tk, TILE, CT);        // q k^T
+            mma_commit(&done);
+        }
+        __syncwarp();
+        if (s == 0)
+            for (int e = tid; e < NH * CT; e += TILE_THREADS) {         // the decays since the chunk's start
+                const int x = e / CT, t = e % CT;
+                float cum = 1.f;
+#pragma unroll 8
+                for (int j = 0; j < CT; ++j) if (j <= t) cum = times_decay<MODE>(cum, s_a[x][j]);
+                s_cum[x][t] = cum;
+            }
+        if (ONES && blockIdx.z == 0 && tid < n) {
+            const float* last = p.chunk_state + (((size_t)c * p.H + h) * p.dk + i0) * p.dvp + dvv;
+            const TI* q = (const TI*)p.q + (size_t)(t0 + tid) * p.ldq + hq * p.dk + i0;
+            for (int i = 0; i < nk; ++i) ones_part = fmaf(to_f32(q[i]), last[(size_t)i * p.dvp], ones_part);
+        }
+    }
+    Raw4<TI> rv[NS];
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+        const int e = tid + x * TILE_THREADS, j = e >> 5, col = (e & 31) * 4, head = NH == 2 ? col >> 6 : 0, at = NH == 2 ? col & 63 : col;
+        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)(h + head) * dvv + (NH == 2 ? 0 : col0), at, nv, j < n, p.vec_v);
+    }
+    if (ok) ok = wait_done(&done, (slices - 1) & 1, p.status);
+    tc_fence_after_sync();
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+        const int e = tid + x * TILE_THREADS, col = (e & 31) * 4;
+        put_terms<QT>(tv + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), 2 * TILE, rv[x].value());
+    }
+    const int older = slices & 1, newer = older ^ 1;    // the sets of the last run but one and of the last
+    if (quad < 2) {                                     // the weights P[t][j]: a thread half of a token's, from the last earlier token back
+        if (slices > 1) take_sums<32>(raw, own + older * 128 + 64, slices == 2);
+        take_sums<32>(raw, own + newer * 128 + 64, slices == 1);
+        const int t = quad * 32 + lane;
+#pragma unroll
+        for (int x = 0; x < NH; ++x) {
+            float d = 1.f, ones = 0.f;
+            if (half == 0)
+#pragma unroll 8
+                for (int j = CT - 2; j >= 32; --j) if (j < t) d = times_decay<MODE>(d, s_a[x][j + 1]);
+#pragma unroll
+            for (int j8 = 24; j8 >= 0; j8 -= 8) {
+                float w[8];
+#pragma unroll
+                for (int y = 7; y >= 0; --y) {
+                    const int j = half * 32 + j8 + y;
+                    if (j < t) d = times_decay<MODE>(d, s_a[x][j + 1]);
+                    // a weight of zero stays zero whatever the product is: a token's q never meets a later token's k
+                    w[y] = j <= t ? s_b[x][j] * d * (raw[j8 + y] * p.q_scale) : 0.f;
+                    if (ONES) ones += w[y];
+                }
+                put_eight(tp + x * 3 * TILE + place_in_tile(t, half * 32 + j8), TILE, w);
+            }
+            if (ONES) s_ones[half][t] = ones;
+        }
+    }
+    if (slices > 1) take_sums<32>(out, own + older * 128, slices == 2);
+    take_sums<32>(out, own + newer * 128, slices == 1);
+    fence_proxy_async_smem();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 0 && elect_one()) {
+        tc_fence_after_sync();
+#pragma unroll
+        for (int x = 0; x < NH; ++x) multiply_tiles<QT, 3, true, false>(tmem + x * 64, tv, 2 * TILE, tp + x * 3 * TILE, TILE, CT);       // V^T P^T
+        mma_commit(&done);
+    }
+    __syncwarp();
+    const int head = NH == 2 ? quad >> 1 : 0, in = quad * 32 + lane, col = NH == 2 ? in & 63 : col0 + in;
+    const float* const S = p.chunk_state + ((size_t)c * p.H + h + head) * p.dk * p.dvp;
+#pragma unroll
+    for (int x = 0; x < 32; ++x) out[x] *= s_cum[head][half * 32 + x] * p.q_scale;
+    if (ONES && blockIdx.z == 0 && tid < n) {
+        float sum = fmaf(s_cum[0][tid] * p.q_scale, ones_part, s_ones[0][tid] + s_ones[1][tid]);
+        if (!is_number(sum)) sum = plain_output<TI, MODE>(p, S, s_a[0], s_b[0], s_cum[0][tid], tp, h, t0, tid, dvv);
+        p.o[(size_t)(t0 + tid) * p.ldo + (size_t)h * p.dv + dvv] = sum;
+    }
+    if (ok) ok = wait_done(&done, slices & 1, p.status);
+    tc_fence_after_sync();
+    take_sums<32>(out, own + head * 64, false);
+    float* const o = p.o + (size_t)t0 * p.ldo + (size_t)(h + head) * p.dv + col;
+    if (col < dvv) {
+        const int rows = n - half * 32;
+        bool odd = false;
+#pragma unroll
+        for (int x = 0; x < 32; ++x) {
+            odd |= !is_number(out[x]);
+            if (x < rows) o[(size_t)(half * 32 + x) * p.ldo] = out[x];
+        }
+        if (odd)
+            for (int t = half * 32; t < min(n, half * 32 + 32); ++t)
+                if (!is_number(o[(size_t)t * p.ldo])) o[(size_t)t * p.ldo] = plain_output<TI, MODE>(p, S, s_a[head], s_b[head], s_cum[head][t], tp + head * 3 * TILE, h + head, t0, t, col);
+    }
+    leave();
+}
+
+template <typename TI, int MODE>
 int launch_added(const Scan& p, int n_chunks, cudaStream_t stream) {
-    const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
-    const size_t smem = (size_t)(CT * 64 + CT * 64 * NC) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(added_state_kernel<TI, MODE, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int tiles = ((dvv + 64 * NC - 1) / (64 * NC)) * ((p.dk + 63) / 64);
-    if (e == cudaSuccess) e = qs_launch_dependent(added_state_kernel<TI, MODE, NC>, dim3(n_chunks, p.H, tiles), dim3(THREADS), smem, stream, p);
+    const int dvv = MODE == 2 ? p.dv - 1 : p.dv, smem = added_smem<TI>();
+    cudaError_t e = cudaFuncSetAttribute(added_state_kernel<TI, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = qs_launch_dependent(added_state_kernel<TI, MODE>, dim3(n_chunks, p.H, (dvv + 127) / 128), dim3(TILE_THREADS), smem, stream, p);
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "state_scan, added states: %s", cudaGetErrorString(e));
     return qs_check_launch("state_scan, added states");
 }
 
+// NC: columns in 64s of a block (per channel), NH: heads of a block (one decay per head)
 template <typename TI, int MODE, int NC, int NH>
 int launch_output(const Scan& p, int n_chunks, cudaStream_t stream) {
     const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
-    const size_t smem = (size_t)(output_body<MODE, NC>() + NH * CT * (CT + 4) + (MODE == 1 || MODE == 4 ? 4 * 64 : 0)) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(chunk_output_kernel<TI, MODE, NC, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int tiles = NH == 2 ? 1 : (dvv + 64 * NC - 1) / (64 * NC);
-    if (e == cudaSuccess)
-        e = qs_launch_dependent(chunk_output_kernel<TI, MODE, NC, NH>, dim3(n_chunks, p.H / NH, tiles), dim3(THREADS), smem, stream, p);
+    cudaError_t e;
+    if constexpr (MODE == 1 || MODE == 4) {
+        const size_t smem = (size_t)(output_body<MODE, NC>() + NH * CT * (CT + 4) + 4 * 64) * sizeof(float);
+        e = cudaFuncSetAttribute(chunk_output_kernel<TI, MODE, NC, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = qs_launch_dependent(chunk_output_kernel<TI, MODE, NC, NH>, dim3(n_chunks, p.H / NH, (dvv + 64 * NC - 1) / (64 * NC)), dim3(THREADS), smem, stream, p);
+    } else {
+        constexpr int smem = tile_smem<TI, NH>();
+        const auto kernel = p.dk > 128 ? tile_output_kernel<TI, MODE, NH, true> : tile_output_kernel<TI, MODE, NH, false>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess)
+            e = qs_launch_dependent(kernel, dim3(n_chunks, p.H / NH, NH == 2 ? 1 : (dvv + 127) / 128), dim3(TILE_THREADS), smem, stream, p);
+    }
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "state_scan, chunk outputs: %s", cudaGetErrorString(e));
     return qs_check_launch("state_scan, chunk outputs");
 }
@@ -564,10 +941,10 @@ int launch_output(const Scan& p, int n_chunks, cudaStream_t stream) {
 template <typename TI, int MODE>
 int run(const Scan& p, int n_chunks, bool outputs, cudaStream_t stream) {
     const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
-    if (!outputs) return dvv > 64 ? launch_added<TI, MODE, 2>(p, n_chunks, stream) : launch_added<TI, MODE, 1>(p, n_chunks, stream);
+    if (!outputs) return launch_added<TI, MODE>(p, n_chunks, stream);
     if constexpr (MODE == 5)                            // two heads that share q and k: their products once
-        if (dvv <= 64 && dvv > 32 && p.qk_group % 2 == 0) return launch_output<TI, MODE, 2, 2>(p, n_chunks, stream);
-    return dvv > 64 ? launch_output<TI, MODE, 2, 1>(p, n_chunks, stream) : launch_output<TI, MODE, 1, 1>(p, n_chunks, stream);
+        if (dvv <= 64 && p.qk_group % 2 == 0) return launch_output<TI, MODE, 2, 2>(p, n_chunks, stream);
+    return dvv > 64 ? launch_output<TI, MODE, 2, 1>(p, n_chunks, stream) : launch_output<TI, MODE, MODE == 1 || MODE == 4 ? 1 : 2, 1>(p, n_chunks, stream);
 }
 
 template <typename TI>
@@ -640,7 +1017,7 @@ QS_API int qs_scan_activate(float* out, const void* q, long long ldq, const void
 int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                    int dtype, const float* dlog, long long ldd, const float* head_decay, const void* bonus, int bonus_dtype, int H, int dk, int dv,
                    const int32_t* chunk_start, int n_chunks, int T_rows, float* chunk_state, float* chunk_decay, const float* ga, const float* gb,
-                   long long ldg, float q_scale, int qk_group, float decay_scale, cudaStream_t stream) {
+                   long long ldg, float q_scale, int qk_group, float decay_scale, int32_t* status, cudaStream_t stream) {
     const size_t item = dtype == QS_F32 ? 4 : 2;
     auto fours = [&](const void* ptr, long long ld, int per_head) { return (int)(per_head % 4 == 0 && ld % 4 == 0 && ((uintptr_t)ptr % (4 * item)) == 0); };
     Scan p = {};
@@ -651,6 +1028,6 @@ int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q
     p.q_scale = q_scale; p.decay_scale = decay_scale;
     p.vec_q = fours(q, ldq, dk); p.vec_k = fours(k, ldk, dk); p.vec_v = fours(v, ldv, mode == 2 ? dv - 1 : dv);
     p.vec_o = mode != 2 && dv % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)o % 16) == 0;
-    p.n_chunks = n_chunks; p.T_rows = T_rows;
+    p.n_chunks = n_chunks; p.T_rows = T_rows; p.status = status;
     return dtype == QS_F32 ? pick<float>(mode, p, n_chunks, outputs != 0, stream) : pick<__nv_bfloat16>(mode, p, n_chunks, outputs != 0, stream);
 }
