@@ -978,6 +978,83 @@ int launch_stream(const void* W, long long ldw, const CUtensorMap& ma, const Epi
     return qs_check_launch("gemm_tc stream");
 }
 
+// ----------------------------------------------------------------------------- few features
+
+// N <= NARROW features (routers, step sizes, gates per head): a block takes 16 tokens, its sixteen warps (eight above 32 features) the k-range in turns of 32
+// elements each, on mma.sync straight from memory.  Within a turn a lane fetches 16 bytes of two rows of A and of one row of W per eight
+// features; the order of k inside the unit is that of the lanes, the same for both operands.  A warp's runs of a few turns are added with
+// rounded additions, the warps' sums in the warps' order: nearer to float64 than a chain over all of K in the unit (K = 4,096: 2e-7 of the norm instead
+// of 5e-7 and, at over 128 tokens, 4e-6).
+//
+// Bound by latency: the whole chain is a fetch of rows, a few turns and one sum over the warps.  The tile kernels put such a product on one
+// column of tiles whose CTAs walk all of K one after the other: 8 x 16 x 4096 15.6 us, 3,000 x 16 x 2048 17, 2,048 x 64 x 2048 15.
+constexpr int NARROW = 64;
+template <int NT> constexpr int narrow_warps() { return NT == 8 ? 8 : 16; }
+template <int NT>
+__global__ void __launch_bounds__(32 * narrow_warps<NT>())
+gemm_narrow_kernel(const __nv_bfloat16* __restrict__ A, size_t lda, const __nv_bfloat16* __restrict__ W, size_t ldw, const Epilogue ep, int K) {
+    constexpr int COLS = 8 * NT, NARROW_WARPS = narrow_warps<NT>();
+    __shared__ float red[NARROW_WARPS][16][COLS + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3, m0 = blockIdx.x * 16;
+    grid_dep_launch();
+    grid_dep_wait();
+    const __nv_bfloat16* a0 = A + (size_t)(m0 + g) * lda;
+    const __nv_bfloat16* a1 = a0 + 8 * lda;
+    const bool has0 = m0 + g < ep.M, has1 = m0 + g + 8 < ep.M;
+    float acc[NT][4], run[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int z = 0; z < 4; ++z) acc[n][z] = run[n][z] = 0.f;
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int TURNS = NT <= 2 ? 4 : 2;              // fetches under way together, and the unit's run: the unit cuts off where it adds
+    for (int k0 = warp * 32; k0 < K; k0 += TURNS * 32 * NARROW_WARPS) {
+        uint4 x[TURNS], y[TURNS], w[TURNS][NT];
+#pragma unroll
+        for (int t = 0; t < TURNS; ++t) {
+            const int k = k0 + t * 32 * NARROW_WARPS + q * 8;
+            const bool in = k < K;
+            x[t] = in && has0 ? *reinterpret_cast<const uint4*>(a0 + k) : none;
+            y[t] = in && has1 ? *reinterpret_cast<const uint4*>(a1 + k) : none;
+#pragma unroll
+            for (int n = 0; n < NT; ++n) w[t][n] = in && n * 8 + g < ep.N ? *reinterpret_cast<const uint4*>(W + (size_t)(n * 8 + g) * ldw + k) : none;
+        }
+#pragma unroll
+        for (int t = 0; t < TURNS; ++t)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                    : "+f"(run[n][0]), "+f"(run[n][1]), "+f"(run[n][2]), "+f"(run[n][3]) : "r"(x[t].x), "r"(y[t].x), "r"(x[t].y), "r"(y[t].y), "r"(w[t][n].x), "r"(w[t][n].y));
+                asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                    : "+f"(run[n][0]), "+f"(run[n][1]), "+f"(run[n][2]), "+f"(run[n][3]) : "r"(x[t].z), "r"(y[t].z), "r"(x[t].w), "r"(y[t].w), "r"(w[t][n].z), "r"(w[t][n].w));
+            }
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int z = 0; z < 4; ++z) { acc[n][z] += run[n][z]; run[n][z] = 0.f; }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int z = 0; z < 4; ++z) red[warp][g + (z >> 1) * 8][n * 8 + q * 2 + (z & 1)] = acc[n][z];
+    __syncthreads();
+    for (int e = threadIdx.x; e < 16 * COLS; e += 32 * NARROW_WARPS) {
+        const int r = e / COLS, n = e % COLS;
+        float v = 0.f;
+#pragma unroll
+        for (int i = 0; i < NARROW_WARPS; ++i) v += red[i][r][n];
+        if (m0 + r < ep.M && n < ep.N) store_out(ep, m0 + r, n, v);
+    }
+}
+
+template <int NT>
+int launch_narrow(const void* A, long long lda, const void* W, long long ldw, const Epilogue& ep, int K, cudaStream_t stream) {
+    const cudaError_t e = qs_launch_dependent(gemm_narrow_kernel<NT>, dim3((ep.M + 15) / 16), dim3(32 * narrow_warps<NT>()), 0, stream, (const __nv_bfloat16*)A, (size_t)lda,
+                                              (const __nv_bfloat16*)W, (size_t)ldw, ep, K);
+    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "gemm_tc narrow: %s", cudaGetErrorString(e));
+    return qs_check_launch("gemm_tc narrow");
+}
+
 // Fewer tiles than CTA pairs (a few hundred tokens against a narrow N): each tile's k-range is cut into
 // equal parts for as many pairs as stand idle, at least 16 k-blocks each; their partial sums meet in the
 // workspace (see the kernel).  The cut depends on M, N, K and the device.
@@ -1097,6 +1174,15 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
     Epilogue ep{C, c_dtype, ldc, bias, bias_dtype, act, (const __nv_bfloat16*)res1, (const __nv_bfloat16*)res2, ldr, M, N};
     CUtensorMap ma, mw;
     int rc;
+    // Few features, microseconds tiles | here (caches flushed): 8 x 16 x 4096 14.3 | 5.4, 128 x 16 x 2048 50 | 4.9, 3,000 x 16 x 2048 13.6 | 7.9, 16,000 x 16 x
+    // 2048 22.3 | 22.3, x 4096 32 | 46; 128 x 64 x 2048 51 | 15, 32 x 64 x 512 4.9 | 5.9, 300 x 64 x 512 7.4 | 5.9, x 2048 11.5 | 13.6,
+    // 8 x 64 x 4096 15 | 23.
+    if (M <= 4096 && (N <= 32 || (N <= NARROW && (M > 128 ? K <= 512 : M >= 64 && K <= 4096)))) {
+        if (N <= 8) return launch_narrow<1>(A, lda, W, ldw, ep, K, stream);
+        if (N <= 16) return launch_narrow<2>(A, lda, W, ldw, ep, K, stream);
+        if (N <= 32) return launch_narrow<4>(A, lda, W, ldw, ep, K, stream);
+        return launch_narrow<8>(A, lda, W, ldw, ep, K, stream);
+    }
     if (M > 128) {
         QS_REQUIRE((M + BM - 1) / BM <= 65535 * 1 && (N + 127) / 128 <= 65535, "gemm_tc: sizes exceed the grid");
         if ((rc = tensor_map(&ma, A, M, K, lda, BM)) != QS_OK) return rc;
