@@ -63,8 +63,11 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
     return false;
 }
 
-template <int BN> constexpr int p_stages() { return SMEM_BUDGET_BIG / stage_bytes<BN>(); }
-template <int BN> constexpr int p_smem_bytes() { return p_stages<BN>() * stage_bytes<BN>() + 1024 + 512; }
+constexpr int P_EPILOGUE_WARPS = 8, P_THREADS = 64 + 32 * P_EPILOGUE_WARPS;
+constexpr int STAGE_PITCH = 36;                     // floats: rows of 16 bytes meet all banks
+constexpr int STAGING = P_EPILOGUE_WARPS * 32 * STAGE_PITCH * 4;
+template <int BN> constexpr int p_stages() { return (SMEM_BUDGET_BIG - STAGING) / stage_bytes<BN>(); }
+template <int BN> constexpr int p_smem_bytes() { return p_stages<BN>() * stage_bytes<BN>() + 1024 + 512 + STAGING; }
 
 // One CTA per SM walks over output tiles of 128 x BN (tile t = n_tile * m_tiles + m_tile, so CTAs that
 // run together share rows of W and all of A stays in L2).  Two accumulators in TMEM: while the four
@@ -75,12 +78,24 @@ template <int BN> constexpr int p_smem_bytes() { return p_stages<BN>() * stage_b
 // ep.N rows one below the other).  The offsets are read on the device, so the host need not know them.  Tiles run through
 // a group's rows first, then its columns, then the groups; a tile's rows beyond its group are computed from the next group's and not
 // stored.
+//
+// GLU (GROUPED): a matrix holds ep.N gate rows above its ep.N up rows, and C = silu(gate) up: a tile takes BN / 2 rows of each, which
+// meet in the epilogue as 32-bit sums.
+//
+// Eight epilogue warps, two to a quarter of the TMEM lanes, half of the columns each: with a short K (the second product of routed experts, K = 512)
+// the drain of a tile takes longer than its main loop, and one warp to a scheduler hides none of its own latencies.  Plain 32-bit sums go through
+// shared memory to whole 128-byte lines: with a row per lane every 16-byte store met 32 lines, 8,192 cycles of the store pipe for a tile whose
+// main loop needs 4,096.  Neither change alone gains (eight warps: 60 us instead of 56 for that product; the lines with four warps made
+// every product slower); together, with the unit in the first product (14 us of its own before), and the kernel as a programmatic dependent, 3,000
+// tokens through 4 of 16 experts of 2048 x 512 take 167 us instead of 193.
 constexpr int MAX_GROUPS = 1024;
-template <int BN, bool GROUPED>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int BN, bool GROUPED, bool GLU>
+__global__ void __launch_bounds__(P_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                           const Epilogue ep, const int K, const int m_tiles, const int n_tiles,
                           int32_t* __restrict__ status, const int32_t* __restrict__ offsets, const int n_groups) {
+    static_assert(GROUPED || !GLU, "the gated unit belongs to the grouped form");
+    constexpr int WIDTH = GLU ? BN / 2 : BN;          // columns of C of a tile
     constexpr int STAGES = p_stages<BN>();
     constexpr int STAGE = stage_bytes<BN>();
     constexpr uint32_t TMEM_COLS = 2 * BN;
@@ -100,15 +115,20 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 128); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 32 * P_EPILOGUE_WARPS); }
         *aborted = 0;
         mbar_fence_init();
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_w);
     }
     if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    grid_dep_launch();                                // behind the allocation: the next kernel's may not take its place
+    grid_dep_wait();
     if (GROUPED) {
-        for (int e = threadIdx.x; e <= n_groups; e += THREADS) first_row[e] = offsets[e];
+        for (int e = threadIdx.x; e <= n_groups; e += P_THREADS) first_row[e] = offsets[e];
         __syncthreads();
         if (warp == 2) {                                // the groups' first tiles: a running sum, 32 groups at a time
             int run = 0;
@@ -123,10 +143,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
             if (lane == 0) first_tile[n_groups] = run;
         }
+        __syncthreads();
     }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     const int total_tiles = GROUPED ? first_tile[n_groups] : m_tiles * n_tiles;
     // a tile's first row of A, the end of its rows, its first column of C and its first row of W; `group` only moves on
@@ -135,8 +153,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         if (!GROUPED) { const int n0 = (t / m_tiles) * BN; return Place{(t % m_tiles) * BM, ep.M, n0, n0}; }
         while (t >= first_tile[group + 1]) ++group;
         const int lo = first_row[group], hi = first_row[group + 1], tiles = (hi - lo + BM - 1) / BM, mine = t - first_tile[group];
-        const int n0 = (mine / tiles) * BN;
-        return Place{lo + (mine % tiles) * BM, hi, n0, group * ep.N + n0};
+        const int n0 = (mine / tiles) * WIDTH;
+        return Place{lo + (mine % tiles) * BM, hi, n0, group * (GLU ? 2 : 1) * ep.N + n0};
     };
 
     if (warp == 0) {
@@ -152,6 +170,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                     mbar_expect_tx(&full[s], STAGE);
                     tma_load_2d(tile, &map_a, &full[s], kb * BK, at.m0);
                     tma_load_2d(tile + BM * BK * 2, &map_w, &full[s], kb * BK, at.w0);
+                    if (GLU) tma_load_2d(tile + BM * BK * 2 + WIDTH * BK * 2, &map_w, &full[s], kb * BK, at.w0 + ep.N);
                 }
             }
         }
@@ -180,13 +199,15 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
         }
     } else {
-        const int quad = warp & 3;
+        const int quad = warp & 3, half = (warp - 2) >> 2;
         const int r = quad * 32 + lane;
         const bool wide = ep.c_dtype == QS_F32;           // 32-bit results: twice as many 16-byte stores
         const bool vec_ok = (ep.ldc % (wide ? 4 : 8)) == 0 && ((uintptr_t)ep.C % 16) == 0 &&
                             (!ep.res1 || ((ep.ldr % 8) == 0 && ((uintptr_t)ep.res1 % 16) == 0)) &&
                             (!ep.res2 || ((uintptr_t)ep.res2 % 16) == 0);
         const bool bias_vec = ep.bias && ((uintptr_t)ep.bias % 32) == 0;
+        const bool plain = vec_ok && !ep.bias && !ep.res1 && !ep.res2 && ep.act == QS_ACT_NONE;
+        float* const stage = reinterpret_cast<float*>(smem + STAGES * STAGE + 512) + (warp - 2) * 32 * STAGE_PITCH;
         int i = 0, group = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++i) {
             const int buf = i & 1;
@@ -195,12 +216,34 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             if (!wait_or_abort(&acc_full[buf], (i >> 1) & 1, aborted)) { atomicExch(status, 124); *aborted = 1; break; }
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
+            for (int c = half * (WIDTH / 64); c < (half + 1) * (WIDTH / 64); ++c) {
                 uint32_t raw[32];
-                tmem_load_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN + c * 32), raw);
-                tmem_load_wait();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN + c * 32);
+                tmem_load_32x32(taddr, raw);
+                if (GLU) {
+                    uint32_t up[32];
+                    tmem_load_32x32(taddr + WIDTH, up);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) raw[j] = __float_as_uint(silu_f32(__uint_as_float(raw[j])) * __uint_as_float(up[j]));
+                } else tmem_load_wait();
                 const int nc = n0 + c * 32;
-                if (m >= at.m_end || nc >= ep.N) continue;
+                if (nc >= ep.N) continue;
+                if (wide && plain && nc + 32 <= ep.N) {
+                    // sums as they are, 32-bit: through shared memory, whole lines of four rows to a store
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(stage + lane * STAGE_PITCH + g * 4) = make_uint4(raw[4 * g], raw[4 * g + 1], raw[4 * g + 2], raw[4 * g + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const int row = g * 4 + (lane >> 3), mr = at.m0 + quad * 32 + row;
+                        const float4 v = *reinterpret_cast<const float4*>(stage + row * STAGE_PITCH + (lane & 7) * 4);
+                        if (mr < at.m_end) *reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.C) + (size_t)mr * ep.ldc + nc + (lane & 7) * 4) = v;
+                    }
+                    __syncwarp();
+                    continue;
+                }
+                if (m >= at.m_end) continue;
                 if (vec_ok && nc + 32 <= ep.N) {
                     // 32 consecutive outputs of one row: bias and activation on the accumulator, residuals
                     // added in 32-bit, one rounding, four 16-byte stores
@@ -1128,13 +1171,13 @@ int launch_pair(const CUtensorMap& ma, const void* W, long long ldw, const Epilo
 }
 
 // offsets null: one product of M rows.  Else `n_groups` products whose rows the device finds in `offsets` (M: all rows together).
-template <int BN, bool GROUPED>
+template <int BN, bool GROUPED, bool GLU>
 int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilogue& ep, int M, int N, int K,
                       int32_t* status, const int32_t* offsets, int n_groups, cudaStream_t stream) {
     static bool configured = false;
     static int sm_count = 0;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, GROUPED, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              p_smem_bytes<BN>());
         int dev = 0;
         if (e == cudaSuccess) e = cudaGetDevice(&dev);
@@ -1143,10 +1186,13 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilog
                                              cudaGetErrorString(e));
         configured = true;
     }
-    const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
+    const int width = GLU ? BN / 2 : BN;
+    const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + width - 1) / width;
     const long long total = (long long)(m_tiles + (GROUPED ? n_groups : 0)) * n_tiles;     // groups: at most a tile row more each
     const int grid = (int)(total < sm_count ? total : sm_count);
-    gemm_tc_persistent_kernel<BN, GROUPED><<<grid, THREADS, p_smem_bytes<BN>(), stream>>>(ma, mw, ep, K, m_tiles, n_tiles, status, offsets, n_groups);
+    const cudaError_t e = qs_launch_dependent(gemm_tc_persistent_kernel<BN, GROUPED, GLU>, dim3(grid), dim3(P_THREADS), p_smem_bytes<BN>(), stream, ma, mw, ep, K,
+                                              m_tiles, n_tiles, status, offsets, n_groups);
+    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "gemm_tc persistent: %s", cudaGetErrorString(e));
     return qs_check_launch("gemm_tc persistent");
 }
 
@@ -1174,8 +1220,8 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
     Epilogue ep{C, c_dtype, ldc, bias, bias_dtype, act, (const __nv_bfloat16*)res1, (const __nv_bfloat16*)res2, ldr, M, N};
     CUtensorMap ma, mw;
     int rc;
-    // Few features, microseconds tiles | here (caches flushed): 8 x 16 x 4096 14.3 | 5.4, 128 x 16 x 2048 50 | 4.9, 3,000 x 16 x 2048 13.6 | 7.9, 16,000 x 16 x
-    // 2048 22.3 | 22.3, x 4096 32 | 46; 128 x 64 x 2048 51 | 15, 32 x 64 x 512 4.9 | 5.9, 300 x 64 x 512 7.4 | 5.9, x 2048 11.5 | 13.6,
+    // Few features, microseconds tiles | here (caches flushed): 8 x 16 x 4096 14.3 | 7.2, 128 x 16 x 2048 50 | 5.6, 3,000 x 16 x 2048 13.6 | 7.2, 16,000 x 16 x
+    // 2048 22.3 | 22.3, x 4096 32 | 46; 128 x 64 x 2048 51 | 9.2, 32 x 64 x 512 4.9 | 5.9, 300 x 64 x 512 7.4 | 5.1, x 2048 11.5 | 13.6,
     // 8 x 64 x 4096 15 | 23.
     if (M <= 4096 && (N <= 32 || (N <= NARROW && (M > 128 ? K <= 512 : M >= 64 && K <= 4096)))) {
         if (N <= 8) return launch_narrow<1>(A, lda, W, ldw, ep, K, stream);
@@ -1208,8 +1254,8 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
         }
         const int bn = N > 128 ? 256 : 128;
         if ((rc = tensor_map(&mw, W, N, K, ldw, bn)) != QS_OK) return rc;
-        if (bn == 256) return launch_persistent<256, false>(ma, mw, ep, M, N, K, status, nullptr, 0, stream);
-        return launch_persistent<128, false>(ma, mw, ep, M, N, K, status, nullptr, 0, stream);
+        if (bn == 256) return launch_persistent<256, false, false>(ma, mw, ep, M, N, K, status, nullptr, 0, stream);
+        return launch_persistent<128, false, false>(ma, mw, ep, M, N, K, status, nullptr, 0, stream);
     }
     const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
     if ((rc = tensor_map(&ma, A, M, K, lda, bn)) != QS_OK) return rc;
@@ -1221,23 +1267,28 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
 
 // C[rows of e] = A[rows of e] W[e]^T for the groups e of rows offsets[e] .. offsets[e + 1] (E + 1 ascending entries on the DEVICE, from 0
 // to at most M), W [E][N][K] contiguous; A [M, K] bfloat16 with row stride lda, C [M, N] bfloat16 or float32.  One launch; rows
-// of no group are left alone.
+// of no group are left alone.  `glu`: W [E][2 N][K], a matrix's gate rows above its up rows, and C = silu(gate) up.
 QS_API int qs_gemm_tc_grouped(void* C, int c_dtype, long long ldc, const void* A, long long lda, const void* W, const int32_t* offsets, int E, int M, int N,
-                              int K, int32_t* status, cudaStream_t stream) {
+                              int K, int glu, int32_t* status, cudaStream_t stream) {
     if (M == 0) return QS_OK;
     QS_REQUIRE(M > 0 && N > 0 && K > 0 && E > 0 && E <= MAX_GROUPS && offsets, "gemm_tc_grouped: bad sizes M=%d N=%d K=%d E=%d", M, N, K, E);
     QS_REQUIRE(K % 8 == 0 && lda % 8 == 0 && lda >= K && ldc >= N, "gemm_tc_grouped: K=%d and the row stride %lld must be multiples of 8", K, lda);
     QS_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0, "gemm_tc_grouped: operands must be 16-byte aligned");
     QS_REQUIRE(c_dtype == QS_F32 || c_dtype == QS_BF16, "gemm_tc_grouped: unknown output type %d", c_dtype);
-    QS_REQUIRE((long long)E * N <= 0x7fffffffll, "gemm_tc_grouped: %d matrices of %d rows", E, N);
+    const long long w_rows = (long long)E * N * (glu ? 2 : 1);
+    QS_REQUIRE(w_rows <= 0x7fffffffll, "gemm_tc_grouped: %d matrices of %d rows", E, N);
     const Epilogue ep{C, c_dtype, ldc, nullptr, 0, QS_ACT_NONE, nullptr, nullptr, N, M, N};
     // tiles half as wide where whole ones would leave SMs without any (few rows: every group still has its tile row)
-    const long long rows = (M + BM - 1) / BM + (E < M ? E : M) / 2, wide = rows * ((N + 255) / 256);
-    const int bn = N > 128 && wide >= 148 ? 256 : 128;
+    const int columns = glu ? 2 * N : N;
+    const long long rows = (M + BM - 1) / BM + (E < M ? E : M) / 2, wide = rows * ((columns + 255) / 256);
+    const int bn = columns > 128 && wide >= 148 ? 256 : 128;
     CUtensorMap ma, mw;
     int rc;
     if ((rc = tensor_map(&ma, A, M, K, lda, BM)) != QS_OK) return rc;
-    if ((rc = tensor_map(&mw, W, (long long)E * N, K, K, bn)) != QS_OK) return rc;
-    return bn == 256 ? launch_persistent<256, true>(ma, mw, ep, M, N, K, status, offsets, E, stream)
-                     : launch_persistent<128, true>(ma, mw, ep, M, N, K, status, offsets, E, stream);
+    if ((rc = tensor_map(&mw, W, w_rows, K, K, glu ? bn / 2 : bn)) != QS_OK) return rc;
+    if (glu)
+        return bn == 256 ? launch_persistent<256, true, true>(ma, mw, ep, M, N, K, status, offsets, E, stream)
+                         : launch_persistent<128, true, true>(ma, mw, ep, M, N, K, status, offsets, E, stream);
+    return bn == 256 ? launch_persistent<256, true, false>(ma, mw, ep, M, N, K, status, offsets, E, stream)
+                     : launch_persistent<128, true, false>(ma, mw, ep, M, N, K, status, offsets, E, stream);
 }

@@ -73,16 +73,35 @@ __global__ void moe_route_kernel(int32_t* __restrict__ idx, float* __restrict__ 
         }
         __syncwarp();
     }
-    if (lane == 0) {
-        for (int j = 0; j < top; ++j) {
-            int best = -1;
-            for (int e = 0; e < E; ++e)
-                if (choice[e] != -INFINITY && (best < 0 || choice[e] > choice[best])) best = e;
-            if (best < 0) best = 0;                         // fewer live experts than `top`: cannot happen with a sound config
+    // The `top` largest, one after the other: lanes look over every 32nd expert, the warp takes the largest of theirs (equal scores: the
+    // lower index).  NaN is larger than nothing and, as the first live expert, beaten by nothing, as in a walk in order.
+    for (int j = 0; j < top; ++j) {
+        float v = -INFINITY;
+        int best = MAX_EXPERTS, first = MAX_EXPERTS;
+        for (int e = lane; e < E; e += 32) {
+            const float c = choice[e];
+            if (c == -INFINITY) continue;
+            if (first == MAX_EXPERTS) first = e;
+            if (c > v) { v = c; best = e; }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, v, off);
+            const int oe = __shfl_xor_sync(0xffffffffu, best, off);
+            if (ov > v || (ov == v && oe < best)) { v = ov; best = oe; }
+            first = min(first, __shfl_xor_sync(0xffffffffu, first, off));
+        }
+        if (first < MAX_EXPERTS && (best == MAX_EXPERTS || choice[first] != choice[first])) best = first;
+        if (best == MAX_EXPERTS) best = 0;              // fewer live experts than `top`: cannot happen with a sound config
+        __syncwarp();
+        if (lane == 0) {
             idx[(size_t)t * top + j] = best;
             wts[(size_t)t * top + j] = s[best] * scale;
             choice[best] = -INFINITY;
         }
+        __syncwarp();
+    }
+    if (lane == 0) {
         if (renorm_eps >= 0.f) {                            // the chosen scores made to sum to one, in the order of choice
             float sum = 0.f;
             for (int j = 0; j < top; ++j) sum += s[idx[(size_t)t * top + j]];
@@ -449,9 +468,18 @@ moe_down_grouped_kernel(float* __restrict__ out, size_t ldo, const __nv_bfloat16
 __global__ void moe_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restrict__ place_token,
                                 int32_t* __restrict__ pair_place, const int32_t* __restrict__ idx, int n_pairs, int top, int E) {
     __shared__ int count[MAX_EXPERTS + 1];
+    grid_dep_launch();
+    grid_dep_wait();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) count[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) atomicAdd(&count[idx[p]], 1);
+    constexpr int AHEAD = 4;                            // choices fetched before the first of them is counted
+    for (int p0 = threadIdx.x; p0 < n_pairs; p0 += AHEAD * blockDim.x) {
+        int e[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) e[i] = p0 + i * (int)blockDim.x < n_pairs ? idx[p0 + i * blockDim.x] : -1;
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) if (e[i] >= 0) atomicAdd(&count[e[i]], 1);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         int run = 0;
@@ -461,10 +489,17 @@ __global__ void moe_sort_kernel(int32_t* __restrict__ offsets, int32_t* __restri
     __syncthreads();
     // a pair's place inside its expert's range is whatever the counter gives it: a row's products do not depend
     // on where the row lies, so the order is free
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-        const int place = atomicAdd(&count[idx[p]], 1);
-        place_token[place] = p / top;
-        pair_place[p] = place;
+    for (int p0 = threadIdx.x; p0 < n_pairs; p0 += AHEAD * blockDim.x) {
+        int e[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) e[i] = p0 + i * (int)blockDim.x < n_pairs ? idx[p0 + i * blockDim.x] : -1;
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            if (e[i] < 0) continue;
+            const int p = p0 + i * blockDim.x, place = atomicAdd(&count[e[i]], 1);
+            place_token[place] = p / top;
+            pair_place[p] = place;
+        }
     }
 }
 
@@ -613,7 +648,8 @@ QS_API int qs_moe_expert_down(float* out, long long ldo, const void* hidden, lon
 QS_API int qs_moe_sort(int32_t* offsets, int32_t* place_token, int32_t* pair_place, const int32_t* idx, int n_pairs,
                        int top, int E, cudaStream_t stream) {
     QS_REQUIRE(n_pairs > 0 && top > 0 && E > 0 && E <= MAX_EXPERTS, "moe_sort: bad sizes");
-    moe_sort_kernel<<<1, 1024, 0, stream>>>(offsets, place_token, pair_place, idx, n_pairs, top, E);
+    const cudaError_t e = qs_launch_dependent(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, offsets, place_token, pair_place, idx, n_pairs, top, E);
+    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "moe_sort: %s", cudaGetErrorString(e));
     return qs_check_launch("moe_sort");
 }
 

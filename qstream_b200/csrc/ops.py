@@ -107,7 +107,7 @@ _SIGNATURES = {
                             c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p], c_int),
     "qs_head_linear": ([c_void_p, c_int, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int,
                         c_int, c_int, c_void_p], c_int),
-    "qs_gemm_tc_grouped": ([c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
+    "qs_gemm_tc_grouped": ([c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     "qs_scan_activate": ([c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p], c_int),
     "qs_moe_route": ([c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                       c_int, c_float, c_int, c_int, c_int, c_float, c_void_p], c_int),
@@ -1089,16 +1089,20 @@ def expert_products(out, x, w_all, offsets) -> None:
     check(rc)
 
 
-def grouped_products(out, x, w_all, offsets) -> None:
+def grouped_products(out, x, w_all, offsets, glu=False) -> None:
     """`expert_products` with the rows' bounds on the device (int32 [>= experts + 1], the first experts + 1 count): one launch, for
-    bfloat16 operands that the tensor-core product takes.  Rows of no expert are left alone."""
+    bfloat16 operands that the tensor-core product takes.  Rows of no expert are left alone.  `glu`: a matrix's gate rows lie above as
+    many up rows, and out (half as wide) = silu(gate) * up, the unit on the 32-bit sums."""
     from . import gemm_tc
     E, N, K = w_all.shape
     rows, K2, lda = _rows(x)
+    if glu and N % 2:
+        raise QStreamError(QsError.INVALID_INPUT, "grouped_products: an odd number of gate and up rows")
+    N = N // 2 if glu else N
     if K2 != K or out.shape != (rows, N) or out.stride(1) != 1 or not w_all.is_contiguous() or offsets.numel() < E + 1:
         raise QStreamError(QsError.INVALID_INPUT, "grouped_products: operands do not fit")
     check(library().qs_gemm_tc_grouped(ptr(out), dtype_code(out), out.stride(0), ptr(x), lda, ptr(w_all), _int32(offsets, "offsets"), E, rows, N, K,
-                                       ptr(gemm_tc.status_word(x.device)), stream()))
+                                       int(bool(glu)), ptr(gemm_tc.status_word(x.device)), stream()))
 
 
 def moe_combine(y, pair_place, wts, tok_slot, add=None, add_scale=None, x=None, n_rows=None) -> torch.Tensor:

@@ -180,15 +180,19 @@ class RoutedExperts(FeedForward):
                 rows = rows[:bounds[-1]]                    # behind them lie the pairs whose expert returns its input
             products = ops.grouped_products if grouped else ops.expert_products
             bounds = offsets if grouped else bounds
-            hidden = torch.empty((rows.shape[0], self.w_up.shape[1]), dtype=h.dtype, device=h.device)
+            in_product = grouped and self.gated == "act" and s.activation == "silu"         # the gated unit in the product's epilogue
+            hidden = torch.empty((rows.shape[0], self.w_up.shape[1] // (2 if in_product else 1)), dtype=h.dtype, device=h.device)
             y = torch.empty((rows.shape[0], s.width), dtype=torch.float32, device=h.device)
-            products(hidden, rows, self.w_up, bounds)
-            if self.gated == "act":
-                hidden = ops.gated_act(hidden, s.activation)            # one launch for all experts' rows
-            elif self.gated:
-                hidden = ops.clamped_glu(hidden, *self.glu)
+            if in_product:
+                ops.grouped_products(hidden, rows, self.w_up, bounds, glu=True)
             else:
-                ops.activate(hidden, s.activation)
+                products(hidden, rows, self.w_up, bounds)
+                if self.gated == "act":
+                    hidden = ops.gated_act(hidden, s.activation)        # one launch for all experts' rows
+                elif self.gated:
+                    hidden = ops.clamped_glu(hidden, *self.glu)
+                else:
+                    ops.activate(hidden, s.activation)
             products(y, hidden, self.w_down, bounds)
             out = ops.moe_combine(y, pair_place, wts, b.tok_slot, shared, gate, x=h if self.outputs > s.n_experts else None,
                                   n_rows=offsets[s.n_experts:s.n_experts + 1] if grouped else None)
