@@ -18,6 +18,7 @@
 // heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 426 (the terms 108, the walk 133, the outputs 56).
 #include "scan.cuh"
 #include "scan_tiles.cuh"
+#include "term_tiles.cuh"
 
 namespace {
 
@@ -277,16 +278,16 @@ delta_terms_kernel(Delta p) {
 }
 
 __host__ __device__ inline int walk_stage(int dkp) { return CT * (dkp + 4) + CT * dkp; }       // W and K of a chunk
-inline int walk_stages(int dkp) { return dkp <= 128 ? 2 : 1; }
 inline size_t walk_smem(int dkp) {
-    return (size_t)(walk_stages(dkp) * walk_stage(dkp) + dkp * WC + CT * WC + (4 * CT * WC > dkp * WC ? 4 * CT * WC : dkp * WC)) * sizeof(float);
+    return (size_t)(walk_stage(dkp) + dkp * WC + CT * WC + (4 * CT * WC > dkp * WC ? 4 * CT * WC : dkp * WC)) * sizeof(float);
 }
 
+// The walk for more than 128 key channels, by multiply-adds.
 __global__ void __launch_bounds__(WALK)
-delta_walk_kernel(Delta p, int stages) {
+delta_walk_kernel(Delta p) {
     extern __shared__ __align__(16) float smem[];
     const int dkp = p.dkp, wp = dkp + 4;
-    float* sS = smem + stages * walk_stage(dkp);        // [dk][16]
+    float* sS = smem + walk_stage(dkp);                 // [dk][16]
     float* sU = sS + dkp * WC;                          // [64][16]
     float* red = sU + CT * WC;                          // [4 parts][64][16], [dk][16]
     grid_dep_launch();
@@ -300,11 +301,11 @@ delta_walk_kernel(Delta p, int stages) {
         const int col = e / dkp, i = e - col * dkp;
         sS[i * WC + col] = col < n_cols && i < p.dk ? own[(size_t)col * p.dk + i] : 0.f;
     }
-    auto fetch = [&](int c, int stage) {
+    auto fetch = [&](int c) {
         const int n = p.chunk_start[c + 1] - p.chunk_start[c];
         if (n <= 0 || n > CT) return;
         const size_t unit = (size_t)c * p.H + h;
-        float* w = smem + stage * walk_stage(dkp);
+        float* w = smem;
         float* k = w + CT * wp;
         const int fours = dkp / 4;
         for (int e = tid; e < CT * fours; e += WALK) {
@@ -313,15 +314,14 @@ delta_walk_kernel(Delta p, int stages) {
             copy16(k + t * dkp + i, p.K + (unit * CT + t) * dkp + i, true);
         }
     };
-    fetch(c0, 0);
+    fetch(c0);
     for (int c = c0; c < c1; ++c) {
         const size_t unit = (size_t)c * p.H + h;
-        const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, stage = stages == 2 ? (c - c0) & 1 : 0;
-        const float* w = smem + stage * walk_stage(dkp);
+        const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0;
+        const float* w = smem;
         const float* k = w + CT * wp;
         copies_done();
         __syncthreads();
-        if (stages == 2 && c + 1 < c1) fetch(c + 1, stage ^ 1);
         if (n <= 0 || n > CT) {                         // token by token: sixteen threads share a column
             const int col = tid >> 4, part = tid & 15, hq = h / p.group;
             for (int t = t0; t < t0 + n; ++t) {
@@ -345,7 +345,7 @@ delta_walk_kernel(Delta p, int stages) {
                 if (part == 0 && col < n_cols) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col0 + col] = o;
             }
             __syncthreads();
-            if (stages == 1 && c + 1 < c1) fetch(c + 1, 0);
+            if (c + 1 < c1) fetch(c + 1);
             continue;
         }
         const int row = tid >> 2, quad = (tid & 3) * 4;  // this thread's four columns of a token's u
@@ -434,10 +434,8 @@ delta_walk_kernel(Delta p, int stages) {
                 }
             }
         }
-        if (stages == 1) {
-            __syncthreads();
-            if (c + 1 < c1) fetch(c + 1, 0);
-        }
+        __syncthreads();
+        if (c + 1 < c1) fetch(c + 1);
     }
     __syncthreads();
     for (int e = tid; e < p.dk * WC; e += WALK) {
@@ -446,99 +444,348 @@ delta_walk_kernel(Delta p, int stages) {
     }
 }
 
-constexpr int OS = 32;                                  // key channels of a slice of the outputs' kernel
-template <int NC>
-constexpr int output_floats() {
-    const int stage = OS * CT + 2 * OS * 64 * NC, values = CT * 64 * NC;
-    return (stage > values ? stage : values) + CT * PP;
+// The walk for up to 128 key channels, on the tensor cores (mma.sync, three bfloat16 terms per number, terms.cuh): a block holds 16 value columns of
+// one head's state, each of its eight warps 16 channels of it in registers; the state's terms, u's and those of W and K lie in shared memory.
+//   1  W S: a warp takes 16 tokens and half of the channels; the halves meet in shared memory, u = U - W S, as terms
+//   2  S <- decay S + K^T u: a warp's 16 channels over all 64 tokens; the state's terms
+// W of the next chunk becomes terms while u is formed, K behind the second step; the one after that is on its way in registers.
+//
+// A chain of 32 steps for 2,000 tokens.  By multiply-adds a step took 4.2 us (shared memory's pipe: eight 16-byte reads per 32 paired
+// multiply-adds), 133 us in all.
+// MC channels, 64 or 128; pitches of W and K, of S and u: rows of 16 bytes meet all banks
+constexpr int SP = WC + 8;
+template <int MC> constexpr int mma_walk_smem() { return (2 * 3 * CT * (MC + 8) + 3 * MC * SP + 3 * CT * SP) * 2 + CT * WC * 4; }
+
+__device__ __forceinline__ void put_four(__nv_bfloat16* at, int term, float4 f) {
+    uint32_t a[3], b[3];
+    terms_of(pack2(f.x, f.y), a[0], a[1], a[2]);
+    terms_of(pack2(f.z, f.w), b[0], b[1], b[2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(at + i * term) = make_uint2(a[i], b[i]);
+}
+__device__ __forceinline__ void put_two(__nv_bfloat16* at, int term, float x, float y) {
+    uint32_t a[3];
+    terms_of(pack2(x, y), a[0], a[1], a[2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(at + i * term) = a[i];
 }
 
-template <int NC>
-__global__ void __launch_bounds__(THREADS, 3)
-delta_output_kernel(Delta p) {
-    constexpr int COLS = 64 * NC, FOURS = OS / 4, NQ = CT * FOURS / THREADS, NV = CT * 16 * NC / THREADS;
+template <int MC>
+__global__ void __launch_bounds__(2 * MC)
+delta_walk_mma_kernel(const __grid_constant__ Delta p) {
+    constexpr int MP = MC + 8, WALKERS = 2 * MC, ROW = MC / 4, PARTS = MC / 64;
     extern __shared__ __align__(16) float smem[];
-    float* sq = smem;                                   // [OS][64 tokens]
-    float* ss = sq + OS * CT;                           // two slices [OS][COLS] of the state in turn
-    float* svv = smem;                                  // [64 tokens][COLS], after the last slice
-    float* sp = smem + output_floats<NC>() - CT * PP;   // [64 j][PP]
+    __nv_bfloat16* const tw = reinterpret_cast<__nv_bfloat16*>(smem);      // [3][64 tokens][MP]
+    __nv_bfloat16* const tk = tw + 3 * CT * MP;
+    __nv_bfloat16* const ts = tk + 3 * CT * MP;         // [3][MC channels][SP]
+    __nv_bfloat16* const tu = ts + 3 * MC * SP;         // [3][64 tokens][SP]
+    float* const red = reinterpret_cast<float*>(tu + 3 * CT * SP);         // [64][16]
     grid_dep_launch();
     grid_dep_wait();
-    const int c = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, nv = min(COLS, p.dv - col0);
-    if (c == 0)                                         // rows behind the last sequence belong to nobody: a defined value
-        for (int r = p.chunk_start[p.n_chunks]; r < p.T_rows; ++r)
-            for (int e = tid; e < nv; e += THREADS) p.o[(size_t)r * p.ldo + (size_t)h * p.dv + col0 + e] = 0.f;
-    if (n <= 0 || n > CT) return;
-    const size_t unit = (size_t)c * p.H + h;
-    Raw4<float> rq[NQ];
-    auto token_of = [&](int e) { return (e >> 5) * 4 + ((e & 31) >> 3); };
-    auto fetch = [&](int i0, float* dst) {
+    const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * WC, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+    const int slot = p.seq_slot[s], c0 = p.seq_chunk[s], c1 = p.seq_chunk[s + 1], dkp = p.dkp;
+    if (slot < 0 || c1 <= c0) return;
+    const int n_cols = min(WC, p.dv - col0);
+    float* own = p.state + (size_t)slot * p.slot_stride + ((size_t)h * p.dv + col0) * p.dk;
+    // the warp's channels warp 16 + g and + 8, columns 8 y + q2 and + 1
+    float S[2][2][2];
+    auto each = [&](auto f) {
 #pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            const int e = tid + x * THREADS;
-            get_four(rq[x], p.Q + (unit * CT + token_of(e)) * p.dkp + i0, (e & 7) * 4, p.dkp - i0, true, 1);
-        }
-#pragma unroll 4
-        for (int e = tid; e < OS * 16 * NC; e += THREADS) {
-            const int i = e / (16 * NC), col = (e % (16 * NC)) * 4;
-            copy16(dst + e * 4, p.start + (unit * p.dk + i0 + i) * p.dvp + col0 + col, i0 + i < p.dk && col < nv);
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                for (int z = 0; z < 2; ++z) f(S[x][y][z], warp * 16 + 8 * x + g, 8 * y + q2 + z);
+    };
+    auto put_state = [&]() {
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) put_two(ts + (warp * 16 + 8 * x + g) * SP + 8 * y + q2, MC * SP, S[x][y][0], S[x][y][1]);
+    };
+    each([&](float& v, int i, int col) { v = i < p.dk && col < n_cols ? own[(size_t)col * p.dk + i] : 0.f; });
+    put_state();
+    constexpr int PIECES = CT * MC / 4 / WALKERS;         // of four channels, of a thread
+    float4 rw[PIECES], rk[PIECES];
+    auto fetch = [&](float4 (&r)[PIECES], const float* from, int c) {
+        const int n = c < c1 ? p.chunk_start[c + 1] - p.chunk_start[c] : 0;
+        const float* base = from + ((size_t)c * p.H + h) * CT * dkp;
+#pragma unroll
+        for (int x = 0; x < PIECES; ++x) {
+            const int e = tid + x * WALKERS, t = e / ROW, i = e % ROW * 4;
+            r[x] = n > 0 && n <= CT && i < dkp ? *reinterpret_cast<const float4*>(base + (size_t)t * dkp + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
-    fetch(0, ss);
-    for (int e = tid; e < CT * 16; e += THREADS)
-        *reinterpret_cast<float4*>(sp + (e >> 4) * PP + (e & 15) * 4) = *reinterpret_cast<const float4*>(p.B + unit * CT * CT + e * 4);
-    f32x2 acc[8][2 * NC];
+    auto put = [&](__nv_bfloat16* to, const float4 (&r)[PIECES]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int x = 0; x < PIECES; ++x) {
+            const int e = tid + x * WALKERS;
+            put_four(to + e / ROW * MP + e % ROW * 4, CT * MP, r[x]);
+        }
+    };
+    fetch(rw, p.W, c0);
+    fetch(rk, p.K, c0);
+    put(tw, rw);
+    put(tk, rk);
+    fetch(rw, p.W, c0 + 1);
+    fetch(rk, p.K, c0 + 1);
+    const uint32_t aw = (uint32_t)__cvta_generic_to_shared(tw), ak = (uint32_t)__cvta_generic_to_shared(tk);
+    const uint32_t as = (uint32_t)__cvta_generic_to_shared(ts), au = (uint32_t)__cvta_generic_to_shared(tu);
+    __syncthreads();
+    for (int c = c0; c < c1; ++c) {
+        const size_t unit = (size_t)c * p.H + h;
+        const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0;
+        if (n <= 0 || n > CT) {                         // token by token on the state in 32-bit, over u's and the state's terms: sixteen threads share a column
+            float* sS = reinterpret_cast<float*>(ts);   // [MC][17]
+            each([&](float& v, int i, int col) { if (i < p.dk) sS[i * 17 + col] = v; });
+            __syncthreads();
+            const int hq = h / p.group, part = tid & 15;
+            for (int col = tid >> 4; col < WC; col += WALKERS / 16)
+            for (int t = t0; t < t0 + n; ++t) {
+                const float* kr = p.k + (size_t)t * p.ldk + hq * p.dk;
+                const float* qr = p.q + (size_t)t * p.ldq + hq * p.dk;
+                const float* gr = p.g + (size_t)t * p.ldg + h * p.dk;
+                float held = 0.f, o = 0.f;
+                for (int i = part; i < p.dk; i += 16) {
+                    sS[i * 17 + col] *= gr[i];
+                    held = fmaf(sS[i * 17 + col], kr[i], held);
+                }
+                for (int x = 8; x > 0; x >>= 1) held += __shfl_xor_sync(0xffffffffu, held, x);
+                const float v = col < n_cols ? p.v[(size_t)t * p.ldv + (size_t)h * p.dv + col0 + col] : 0.f;
+                const float u = p.beta[(size_t)t * p.ldb + h] * (v - held);
+                for (int i = part; i < p.dk; i += 16) {
+                    const float now = fmaf(kr[i], u, sS[i * 17 + col]);
+                    sS[i * 17 + col] = now;
+                    o = fmaf(now, qr[i], o);
+                }
+                for (int x = 8; x > 0; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+                if (part == 0 && col < n_cols) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col0 + col] = o;
+            }
+            __syncthreads();
+            each([&](float& v, int i, int at) { v = i < p.dk ? sS[i * 17 + at] : 0.f; });
+            __syncthreads();
+            put_state();
+            put(tw, rw);
+            put(tk, rk);
+            fetch(rw, p.W, c + 2);
+            fetch(rk, p.K, c + 2);
+            __syncthreads();
+            continue;
+        }
+        // 1
+        const int tile = warp & 3, part = warp >> 2;
+        float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, u[2][2][2];
+        if (part == 0)                                  // what the tokens write from nothing
 #pragma unroll
-        for (int j = 0; j < 2 * NC; ++j) acc[i][j] = 0ull;
-    for (int i0 = 0; i0 < p.dk; i0 += OS) {
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {
+                    const float2 two = 8 * z + q2 < n_cols ? *reinterpret_cast<const float2*>(p.U + (unit * CT + tile * 16 + 8 * x + g) * p.dvp + col0 + 8 * z + q2)
+                                                           : make_float2(0.f, 0.f);
+                    u[x][z][0] = two.x;
+                    u[x][z][1] = two.y;
+                }
+        float d[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int i = warp * 16 + 8 * x + g;
+            d[x] = i < dkp ? p.decay[unit * dkp + i] : 0.f;
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)                     // the state this chunk starts from
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+                const int i = warp * 16 + 8 * x + g, col = 8 * z + q2;
+                if (i < p.dk && col < n_cols) *reinterpret_cast<float2*>(p.start + (unit * p.dk + i) * p.dvp + col0 + col) = make_float2(S[x][z][0], S[x][z][1]);
+            }
+#pragma unroll
+        for (int i = part * 64; i < part * 64 + 64; i += 16) {
+            uint32_t a[3][4], b[3][4];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                load_matrices(a[x], aw + x * CT * MP * 2 + rows_first(tile * 16, i, MP, lane));
+                load_matrices_turned(b[x], as + x * MC * SP * 2 + rows_first(i, 0, SP, lane));
+            }
+            add_product<3, 3>(y[0], a, b, 0);
+            add_product<3, 3>(y[1], a, b, 1);
+        }
+        if (PARTS > 1 && part)
+#pragma unroll
+            for (int z = 0; z < 2; ++z)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(red + (tile * 16 + 8 * x + g) * WC + 8 * z + q2) = make_float2(y[z][2 * x], y[z][2 * x + 1]);
         __syncthreads();
+        if (part == 0)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {
+                    const int t = tile * 16 + 8 * x + g, col = 8 * z + q2;
+                    const float2 more = PARTS > 1 ? *reinterpret_cast<const float2*>(red + t * WC + col) : make_float2(0.f, 0.f);
+                    const float2 v = make_float2(u[x][z][0] - (y[z][2 * x] + more.x), u[x][z][1] - (y[z][2 * x + 1] + more.y));
+                    put_two(tu + t * SP + col, CT * SP, v.x, v.y);
+                    if (col < n_cols) *reinterpret_cast<float2*>(p.U + (unit * CT + t) * p.dvp + col0 + col) = v;
+                }
+        put(tw, rw);
+        fetch(rw, p.W, c + 2);
+        __syncthreads();
+        // 2
+        float more[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int t = 0; t < CT; t += 16) {
+            uint32_t a[3][4], b[3][4];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                load_matrices_turned(a[x], ak + x * CT * MP * 2 + columns_first(t, warp * 16, MP, lane));
+                load_matrices_turned(b[x], au + x * CT * SP * 2 + rows_first(t, 0, SP, lane));
+            }
+            add_product<3, 3>(more[0], a, b, 0);
+            add_product<3, 3>(more[1], a, b, 1);
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int z = 0; z < 2; ++z)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) S[x][z][e] = fmaf(d[x], S[x][z][e], more[z][2 * x + e]);
+        put_state();
+        __syncthreads();
+        put(tk, rk);
+        fetch(rk, p.K, c + 2);
+    }
+    each([&](float& v, int i, int col) { if (i < p.dk && col < n_cols) own[(size_t)col * p.dk + i] = v; });
+}
+
+// The outputs on tcgen05, three terms per number: a block takes a chunk's 64 tokens and 128 value columns (on the TMEM lanes, so that a warp stores 32
+// neighbouring ones).  Slices of 64 channels are runs in the unit, summed up in registers; then the weights against u.
+constexpr int OUT_THREADS = 256, OUT_SMEM = 1024 + 9 * TILE;
+// MANY: more than 128 channels, more than two runs.
+template <bool MANY>
+__global__ void __launch_bounds__(OUT_THREADS, 2)
+delta_output_kernel(const __grid_constant__ Delta p, int32_t* __restrict__ status) {
+    constexpr int NQ = CT * 16 / OUT_THREADS, NS = 2 * NQ;
+    constexpr uint32_t TMEM = 128;                      // two runs' sums [128 columns][64 tokens]
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t done;
+    __shared__ uint32_t tmem_slot;
+    const int c = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * 128, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
+    if (tid == 0) { mbar_init(&done, 1); mbar_fence_init(); }
+    if (warp == 0) { tmem_alloc(&tmem_slot, TMEM); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem = tmem_slot, own = tmem + ((uint32_t)(quad * 32) << 16) + half * 32;
+    const uint32_t tq = (smem_u32(smem_raw) + 1023) & ~1023u, ts = tq + 3 * TILE;       // [3][tokens], [3][2 halves of the columns][channels]
+    const uint32_t tb = tq, tu = tb + 3 * TILE;         // after the slices: the weights [3][earlier tokens], u [3][2][tokens]
+    const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, nv = min(128, p.dv - col0);
+    const size_t unit = (size_t)c * p.H + h;
+    auto leave = [&]() {
+        tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(tmem, TMEM);
+    };
+    if (c == 0)                                         // rows behind the last sequence belong to nobody: a defined value
+        for (int r = p.chunk_start[p.n_chunks]; r < p.T_rows; ++r)
+            for (int e = tid; e < nv; e += OUT_THREADS) p.o[(size_t)r * p.ldo + (size_t)h * p.dv + col0 + e] = 0.f;
+    if (n <= 0 || n > CT) { leave(); return; }
+    const int slices = (p.dk + 63) / 64;
+    float out[32];
+    bool ok = true;
+    for (int s = 0; s < slices; ++s) {
+        const int i0 = s * 64;
+        float4 rq[NQ], rs[NS];
 #pragma unroll
         for (int x = 0; x < NQ; ++x) {
-            const int e = tid + x * THREADS, t = token_of(e), i = (e & 7) * 4;
-            const float4 a = rq[x].value();
-            sq[at_ct(i, t)] = a.x; sq[at_ct(i + 1, t)] = a.y; sq[at_ct(i + 2, t)] = a.z; sq[at_ct(i + 3, t)] = a.w;
+            const int e = tid + x * OUT_THREADS, i = i0 + (e & 15) * 4;
+            rq[x] = i < p.dkp ? *reinterpret_cast<const float4*>(p.Q + (unit * CT + (e >> 4)) * p.dkp + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        copies_done();
+#pragma unroll
+        for (int x = 0; x < NS; ++x) {
+            const int e = tid + x * OUT_THREADS, i = i0 + (e >> 5), col = col0 + (e & 31) * 4;
+            rs[x] = i < p.dk && col < p.dvp ? *reinterpret_cast<const float4*>(p.start + (unit * p.dk + i) * p.dvp + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (s && ok) ok = wait_done(&done, (s - 1) & 1, status);
+        if (MANY && s >= 2) {
+            tc_fence_after_sync();
+            take_sums<32>(out, own + (s & 1) * 64, s == 2);
+        }
+#pragma unroll
+        for (int x = 0; x < NQ; ++x) {
+            const int e = tid + x * OUT_THREADS;
+            put_terms<3>(tq + place_in_tile(e >> 4, (e & 15) * 4), TILE, rq[x]);
+        }
+#pragma unroll
+        for (int x = 0; x < NS; ++x) {
+            const int e = tid + x * OUT_THREADS, col = (e & 31) * 4;
+            put_terms<3>(ts + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), 2 * TILE, rs[x]);
+        }
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
         __syncthreads();
-        const float* now = ss + (i0 / OS & 1) * OS * COLS;
-        if (i0 + OS < p.dk) fetch(i0 + OS, ss + ((i0 / OS + 1) & 1) * OS * COLS);
-        tile_product<NC, true>(acc, sq, now, OS, ty, tx);
-    }
-    Raw4<float> rv[NV];
-#pragma unroll
-    for (int x = 0; x < NV; ++x) {
-        const int e = tid + x * THREADS, j = e / (16 * NC), col = (e % (16 * NC)) * 4;
-        get_four(rv[x], p.U + (unit * CT + j) * p.dvp + col0, col, (nv + 3) / 4 * 4, j < n, 1);
-    }
-    __syncthreads();
-    bool odd = false;                                   // a value that is not finite must not meet the weights of zero of earlier tokens
-#pragma unroll
-    for (int x = 0; x < NV; ++x) {
-        const float4 f = rv[x].value();
-        odd |= !(fabsf(f.x) <= 3.402823466e38f && fabsf(f.y) <= 3.402823466e38f && fabsf(f.z) <= 3.402823466e38f && fabsf(f.w) <= 3.402823466e38f);
-        *reinterpret_cast<float4*>(svv + (tid + x * THREADS) * 4) = f;
-    }
-    odd = __syncthreads_or(odd);
-    if (odd) add_values<NC, 1, true>(acc, sp, svv, n, ty, tx);
-    else add_values<NC, 1, false>(acc, sp, svv, n, ty, tx);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = (i >> 2) * 32 + ty * 4 + (i & 3);
-        if (t >= n) continue;
-#pragma unroll
-        for (int g = 0; g < NC; ++g) {
-            const int own = g * 64 + tx * 4;
-            float* dst = p.o + (size_t)(t0 + t) * p.ldo + (size_t)h * p.dv + col0 + own;
-            const float2 a = unpack2(acc[i][2 * g]), b = unpack2(acc[i][2 * g + 1]);
-            if (own < nv) dst[0] = a.x;
-            if (own + 1 < nv) dst[1] = a.y;
-            if (own + 2 < nv) dst[2] = b.x;
-            if (own + 3 < nv) dst[3] = b.y;
+        if (warp == 0 && elect_one()) {
+            tc_fence_after_sync();
+            multiply_tiles<3, 3, true, false>(tmem + (s & 1) * 64, ts, 2 * TILE, tq, TILE, CT);       // S0^T Q
+            mma_commit(&done);
         }
+        __syncwarp();
     }
+    float4 rb[NQ], ru[NS];
+#pragma unroll
+    for (int x = 0; x < NQ; ++x) rb[x] = *reinterpret_cast<const float4*>(p.B + unit * CT * CT + (tid + x * OUT_THREADS) * 4);
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+        const int e = tid + x * OUT_THREADS, j = e >> 5, col = col0 + (e & 31) * 4;
+        ru[x] = j < n && col < p.dvp ? *reinterpret_cast<const float4*>(p.U + (unit * CT + j) * p.dvp + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (ok) ok = wait_done(&done, (slices - 1) & 1, status);
+    tc_fence_after_sync();
+#pragma unroll
+    for (int x = 0; x < NQ; ++x) {
+        const int e = tid + x * OUT_THREADS;
+        put_terms<3>(tb + place_in_tile(e >> 4, (e & 15) * 4), TILE, rb[x]);
+    }
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+        const int e = tid + x * OUT_THREADS, col = (e & 31) * 4;
+        put_terms<3>(tu + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), 2 * TILE, ru[x]);
+    }
+    const int older = slices & 1, newer = older ^ 1;
+    if (slices > 1) take_sums<32>(out, own + older * 64, slices == 2);
+    take_sums<32>(out, own + newer * 64, slices == 1);
+    fence_proxy_async_smem();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 0 && elect_one()) {
+        tc_fence_after_sync();
+        multiply_tiles<3, 3, true, true>(tmem, tu, 2 * TILE, tb, TILE, CT);       // u^T B
+        mma_commit(&done);
+    }
+    __syncwarp();
+    if (ok) ok = wait_done(&done, slices & 1, status);
+    tc_fence_after_sync();
+    take_sums<32>(out, own, false);
+    const int in = quad * 32 + lane, rows = n - half * 32;
+    if (in < nv) {
+        float* o = p.o + (size_t)t0 * p.ldo + (size_t)h * p.dv + col0 + in;
+        bool odd = false;
+#pragma unroll
+        for (int x = 0; x < 32; ++x) {
+            odd |= !is_number(out[x]);
+            if (x < rows) o[(size_t)(half * 32 + x) * p.ldo] = out[x];
+        }
+        if (odd)                                        // by multiply-adds, where the terms gave no number: a later token's u meets no earlier one
+            for (int t = half * 32; t < min(n, half * 32 + 32); ++t) {
+                float v = o[(size_t)t * p.ldo];
+                if (is_number(v)) continue;
+                v = 0.f;
+                for (int i = 0; i < p.dk && v == v; ++i) v = fmaf(p.Q[(unit * CT + t) * p.dkp + i], p.start[(unit * p.dk + i) * p.dvp + col0 + in], v);
+                for (int j = 0; j <= t && v == v; ++j) v = fmaf(p.B[unit * CT * CT + j * CT + t], p.U[(unit * CT + j) * p.dvp + col0 + in], v);
+                o[(size_t)t * p.ldo] = v;
+            }
+    }
+    leave();
 }
 
 }  // namespace
@@ -553,7 +800,7 @@ QS_API long long qs_delta_chunks_scratch(int n_chunks, int H, int dk, int dv) {
 QS_API int qs_delta_chunks(float* o, long long ldo, const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, const float* g,
                            long long ldg, const float* beta, long long ldb, float* state, long long slot_stride, const int32_t* seq_slot, int n_seq, int T_rows,
                            int H, int group, int dk, int dv, const int32_t* chunk_start, int n_chunks, const int32_t* seq_chunk, float* scratch,
-                           cudaStream_t stream) {
+                           int32_t* status, cudaStream_t stream) {
     if (n_seq == 0 || T_rows == 0) return QS_OK;
     QS_REQUIRE(n_seq > 0 && T_rows > 0 && H > 0 && dk > 0 && dv > 0 && n_chunks > 0 && group > 0 && H % group == 0, "delta_chunks: bad sizes");
     QS_REQUIRE(dk <= 256 && H <= 65535 && (dv + WC - 1) / WC <= 65535, "delta_chunks: %d key channels per head above 256", dk);
@@ -574,16 +821,20 @@ QS_API int qs_delta_chunks(float* o, long long ldo, const float* q, long long ld
     p.start = p.decay + units * p.dkp;
     cudaError_t e = cudaFuncSetAttribute(delta_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TERMS_SMEM);
     if (e == cudaSuccess) e = qs_launch_dependent(delta_terms_kernel, dim3(n_chunks, H), dim3(TERMS), TERMS_SMEM, stream, p);
-    const size_t walk = walk_smem(p.dkp);
-    // the most any head takes (two stages of 128 channels or one of 256), so that threads with models of other sizes set the same
-    const size_t most = walk_smem(256) > walk_smem(128) ? walk_smem(256) : walk_smem(128);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (e == cudaSuccess) e = qs_launch_dependent(delta_walk_kernel, dim3(n_seq, H, (dv + WC - 1) / WC), dim3(WALK), walk, stream, p, walk_stages(p.dkp));
-#define GO(NC) do { const size_t smem = output_floats<NC>() * sizeof(float); \
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_output_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (e == cudaSuccess) e = qs_launch_dependent(delta_output_kernel<NC>, dim3(n_chunks, H, (dv + 64 * NC - 1) / (64 * NC)), dim3(THREADS), smem, stream, p); } while (0)
-    if (dv > 64) GO(2); else GO(1);
-#undef GO
+    const dim3 blocks(n_seq, H, (dv + WC - 1) / WC);
+    if (p.dkp <= 64) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_walk_smem<64>());
+        if (e == cudaSuccess) e = qs_launch_dependent(delta_walk_mma_kernel<64>, blocks, dim3(128), mma_walk_smem<64>(), stream, p);
+    } else if (p.dkp <= 128) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_walk_smem<128>());
+        if (e == cudaSuccess) e = qs_launch_dependent(delta_walk_mma_kernel<128>, blocks, dim3(256), mma_walk_smem<128>(), stream, p);
+    } else {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem(256));
+        if (e == cudaSuccess) e = qs_launch_dependent(delta_walk_kernel, blocks, dim3(WALK), walk_smem(p.dkp), stream, p);
+    }
+    const auto output = dk > 128 ? delta_output_kernel<true> : delta_output_kernel<false>;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(output, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_SMEM);
+    if (e == cudaSuccess) e = qs_launch_dependent(output, dim3(n_chunks, H, (dv + 127) / 128), dim3(OUT_THREADS), OUT_SMEM, stream, p, status);
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "delta_chunks: %s", cudaGetErrorString(e));
     return qs_check_launch("delta_chunks");
 }

@@ -66,8 +66,8 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 constexpr int P_EPILOGUE_WARPS = 8, P_THREADS = 64 + 32 * P_EPILOGUE_WARPS;
 constexpr int STAGE_PITCH = 36;                     // floats: rows of 16 bytes meet all banks
 constexpr int STAGING = P_EPILOGUE_WARPS * 32 * STAGE_PITCH * 4;
-template <int BN> constexpr int p_stages() { return (SMEM_BUDGET_BIG - STAGING) / stage_bytes<BN>(); }
-template <int BN> constexpr int p_smem_bytes() { return p_stages<BN>() * stage_bytes<BN>() + 1024 + 512 + STAGING; }
+template <int BN, bool WIDE> constexpr int p_stages() { return (SMEM_BUDGET_BIG - (WIDE ? STAGING : 0)) / stage_bytes<BN>(); }
+template <int BN, bool WIDE> constexpr int p_smem_bytes() { return p_stages<BN, WIDE>() * stage_bytes<BN>() + 1024 + 512 + (WIDE ? STAGING : 0); }
 
 // One CTA per SM walks over output tiles of 128 x BN (tile t = n_tile * m_tiles + m_tile, so CTAs that
 // run together share rows of W and all of A stays in L2).  Two accumulators in TMEM: while the four
@@ -89,14 +89,14 @@ template <int BN> constexpr int p_smem_bytes() { return p_stages<BN>() * stage_b
 // every product slower); together, with the unit in the first product (14 us of its own before), and the kernel as a programmatic dependent, 3,000
 // tokens through 4 of 16 experts of 2048 x 512 take 167 us instead of 193.
 constexpr int MAX_GROUPS = 1024;
-template <int BN, bool GROUPED, bool GLU>
+template <int BN, bool GROUPED, bool GLU, bool WIDE>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                           const Epilogue ep, const int K, const int m_tiles, const int n_tiles,
                           int32_t* __restrict__ status, const int32_t* __restrict__ offsets, const int n_groups) {
     static_assert(GROUPED || !GLU, "the gated unit belongs to the grouped form");
     constexpr int WIDTH = GLU ? BN / 2 : BN;          // columns of C of a tile
-    constexpr int STAGES = p_stages<BN>();
+    constexpr int STAGES = p_stages<BN, WIDE>();
     constexpr int STAGE = stage_bytes<BN>();
     constexpr uint32_t TMEM_COLS = 2 * BN;
 
@@ -206,7 +206,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                             (!ep.res1 || ((ep.ldr % 8) == 0 && ((uintptr_t)ep.res1 % 16) == 0)) &&
                             (!ep.res2 || ((uintptr_t)ep.res2 % 16) == 0);
         const bool bias_vec = ep.bias && ((uintptr_t)ep.bias % 32) == 0;
-        const bool plain = vec_ok && !ep.bias && !ep.res1 && !ep.res2 && ep.act == QS_ACT_NONE;
+        const bool plain = WIDE && vec_ok && !ep.bias && !ep.res1 && !ep.res2 && ep.act == QS_ACT_NONE;
         float* const stage = reinterpret_cast<float*>(smem + STAGES * STAGE + 512) + (warp - 2) * 32 * STAGE_PITCH;
         int i = 0, group = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++i) {
@@ -229,7 +229,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 } else tmem_load_wait();
                 const int nc = n0 + c * 32;
                 if (nc >= ep.N) continue;
-                if (wide && plain && nc + 32 <= ep.N) {
+                if (WIDE && plain && nc + 32 <= ep.N) {
                     // sums as they are, 32-bit: through shared memory, whole lines of four rows to a store
 #pragma unroll
                     for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(stage + lane * STAGE_PITCH + g * 4) = make_uint4(raw[4 * g], raw[4 * g + 1], raw[4 * g + 2], raw[4 * g + 3]);
@@ -1171,14 +1171,15 @@ int launch_pair(const CUtensorMap& ma, const void* W, long long ldw, const Epilo
 }
 
 // offsets null: one product of M rows.  Else `n_groups` products whose rows the device finds in `offsets` (M: all rows together).
-template <int BN, bool GROUPED, bool GLU>
-int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilogue& ep, int M, int N, int K,
+// WIDE: results of 32 bits, whose way through shared memory takes a stage of the ring.
+template <int BN, bool GROUPED, bool GLU, bool WIDE>
+int launch_persistent_as(const CUtensorMap& ma, const CUtensorMap& mw, const Epilogue& ep, int M, int N, int K,
                       int32_t* status, const int32_t* offsets, int n_groups, cudaStream_t stream) {
     static bool configured = false;
     static int sm_count = 0;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, GROUPED, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             p_smem_bytes<BN>());
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, GROUPED, GLU, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             p_smem_bytes<BN, WIDE>());
         int dev = 0;
         if (e == cudaSuccess) e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
@@ -1190,10 +1191,16 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilog
     const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + width - 1) / width;
     const long long total = (long long)(m_tiles + (GROUPED ? n_groups : 0)) * n_tiles;     // groups: at most a tile row more each
     const int grid = (int)(total < sm_count ? total : sm_count);
-    const cudaError_t e = qs_launch_dependent(gemm_tc_persistent_kernel<BN, GROUPED, GLU>, dim3(grid), dim3(P_THREADS), p_smem_bytes<BN>(), stream, ma, mw, ep, K,
+    const cudaError_t e = qs_launch_dependent(gemm_tc_persistent_kernel<BN, GROUPED, GLU, WIDE>, dim3(grid), dim3(P_THREADS), p_smem_bytes<BN, WIDE>(), stream, ma, mw, ep, K,
                                               m_tiles, n_tiles, status, offsets, n_groups);
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "gemm_tc persistent: %s", cudaGetErrorString(e));
     return qs_check_launch("gemm_tc persistent");
+}
+template <int BN, bool GROUPED, bool GLU>
+int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, const Epilogue& ep, int M, int N, int K,
+                      int32_t* status, const int32_t* offsets, int n_groups, cudaStream_t stream) {
+    return ep.c_dtype == QS_F32 ? launch_persistent_as<BN, GROUPED, GLU, true>(ma, mw, ep, M, N, K, status, offsets, n_groups, stream)
+                                : launch_persistent_as<BN, GROUPED, GLU, false>(ma, mw, ep, M, N, K, status, offsets, n_groups, stream);
 }
 
 }  // namespace

@@ -77,7 +77,7 @@ _SIGNATURES = {
                        c_void_p, c_void_p, c_longlong, c_float, c_int, c_float, c_void_p, c_void_p], c_int),
     "qs_delta_chunks_scratch": ([c_int, c_int, c_int, c_int], c_longlong),
     "qs_delta_chunks": ([c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
-                         c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p], c_int),
+                         c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p], c_int),
     "qs_mlstm_gates": ([c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_float, c_void_p, c_longlong,
                         c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     "qs_mlstm_output": ([c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int,
@@ -681,6 +681,7 @@ def _activated(q, k, v, activation):
 def _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_dim, key_decay, token_weight, qk_group, chunks):
     """The delta rule of a long prompt, its chunks as matrix products (csrc/delta_chunks.cu): what each chunk's tokens ask of the
     state it starts from and what they write, side by side; the chunks' states in order; the outputs, side by side."""
+    from . import gemm_tc
     chunk_start, chunk_ids, seq_chunk, n_chunks = chunks
     T = q.shape[0]
     if any(t.dtype != torch.float32 or t.stride(1) != 1 for t in (key_decay, token_weight)):
@@ -695,7 +696,7 @@ def _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_di
     check(lib.qs_delta_chunks(ptr(o), o.stride(0), ptr(q), q.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), ptr(key_decay), key_decay.stride(0),
                               ptr(token_weight), token_weight.stride(0), ptr(state), state.stride(0), _int32(seq_slot, "seq_slot"), int(n_seq), T,
                               n_heads, int(qk_group), key_dim, value_dim, _int32(chunk_start, "chunk_start"), int(n_chunks),
-                              _int32(seq_chunk, "seq_chunk"), ptr(scratch), stream()))
+                              _int32(seq_chunk, "seq_chunk"), ptr(scratch), ptr(gemm_tc.status_word(q.device)), stream()))
     count_launches(2)
     return o
 
