@@ -541,26 +541,26 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
             __syncthreads();
             const int hq = h / p.group, part = tid & 15;
             for (int col = tid >> 4; col < WC; col += WALKERS / 16)
-            for (int t = t0; t < t0 + n; ++t) {
-                const float* kr = p.k + (size_t)t * p.ldk + hq * p.dk;
-                const float* qr = p.q + (size_t)t * p.ldq + hq * p.dk;
-                const float* gr = p.g + (size_t)t * p.ldg + h * p.dk;
-                float held = 0.f, o = 0.f;
-                for (int i = part; i < p.dk; i += 16) {
-                    sS[i * 17 + col] *= gr[i];
-                    held = fmaf(sS[i * 17 + col], kr[i], held);
+                for (int t = t0; t < t0 + n; ++t) {
+                    const float* kr = p.k + (size_t)t * p.ldk + hq * p.dk;
+                    const float* qr = p.q + (size_t)t * p.ldq + hq * p.dk;
+                    const float* gr = p.g + (size_t)t * p.ldg + h * p.dk;
+                    float held = 0.f, o = 0.f;
+                    for (int i = part; i < p.dk; i += 16) {
+                        sS[i * 17 + col] *= gr[i];
+                        held = fmaf(sS[i * 17 + col], kr[i], held);
+                    }
+                    for (int x = 8; x > 0; x >>= 1) held += __shfl_xor_sync(0xffffffffu, held, x);
+                    const float v = col < n_cols ? p.v[(size_t)t * p.ldv + (size_t)h * p.dv + col0 + col] : 0.f;
+                    const float u = p.beta[(size_t)t * p.ldb + h] * (v - held);
+                    for (int i = part; i < p.dk; i += 16) {
+                        const float now = fmaf(kr[i], u, sS[i * 17 + col]);
+                        sS[i * 17 + col] = now;
+                        o = fmaf(now, qr[i], o);
+                    }
+                    for (int x = 8; x > 0; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+                    if (part == 0 && col < n_cols) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col0 + col] = o;
                 }
-                for (int x = 8; x > 0; x >>= 1) held += __shfl_xor_sync(0xffffffffu, held, x);
-                const float v = col < n_cols ? p.v[(size_t)t * p.ldv + (size_t)h * p.dv + col0 + col] : 0.f;
-                const float u = p.beta[(size_t)t * p.ldb + h] * (v - held);
-                for (int i = part; i < p.dk; i += 16) {
-                    const float now = fmaf(kr[i], u, sS[i * 17 + col]);
-                    sS[i * 17 + col] = now;
-                    o = fmaf(now, qr[i], o);
-                }
-                for (int x = 8; x > 0; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
-                if (part == 0 && col < n_cols) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col0 + col] = o;
-            }
             __syncthreads();
             each([&](float& v, int i, int at) { v = i < p.dk ? sS[i * 17 + at] : 0.f; });
             __syncthreads();

@@ -74,7 +74,7 @@ _SIGNATURES = {
     "qs_state_scan": ([c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int,
                        c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
                        c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_longlong, c_float, c_int, c_float, c_void_p, c_void_p], c_int),
+                       c_void_p, c_void_p, c_longlong, c_float, c_int, c_float, c_void_p, c_void_p, c_void_p], c_int),
     "qs_delta_chunks_scratch": ([c_int, c_int, c_int, c_int], c_longlong),
     "qs_delta_chunks": ([c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
                          c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p], c_int),
@@ -639,7 +639,7 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
     if mode == "delta" and chunks is not None:
         return _delta_in_chunks(q, k, v, state, seq_slot, n_seq, n_heads, key_dim, value_dim, key_decay, token_weight, qk_group, chunks)
     o = torch.empty((T, n_heads * value_dim), dtype=torch.float32, device=q.device)
-    chunk_start = chunk_ids = seq_chunk = chunk_state = chunk_decay = None
+    chunk_start = chunk_ids = seq_chunk = chunk_state = chunk_decay = chunk_factors = None
     n_chunks = 0
     if chunks is not None and ACTIVATIONS[in_activation] != ACT_NONE:
         q, k, v = _activated(q, k, v, in_activation)
@@ -648,6 +648,8 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
         chunk_start, chunk_ids, seq_chunk, n_chunks = chunks
         chunk_state = torch.empty((n_chunks, n_heads * key_dim * (-(-value_dim // 4) * 4)), dtype=torch.float32, device=q.device)
         chunk_decay = torch.empty((n_chunks, n_heads * key_dim), dtype=torch.float32, device=q.device)
+        if mode in ("wkv", "gla"):                     # the channels' decays, taken once for two kernels
+            chunk_factors = torch.empty((T, n_heads * key_dim), dtype=torch.float32, device=q.device)
     per_token = token_decay if token_decay is not None else token_weight
     if mode == "gla" and (decay_logits is None or decay_logits.dtype != torch.float32 or not decay_power > 0):
         raise QStreamError(QsError.INVALID_INPUT, "state_scan: gated linear attention takes float32 decay logits and a positive power")
@@ -665,7 +667,7 @@ def state_scan(mode: str, q, k, v, state, seq_start, seq_slot, n_seq, n_heads, k
         _int32(seq_slot, "seq_slot"), int(n_seq), T, n_heads, key_dim, value_dim, ACTIVATIONS[in_activation],
         ptr(chunk_start), ptr(chunk_ids), int(n_chunks), ptr(seq_chunk), ptr(chunk_state), ptr(chunk_decay),
         ptr(token_decay), ptr(token_weight), per_token.stride(0) if per_token is not None else 0, float(q_scale),
-        int(qk_group), float(decay_power), ptr(gemm_tc.status_word(q.device)), stream()))
+        int(qk_group), float(decay_power), ptr(chunk_factors), ptr(gemm_tc.status_word(q.device)), stream()))
     return o if want_output else None
 
 

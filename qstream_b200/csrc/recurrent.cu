@@ -625,9 +625,10 @@ QS_API int qs_state_scan(int mode, float* o, long long ldo, const void* q, long 
                          const int32_t* seq_slot, int n_seq, int T_rows, int H, int dk, int dv, int in_act,
                          const int32_t* chunk_start, const int32_t* chunk_ids, int n_chunks, const int32_t* seq_chunk,
                          float* chunk_state, float* chunk_decay, const float* ga, const float* gb, long long ldg,
-                         float q_scale, int qk_group, float decay_scale, int32_t* status, cudaStream_t stream) {
+                         float q_scale, int qk_group, float decay_scale, float* chunk_factors, int32_t* status, cudaStream_t stream) {
     if (n_seq == 0 || T_rows == 0) return QS_OK;
     QS_REQUIRE(n_seq > 0 && T_rows > 0 && H > 0 && dk > 0 && dv > 0, "state_scan: bad sizes");
+    QS_REQUIRE(!chunk_start || (mode != 1 && mode != 4) || chunk_factors, "state_scan: chunks with a decay per channel take room for the decays");
     QS_REQUIRE(dk <= 16 * RK, "state_scan: %d key channels per head above %d", dk, 16 * RK);
     QS_REQUIRE(H <= 65535, "state_scan: %d heads exceed the grid", H);
     QS_REQUIRE(mode == 0 ? head_decay != nullptr : mode == 1 ? (dlog && bonus) : mode == 2 ? (ga && gb && dv > 1)
@@ -646,7 +647,7 @@ QS_API int qs_state_scan(int mode, float* o, long long ldo, const void* q, long 
     QS_REQUIRE(((uintptr_t)chunk_state % 16) == 0 && in_act == QS_ACT_NONE, "state_scan: chunks take activated operands and aligned scratch");
     auto chunks = [&](int outputs) {
         return qs_scan_chunks(mode, outputs, o, ldo, q, ldq, k, ldk, v, ldv, dtype, dlog, ldd, head_decay, bonus, bonus_dtype, H, dk, dv,
-                              chunk_start, n_chunks, T_rows, chunk_state, chunk_decay, ga, gb, ldg, q_scale, qk_group, decay_scale, status, stream);
+                              chunk_start, n_chunks, T_rows, chunk_state, chunk_decay, ga, gb, ldg, q_scale, qk_group, decay_scale, chunk_factors, status, stream);
     };
     int rc = chunks(0);
     if (rc != QS_OK) return rc;

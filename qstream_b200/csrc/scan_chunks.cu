@@ -7,7 +7,7 @@
 // take a prompt's chunks side by side:
 //   added_state_kernel      what each chunk adds to the state it starts from, and its decays
 //   chunk_prefix_kernel     (recurrent.cu) the state each chunk starts from, and the sequence's last one
-//   chunk_output_kernel     every token's o, written once
+//   tile_output_kernel, channel_output_kernel     every token's o, written once: one decay per head, one per key channel
 // Decays enter as products of at most 64 factors up to one, never as quotients, so small ones cost no precision: per token and head by a
 // recursion from a token back over the earlier ones; per channel in blocks of 16 tokens, a block's own pairs walked in order, pairs of blocks
 // through the products up to the blocks' common edge.
@@ -19,9 +19,9 @@
 // for the outputs, 42 of 47 for what the chunks add, at 4,096 tokens of 16 heads of 128 x 128, float32 operands); the split needs half of
 // the issue slots.  On mma.sync the same products took 138 and 59 us, multiply-adds 139 and 66.
 //
-// Microseconds of the scan alone (multiply-adds | now; caches flushed): decay per head, 4,096 tokens, 16 heads of 128 x 128, float32: 236 | 151; 1,000
-// tokens, bfloat16: 85 | 38; state-space form, 2,048 tokens, 64 heads of 128 x 64: 237 | 142; gated memory, 1,000 tokens, 4 heads of 256 x 256:
-// 136 | 79; per channel (its outputs on the CUDA cores), 3,401 tokens, 16 heads of 64 x 128: 175 | 163.
+// Microseconds of the scan alone (multiply-adds | now; caches flushed): decay per head, 4,096 tokens, 16 heads of 128 x 128, float32: 236 | 150; 1,000
+// tokens, bfloat16: 85 | 38; state-space form, 2,048 tokens, 64 heads of 128 x 64: 237 | 134; gated memory, 1,000 tokens, 4 heads of 256 x 256:
+// 136 | 79; per channel, 3,401 tokens, 16 heads of 64 x 128: 175 | 140, 600 tokens, float32: 103 | 58; wkv, 1,000 tokens, 16 of 64 x 64: 60 | 50.
 #include "scan.cuh"
 #include "scan_tiles.cuh"
 #include "term_tiles.cuh"
@@ -32,6 +32,7 @@ struct Scan {
     const void *q, *k, *v;
     size_t ldq, ldk, ldv;
     const float *dlog; size_t ldd;                      // per channel: logits of the decays
+    float* factors;                                     // and, from the first kernel on, the decays themselves [T_rows][H dk]
     const float *head_decay;                            // one decay per head
     const float *ga, *gb; size_t ldg;                   // per token and head: decays (less one in mode 5), input weights
     const void* bonus; int bonus_dtype;
@@ -40,7 +41,7 @@ struct Scan {
     float* o; size_t ldo;
     int H, dk, dv, dvp, qk_group, n_chunks, T_rows;       // dvp: dv rounded up to a multiple of four
     float q_scale, decay_scale;
-    int vec_q, vec_k, vec_v, vec_o;                    // whether rows may be read (written) in pieces of four
+    int vec_q, vec_k, vec_v, vec_d;                     // whether rows may be read in pieces of four
     int32_t* status;                                    // receives a code if a bounded wait ran out
 };
 
@@ -111,6 +112,8 @@ __device__ __noinline__ void mend_added(const Scan& p, float* to, int rows, int 
 
 template <typename TI> constexpr int added_smem() { return 1024 + (3 + (sizeof(TI) == 2 ? 1 : 3)) * 2 * TILE; }
 
+// Three blocks per SM for the state-space form in bfloat16 (2,048 tokens of 64 heads of 128 x 64: 64 -> 56 us); in the other forms they were slower
+// (gated memory, 1,000 tokens: 79 -> 97 us for the scan; decay per head 38 -> 40).
 template <typename TI, int MODE>
 __global__ void __launch_bounds__(TILE_THREADS, sizeof(TI) == 2 && MODE == 5 ? 3 : 2)
 added_state_kernel(const __grid_constant__ Scan p) {
@@ -218,7 +221,10 @@ added_state_kernel(const __grid_constant__ Scan p) {
 #pragma unroll
                 for (int x = LEN - 1; x >= 0; --x) {
                     behind[(g * LEN + x) * 64 + i] = run;
-                    run *= g * LEN + x < n && i < nk ? channel_decay<MODE>(a[x], p.decay_scale) : 1.f;
+                    if (g * LEN + x >= n || i >= nk) continue;
+                    const float d = channel_decay<MODE>(a[x], p.decay_scale);
+                    run *= d;
+                    if (col0 == 0) p.factors[(size_t)(t0 + g * LEN + x) * p.H * p.dk + (size_t)h * p.dk + i0 + i] = d;
                 }
                 part[g * 64 + i] = run;
                 __syncthreads();
@@ -274,337 +280,307 @@ added_state_kernel(const __grid_constant__ Scan p) {
     leave();
 }
 
-// ----------------------------------------------------------------------------- a chunk's outputs
+// ----------------------------------------------------------------------------- a chunk's outputs, a decay per key channel
 
-// A block takes the 64 tokens of a chunk and 64 NC value columns: of one head, or (NH = 2) 64 of each of two neighbouring heads
-// that share q and k, whose products q k^T are then taken once.  The key channels pass in slices through shared memory.
-// Three blocks per SM leave a thread 168 registers.  The bfloat16 forms fit (at most 16 bytes spilled); the float32 ones, which a decay per head
-// behind an activation takes too, hold a slice of q and k on its way in twice the room and spill 340 bytes, 700 to 780 per channel and with
-// the column of ones.
-template <int MODE, int NC>
-constexpr int output_body() {                           // floats of shared memory before the weights
-    const int sl = MODE == 1 || MODE == 4 ? 64 : 32, stage = sl == 64 ? (3 * sl * CT > sl * CT + sl * 64 * NC ? 3 * sl * CT : sl * CT + sl * 64 * NC)
-                                                                      : 2 * sl * CT + 2 * sl * 64 * NC;
-    return stage > CT * 64 * NC ? stage : CT * 64 * NC;
+// The same with a decay per token and key channel: a block takes the 64 tokens of a chunk and 128 value columns of one head.  The weights P come from
+// multiply-adds: pairs of tokens within a block of 16 with their decays as running products (a warp a block and half of the channels), a block's tokens
+// against all earlier ones as products of q times the decays since the block's start with k taken on to it (a warp eight channels).  The products with the
+// state and with the values run on tcgen05, in three terms per number (one for values that come as bfloat16).
+//
+// Bound by instruction issue (7,100 per warp when the decays were still taken here from their logits: 103 us for 3,401 tokens of 16 heads of 64 x 128;
+// by multiply-adds alone 114): so the first kernel leaves the decays behind.
+constexpr int SL = 64;                                  // channels of a slice
+// ts, with k, the decays and the warps' sums over it; tq; q; the weights; the blocks' whole decays
+constexpr int CHANNEL_SMEM = 1024 + 6 * TILE + 3 * TILE + (SL * CT + CT * PP + 4 * SL) * 4;
+static_assert(8 * CROSS * 4 <= 9 * TILE && 2 * SL * CT * 4 <= 6 * TILE, "what lies over the tiles");
+
+// The part of an output that the state gives, by multiply-adds.
+template <typename TI, int MODE>
+__device__ __noinline__ float plain_from_state(const Scan& p, const float* __restrict__ S, int h, int t0, int t, int col) {
+    const TI* q = (const TI*)p.q + (size_t)(t0 + t) * p.ldq + (size_t)(h / p.qk_group) * p.dk;
+    float o = 0.f;
+    for (int i = 0; i < p.dk && o == o; ++i) {          // NaN stays NaN
+        float x = to_f32(q[i]) * (MODE == 1 ? 1.f : p.q_scale);
+        for (int j = 0; j < (MODE == 1 ? t : t + 1); ++j) x *= decay_at<MODE>(p, t0 + j, h, i);
+        o = fmaf(x, S[(size_t)i * p.dvp + col], o);
+    }
+    return o;
 }
 
-template <typename TI, int MODE, int NC, int NH>
-__global__ void __launch_bounds__(THREADS, 3)
-chunk_output_kernel(Scan p) {
-    constexpr bool PER_CHANNEL = MODE == 1 || MODE == 4, ONES = MODE == 2, WKV = MODE == 1;
-    constexpr int SL = PER_CHANNEL ? 64 : 32;           // channels of a slice
-    constexpr int COLS = 64 * NC, NQ = CT * SL / 4 / THREADS, NV = CT * 16 * NC / THREADS;
-    extern __shared__ __align__(16) float smem[];
-    float* sq = smem;                                   // [SL][64 tokens]
-    float* sk = sq + SL * CT;                           // [SL][64 tokens]
-    float* sw = sk + SL * CT;                           // PER_CHANNEL: the decays [SL][64 tokens]; then the state lies over sk, sw
-    float* ss = PER_CHANNEL ? sk : sw;                  // [SL][COLS]: a slice of the states the chunk starts from; two of them in turn per head
-    float* svv = smem;                                  // [64 tokens][COLS]: the values, after the last slice
-    float* sp = smem + output_body<MODE, NC>();         // [NH][64 j][PP]
-    float* edge = sp + NH * CT * PP;                    // PER_CHANNEL: [4][SL] the decays of a block of 16 tokens
-    __shared__ float s_a[NH][CT], s_cum[NH][CT], s_b[NH][CT];
+// MANY: more than 128 key channels, more than two runs.
+template <typename TI, int MODE, bool MANY>
+__global__ void __launch_bounds__(TILE_THREADS, 2)
+channel_output_kernel(const __grid_constant__ Scan p) {
+    constexpr bool WKV = MODE == 1;
+    constexpr int VT = sizeof(TI) == 2 ? 1 : 3, NQ = CT * SL / 4 / TILE_THREADS, NS = 2 * NQ;
+    constexpr uint32_t TMEM = 128;                      // two runs' sums [128 columns][64 tokens]
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t done;
+    __shared__ uint32_t tmem_slot;
+    uint8_t* const base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    float* const sk = reinterpret_cast<float*>(base);   // [SL][64 tokens]
+    float* const sw = sk + SL * CT;                     // the decays [SL][64 tokens]
+    float* const sums = sk;                             // [8 warps][CROSS], over k and the decays
+    float* const sq = reinterpret_cast<float*>(base + 9 * TILE);         // [SL][64 tokens]
+    float* const sp = sq + SL * CT;                     // [64 j][PP]
+    float* const edge = sp + CT * PP;                   // [4][SL] the decays of a block of 16 tokens
+    const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
+    if (tid == 0) { mbar_init(&done, 1); mbar_fence_init(); }
+    if (warp == 0) { tmem_alloc(&tmem_slot, TMEM); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
     grid_dep_launch();
     grid_dep_wait();
-    const int c = blockIdx.x, h = blockIdx.y * NH, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int dvv = ONES ? p.dv - 1 : p.dv, col0 = blockIdx.z * 64 * NC, nv = NH == 2 ? dvv : min(64 * NC, dvv - col0);
+    const uint32_t tmem = tmem_slot, own = tmem + ((uint32_t)(quad * 32) << 16) + half * 32;
+    const uint32_t ts = smem_u32(base), tq = ts + 6 * TILE;     // [3][2 halves of the columns][channels], [3][tokens]
+    const uint32_t tv = ts, tp = tq;                    // after the slices: [VT][2][tokens], [3][tokens][earlier tokens]
+    const int col0 = blockIdx.z * 128, nv = min(128, p.dv - col0);
     const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0, hq = h / p.qk_group;
+    float* const S = p.chunk_state + ((size_t)c * p.H + h) * p.dk * p.dvp;
+    auto leave = [&]() {
+        tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(tmem, TMEM);
+    };
     if (c == 0)                                         // rows behind the last sequence belong to nobody: a defined value
-        for (int t = p.chunk_start[p.n_chunks]; t < p.T_rows; ++t) {
-            for (int e = tid; e < NH * nv; e += THREADS) p.o[(size_t)t * p.ldo + (size_t)(h + e / nv) * p.dv + (NH == 2 ? 0 : col0) + e % nv] = 0.f;
-            if (ONES && col0 == 0 && tid == 0) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + dvv] = 0.f;
-        }
-    if (n <= 0) return;
-    if (n > CT) {
-        for (int x = 0; x < NH; ++x) {
-            float* S = p.chunk_state + ((size_t)c * p.H + h + x) * p.dk * p.dvp;
-            walk_in_order<TI, MODE>(p, S, c, h + x, col0, nv, true);
-            if (ONES && col0 == 0) walk_in_order<TI, MODE>(p, S, c, h + x, dvv, 1, true);
-        }
+        for (int t = p.chunk_start[p.n_chunks]; t < p.T_rows; ++t)
+            for (int e = tid; e < nv; e += TILE_THREADS) p.o[(size_t)t * p.ldo + (size_t)h * p.dv + col0 + e] = 0.f;
+    if (n <= 0 || n > CT) {
+        if (n > CT) walk_in_order<TI, MODE>(p, S, c, h, col0, nv, true);
+        leave();
         return;
     }
-    if (!PER_CHANNEL) {                                 // the tokens' decays and weights
-        for (int e = tid; e < NH * CT; e += THREADS) {
-            const int x = e / CT, t = e % CT;
-            s_a[x][t] = t < n ? decay_at<MODE>(p, t0 + t, h + x, 0) : (MODE == 5 ? 0.f : 1.f);
-            s_b[x][t] = t >= n ? 0.f : (MODE == 2 || MODE == 5) ? p.gb[(size_t)(t0 + t) * p.ldg + h + x] : 1.f;
-        }
-    }
-    f32x2 acc[8][2 * NC], raw[8][2];
+    for (int e = tid; e < CT * PP; e += TILE_THREADS) sp[e] = 0.f;
+    const int slices = (p.dk + SL - 1) / SL;
+    float out[32];
+    bool ok = true;
+    for (int s = 0; s < slices; ++s) {
+        const int i0 = s * SL, nk = min(SL, p.dk - i0);
+        Raw4<TI> rq[NQ], rk[NQ];
+        Raw4<float> rd[NQ], rs[NS];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        raw[i][0] = raw[i][1] = 0ull;
-#pragma unroll
-        for (int j = 0; j < 2 * NC; ++j) acc[i][j] = 0ull;
-    }
-    float ones_part = 0.f;                              // ONES: q_t . S0's last column, token tid
-    if (PER_CHANNEL)
-        for (int e = tid; e < CT * PP; e += THREADS) sp[e] = 0.f;
-
-    // q and k of a slice on their way to registers; the states' slice on its way to shared memory
-    Raw4<TI> rq[NQ], rk[NQ];
-    constexpr int LANES = SL / 4;                       // lanes that share a token's slice; a warp writes every bank of the staged tile once
-    auto token_of = [&](int e) { return PER_CHANNEL ? e / LANES : (e >> 5) * 4 + ((e & 31) >> 3); };
-    auto channel_of = [&](int e) { return PER_CHANNEL ? (e % LANES) * 4 : (e & 7) * 4; };
-    auto fetch = [&](int i0) {
-        const int nk = min(SL, p.dk - i0);
-#pragma unroll
-        for (int x = 0; x < NQ; ++x) {
-            const int e = tid + x * THREADS, t = token_of(e), i = channel_of(e);
+        for (int x = 0; x < NQ; ++x) {                  // a warp takes four tokens by 32 channels: no two lanes of a store on one bank
+            const int e = tid + x * TILE_THREADS, t = (e >> 6) * 4 + (e >> 3 & 3), i = (e >> 5 & 1) * 32 + (e & 7) * 4;
             get_four(rq[x], (const TI*)p.q + (size_t)(t0 + t) * p.ldq + hq * p.dk + i0, i, nk, t < n, p.vec_q);
             get_four(rk[x], (const TI*)p.k + (size_t)(t0 + t) * p.ldk + hq * p.dk + i0, i, nk, t < n, p.vec_k);
+            get_four(rd[x], (const float*)p.factors + (size_t)(t0 + t) * p.H * p.dk + (size_t)h * p.dk + i0, i, nk, t < n, p.vec_d);
         }
-    };
-    auto fetch_state = [&](int i0, float* dst) {
-        const int nk = min(SL, p.dk - i0);
-#pragma unroll 4
-        for (int e = tid; e < SL * 16 * NC; e += THREADS) {
-            const int i = e / (16 * NC), col = (e % (16 * NC)) * 4, x = NH == 2 ? col >> 6 : 0, own = NH == 2 ? col & 63 : col0 + col;
-            copy16(dst + e * 4, p.chunk_state + (((size_t)c * p.H + h + x) * p.dk + i0 + i) * p.dvp + own, i < nk && own < dvv);
+        if (s && ok) ok = wait_done(&done, (s - 1) & 1, p.status);
+        if (MANY && s >= 2) {
+            tc_fence_after_sync();
+            take_sums<32>(out, own + (s & 1) * 64, s == 2);
+            tc_fence_before_sync();
         }
-    };
-    fetch(0);
-    if (!PER_CHANNEL) {
-        fetch_state(0, ss);
-        __syncthreads();
-        for (int e = tid; e < NH * CT; e += THREADS) {  // the decays between two tokens, with the earlier one's weight; those since the start
-            const int x = e / CT, j = e % CT;
-            float w = s_b[x][j], cum = 1.f;
-#pragma unroll 8
-            for (int t = 0; t < CT; ++t) {
-                const float a = s_a[x][t];
-                if (t > j) w = times_decay<MODE>(w, a);
-                if (t <= j) cum = times_decay<MODE>(cum, a);
-                sp[(x * CT + j) * PP + t] = t >= j ? w : 0.f;
-            }
-            s_cum[x][j] = cum;
-        }
-    }
-    for (int i0 = 0; i0 < p.dk; i0 += SL) {
-        const int nk = min(SL, p.dk - i0);
-        float* const s_now = PER_CHANNEL ? ss : ss + (i0 / SL & 1) * SL * COLS;
-        __syncthreads();
+        if (s) __syncthreads();                         // every warp has seen the products that read what is written over now
 #pragma unroll
         for (int x = 0; x < NQ; ++x) {
-            const int e = tid + x * THREADS, t = token_of(e), i = channel_of(e);
-            const float4 q4 = rq[x].value(), k4 = rk[x].value();
-            const float fq[4] = {q4.x, q4.y, q4.z, q4.w}, fk[4] = {k4.x, k4.y, k4.z, k4.w};
+            const int e = tid + x * TILE_THREADS, t = (e >> 6) * 4 + (e >> 3 & 3), i = (e >> 5 & 1) * 32 + (e & 7) * 4;
+            const float4 q4 = rq[x].value(), k4 = rk[x].value(), d4 = rd[x].value();
+            const float fq[4] = {q4.x, q4.y, q4.z, q4.w}, fk[4] = {k4.x, k4.y, k4.z, k4.w}, fd[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
             for (int y = 0; y < 4; ++y) {
-                sq[at_ct(i + y, t)] = WKV ? fq[y] : fq[y] * p.q_scale;
-                sk[at_ct(i + y, t)] = fk[y];
-            }
-            if (PER_CHANNEL) {
-#pragma unroll
-                for (int y = 0; y < 4; ++y) sw[at_ct(i + y, t)] = t < n && i + y < nk ? decay_at<MODE>(p, t0 + t, h, i0 + i + y) : 1.f;
+                const int at = at_ct(i + y, t);
+                sq[at] = WKV ? fq[y] : fq[y] * p.q_scale;
+                sk[at] = fk[y];
+                sw[at] = t < n && i + y < nk ? fd[y] : 1.f;
             }
         }
-        if (!PER_CHANNEL) {
-            copies_done();
-            __syncthreads();
-            if (i0 + SL < p.dk) {
-                fetch_state(i0 + SL, ss + ((i0 / SL + 1) & 1) * SL * COLS);
-                fetch(i0 + SL);
-            }
-            // q k^T and q S0 of this slice
-#pragma unroll 4
-            for (int k = 0; k < SL; ++k) {
-                const float4 x = *reinterpret_cast<const float4*>(sq + at_ct(k, ty * 4)), y = *reinterpret_cast<const float4*>(sq + at_ct(k, 32 + ty * 4));
-                const float a[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(sk + at_ct(k, tx * 4));
-                f32x2 b[2 * NC];
+        // the state's slice on its way to registers
 #pragma unroll
-                for (int g = 0; g < NC; ++g) {
-                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(s_now + k * COLS + g * 64 + tx * 4);
-                    b[2 * g] = w.x;
-                    b[2 * g + 1] = w.y;
+        for (int x = 0; x < NS; ++x) {
+            const int e = tid + x * TILE_THREADS, i = e >> 5;
+            get_four(rs[x], S + (size_t)(i0 + i) * p.dvp, col0 + (e & 31) * 4, (p.dv + 3) / 4 * 4, i < nk, 1);
+        }
+        __syncthreads();
+        // pairs of tokens within a block of 16: lane = token j and a quarter of the channels
+        {
+            const int jj = lane & 15, b0 = quad * 16, e0 = (half * 2 + (lane >> 4)) * (SL / 4);
+            float d[16];
+#pragma unroll
+            for (int x = 0; x < 16; ++x) d[x] = 0.f;
+            for (int i = e0; i < e0 + SL / 4; ++i) {
+                float fq[16], fw[16];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const float4 x = *reinterpret_cast<const float4*>(sq + at_ct(i, b0 + 4 * g)), y = *reinterpret_cast<const float4*>(sw + at_ct(i, b0 + 4 * g));
+                    fq[4 * g] = x.x; fq[4 * g + 1] = x.y; fq[4 * g + 2] = x.z; fq[4 * g + 3] = x.w;
+                    fw[4 * g] = y.x; fw[4 * g + 1] = y.y; fw[4 * g + 2] = y.z; fw[4 * g + 3] = y.w;
                 }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const f32x2 aa = pack2(a[i], a[i]);
-                    raw[i][0] = fma2(aa, kk.x, raw[i][0]);
-                    raw[i][1] = fma2(aa, kk.y, raw[i][1]);
-#pragma unroll
-                    for (int j = 0; j < 2 * NC; ++j) acc[i][j] = fma2(aa, b[j], acc[i][j]);
-                }
-            }
-            if (ONES && blockIdx.z == 0 && tid < CT) {
-                const float* last = p.chunk_state + (((size_t)c * p.H + h) * p.dk + i0) * p.dvp + dvv;
-                for (int i = 0; i < nk; ++i) ones_part = fmaf(sq[at_ct(i, tid)], last[(size_t)i * p.dvp], ones_part);
-            }
-        } else {
-            __syncthreads();
-            // pairs of tokens within a block of 16, a warp per block: lane = token j and half of the channels
-            const int blk = tid >> 5, lane = tid & 31, jj = lane & 15, b0 = blk * 16;
-            {
-                float d[16];
-#pragma unroll
-                for (int x = 0; x < 16; ++x) d[x] = 0.f;
-                for (int i = (lane >> 4) * (SL / 2); i < (lane >> 4) * (SL / 2) + SL / 2; ++i) {
-                    float fq[16], fw[16];
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const float4 x = *reinterpret_cast<const float4*>(sq + at_ct(i, b0 + 4 * g)), y = *reinterpret_cast<const float4*>(sw + at_ct(i, b0 + 4 * g));
-                        fq[4 * g] = x.x; fq[4 * g + 1] = x.y; fq[4 * g + 2] = x.z; fq[4 * g + 3] = x.w;
-                        fw[4 * g] = y.x; fw[4 * g + 1] = y.y; fw[4 * g + 2] = y.z; fw[4 * g + 3] = y.w;
-                    }
-                    const float kj = sk[at_ct(i, b0 + jj)];
-                    const float u = WKV && i < nk ? load_as_f32(p.bonus, p.bonus_dtype, (size_t)h * p.dk + i0 + i) : 1.f;
-                    float run = kj;
-#pragma unroll
-                    for (int x = 0; x < 16; ++x) {
-                        if (x > jj && !WKV) run *= fw[x];
-                        d[x] = fmaf(fq[x], WKV && x == jj ? u * kj : run, d[x]);         // means nothing where x < jj
-                        if (x > jj && WKV) run *= fw[x];
-                    }
-                }
+                const float kj = sk[at_ct(i, b0 + jj)];
+                const float u = WKV && i < nk ? load_as_f32(p.bonus, p.bonus_dtype, (size_t)h * p.dk + i0 + i) : 1.f;
+                float run = kj;
 #pragma unroll
                 for (int x = 0; x < 16; ++x) {
-                    const float sum = d[x] + __shfl_xor_sync(0xffffffffu, d[x], 16);
-                    if (lane < 16 && x >= jj) sp[(b0 + jj) * PP + b0 + x] += sum;
+                    if (x > jj && !WKV) run *= fw[x];
+                    d[x] = fmaf(fq[x], WKV && x == jj ? u * kj : run, d[x]);         // means nothing where x < jj
+                    if (x > jj && WKV) run *= fw[x];
                 }
             }
-            __syncthreads();
-            // q times the decays since the start of its block of 16, k times those up to the block's end, the block's whole decay
-            for (int e = tid; e < SL * 4; e += THREADS) {        // neighbouring lanes four channels apart: other banks
-                const int i = (e & 15) * 4 + (e >> 4 & 3), g = e >> 6;
-                float4 w[4];
-                float run = 1.f;
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    w[x] = *reinterpret_cast<const float4*>(sw + at_ct(i, g * 16 + 4 * x));
-                    float4* at = reinterpret_cast<float4*>(sq + at_ct(i, g * 16 + 4 * x));
-                    float4 f = *at;
-                    if (!WKV) run *= w[x].x;
-                    f.x *= run; run *= WKV ? w[x].x : w[x].y;
-                    f.y *= run; run *= WKV ? w[x].y : w[x].z;
-                    f.z *= run; run *= WKV ? w[x].z : w[x].w;
-                    f.w *= run;
-                    if (WKV) run *= w[x].w;
-                    *at = f;
-                }
-                edge[g * SL + i] = run;
-                run = 1.f;
+            for (int x = 0; x < 16; ++x) d[x] += __shfl_xor_sync(0xffffffffu, d[x], 16);
 #pragma unroll
-                for (int x = 3; x >= 0; --x) {
-                    float4* at = reinterpret_cast<float4*>(sk + at_ct(i, g * 16 + 4 * x));
-                    float4 f = *at;
-                    f.w *= run; run *= w[x].w;
-                    f.z *= run; run *= w[x].z;
-                    f.y *= run; run *= w[x].y;
-                    f.x *= run; run *= w[x].x;
-                    *at = f;
-                }
+            for (int turn = 0; turn < 2; ++turn) {      // the channels' halves one after the other
+                if (half == turn && lane < 16)
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) if (x >= jj) sp[(b0 + jj) * PP + b0 + x] += d[x];
+                __syncthreads();
             }
-            __syncthreads();
-            // a block's tokens against all earlier ones, whose k are taken on to this block's start; a warp has 16 of the channels
-            f32x2 x1[2][2], x2[4][2], x3[6][2];
-#pragma unroll
-            for (int x = 0; x < 6; ++x) {
-                if (x < 2) x1[x][0] = x1[x][1] = 0ull;
-                if (x < 4) x2[x][0] = x2[x][1] = 0ull;
-                x3[x][0] = x3[x][1] = 0ull;
-            }
-            const int ch = blk * 16 + (jj & 3) * 4 + (jj >> 2), eighth = (lane >> 4) * 8;
-            cross_product<1, 16, at_ct>(x1, sq, sk, blk * 16, lane);
-            __syncwarp();
-#pragma unroll
-            for (int x = 0; x < 2; ++x) scale_four(sk + at_ct(ch, eighth + 4 * x), edge[SL + ch]);
-            __syncwarp();
-            cross_product<2, 16, at_ct>(x2, sq, sk, blk * 16, lane);
-            __syncwarp();
-#pragma unroll
-            for (int x = 0; x < 4; ++x) scale_four(sk + at_ct(ch, 2 * eighth + 4 * x), edge[2 * SL + ch]);
-            __syncwarp();
-            cross_product<3, 16, at_ct>(x3, sq, sk, blk * 16, lane);
-            __syncthreads();
-            // the warps' sums over k and the decays, then added up; q times the decays since the chunk's start
-            cross_store<1>(sk + blk * CROSS, x1, lane);
-            cross_store<2>(sk + blk * CROSS, x2, lane);
-            cross_store<3>(sk + blk * CROSS, x3, lane);
-            for (int e = tid; e < SL * 12; e += THREADS) {
-                const int i = (e & 15) * 4 + (e >> 4 & 3), t = 16 + (e >> 6) * 4;
-                float x = 1.f;
-                for (int m = 0; m < t / 16; ++m) x *= edge[m * SL + i];
-                scale_four(sq + at_ct(i, t), x);
-            }
-            __syncthreads();
-#pragma unroll
-            for (int pair = 0; pair < 6; ++pair) {      // blocks (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
-                const int I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
-                for (int e = tid; e < 256; e += THREADS) {
-                    const int t = e & 15, j = J * 16 + (e >> 4);
-                    const float* at = sk + cross_at(I) + t * (16 * I + 1) + j;
-                    sp[j * PP + I * 16 + t] += (at[0] + at[CROSS]) + (at[2 * CROSS] + at[3 * CROSS]);
-                }
-            }
-            __syncthreads();
-            fetch_state(i0, ss);                        // over k and the decays
-            if (i0 + SL < p.dk) fetch(i0 + SL);
-            copies_done();
-            __syncthreads();
-            tile_product<NC, true>(acc, sq, ss, SL, ty, tx);
         }
-    }
-    Raw4<TI> rv[NV];
+        // q times the decays since the start of its block of 16, k times those up to the block's end, the block's whole decay
+        {
+            const int i = (tid & 15) * 4 + (tid >> 4 & 3), g = tid >> 6;       // neighbouring lanes four channels apart: other banks
+            float4 w[4];
+            float run = 1.f;
 #pragma unroll
-    for (int x = 0; x < NV; ++x) {
-        const int e = tid + x * THREADS, j = e / (16 * NC), col = (e % (16 * NC)) * 4, head = NH == 2 ? col >> 6 : 0, own = NH == 2 ? col & 63 : col;
-        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)(h + head) * dvv + (NH == 2 ? 0 : col0), own, nv, j < n, p.vec_v);
+            for (int x = 0; x < 4; ++x) {
+                w[x] = *reinterpret_cast<const float4*>(sw + at_ct(i, g * 16 + 4 * x));
+                float4* at = reinterpret_cast<float4*>(sq + at_ct(i, g * 16 + 4 * x));
+                float4 f = *at;
+                if (!WKV) run *= w[x].x;
+                f.x *= run; run *= WKV ? w[x].x : w[x].y;
+                f.y *= run; run *= WKV ? w[x].y : w[x].z;
+                f.z *= run; run *= WKV ? w[x].z : w[x].w;
+                f.w *= run;
+                if (WKV) run *= w[x].w;
+                *at = f;
+            }
+            edge[g * SL + i] = run;
+            run = 1.f;
+#pragma unroll
+            for (int x = 3; x >= 0; --x) {
+                float4* at = reinterpret_cast<float4*>(sk + at_ct(i, g * 16 + 4 * x));
+                float4 f = *at;
+                f.w *= run; run *= w[x].w;
+                f.z *= run; run *= w[x].z;
+                f.y *= run; run *= w[x].y;
+                f.x *= run; run *= w[x].x;
+                *at = f;
+            }
+        }
+        __syncthreads();
+        // a block's tokens against all earlier ones, whose k are taken on to this block's start; a warp has eight of the channels
+        f32x2 x1[2][2], x2[4][2], x3[6][2];
+#pragma unroll
+        for (int x = 0; x < 6; ++x) {
+            if (x < 2) x1[x][0] = x1[x][1] = 0ull;
+            if (x < 4) x2[x][0] = x2[x][1] = 0ull;
+            x3[x][0] = x3[x][1] = 0ull;
+        }
+        const int ch = warp * 8 + (lane & 7), piece = (lane >> 3) * 4;
+        cross_product<1, 8, at_ct>(x1, sq, sk, warp * 8, lane);
+        __syncwarp();
+        scale_four(sk + at_ct(ch, piece), edge[SL + ch]);
+        __syncwarp();
+        cross_product<2, 8, at_ct>(x2, sq, sk, warp * 8, lane);
+        __syncwarp();
+        scale_four(sk + at_ct(ch, piece), edge[2 * SL + ch]);
+        scale_four(sk + at_ct(ch, 16 + piece), edge[2 * SL + ch]);
+        __syncwarp();
+        cross_product<3, 8, at_ct>(x3, sq, sk, warp * 8, lane);
+        __syncthreads();
+        // the warps' sums over k and the decays, then added up
+        cross_store<1>(sums + warp * CROSS, x1, lane);
+        cross_store<2>(sums + warp * CROSS, x2, lane);
+        cross_store<3>(sums + warp * CROSS, x3, lane);
+        __syncthreads();
+#pragma unroll
+        for (int pair = 0; pair < 6; ++pair) {          // blocks (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+            const int I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
+            const int t = tid & 15, j = J * 16 + (tid >> 4);
+            const float* at = sums + cross_at(I) + t * (16 * I + 1) + j;
+            float sum = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w += 2) sum += at[w * CROSS] + at[(w + 1) * CROSS];
+            sp[j * PP + I * 16 + t] += sum;
+        }
+        __syncthreads();
+        // the state, and q times the decays since the chunk's start, as terms
+#pragma unroll
+        for (int x = 0; x < NS; ++x) {
+            const int e = tid + x * TILE_THREADS, col = (e & 31) * 4;
+            put_terms<3>(ts + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), 2 * TILE, rs[x].value());
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {                   // a thread takes a token's eight channels, lanes neighbouring tokens
+            const int e = tid + x * TILE_THREADS, t = e & 63, i = (e >> 6) * 8;
+            float f[8];
+#pragma unroll
+            for (int y = 0; y < 8; ++y) {
+                float before = 1.f;
+                for (int m = 0; m < t / 16; ++m) before *= edge[m * SL + i + y];
+                f[y] = sq[at_ct(i + y, t)] * before;
+            }
+            put_eight(tq + place_in_tile(t, i), TILE, f);
+        }
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
+        __syncthreads();
+        if (warp == 0 && elect_one()) {
+            tc_fence_after_sync();
+            multiply_tiles<3, 3, true, false>(tmem + (s & 1) * 64, ts, 2 * TILE, tq, TILE, CT);       // S0^T q
+            mma_commit(&done);
+        }
+        __syncwarp();
     }
+    Raw4<TI> rv[NS];
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+        const int e = tid + x * TILE_THREADS, j = e >> 5;
+        get_four(rv[x], (const TI*)p.v + (size_t)(t0 + j) * p.ldv + (size_t)h * p.dv + col0, (e & 31) * 4, nv, j < n, p.vec_v);
+    }
+    if (ok) ok = wait_done(&done, (slices - 1) & 1, p.status);
+    tc_fence_after_sync();
+    const int older = slices & 1, newer = older ^ 1;
+    if (slices > 1) take_sums<32>(out, own + older * 64, slices == 2);
+    take_sums<32>(out, own + newer * 64, slices == 1);
+    tc_fence_before_sync();
+    __syncthreads();                                    // every warp has seen the products: their tiles may be written over
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+        const int e = tid + x * TILE_THREADS, col = (e & 31) * 4;
+        put_terms<VT>(tv + (col >> 6) * TILE + place_in_tile(e >> 5, col & 63), 2 * TILE, rv[x].value());
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const int e = tid + x * TILE_THREADS, t = e & 63, j = (e >> 6) * 8;
+        float f[8];
+#pragma unroll
+        for (int y = 0; y < 8; ++y) f[y] = sp[(j + y) * PP + t];
+        put_eight(tp + place_in_tile(t, j), TILE, f);
+    }
+    fence_proxy_async_smem();
+    tc_fence_before_sync();
     __syncthreads();
-    // the weights P[j][t], and acc times the decays since the chunk's start
-    if (!PER_CHANNEL) {
+    if (warp == 0 && elect_one()) {
+        tc_fence_after_sync();
+        multiply_tiles<VT, 3, true, false>(tmem, tv, 2 * TILE, tp, TILE, CT);       // V^T P^T
+        mma_commit(&done);
+    }
+    __syncwarp();
+    if (ok) ok = wait_done(&done, slices & 1, p.status);
+    tc_fence_after_sync();
+    float more[32];
+    take_sums<32>(more, own, true);
+    const int in = quad * 32 + lane, rows = n - half * 32;
+    if (in < nv) {
+        float* const o = p.o + (size_t)t0 * p.ldo + (size_t)h * p.dv + col0 + in;
+        bool odd = false;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int t = (i >> 2) * 32 + ty * 4 + (i & 3);
-            const float2 r0 = unpack2(raw[i][0]), r1 = unpack2(raw[i][1]);
-#pragma unroll
-            for (int x = 0; x < NH; ++x) {
-                float* w = sp + (x * CT + tx * 4) * PP + t;
-                // a weight of zero stays zero whatever the product is: a token's q never meets a later token's k
-                w[0] = tx * 4 <= t ? w[0] * r0.x : 0.f; w[PP] = tx * 4 + 1 <= t ? w[PP] * r0.y : 0.f;
-                w[2 * PP] = tx * 4 + 2 <= t ? w[2 * PP] * r1.x : 0.f; w[3 * PP] = tx * 4 + 3 <= t ? w[3 * PP] * r1.y : 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < 2 * NC; ++j) {
-                const float cum = s_cum[NH == 2 ? j >> 1 : 0][t];
-                acc[i][j] = mul2(pack2(cum, cum), acc[i][j]);
-            }
+        for (int x = 0; x < 32; ++x) {
+            odd |= !is_number(out[x] + more[x]);
+            if (x < rows) o[(size_t)(half * 32 + x) * p.ldo] = out[x] + more[x];
         }
-    }
-    bool odd = false;                                   // a value that is not finite must not meet the weights of zero of earlier tokens
-#pragma unroll
-    for (int x = 0; x < NV; ++x) {
-        const float4 f = rv[x].value();
-        odd |= !(fabsf(f.x) <= 3.402823466e38f && fabsf(f.y) <= 3.402823466e38f && fabsf(f.z) <= 3.402823466e38f && fabsf(f.w) <= 3.402823466e38f);
-        *reinterpret_cast<float4*>(svv + (tid + x * THREADS) * 4) = f;
-    }
-    odd = __syncthreads_or(odd);
-    if (odd) add_values<NC, NH, true>(acc, sp, svv, n, ty, tx);
-    else add_values<NC, NH, false>(acc, sp, svv, n, ty, tx);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = (i >> 2) * 32 + ty * 4 + (i & 3);
-        if (t >= n) continue;
-#pragma unroll
-        for (int g = 0; g < NC; ++g) {
-            const int own = NH == 2 ? tx * 4 : g * 64 + tx * 4;
-            float* dst = p.o + (size_t)(t0 + t) * p.ldo + (size_t)(NH == 2 ? h + g : h) * p.dv + (NH == 2 ? 0 : col0) + own;
-            const float2 a = unpack2(acc[i][2 * g]), b = unpack2(acc[i][2 * g + 1]);
-            if (p.vec_o && own < nv) *reinterpret_cast<float4*>(dst) = make_float4(a.x, a.y, b.x, b.y);
-            else {
-                if (own < nv) dst[0] = a.x;
-                if (own + 1 < nv) dst[1] = a.y;
-                if (own + 2 < nv) dst[2] = b.x;
-                if (own + 3 < nv) dst[3] = b.y;
+        if (odd)                                        // by multiply-adds, where the terms gave no number: a later token's value meets no earlier one
+            for (int t = half * 32; t < min(n, half * 32 + 32); ++t) {
+                if (is_number(o[(size_t)t * p.ldo])) continue;
+                float v = plain_from_state<TI, MODE>(p, S, h, t0, t, col0 + in);
+                for (int j = 0; j <= t && v == v; ++j)
+                    v = fmaf(sp[j * PP + t], to_f32(((const TI*)p.v)[(size_t)(t0 + j) * p.ldv + (size_t)h * p.dv + col0 + in]), v);
+                o[(size_t)t * p.ldo] = v;
             }
-        }
     }
-    if (ONES && blockIdx.z == 0 && tid < n) {
-        float sum = s_cum[0][tid] * ones_part;
-        for (int j = 0; j <= tid; ++j) sum += sp[j * PP + tid];
-        p.o[(size_t)(t0 + tid) * p.ldo + (size_t)h * p.dv + dvv] = sum;
-    }
+    leave();
 }
 
 // ----------------------------------------------------------------------------- a chunk's outputs, one decay per head
@@ -846,22 +822,20 @@ int launch_added(const Scan& p, int n_chunks, cudaStream_t stream) {
     return qs_check_launch("state_scan, added states");
 }
 
-// NC: columns in 64s of a block (per channel), NH: heads of a block (one decay per head)
-template <typename TI, int MODE, int NC, int NH>
+template <typename TI, int MODE, int NH>
 int launch_output(const Scan& p, int n_chunks, cudaStream_t stream) {
     const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
+    const dim3 grid(n_chunks, p.H / NH, NH == 2 ? 1 : (dvv + 127) / 128);
     cudaError_t e;
     if constexpr (MODE == 1 || MODE == 4) {
-        const size_t smem = (size_t)(output_body<MODE, NC>() + NH * CT * (CT + 4) + 4 * 64) * sizeof(float);
-        e = cudaFuncSetAttribute(chunk_output_kernel<TI, MODE, NC, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = qs_launch_dependent(chunk_output_kernel<TI, MODE, NC, NH>, dim3(n_chunks, p.H / NH, (dvv + 64 * NC - 1) / (64 * NC)), dim3(THREADS), smem, stream, p);
+        const auto kernel = p.dk > 128 ? channel_output_kernel<TI, MODE, true> : channel_output_kernel<TI, MODE, false>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHANNEL_SMEM);
+        if (e == cudaSuccess) e = qs_launch_dependent(kernel, grid, dim3(TILE_THREADS), CHANNEL_SMEM, stream, p);
     } else {
         constexpr int smem = tile_smem<TI, NH>();
         const auto kernel = p.dk > 128 ? tile_output_kernel<TI, MODE, NH, true> : tile_output_kernel<TI, MODE, NH, false>;
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess)
-            e = qs_launch_dependent(kernel, dim3(n_chunks, p.H / NH, NH == 2 ? 1 : (dvv + 127) / 128), dim3(TILE_THREADS), smem, stream, p);
+        if (e == cudaSuccess) e = qs_launch_dependent(kernel, grid, dim3(TILE_THREADS), smem, stream, p);
     }
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "state_scan, chunk outputs: %s", cudaGetErrorString(e));
     return qs_check_launch("state_scan, chunk outputs");
@@ -869,11 +843,10 @@ int launch_output(const Scan& p, int n_chunks, cudaStream_t stream) {
 
 template <typename TI, int MODE>
 int run(const Scan& p, int n_chunks, bool outputs, cudaStream_t stream) {
-    const int dvv = MODE == 2 ? p.dv - 1 : p.dv;
     if (!outputs) return launch_added<TI, MODE>(p, n_chunks, stream);
     if constexpr (MODE == 5)                            // two heads that share q and k: their products once
-        if (dvv <= 64 && p.qk_group % 2 == 0) return launch_output<TI, MODE, 2, 2>(p, n_chunks, stream);
-    return dvv > 64 ? launch_output<TI, MODE, 2, 1>(p, n_chunks, stream) : launch_output<TI, MODE, MODE == 1 || MODE == 4 ? 1 : 2, 1>(p, n_chunks, stream);
+        if (p.dv <= 64 && p.qk_group % 2 == 0) return launch_output<TI, MODE, 2>(p, n_chunks, stream);
+    return launch_output<TI, MODE, 1>(p, n_chunks, stream);
 }
 
 template <typename TI>
@@ -946,7 +919,7 @@ QS_API int qs_scan_activate(float* out, const void* q, long long ldq, const void
 int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                    int dtype, const float* dlog, long long ldd, const float* head_decay, const void* bonus, int bonus_dtype, int H, int dk, int dv,
                    const int32_t* chunk_start, int n_chunks, int T_rows, float* chunk_state, float* chunk_decay, const float* ga, const float* gb,
-                   long long ldg, float q_scale, int qk_group, float decay_scale, int32_t* status, cudaStream_t stream) {
+                   long long ldg, float q_scale, int qk_group, float decay_scale, float* chunk_factors, int32_t* status, cudaStream_t stream) {
     const size_t item = dtype == QS_F32 ? 4 : 2;
     auto fours = [&](const void* ptr, long long ld, int per_head) { return (int)(per_head % 4 == 0 && ld % 4 == 0 && ((uintptr_t)ptr % (4 * item)) == 0); };
     Scan p = {};
@@ -956,7 +929,8 @@ int qs_scan_chunks(int mode, int outputs, float* o, long long ldo, const void* q
     p.o = o; p.ldo = (size_t)ldo; p.H = H; p.dk = dk; p.dv = dv; p.dvp = (dv + 3) / 4 * 4; p.qk_group = qk_group;
     p.q_scale = q_scale; p.decay_scale = decay_scale;
     p.vec_q = fours(q, ldq, dk); p.vec_k = fours(k, ldk, dk); p.vec_v = fours(v, ldv, mode == 2 ? dv - 1 : dv);
-    p.vec_o = mode != 2 && dv % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)o % 16) == 0;
+    p.factors = chunk_factors;
+    p.vec_d = dk % 4 == 0 && ((uintptr_t)chunk_factors % 16) == 0;
     p.n_chunks = n_chunks; p.T_rows = T_rows; p.status = status;
     return dtype == QS_F32 ? pick<float>(mode, p, n_chunks, outputs != 0, stream) : pick<__nv_bfloat16>(mode, p, n_chunks, outputs != 0, stream);
 }

@@ -1,4 +1,4 @@
-// Tiles of 64 tokens as operands of 32-bit products on the CUDA cores: what the kernels over a prompt's chunks share.
+// Chunks of 64 tokens: loads, staged tiles and the sums over pairs of tokens with a decay per channel, on the CUDA cores.
 #pragma once
 
 #include "common.cuh"
@@ -6,7 +6,6 @@
 namespace {
 
 constexpr int CT = 64;                                  // tokens of a chunk
-constexpr int THREADS = 128;
 constexpr int PP = CT + 4;                              // pitch of a chunk's weights P[j][t]
 
 // Where channel c's column of a staged [channels][64 tokens] tile lies: tokens in groups of four, permuted by the channel's
@@ -88,65 +87,6 @@ __device__ __forceinline__ void scale_four(float* at, float d) {
     float4 v = *reinterpret_cast<float4*>(at);
     v.x *= d; v.y *= d; v.z *= d; v.w *= d;
     *reinterpret_cast<float4*>(at) = v;
-}
-
-// acc[8][4 NC] += A[k][8 rows] B[k][4 NC columns] over k < n: A a [k][64] tile (rows 4 ty .. and 32 + 4 ty ..; SKEW: swizzled as by
-// at_ct), B rows of 64 NC columns (4 tx .. of every 64).
-template <int NC, bool SKEW>
-__device__ __forceinline__ void tile_product(f32x2 (&acc)[8][2 * NC], const float* __restrict__ A, const float* __restrict__ B, int n, int ty, int tx) {
-#pragma unroll 4
-    for (int k = 0; k < n; ++k) {
-        const float4 x = *reinterpret_cast<const float4*>(A + (SKEW ? at_ct(k, ty * 4) : k * CT + ty * 4));
-        const float4 y = *reinterpret_cast<const float4*>(A + (SKEW ? at_ct(k, 32 + ty * 4) : k * CT + 32 + ty * 4));
-        const float a[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-        f32x2 b[2 * NC];
-#pragma unroll
-        for (int g = 0; g < NC; ++g) {
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(B + k * 64 * NC + g * 64 + tx * 4);
-            b[2 * g] = w.x;
-            b[2 * g + 1] = w.y;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const f32x2 aa = pack2(a[i], a[i]);
-#pragma unroll
-            for (int j = 0; j < 2 * NC; ++j) acc[i][j] = fma2(aa, b[j], acc[i][j]);
-        }
-    }
-}
-
-// acc[t][columns] += sum over j <= t of P[j][t] V[j][columns]: tokens j of the first 32 meet every t, the others only the last 32.  NH = 2: the
-// columns' halves have weights of their own, one below the other.  LATER_ONLY: a weight of zero is not multiplied, for values that
-// are not finite.
-template <int NC, int NH, bool LATER_ONLY>
-__device__ __forceinline__ void add_values(f32x2 (&acc)[8][2 * NC], const float* __restrict__ P, const float* __restrict__ V, int n, int ty, int tx) {
-#pragma unroll 2
-    for (int j = 0; j < n; ++j) {
-        f32x2 b[2 * NC];
-#pragma unroll
-        for (int g = 0; g < NC; ++g) {
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(V + j * 64 * NC + g * 64 + tx * 4);
-            b[2 * g] = w.x;
-            b[2 * g + 1] = w.y;
-        }
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            if (g == 0 && j >= 32) continue;
-#pragma unroll
-            for (int x = 0; x < NH; ++x) {
-                const float4 w = *reinterpret_cast<const float4*>(P + (x * CT + j) * PP + g * 32 + ty * 4);
-                const float a[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (LATER_ONLY && g * 32 + ty * 4 + i < j) continue;
-                    const f32x2 aa = pack2(a[i], a[i]);
-#pragma unroll
-                    for (int y = 0; y < 2 * NC; ++y)
-                        if (NH == 1 || (y >> 1) == x) acc[g * 4 + i][y] = fma2(aa, b[y], acc[g * 4 + i][y]);
-                }
-            }
-        }
-    }
 }
 
 }  // namespace
