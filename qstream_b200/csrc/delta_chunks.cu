@@ -15,7 +15,7 @@
 //
 // All 32-bit; decays only as products of factors up to one.  Three walks of every chunk token by token (what it does to an
 // identity, what it writes from nothing, its outputs) and a product of dk x dk matrices in the prefix stood here before: 2,000 tokens, 16
-// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 426 (the terms 108, the walk 133, the outputs 56).
+// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 375 (the terms 108, the walk 113, the outputs 30).
 #include "scan.cuh"
 #include "scan_tiles.cuh"
 #include "term_tiles.cuh"
@@ -30,13 +30,14 @@ struct Delta {
     size_t ldq, ldk, ldv, ldg, ldb;
     const int32_t *chunk_start, *seq_chunk, *seq_slot;
     float *W, *K, *Q;                                   // [chunks][H][64][dkp]: the solution's W, k times the decays behind it, q times those before
+    __nv_bfloat16 *K3;                                  // up to 128 channels, instead of K: its terms [chunks][H][3][64][dk8]
     float *U;                                           // [chunks][H][64][dvp]
     float *B;                                           // [chunks][H][64 j][64 t]
     float *decay;                                       // [chunks][H][dkp]
     float *start;                                       // [chunks][H][dk][dvp]: the states the chunks start from
     float *state; size_t slot_stride;
     float *o; size_t ldo;
-    int H, dk, dv, dkp, dvp, group, n_chunks, T_rows;
+    int H, dk, dv, dkp, dvp, dk8, group, n_chunks, T_rows;
     int vec_q, vec_k, vec_g;
 };
 
@@ -57,6 +58,9 @@ static_assert(GROUPS * (2 * CROSS + 4 * OWN) + CT * CT <= 3 * PASS * CT, "the gr
 __device__ __forceinline__ int at_pass(int c, int t) { return c * CT + (t ^ (((c ^ (c >> 2)) & 7) << 2)); }
 __device__ __forceinline__ void group_wait(int group) { asm volatile("bar.sync %0, 64;" :: "r"(1 + group) : "memory"); }
 
+// TERM_PLANES: K goes on as terms, split once instead of by every block of the walk (W as terms too: six 2-byte stores for two 4-byte ones in
+// the unrolled substitution, 130 us instead of 106).
+template <bool TERM_PLANES>
 __global__ void __launch_bounds__(TERMS, 2)
 delta_terms_kernel(Delta p) {
     extern __shared__ __align__(16) float smem[];
@@ -185,7 +189,7 @@ delta_terms_kernel(Delta p) {
         group_wait(group);
         cross_product<3, GCH, at_pass>(x3, X, sk, c0, lane);
         // relative to the chunk's ends, for the products with the states
-        if (i0 + i < p.dkp) {
+        if (i0 + i < (TERM_PLANES ? p.dk8 : p.dkp)) {  // zeros from dk on
             float e0[4], e1[4], e2[4], e3[4];
 #pragma unroll
             for (int y = 0; y < 4; ++y) {
@@ -194,7 +198,8 @@ delta_terms_kernel(Delta p) {
                 e2[y] = e1[y] * edge[2 * PASS + i + y];
                 e3[y] = edge[3 * PASS + i + y];
             }
-            if (second && lane < 8)
+            const bool in = !TERM_PLANES || i0 + i < p.dkp;
+            if (second && lane < 8 && in)
                 *reinterpret_cast<float4*>(p.decay + unit * p.dkp + i0 + i) = make_float4(e2[0] * e3[0], e2[1] * e3[1], e2[2] * e3[2], e2[3] * e3[3]);
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
@@ -209,9 +214,18 @@ delta_terms_kernel(Delta p) {
                     w[y] = sw[from] * before;
                     k[y] = sk[from] * (b == 3 ? 1.f : e3[y]);
                 }
-                *reinterpret_cast<float4*>(p.Q + at) = make_float4(q[0], q[1], q[2], q[3]);
-                *reinterpret_cast<float4*>(p.W + at) = make_float4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<float4*>(p.K + at) = make_float4(k[0], k[1], k[2], k[3]);
+                if (in) {
+                    *reinterpret_cast<float4*>(p.Q + at) = make_float4(q[0], q[1], q[2], q[3]);
+                    *reinterpret_cast<float4*>(p.W + at) = make_float4(w[0], w[1], w[2], w[3]);
+                }
+                if (TERM_PLANES) {
+                    uint32_t a[3], b[3];
+                    terms_of(pack2(k[0], k[1]), a[0], a[1], a[2]);
+                    terms_of(pack2(k[2], k[3]), b[0], b[1], b[2]);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                        *reinterpret_cast<uint2*>(p.K3 + ((unit * 3 + x) * CT + t) * p.dk8 + i0 + i) = make_uint2(a[x], b[x]);
+                } else *reinterpret_cast<float4*>(p.K + at) = make_float4(k[0], k[1], k[2], k[3]);
             }
         }
         group_wait(group);
@@ -448,10 +462,12 @@ delta_walk_kernel(Delta p) {
 // one head's state, each of its eight warps 16 channels of it in registers; the state's terms, u's and those of W and K lie in shared memory.
 //   1  W S: a warp takes 16 tokens and half of the channels; the halves meet in shared memory, u = U - W S, as terms
 //   2  S <- decay S + K^T u: a warp's 16 channels over all 64 tokens; the state's terms
-// W of the next chunk becomes terms while u is formed, K behind the second step; the one after that is on its way in registers.
+// W of the next chunk becomes terms while u is formed (the one after that is on its way in registers), K is copied in behind the second
+// step, as terms that the kernel before has split.
 //
-// A chain of 32 steps for 2,000 tokens.  By multiply-adds a step took 4.2 us (shared memory's pipe: eight 16-byte reads per 32 paired
-// multiply-adds), 133 us in all.
+// A chain of 32 steps for 2,000 tokens of 16 heads of 128 x 128.  By multiply-adds a step took 4.2 us (shared memory's pipe: eight 16-byte reads per 32 paired
+// multiply-adds), 133 us in all; with each block splitting W and K for itself 119; now
+// 113.  With sixteen warps, each half of the columns: 119 (64 channels: 4 us less of 73).
 // MC channels, 64 or 128; pitches of W and K, of S and u: rows of 16 bytes meet all banks
 constexpr int SP = WC + 8;
 template <int MC> constexpr int mma_walk_smem() { return (2 * 3 * CT * (MC + 8) + 3 * MC * SP + 3 * CT * SP) * 2 + CT * WC * 4; }
@@ -473,7 +489,7 @@ __device__ __forceinline__ void put_two(__nv_bfloat16* at, int term, float x, fl
 template <int MC>
 __global__ void __launch_bounds__(2 * MC)
 delta_walk_mma_kernel(const __grid_constant__ Delta p) {
-    constexpr int MP = MC + 8, WALKERS = 2 * MC, ROW = MC / 4, PARTS = MC / 64;
+    constexpr int MP = MC + 8, WALKERS = 2 * MC, PARTS = MC / 64;
     extern __shared__ __align__(16) float smem[];
     __nv_bfloat16* const tw = reinterpret_cast<__nv_bfloat16*>(smem);      // [3][64 tokens][MP]
     __nv_bfloat16* const tk = tw + 3 * CT * MP;
@@ -505,30 +521,44 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
     };
     each([&](float& v, int i, int col) { v = i < p.dk && col < n_cols ? own[(size_t)col * p.dk + i] : 0.f; });
     put_state();
-    constexpr int PIECES = CT * MC / 4 / WALKERS;         // of four channels, of a thread
-    float4 rw[PIECES], rk[PIECES];
-    auto fetch = [&](float4 (&r)[PIECES], const float* from, int c) {
+    // W of a chunk on its way to registers, and as terms to shared memory; the terms of K on their way there (columns behind dk8 stay zeros)
+    constexpr int ROW = MC / 4, PIECES = CT * ROW / WALKERS;
+    float4 rw[PIECES];
+    auto whole = [&](int c) {
         const int n = c < c1 ? p.chunk_start[c + 1] - p.chunk_start[c] : 0;
-        const float* base = from + ((size_t)c * p.H + h) * CT * dkp;
+        return n > 0 && n <= CT;
+    };
+    const int w_at = tid / ROW, w_i = tid % ROW * 4;
+    auto fetch_w = [&](int c) {
+        const bool have = whole(c) && w_i < dkp;
+        const float* from = p.W + (((size_t)c * p.H + h) * CT + w_at) * dkp + w_i;
 #pragma unroll
-        for (int x = 0; x < PIECES; ++x) {
-            const int e = tid + x * WALKERS, t = e / ROW, i = e % ROW * 4;
-            r[x] = n > 0 && n <= CT && i < dkp ? *reinterpret_cast<const float4*>(base + (size_t)t * dkp + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int x = 0; x < PIECES; ++x) rw[x] = have ? *reinterpret_cast<const float4*>(from + x * (WALKERS / ROW) * dkp) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto put_w = [&]() {
+#pragma unroll
+        for (int x = 0; x < PIECES; ++x) put_four(tw + (w_at + x * (WALKERS / ROW)) * MP + w_i, CT * MP, rw[x]);
+    };
+    constexpr int KROW = MC / 8;
+    const int k_at = tid / KROW, k_i = tid % KROW * 8;
+    const uint32_t k_to = (uint32_t)__cvta_generic_to_shared(tk) + (k_at * MP + k_i) * 2;
+    auto copy_k = [&](int c) {
+        if (whole(c) && k_i < p.dk8) {
+            const __nv_bfloat16* from = p.K3 + (((size_t)c * p.H + h) * 3 * CT + k_at) * p.dk8 + k_i;
+#pragma unroll
+            for (int x = 0; x < 3 * CT * KROW / WALKERS; ++x)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(k_to + x * (WALKERS / KROW) * MP * 2), "l"(from + x * (WALKERS / KROW) * p.dk8) : "memory");
         }
     };
-    auto put = [&](__nv_bfloat16* to, const float4 (&r)[PIECES]) {
-#pragma unroll
-        for (int x = 0; x < PIECES; ++x) {
-            const int e = tid + x * WALKERS;
-            put_four(to + e / ROW * MP + e % ROW * 4, CT * MP, r[x]);
-        }
-    };
-    fetch(rw, p.W, c0);
-    fetch(rk, p.K, c0);
-    put(tw, rw);
-    put(tk, rk);
-    fetch(rw, p.W, c0 + 1);
-    fetch(rk, p.K, c0 + 1);
+    if (p.dk8 < MC) {
+        for (int e = tid; e < 3 * CT * MP / 2; e += WALKERS) reinterpret_cast<uint32_t*>(tk)[e] = 0u;
+        __syncthreads();
+    }
+    fetch_w(c0);
+    copy_k(c0);
+    put_w();
+    fetch_w(c0 + 1);
+    copies_done();
     const uint32_t aw = (uint32_t)__cvta_generic_to_shared(tw), ak = (uint32_t)__cvta_generic_to_shared(tk);
     const uint32_t as = (uint32_t)__cvta_generic_to_shared(ts), au = (uint32_t)__cvta_generic_to_shared(tu);
     __syncthreads();
@@ -565,10 +595,10 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
             each([&](float& v, int i, int at) { v = i < p.dk ? sS[i * 17 + at] : 0.f; });
             __syncthreads();
             put_state();
-            put(tw, rw);
-            put(tk, rk);
-            fetch(rw, p.W, c + 2);
-            fetch(rk, p.K, c + 2);
+            put_w();
+            fetch_w(c + 2);
+            copy_k(c + 1);
+            copies_done();
             __syncthreads();
             continue;
         }
@@ -626,8 +656,9 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
                     put_two(tu + t * SP + col, CT * SP, v.x, v.y);
                     if (col < n_cols) *reinterpret_cast<float2*>(p.U + (unit * CT + t) * p.dvp + col0 + col) = v;
                 }
-        put(tw, rw);
-        fetch(rw, p.W, c + 2);
+        put_w();                                        // behind the barrier: nobody reads W any more
+        fetch_w(c + 2);
+        copies_done();                                  // this chunk's K
         __syncthreads();
         // 2
         float more[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -650,8 +681,7 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
                 for (int e = 0; e < 2; ++e) S[x][z][e] = fmaf(d[x], S[x][z][e], more[z][2 * x + e]);
         put_state();
         __syncthreads();
-        put(tk, rk);
-        fetch(rk, p.K, c + 2);
+        copy_k(c + 1);
     }
     each([&](float& v, int i, int col) { if (i < p.dk && col < n_cols) own[(size_t)col * p.dk + i] = v; });
 }
@@ -793,7 +823,8 @@ delta_output_kernel(const __grid_constant__ Delta p, int32_t* __restrict__ statu
 // Floats of scratch that `qs_delta_chunks` takes.
 QS_API long long qs_delta_chunks_scratch(int n_chunks, int H, int dk, int dv) {
     const long long dkp = (dk + 3) / 4 * 4, dvp = (dv + 3) / 4 * 4;
-    return (long long)n_chunks * H * (CT * (3 * dkp + dvp + CT) + dkp + dk * dvp);
+    const long long k_or_terms = dk <= 128 ? (3 * ((dk + 7) / 8 * 8) + 1) / 2 : dkp;       // K, or its terms
+    return (long long)n_chunks * H * (CT * (2 * dkp + k_or_terms + dvp + CT) + dkp + dk * dvp);
 }
 
 // q, k [T, (H / group) dk], v [T, H dv], g [T, H dk] (decays), beta [T, H], all float32; o [T, H dv]; state float32 [slots][H][dv][dk].
@@ -809,18 +840,21 @@ QS_API int qs_delta_chunks(float* o, long long ldo, const float* q, long long ld
     Delta p = {};
     p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta; p.ldq = (size_t)ldq; p.ldk = (size_t)ldk; p.ldv = (size_t)ldv; p.ldg = (size_t)ldg; p.ldb = (size_t)ldb;
     p.chunk_start = chunk_start; p.seq_chunk = seq_chunk; p.seq_slot = seq_slot; p.state = state; p.slot_stride = (size_t)slot_stride;
-    p.o = o; p.ldo = (size_t)ldo; p.H = H; p.dk = dk; p.dv = dv; p.dkp = (dk + 3) / 4 * 4; p.dvp = (dv + 3) / 4 * 4; p.group = group;
+    p.o = o; p.ldo = (size_t)ldo; p.H = H; p.dk = dk; p.dv = dv; p.dkp = (dk + 3) / 4 * 4; p.dvp = (dv + 3) / 4 * 4; p.dk8 = (dk + 7) / 8 * 8; p.group = group;
     p.n_chunks = n_chunks; p.T_rows = T_rows; p.vec_q = fours(q, ldq); p.vec_k = fours(k, ldk); p.vec_g = fours(g, ldg);
     const size_t units = (size_t)n_chunks * H;
     p.W = scratch;
+    const bool terms = dk <= 128;
     p.K = p.W + units * CT * p.dkp;
-    p.Q = p.K + units * CT * p.dkp;
+    p.K3 = reinterpret_cast<__nv_bfloat16*>(p.K);
+    p.Q = p.K + units * CT * (terms ? (3 * p.dk8 + 1) / 2 : p.dkp);
     p.U = p.Q + units * CT * p.dkp;
     p.B = p.U + units * CT * p.dvp;
     p.decay = p.B + units * CT * CT;
     p.start = p.decay + units * p.dkp;
-    cudaError_t e = cudaFuncSetAttribute(delta_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TERMS_SMEM);
-    if (e == cudaSuccess) e = qs_launch_dependent(delta_terms_kernel, dim3(n_chunks, H), dim3(TERMS), TERMS_SMEM, stream, p);
+    const auto terms_kernel = terms ? delta_terms_kernel<true> : delta_terms_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TERMS_SMEM);
+    if (e == cudaSuccess) e = qs_launch_dependent(terms_kernel, dim3(n_chunks, H), dim3(TERMS), TERMS_SMEM, stream, p);
     const dim3 blocks(n_seq, H, (dv + WC - 1) / WC);
     if (p.dkp <= 64) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_walk_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_walk_smem<64>());
