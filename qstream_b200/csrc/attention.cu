@@ -8,6 +8,8 @@
 // p % page_tokens.  A token with slot < 0 is padding: nothing is read or written for it.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace {
 
 // ----------------------------------------------------------------------------- rotary + store
@@ -197,8 +199,8 @@ __device__ __forceinline__ void rotate_halves(uint4& lo, uint4& hi, const float*
     hi = make_uint4(b[0], b[1], b[2], b[3]);
 }
 
-// HALF: the pairs are (i, i + R / 2); R / 2 is then a multiple of 8 (other widths go the general way, an element at a time: 14 us for 2,047 rows of
-// 16 + 4 heads of 128 with 64 rotated dims against 10 in pieces, of which the call sees 4).
+// HALF: the pairs are (i, i + R / 2); R / 2 is then a multiple of 8 (other widths go the general way, an element at a time: attention over
+// 2,047 rows of 16 + 4 heads of 128 with 64 rotated dims, projections included, takes 121 us with that and 117 with this).
 template <bool HALF>
 __global__ void rope_store_vec_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                                       const __nv_bfloat16* __restrict__ v, size_t ldq, size_t ldk, size_t ldv,
@@ -409,28 +411,35 @@ attention_kernel(TO* __restrict__ out, const T* __restrict__ q, size_t ldo, size
     }
 }
 
-// The same for steps that bring many tokens per sequence, in the float32 engine: a block takes up to 64 consecutive rows of the
+// The same for steps that bring many tokens per sequence, in the float32 engine: a block takes up to 32 consecutive rows of the
 // packed batch and one query head, and walks the sequence's keys 64 at a time with q, keys and values in shared memory.
 // Every sum has the order of `attention_kernel` (groups of 32 keys, ascending dims, the same tree over a group's
 // weights), so a row's result is the same bits whichever of the two kernels computes it.  With `seq_start` a block's rows are
-// those of one sequence (its first 64, its next 64 ..), so that the walks of short sequences run side by side; without, the batch is cut
-// every 64 rows and a block makes one walk per sequence, the other rows masked.
+// those of one sequence (its first 32, its next 32 ..), so that the walks of short sequences run side by side; without, the batch is cut
+// every 32 rows and a block makes one walk per sequence, the other rows masked.
 //
-// 128 threads as 8 row groups x 16: a thread scores 8 rows x 4 keys and then accumulates 8 rows x 4 NG dims.  Within a group of
-// 32 keys lane l of eight holds keys l, l + 8, l + 16, l + 24, so that the sum over the group has the butterfly's order.
-// Bound by shared-memory reads and multiply-add issue; the warp-per-query kernel reads every key from L1 once per
-// query.  Two prompts of 400 and 300 tokens, 16 heads of 128: 181 us; `attention_kernel`: 1,150 us.
+// A thread scores 4 rows x 4 keys and then accumulates 4 rows x 4 NG dims, of heads above 128 two rows.  Within a group of
+// 32 keys lane l of eight holds keys l, l + 8, l + 16, l + 24, so that the sum over the group has the butterfly's order; the groups' maxima and
+// sums meet in shared memory.
+//
+// Long prompts are bound by shared memory's pipe (a cycle per register that a warp fills, broadcast or not: 56 % of its rate at 4 rows a
+// thread, 82 % at two), short ones by the longest walk and by what SM two long walks meet on: with 64 rows to a block, all blocks of a head side by
+// side and 8 rows to a thread half of the SMs stood idle.  Microseconds, 16 heads, before | 32 rows and 256 threads | 32 rows and 128 threads:
+//   heads of 128: 400 + 300 tokens 161 | 96 | 96, 2,000 tokens 1,065 | 745 | 674; heads of 64: 101 | 68 | 68, 2,000 tokens - | 440 | 336;
+//   heads of 256: 302 | 162 | 193, 2,000 tokens - | 1,630 | 1,741.  `attention_kernel` takes 1,150 for the first.
 //
 // Weights of keys that a row does not see are stored as -1 and skipped, as there, so that a value that is not finite
 // reaches only the rows that see it.
-constexpr int TQ = 64, TK = 64;
+constexpr int TQ = 32, TK = 64;
+template <int NG> constexpr int tile_threads() { return NG == 4 ? 256 : 128; }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
 template <int NG>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(tile_threads<NG>(), NG == 4 ? 1 : NG == 2 ? 2 : 4)
 attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size_t ldo, size_t ldq,
                       const float* __restrict__ k_cache, const float* __restrict__ v_cache,
                       const int32_t* __restrict__ page_table, int max_pages, int page_shift,
@@ -438,30 +447,33 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
                       int T_tokens, int n_heads, int n_kv_heads, int dh, float scale, int window,
                       int32_t* __restrict__ status, int dv, float softcap, int chunk, int keep_first,
                       const float* __restrict__ sink, int maps, const int32_t* __restrict__ seq_start, int n_seq) {
+    constexpr int TILE_THREADS = tile_threads<NG>(), RT = TQ * 16 / TILE_THREADS, ROW_WARPS = TILE_THREADS / 64;        // RT: rows of a thread
+    struct __align__(RT * 4) Rows { float x[RT]; };
     extern __shared__ __align__(16) float tile_smem[];
-    __shared__ int s_slot[TQ], s_pos[TQ], s_first[TQ], s_kept[TQ], s_ok[TK], s_end;
-    __shared__ float s_alpha[2][TQ];
+    __shared__ int s_slot[TQ], s_pos[TQ], s_first[TQ], s_kept[TQ], s_at[2][TK];
+    __shared__ float s_top[2][TQ], s_sum[2][TQ];
     const int pitch = dh + 4, vp = NG * 64;
     float* sq = tile_smem;                              // [dh][TQ + 4]: transposed, so that neighbouring rows form pairs
-    float* sk = sq + dh * (TQ + 4);                      // [TK][pitch]; after the scores the weights [TK][TQ + 4] lie here
-    float* sp = sk;
-    float* sv = sk + TK * (pitch > TQ + 4 ? pitch : TQ + 4);      // [TK][vp]
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int head = blockIdx.y;
-    int row0 = (gridDim.x - 1 - blockIdx.x) * TQ, n_rows = min(TQ, T_tokens - row0);     // the longest contexts first
+    float* sk = sq + dh * (TQ + 4);                      // [TK][pitch]
+    float* sv = sk + TK * pitch;                        // [TK][vp]
+    float* sp = sv + TK * vp;                           // [TK][TQ + 4]: the weights
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // neighbouring blocks take the heads of one tile of rows
+    const int head = blockIdx.x % n_heads, number = blockIdx.x / n_heads;
+    int row0 = (gridDim.x / n_heads - 1 - number) * TQ, n_rows = min(TQ, T_tokens - row0);     // the longest contexts first
     if (seq_start) {                                    // the block's sequence: tiles counted from the last rows, a lane per sequence
         __shared__ int s_row0, s_rows;
         if (tid == 0) s_rows = 0;
         if (tid < 32) {
             int run = 0;
-            for (int base = 0; base <= n_seq && run <= (int)blockIdx.x; base += 32) {
+            for (int base = 0; base <= n_seq && run <= number; base += 32) {
                 const int s = n_seq - base - tid;       // number n_seq: the rows behind the last sequence
                 const int lo = s >= 0 ? seq_start[s] : 0, hi = s < 0 ? 0 : s < n_seq ? min(seq_start[s + 1], T_tokens) : T_tokens;
                 const int tiles = hi > lo ? (hi - lo + TQ - 1) / TQ : 0;
                 int sum = tiles;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (tid >= o) sum += v; }
-                const int at = (int)blockIdx.x - (run + sum - tiles);
+                const int at = number - (run + sum - tiles);
                 if (at >= 0 && at < tiles) {
                     s_row0 = lo + (tiles - 1 - at) * TQ;
                     s_rows = min(TQ, hi - s_row0);
@@ -484,180 +496,215 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
         s_first[tid] = first;
         s_kept[tid] = min(keep_first, first);
     }
-    for (int e = tid; e < TQ * (dh / 4); e += 128) {
+    for (int e = tid; e < TQ * (dh / 4); e += TILE_THREADS) {
         const int r = e % TQ, d = e / TQ * 4;           // neighbouring lanes on neighbouring rows: their stores meet different banks
         const float4 x = r < n_rows ? *reinterpret_cast<const float4*>(q + (size_t)(row0 + r) * ldq + (size_t)head * dh + d) : make_float4(0.f, 0.f, 0.f, 0.f);
         float* dst = sq + d * (TQ + 4) + r;
         dst[0] = x.x; dst[TQ + 4] = x.y; dst[2 * (TQ + 4)] = x.z; dst[3 * (TQ + 4)] = x.w;
     }
     if (vp > dv)                                        // columns of no value: zeros, once
-        for (int e = tid; e < TK * (vp - dv); e += 128) sv[(e / (vp - dv)) * vp + dv + e % (vp - dv)] = 0.f;
-    auto row_of = [&](int i) { return (i >> 2) * 32 + ty * 4 + (i & 3); };
-    const int half = tx >> 3, sub = tx & 7;
+        for (int e = tid; e < TK * (vp - dv); e += TILE_THREADS) sv[(e / (vp - dv)) * vp + dv + e % (vp - dv)] = 0.f;
+    // a warp: its rows against one half of the keys, and against one half of the dims
+    const int half = warp / ROW_WARPS, column = half * (NG * 32) + (lane & 7) * 4, sub = lane & 7, row = warp % ROW_WARPS * 4 * RT + (lane >> 3) * RT;
+    // 64 rows of `pieces` 16-byte pieces from the cache to shared memory, zeros where there is no key
+    auto copy_rows = [&](float* to, int to_pitch, const float* from, size_t from_pitch, const int* at, int pieces) {
+        int r = tid / pieces, d = tid % pieces;
+        const int step_r = TILE_THREADS / pieces, step_d = TILE_THREADS % pieces;
+        while (r < TK) {
+            float* dst = to + r * to_pitch + d * 4;
+            if (at[r] >= 0) cp_async16(dst, from + (size_t)at[r] * from_pitch + d * 4);
+            else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+            r += step_r;
+            d += step_d;
+            if (d >= pieces) { d -= pieces; ++r; }
+        }
+        cp_async_commit();
+    };
 
     for (int r0 = 0; r0 < n_rows;) {
         __syncthreads();
         const int slot = s_slot[r0];
-        if (tid == 0) {
-            int r = r0 + 1;
-            while (r < n_rows && s_slot[r] == slot) ++r;
-            s_end = r;
-        }
-        __syncthreads();
-        const int r1 = s_end;
+        int r1 = n_rows;
+#pragma unroll
+        for (int r = lane; r < TQ; r += 32)
+            if (r > r0 && r < n_rows && s_slot[r] != slot) r1 = min(r1, r);
+        r1 = __reduce_min_sync(0xffffffffu, r1);
         if (slot < 0) {                                 // padding: defined output, no cache access
-            for (int e = tid; e < (r1 - r0) * dv; e += 128) out[(size_t)(row0 + r0 + e / dv) * ldo + (size_t)head * dv + e % dv] = 0.f;
+            for (int e = tid; e < (r1 - r0) * dv; e += TILE_THREADS) out[(size_t)(row0 + r0 + e / dv) * ldo + (size_t)head * dv + e % dv] = 0.f;
             r0 = r1;
             continue;
         }
         int lo = 0x7fffffff, hi = 0, kept = 0, all_from = 0, all_to = 0x7fffffff;     // keys some row sees; keys all rows see
-        for (int r = r0; r < r1; ++r) {
+#pragma unroll
+        for (int r = lane; r < TQ; r += 32) {
+            if (r < r0 || r >= r1) continue;
             lo = min(lo, s_first[r]);
             hi = max(hi, s_pos[r] + 1);
             kept = max(kept, s_kept[r]);
             all_from = max(all_from, s_first[r]);
             all_to = min(all_to, s_pos[r] + 1);
         }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        kept = __reduce_max_sync(0xffffffffu, kept);
+        all_from = __reduce_max_sync(0xffffffffu, all_from);
+        all_to = __reduce_min_sync(0xffffffffu, all_to);
         const int32_t* pages = page_table + (size_t)slot * max_pages;
-        float m[8], l[8];
-        f32x2 acc[8][2 * NG];
+        float m[RT], l[RT];
+        f32x2 acc[RT][2 * NG];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < RT; ++i) {
             m[i] = -INFINITY;
             l[i] = 0.f;
 #pragma unroll
             for (int j = 0; j < 2 * NG; ++j) acc[i][j] = 0ull;
         }
-        for (int base = kept > 0 ? 0 : lo / TK * TK; base < hi; base += TK) {
-            if (base >= kept && base + TK <= lo) base = lo / TK * TK;
-            __syncthreads();                            // the last block's weights and values have been used
-            if (tid < TK) {
-                const int key = base + tid;
-                int at = -1;
-                if (key < hi && (key >= lo || key < kept)) {
-                    const int page = pages[key >> page_shift];
-                    if (page < 0) atomicExch(status, 3);
-                    else at = (page * n_kv_heads + kvh) * page_tokens + (key & (page_tokens - 1));
-                }
-                s_ok[tid] = at;
+        // tiles that hold only keys between the kept ones and the first are stepped over
+        auto tile_from = [&](int base) { return base >= kept && base + TK <= lo ? lo / TK * TK : base; };
+        auto held = [&](int key) { return key < hi && (key >= lo || key < kept); };
+        int page = 0;
+        auto next_page = [&](int base) { if (tid < TK && held(base + tid)) page = pages[(base + tid) >> page_shift]; };
+        auto put_places = [&](int* at, int base) {      // where the tile's keys lie, from the pages fetched before
+            if (tid >= TK) return;
+            const int key = base + tid;
+            int place = -1;
+            if (held(key)) {
+                if (page < 0) atomicExch(status, 3);
+                else place = (page * n_kv_heads + kvh) * page_tokens + (key & (page_tokens - 1));
             }
+            at[tid] = place;
+        };
+        int base = tile_from(kept > 0 ? 0 : lo / TK * TK), buf = 0;
+        next_page(base);
+        put_places(s_at[0], base);
+        next_page(tile_from(base + TK));
+        __syncthreads();
+        copy_rows(sk, pitch, k_cache + k_off, krow_width, s_at[0], dh / 4);
+        for (; base < hi; buf ^= 1) {
+            // on their way: this tile's values while it is scored, the next one's keys while the values are added, the pages of the one after that
+            const int next = tile_from(base + TK);
+            const int* s_ok = s_at[buf];
+            __syncthreads();                            // the last tile's weights and values have been used
+            copy_rows(sv, vp, v_cache, dv, s_ok, dv / 4);
+            put_places(s_at[buf ^ 1], next);
+            next_page(tile_from(next + TK));
+            cp_async_wait<1>();                         // the keys
             __syncthreads();
-            const int d4 = dh / 4, v4 = dv / 4;
-            for (int e = tid; e < TK * d4; e += 128) {
-                const int r = e / d4, d = (e - r * d4) * 4;
-                float* dst = sk + r * pitch + d;
-                if (s_ok[r] >= 0) cp_async16(dst, k_cache + (size_t)s_ok[r] * krow_width + k_off + d);
-                else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            for (int e = tid; e < TK * v4; e += 128) {
-                const int r = e / v4, d = (e - r * v4) * 4;
-                float* dst = sv + r * vp + d;
-                if (s_ok[r] >= 0) cp_async16(dst, v_cache + (size_t)s_ok[r] * dv + d);
-                else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            cp_async_wait();
-            __syncthreads();
-            f32x2 s2[4][4];                             // rows 2 i, 2 i + 1 of this thread's eight against its four keys
+            float sums[RT][4];                          // this thread's rows against its four keys
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RT; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
+                for (int j = 0; j < 4; ++j) sums[i][j] = 0.f;
+#pragma unroll 2
             for (int d = 0; d < dh; d += 4) {
                 float4 kk[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const float4*>(sk + (half * 32 + j * 8 + sub) * pitch + d);
 #pragma unroll
                 for (int y = 0; y < 4; ++y) {
-                    const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(sq + (d + y) * (TQ + 4) + ty * 4);
-                    const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(sq + (d + y) * (TQ + 4) + 32 + ty * 4);
+                    const Rows qv = *reinterpret_cast<const Rows*>(sq + (d + y) * (TQ + 4) + row);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float kv = y == 0 ? kk[j].x : y == 1 ? kk[j].y : y == 2 ? kk[j].z : kk[j].w;
-                        const f32x2 k2 = pack2(kv, kv);
-                        s2[0][j] = fma2(qa.x, k2, s2[0][j]);
-                        s2[1][j] = fma2(qa.y, k2, s2[1][j]);
-                        s2[2][j] = fma2(qb.x, k2, s2[2][j]);
-                        s2[3][j] = fma2(qb.y, k2, s2[3][j]);
+#pragma unroll
+                        for (int i = 0; i < RT; ++i) sums[i][j] = fmaf(qv.x[i], kv, sums[i][j]);
                     }
                 }
             }
-            __syncthreads();                            // the keys have been read: the weights go where they were
+            int ok[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = row_of(i), pos = s_pos[r], first = s_first[r], row_kept = s_kept[r];
+            for (int j = 0; j < 4; ++j) ok[j] = s_ok[half * 32 + j * 8 + sub];
+            bool live[RT][4];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const int r = row + i, pos = s_pos[r], first = s_first[r], row_kept = s_kept[r];
                 const bool mine = r >= r0 && r < r1;
-                float s[4];
-                bool live[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int at = half * 32 + j * 8 + sub, key = base + at;
-                    live[j] = mine && key <= pos && (key >= first || key < row_kept) && s_ok[at] >= 0;
-                    const float2 two = unpack2(s2[i >> 1][j]);
-                    s[j] = (i & 1 ? two.y : two.x) * scale;
-                    if (softcap > 0.f) s[j] = softcap * tanhf(s[j] / softcap);
-                    if (!live[j]) s[j] = -INFINITY;
+                    const int key = base + half * 32 + j * 8 + sub;
+                    live[i][j] = mine && key <= pos && (key >= first || key < row_kept) && ok[j] >= 0;
+                    float x = sums[i][j] * scale;
+                    if (softcap > 0.f) x = softcap * tanhf(x / softcap);
+                    sums[i][j] = live[i][j] ? x : -INFINITY;
                 }
-                float top = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+                float top = fmaxf(fmaxf(sums[i][0], sums[i][1]), fmaxf(sums[i][2], sums[i][3]));
 #pragma unroll
                 for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-                const float other = __shfl_xor_sync(0xffffffffu, top, 8);
-                const float m1 = fmaxf(m[i], half ? other : top), m2 = fmaxf(m1, half ? top : other);     // after the first, the second 32 keys
-                const float a1 = m[i] == -INFINITY ? 0.f : expf(m[i] - m1), a2 = m1 == -INFINITY ? 0.f : expf(m1 - m2);
+                if (sub == 0) s_top[half][r] = top;
+            }
+            __syncthreads();                            // the keys have been read
+            if (next < hi) copy_rows(sk, pitch, k_cache + k_off, krow_width, s_at[buf ^ 1], dh / 4);
+            else cp_async_commit();
+            Rows weight[4];
+            float a1[RT], a2[RT];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const int r = row + i;
+                const float m1 = fmaxf(m[i], s_top[0][r]), m2 = fmaxf(m1, s_top[1][r]);       // after the first, the second 32 keys
+                a1[i] = m[i] == -INFINITY ? 0.f : expf(m[i] - m1);
+                a2[i] = m1 == -INFINITY ? 0.f : expf(m1 - m2);
                 const float mm = half ? m2 : m1;
                 float p[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) p[j] = live[j] ? expf(s[j] - mm) : 0.f;
+                for (int j = 0; j < 4; ++j) p[j] = live[i][j] ? expf(sums[i][j] - mm) : 0.f;
                 float sum = (p[0] + p[2]) + (p[1] + p[3]);
 #pragma unroll
                 for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                const float osum = __shfl_xor_sync(0xffffffffu, sum, 8);
-                l[i] = l[i] * a1 + (half ? osum : sum);
-                l[i] = l[i] * a2 + (half ? sum : osum);
                 m[i] = m2;
-                if (tx == 0) { s_alpha[0][r] = a1; s_alpha[1][r] = a2; }
+                if (sub == 0) s_sum[half][r] = sum;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) sp[(half * 32 + j * 8 + sub) * (TQ + 4) + r] = live[j] ? p[j] : -1.f;
+                for (int j = 0; j < 4; ++j) weight[j].x[i] = live[i][j] ? p[j] : -1.f;
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<Rows*>(sp + (half * 32 + j * 8 + sub) * (TQ + 4) + row) = weight[j];
+            cp_async_wait<1>();                         // the values
             __syncthreads();
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                l[i] = l[i] * a1[i] + s_sum[0][row + i];
+                l[i] = l[i] * a2[i] + s_sum[1][row + i];
+            }
             const bool whole = r0 == 0 && r1 == TQ && base >= all_from && base + TK <= all_to;      // every row sees every key
-#pragma unroll 1
-            for (int g = 0; g < 2; ++g) {
-                if (base + g * 32 >= hi) break;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float a = s_alpha[g][row_of(i)];
-                    const f32x2 aa = pack2(a, a);
-#pragma unroll
-                    for (int j = 0; j < 2 * NG; ++j) acc[i][j] = mul2(aa, acc[i][j]);
-                }
+            auto add_values = [&](auto tested, int g) {
 #pragma unroll 4
                 for (int key = g * 32; key < g * 32 + 32; ++key) {
-                    float p[8];
                     f32x2 vv[2 * NG];
-                    const float4 pa = *reinterpret_cast<const float4*>(sp + key * (TQ + 4) + ty * 4);
-                    const float4 pb = *reinterpret_cast<const float4*>(sp + key * (TQ + 4) + 32 + ty * 4);
-                    p[0] = pa.x; p[1] = pa.y; p[2] = pa.z; p[3] = pa.w; p[4] = pb.x; p[5] = pb.y; p[6] = pb.z; p[7] = pb.w;
+                    const Rows p = *reinterpret_cast<const Rows*>(sp + key * (TQ + 4) + row);
 #pragma unroll
                     for (int j = 0; j < NG; ++j) {
-                        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sv + key * vp + j * 64 + tx * 4);
+                        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sv + key * vp + column + j * 32);
                         vv[2 * j] = x.x;
                         vv[2 * j + 1] = x.y;
                     }
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const f32x2 pp = pack2(p[i], p[i]);
-                        if (whole || !(p[i] < 0.f)) {
+                    for (int i = 0; i < RT; ++i) {
+                        const f32x2 pp = pack2(p.x[i], p.x[i]);
+                        if (!decltype(tested)::value || !(p.x[i] < 0.f)) {
 #pragma unroll
                             for (int j = 0; j < 2 * NG; ++j) acc[i][j] = fma2(pp, vv[j], acc[i][j]);
                         }
                     }
                 }
+            };
+#pragma unroll 1
+            for (int g = 0; g < 2; ++g) {
+                if (base + g * 32 >= hi) break;
+#pragma unroll
+                for (int i = 0; i < RT; ++i) {
+                    const float a = g ? a2[i] : a1[i];
+                    const f32x2 aa = pack2(a, a);
+#pragma unroll
+                    for (int j = 0; j < 2 * NG; ++j) acc[i][j] = mul2(aa, acc[i][j]);
+                }
+                if (whole) add_values(std::false_type{}, g);
+                else add_values(std::true_type{}, g);
             }
+            base = next;
         }
         const float sk_score = sink ? sink[head] : 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int r = row_of(i);
+        for (int i = 0; i < RT; ++i) {
+            const int r = row + i;
             if (r < r0 || r >= r1) continue;
             float alpha = 1.f;
             if (sink) {
@@ -669,7 +716,7 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
             float* o = out + (size_t)(row0 + r) * ldo + (size_t)head * dv;
 #pragma unroll
             for (int j = 0; j < 2 * NG; ++j) {
-                const int c = (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
+                const int c = column + (j >> 1) * 32 + (j & 1) * 2;
                 const float2 v = unpack2(acc[i][j]);
                 if (c < dv) o[c] = v.x * alpha * inv;
                 if (c + 1 < dv) o[c + 1] = v.y * alpha * inv;
@@ -680,7 +727,8 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
 }
 
 // Where the tile kernel serves: from 16 rows per sequence on (the mean: a tile of fewer rows is a block of its own), and with no more keys
-// than one group of 32 from 32 rows on.  Microseconds (tiles | a warp per query), heads of 128, 1 and 16 sequences of so many rows
+// than one group of 32 from 32 rows on.  Microseconds (tiles, with 64 rows to a block | a warp per query; with 32 rows 16 x 16 rows behind 500 keys take
+// 131 instead of 221, one prompt of 64 rows 18), heads of 128, 1 and 16 sequences of so many rows
 // behind so many cached keys:
 //              1 sequence, 16 heads                                         16 sequences, 16 heads
 //   rows       0 keys    48        112       500        2,000               0 keys     48         500          2,000
@@ -695,8 +743,7 @@ bool tiles_serve(long long rows, int n_seq, int longest) {
 }
 
 size_t tile_smem_bytes(int dh, int ng) {
-    const int pitch = dh + 4 > TQ + 4 ? dh + 4 : TQ + 4;
-    return (size_t)(dh * (TQ + 4) + TK * pitch + TK * ng * 64) * sizeof(float);
+    return (size_t)(dh * (TQ + 4) + TK * (dh + 4) + TK * ng * 64 + TK * (TQ + 4)) * sizeof(float);
 }
 
 template <typename T, typename TO>
@@ -707,7 +754,7 @@ int launch_attention(void* out, const void* q, long long ldo, long long ldq, con
                      int chunk, int keep_first, const float* sink, int maps, int n_seq, const int32_t* seq_start, int longest,
                      cudaStream_t stream) {
     // the tile kernel copies 16-byte pieces and holds the tiles of a head in shared memory
-    if (sizeof(T) == 4 && sizeof(TO) == 4 && tiles_serve(T_tokens, n_seq, longest) && n_heads <= 65535 &&
+    if (sizeof(T) == 4 && sizeof(TO) == 4 && tiles_serve(T_tokens, n_seq, longest) && ((long long)T_tokens / TQ + n_seq + 1) * n_heads <= 0x7fffffffll &&
         dh % 4 == 0 && dv % 4 == 0 && dh <= 256 && dv <= 256 && ldq % 4 == 0 && ((uintptr_t)q % 16) == 0 &&
         ((uintptr_t)k_cache % 16) == 0 && ((uintptr_t)v_cache % 16) == 0) {
         const int ng = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4);
@@ -717,7 +764,7 @@ int launch_attention(void* out, const void* q, long long ldo, long long ldq, con
         cudaError_t e = cudaSuccess;
         // the limit is set to what the widest heads need, whatever these need: another thread's launch may come between it and this one's
 #define GOT(NG_) do { e = cudaFuncSetAttribute(attention_tile_kernel<NG_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem_bytes(256, NG_)); \
-        if (e == cudaSuccess) attention_tile_kernel<NG_><<<dim3(blocks, n_heads), 128, bytes, stream>>>( \
+        if (e == cudaSuccess) attention_tile_kernel<NG_><<<dim3(blocks * n_heads), tile_threads<NG_>(), bytes, stream>>>( \
             (float*)out, (const float*)q, (size_t)ldo, (size_t)ldq, (const float*)k_cache, (const float*)v_cache, page_table, max_pages, \
             page_shift, tok_slot, tok_pos, T_tokens, n_heads, n_kv_heads, dh, scale, window, status, dv, softcap, chunk, keep_first, sink, maps, \
             seq_start, n_seq); } while (0)
