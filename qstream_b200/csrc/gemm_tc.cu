@@ -87,7 +87,7 @@ template <int BN, bool WIDE> constexpr int p_smem_bytes() { return p_stages<BN, 
 // shared memory to whole 128-byte lines: with a row per lane every 16-byte store met 32 lines, 8,192 cycles of the store pipe for a tile whose
 // main loop needs 4,096.  Neither change alone gains (eight warps: 60 us instead of 56 for that product; the lines with four warps made
 // every product slower); together, with the unit in the first product (14 us of its own before), and the kernel as a programmatic dependent, 3,000
-// tokens through 4 of 16 experts of 2048 x 512 take 167 us instead of 193.
+// tokens through 4 of 16 experts of 2048 x 512 take 163 us instead of 193.
 constexpr int MAX_GROUPS = 1024;
 template <int BN, bool GROUPED, bool GLU, bool WIDE>
 __global__ void __launch_bounds__(P_THREADS, 1)

@@ -43,7 +43,8 @@ from .linear import linear
 
 CHUNK_TOKENS = 64            # a long prompt is cut into chunks of this many tokens that run side by side
 # The longest sequence of a step from which the chunks serve: all forms gain there, with one sequence as with several.  Shorter prompts would
-# gain in some of them already.  Microseconds of the scan, walk | chunks, one sequence at 64, 128 and 256 tokens, then four sequences:
+# gain in some of them already.  Microseconds of the scan, walk | chunks (with their products on the CUDA cores; on the
+# tensor cores they take up to a third less), one sequence at 64, 128 and 256 tokens, then four sequences:
 #   decay per head, 16 heads of 128 x 128   59 | 44, 111 | 44, 213 | 70      53 | 83,  96 | 85,  182 | 95
 #   per channel (gla), 16 of 64 x 128       78 | 93, 147 | 97, 289 | 101     78 | 99,  147 | 101, 285 | 103
 #   per channel (wkv), 16 of 64 x 64        82 | 46, 156 | 46, 306 | 44      82 | 58,  156 | 56, 305 | 58
