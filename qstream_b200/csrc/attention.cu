@@ -727,16 +727,15 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
 }
 
 // Where the tile kernel serves: from 16 rows per sequence on (the mean: a tile of fewer rows is a block of its own), and with no more keys
-// than one group of 32 from 32 rows on.  Microseconds (tiles, with 64 rows to a block | a warp per query; with 32 rows 16 x 16 rows behind 500 keys take
-// 131 instead of 221, one prompt of 64 rows 18), heads of 128, 1 and 16 sequences of so many rows
+// than one group of 32 from 32 rows on.  Microseconds (tiles | a warp per query), heads of 128, 1 and 16 sequences of so many rows
 // behind so many cached keys:
 //              1 sequence, 16 heads                                         16 sequences, 16 heads
 //   rows       0 keys    48        112       500        2,000               0 keys     48         500          2,000
-//   16         25 | 20   29 | 51   45 | 96   158 | 369  543 | 1,393         31 | 35    37 | 137   221 | 1,071  771 | 4,075
-//   24         25 | 23   41 | 60   59 | 104  158 | 373  547 | 1,393         31 | 68    55 | 258   223 | 2,014  780 | 7,560
-//   32         27 | 28   43 | 63   59 | 109  164 | 375  562 | 1,397         33 | 100   57 | 322   227 | 2,404  786 | 9,232
-// A prompt of 2,000 tokens beside 64 sequences that bring one token behind 2,000 keys: 3.4 ms, 17.2 with a warp per query, 28.9 with
-// tiles cut every 64 rows, whose blocks walk sequence after sequence.
+//   16         25 | 20   20 | 51   29 | 96   96 | 371   322 | 1,395         31 | 35    25 | 139   131 | 1,075  440 | 4,063
+//   24         25 | 23   29 | 61   37 | 104  98 | 373   330 | 1,401         31 | 68    37 | 246   135 | 2,021  459 | 7,581
+//   32         18 | 29   27 | 63   37 | 109  88 | 377   287 | 1,401         22 | 100   37 | 317   121 | 2,409  383 | 9,252
+// (fewer than 32 rows behind no keys: measured with 64 rows to a block).  A prompt of 2,000 tokens beside 64 sequences that bring one token
+// behind 2,000 keys: 2.0 ms, 17.1 with a warp per query, 28.9 with tiles cut every 64 rows, whose blocks walk sequence after sequence.
 constexpr int TILE_ROWS = 16, TILE_ROWS_SHORT = 32, TILE_KEYS = 33;
 bool tiles_serve(long long rows, int n_seq, int longest) {
     return n_seq > 0 && rows >= (longest == 0 || longest >= TILE_KEYS ? TILE_ROWS : TILE_ROWS_SHORT) * (long long)n_seq;
