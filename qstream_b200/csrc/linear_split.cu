@@ -25,6 +25,7 @@
 // Numbers that are not finite (or round to infinity as bfloat16) have no such terms: their last one is NaN, and with it every sum they
 // take part in.  Such a sum is computed again with multiply-adds, so that it becomes what a plain product gives.
 #include "linear_finish.cuh"
+#include "per_device.h"
 #include "sm100.cuh"
 #include "terms.cuh"
 
@@ -290,10 +291,13 @@ linear_split_kernel(const Product p) {
     if (warp == 0) tmem_dealloc_pair(tmem_base, T::TMEM);
 }
 
+// Pairs of these blocks that the current device runs at once.  The kernel's limit of shared memory, set on the way, is the device's own too.
 template <int NT>
-int max_pairs() {
-    static int state = 0, pairs = 0;                    // 0: not asked yet
-    if (state == 0) {
+int max_pairs(int* pairs) {
+    static PerDevice known;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) *pairs = known.get(dev, [&] {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = Tile<NT>::SMEM;
         cudaLaunchAttribute attr[1];
@@ -301,18 +305,19 @@ int max_pairs() {
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(linear_split_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<NT>::SMEM) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&n, linear_split_kernel<NT>, &cfg) == cudaSuccess) pairs = n;
-        cudaGetLastError();
-        state = 1;
-    }
-    return pairs;
+        e = cudaFuncSetAttribute(linear_split_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<NT>::SMEM);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, linear_split_kernel<NT>, &cfg);
+        return e == cudaSuccess ? n : 0;
+    });
+    if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "linear_split: %s", cudaGetErrorString(e));
+    return *pairs > 0 ? QS_OK : qs_fail(QS_ERR_INTERNAL, "linear_split: this device runs no pair of these blocks");
 }
 
 template <int NT>
 int launch(Product p, cudaStream_t stream) {
-    const int pairs = max_pairs<NT>();
-    if (pairs <= 0) return qs_fail(QS_ERR_INTERNAL, "linear_split: this device runs no pair of these blocks");
+    int pairs = 0;
+    const int rc = max_pairs<NT>(&pairs);
+    if (rc != QS_OK) return rc;
     const long long units = (long long)p.m_tiles * p.n_tiles * p.splits;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (unsigned)std::min<long long>(units, pairs)); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = Tile<NT>::SMEM; cfg.stream = stream;
