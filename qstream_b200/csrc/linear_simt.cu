@@ -1,9 +1,9 @@
 // C = act(A W^T + bias) + res1 + res2 on the CUDA cores, accumulating in true
 // 32-bit (FFMA; no tensor-core or reduced-precision matrix mode).
 //
-// This is the matrix product of the float32 engine, and the product for operand
-// type pairs the tensor-core kernel does not take (a matrix stored in 32-bit used
-// with bfloat16 activations).  A: [M, K] row-major (row stride lda), W: [N, K]
+// This is the product for what the tensor-core kernels do not take: a matrix stored
+// in 32-bit used with bfloat16 activations, short sums and odd row strides of the
+// float32 engine (whose other products linear_split.cu takes), its routed experts.  A: [M, K] row-major (row stride lda), W: [N, K]
 // row-major, weight rows = outputs, QStream's matvec convention
 // (include/qsf/kernels.h:53-58).  Each output element sums its K products in
 // ascending k inside one thread, so a row's result does not depend on M or on

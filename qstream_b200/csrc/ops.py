@@ -37,6 +37,7 @@ _SIGNATURES = {
     "qs_linear_split": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                          c_longlong, c_void_p, c_longlong, c_void_p, c_void_p], c_int),
     "qs_linear_split_scratch": ([c_int, c_int, c_int], c_longlong),
+    "qs_linear_split_form": ([c_int, c_int, c_int, c_void_p], c_int),
     "qs_rope_store": ([c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_longlong,
                        c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                        c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_float, c_int, c_void_p], c_int),
@@ -330,6 +331,13 @@ def _linear_split_scratch(M: int, N: int, K: int) -> int:
     return int(library().qs_linear_split_scratch(M, N, K))
 
 
+def linear_split_form(M: int, N: int, K: int):
+    """How `linear_split` works on a product: (tokens of a tile, parts of K, units of a tile side by side, whether these hand on runs)."""
+    form = (c_int * 4)()
+    check(library().qs_linear_split_form(M, N, K, form))
+    return form[0], form[1], form[2], bool(form[3])
+
+
 def split_takes(x, weight, out=None) -> bool:
     """Whether the float32 product on the tensor cores takes these operands: rows in 16-byte pieces."""
     return (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2 and x.shape[1] % 4 == 0
@@ -338,8 +346,8 @@ def split_takes(x, weight, out=None) -> bool:
 
 
 def linear_split(x, weight, bias=None, activation=None, residuals=(), out=None) -> torch.Tensor:
-    """act(x W^T + bias) + residuals, all float32, on the tensor cores: every number as three bfloat16 terms, sums no further from
-    64 bits than those of `linear_simt`."""
+    """act(x W^T + bias) + residuals, all float32, on the tensor cores: every number as three bfloat16 terms, in an order of sums that
+    depends on the matrix's sizes alone."""
     from . import gemm_tc
     M, K, lda = _rows(x)
     N = weight.shape[0]

@@ -2,10 +2,13 @@
 
 bfloat16 activations with a bfloat16 matrix run on the tensor cores (tcgen05, fed by
 TMA, 32-bit accumulation).  float32 activations with a float32 matrix run there too, every
-number as three bfloat16 terms and the sums rounded in 32 bits outside the unit, where more than a
-few rows meet enough products; everything else (few rows, mixed types) runs on the CUDA cores in
-true 32-bit.  Each kernel sums a row's products in an order that does not depend on
-the other rows' contents.
+number as three bfloat16 terms and the sums rounded in 32 bits outside the unit, where a result is the
+sum of 256 products or more and rows come in 16-byte pieces; everything else (short sums, mixed types)
+runs on the CUDA cores in true 32-bit.
+
+A row's result does not depend on the contents of the other rows.  Neither does it depend on their number in
+the float32 engine, where the matrix alone decides the kernel and the order of the sums; the bfloat16
+products change their order between up to 128 rows and more (and with the number beyond), by rounding.
 """
 from __future__ import annotations
 
@@ -14,10 +17,12 @@ import torch
 from ..csrc import ops
 
 TENSOR_CORE_ACTIVATIONS = (None, "none", "gelu_new", "gelu")
-# float32: from how many rows and products per result on the tensor cores serve.  Microseconds, CUDA cores | tensor cores (caches
-# flushed, launches included): 16 rows, 6144 x 2048: 32 | 34; 17 rows, 2048 x 8192: 54 | 40; 32, 2048 x 2048: 28 | 21; 64, 6144 x 2048: 60 | 36; 700,
-# 64 x 1024: 24 | 24; 700, 2048 x 64: 49 | 18, but 64 x 64: 12 | 12; 128, 256 x 256: 20 | 15; 700, 6144 x 2048: 412 | 99; 2048, 16384 x 4096: 5159 | 1138.
-SPLIT_ROWS, SPLIT_PRODUCTS = 17, 256
+# float32: from how many products per result on the tensor cores serve, whatever the number of rows, so that a row's result is the same bits in any
+# batch.  Microseconds, CUDA cores | tensor cores (caches flushed, launches included): 1, 16, 17, 64 and 700 rows, 6144 x 2048: 29 | 31, 31 | 33,
+# 49 | 33, 57 | 35, 410 | 115; 2048 x 2048: 23 | 23, 23 | 25, 25 | 25, 33 | 31, 187 | 51; 2048 x 8192: 35 | 37, 37 | 39, 53 | 39, 70 | 41, 551 | 143;
+# 32000 x 2048: 94 | 102, 100 | 109, 176 | 111, 244 | 111, 2211 | 520; 64 x 2048: 18 | 15, 18 | 16, 18 | 16, 18 | 16, 27 | 29; 128 x 256: 20 | 14, 21 | 14,
+# 20 | 14, 23 | 14, 22 | 16.
+SPLIT_PRODUCTS = 256
 OWN_KERNEL_ACTIVATIONS = ("relu2",)         # in no product's epilogue: applied by a kernel of their own behind the product
 
 
@@ -31,8 +36,8 @@ def linear(x, weight, bias=None, activation=None, residuals=(), out_dtype=None, 
                 return gemm_tc.linear(x, weight, bias, activation, residuals, out_dtype, out)
             if not residuals:       # an activation that the tensor-core epilogue does not offer: a kernel of its own behind it
                 return ops.activate(gemm_tc.linear(x, weight, bias, None, (), out_dtype, out), activation)
-    if x.dtype == torch.float32 and out_dtype in (None, torch.float32) and x.dim() == 2 and x.shape[0] >= SPLIT_ROWS \
-            and x.shape[1] >= SPLIT_PRODUCTS and ops.split_takes(x, weight, out):
+    if x.dtype == torch.float32 and out_dtype in (None, torch.float32) and x.dim() == 2 and x.shape[1] >= SPLIT_PRODUCTS \
+            and ops.split_takes(x, weight, out):
         own = activation in OWN_KERNEL_ACTIVATIONS and not residuals
         y = ops.linear_split(x, weight, bias, None if own else activation, residuals, out)
         return ops.activate(y, activation) if own else y

@@ -9,8 +9,8 @@ pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -24
 
 
-# rows at the edges of the four tiles (32, 64, 128, 256 tokens) and of several, features at the edge of 256 and of a CTA's 128, K of one
-# block of 64, with tails, and cut over many pairs of blocks
+# rows and features at the edges of tiles and of a CTA's 128 features, K of one block of 64, with tails, and cut over many pairs of blocks
+# (tiles of 256 tokens, and pairs that take several units: below)
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (17, 16, 256), (32, 256, 64), (33, 257, 68), (64, 300, 260), (65, 129, 2048), (128, 2048, 1024), (129, 128, 516),
                                    (255, 520, 320), (257, 2048, 2048), (700, 1000, 512), (300, 64, 8192)])
 def test_product_against_float64(M, N, K):
@@ -74,3 +74,89 @@ def test_rows_that_are_no_whole_pieces_are_refused(K):
     with pytest.raises(QStreamError):
         ops.linear_split(x, w)
     assert linear(x, w).shape == (40, 64)
+
+
+# (N, K): the forms that their row counts below reach, as (tokens of a tile, whether units of a tile run side by side, whether these hand on runs).
+# Tails of rows, features and K; pairs with one unit and with several (over 74), of one tile's parts and of other tiles
+FORMS = {(2570, 2564): {(32, True, True), (64, True, True), (128, True, False), (64, True, False), (256, True, False)},
+         (6200, 1284): {(32, True, False), (64, True, False), (128, True, False), (256, True, False), (64, False, False), (128, False, False)},
+         (4100, 1284): {(32, True, True), (64, True, False), (256, False, False), (256, True, False)},
+         (9500, 644): {(32, False, False), (64, False, False), (128, False, False), (256, False, False)},
+         (64, 2052): {(32, True, True), (64, True, True)}, (300, 260): {(32, True, True), (64, True, True), (32, False, False)}}
+ROWS = (1, 2, 16, 17, 33, 64, 65, 100, 129, 257, 300, 513, 700, 1100)
+
+
+@pytest.mark.parametrize("N,K", list(FORMS))
+def test_a_row_is_the_same_bits_whatever_else_is_in_the_batch(N, K):
+    """Every form a product can take, by its number of rows: against float64, and the same bits for each row; among them pairs with several
+    units (barriers and stages used on), tiles of 256 tokens, and a number that is not finite in the last unit."""
+    forms = {M: ops.linear_split_form(M, N, K) for M in ROWS}
+    assert FORMS[N, K] <= {(f[0], f[2] > 1, f[3]) for f in forms.values()}
+    assert len({f[1] for f in forms.values()}) == 1
+    if N > 2500:
+        assert any(-(-M // f[0]) * -(-N // 256) * f[2] > 74 for M, f in forms.items())
+    M = max(ROWS)
+    g = torch.Generator().manual_seed(N + K)
+    x, w, bias = torch.randn(M, K, generator=g).cuda(), (torch.randn(N, K, generator=g) * K ** -0.5).cuda(), torch.randn(N, generator=g).cuda()
+    res = (torch.randn(M, N, generator=g).cuda(),)
+    whole = linear(x, w, bias, "gelu_new", res)
+    ref, size = x.double() @ w.double().T + bias.double(), x.double().abs() @ w.double().abs().T + bias.double().abs()
+    ref = torch.nn.functional.gelu(ref, approximate="tanh") + res[0].double()
+    # as above for the sum; gelu's slope is below 1.2, its own roundings and those behind it act on values of the size of the sums
+    runs = -(-K // 64)
+    assert ((whole.double() - ref).abs() <= 1.2 * (2 * 24 + 4 + 2 * runs) * EPS * size + 16 * EPS * (ref.abs() + res[0].abs() + 1)).all()
+    for n in ROWS:
+        for at in {0, M - n}:
+            assert torch.equal(linear(x[at:at + n], w, bias, "gelu_new", (res[0][at:at + n],)), whole[at:at + n]), (n, at, forms[n])
+    gemm_tc.check_status("cuda:0")
+    x[M - 2, K - 3], x[M - 1, 5] = float("inf"), 3.4e38                 # the second: infinity as a bfloat16 only
+    odd = linear(x, w, bias)
+    plain = ops.linear_simt(x[M - 2:], w, bias)
+    assert torch.equal(torch.isnan(odd[M - 2:]), torch.isnan(plain)) and torch.equal(torch.isinf(odd[M - 2:]), torch.isinf(plain))
+    for n in ROWS:
+        torch.testing.assert_close(linear(x[M - n:], w, bias), odd[M - n:], rtol=0, atol=0, equal_nan=True)
+    gemm_tc.check_status("cuda:0")
+
+
+def test_the_workspace_that_a_product_takes_is_asked_for():
+    from qstream_b200 import QStreamError
+    x, w, out = torch.zeros(16, 2048, device="cuda"), torch.zeros(2048, 2048, device="cuda"), torch.zeros(16, 2048, device="cuda")
+    lib = ops.library()
+    floats = lib.qs_linear_split_scratch(16, 2048, 2048)
+    assert floats > 0
+    with pytest.raises(QStreamError):
+        ops.check(lib.qs_linear_split(ops.ptr(out), ops.ptr(x), ops.ptr(w), None, 0, 0, None, None, 16, 2048, 2048, 2048, 2048, 2048, None, 0,
+                                      ops.ptr(gemm_tc.status_word(x.device)), ops.stream()))
+
+
+def test_a_float32_request_is_the_same_bits_alone_in_a_batch_and_in_portions(tmp_path):
+    import qstream_b200 as qs
+    cfg = qs.GptjConfig.from_dict(dict(n_layer=2, n_embd=1024, n_head=8, n_positions=256, vocab_size=512, rotary_dim=16,
+                                       architectures=["GPTJForCausalLM"]))
+    model = qs.load_model(qs.write_model_folder(str(tmp_path / "m"), cfg, seed=3, dtype="float32"), dtype="float32", device="cuda:0")
+    g = torch.Generator().manual_seed(1)
+    prompts = [torch.randint(0, 512, (n,), generator=g).tolist() for n in (7, 40, 100)]
+    engine = qs.Engine(model, max_tokens=1024, max_batch=3)
+
+    def serve(which, portion):
+        slots = [engine.acquire() for _ in which]
+        rest = [list(prompts[i]) for i in which]
+        while any(len(r) > portion for r in rest):          # all but the last portions, a sequence at a time
+            for k, r in enumerate(rest):
+                if len(r) > portion:
+                    engine.step([slots[k]], [r[:portion]])
+                    rest[k] = r[portion:]
+        out = [engine.step(slots, rest).clone()]
+        for t in (5, 17):
+            out.append(engine.step(slots, [[t]] * len(which)).clone())
+        for s in slots:
+            engine.release(s)
+        return out
+
+    together = serve((0, 1, 2), 1000)
+    for got in (serve((0, 1, 2), 30), serve((0, 1, 2), 9)):
+        assert all(torch.equal(a, b) for a, b in zip(together, got))
+    for i in range(3):
+        for a, b in zip(together, serve((i,), 1000)):
+            assert torch.equal(a[i], b[0])
+    engine.check_status()
