@@ -799,16 +799,16 @@ delta_output_kernel(const __grid_constant__ Delta p, int32_t* __restrict__ statu
     const int in = quad * 32 + lane, rows = n - half * 32;
     if (in < nv) {
         float* o = p.o + (size_t)t0 * p.ldo + (size_t)h * p.dv + col0 + in;
-        bool odd = false;
+        uint32_t odd = 0;
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
-            odd |= !is_number(out[x]);
+            odd = max(odd, beyond(out[x]));
             if (x < rows) o[(size_t)(half * 32 + x) * p.ldo] = out[x];
         }
-        if (odd)                                        // by multiply-adds, where the terms gave no number: a later token's u meets no earlier one
+        if (odd > HELD)                                 // by multiply-adds, where the terms did not hold the operands: a later token's u meets no earlier one
             for (int t = half * 32; t < min(n, half * 32 + 32); ++t) {
                 float v = o[(size_t)t * p.ldo];
-                if (is_number(v)) continue;
+                if (held(v)) continue;
                 v = 0.f;
                 for (int i = 0; i < p.dk && v == v; ++i) v = fmaf(p.Q[(unit * CT + t) * p.dkp + i], p.start[(unit * p.dk + i) * p.dvp + col0 + in], v);
                 for (int j = 0; j <= t && v == v; ++j) v = fmaf(p.B[unit * CT * CT + j * CT + t], p.U[(unit * CT + j) * p.dvp + col0 + in], v);

@@ -27,8 +27,8 @@
 // That costs many tokens some time: microseconds with the cut by M as well | now: 700 x 6144 x 2048 91 | 108, x 2048 x 8192 119 | 138, 350 x 8192 x 2048 93 | 100,
 // 2,048 x 6144 x 2048 258 | 324, 700 x 8192 x 2048 174 | 170, 700 x 14336 x 2048 263 | 262; 16 x 6144 x 2048 23.3 | 24.2.
 //
-// Numbers that are not finite (or round to infinity as bfloat16) have no such terms: their last one is NaN, and with it every sum they
-// take part in.  Such a sum is computed again with multiply-adds, so that it becomes what a plain product gives.
+// A part's sum whose operands the terms may not have held (`held`: numbers that are not finite, and very small ones) is computed again with
+// multiply-adds, so that it becomes what a plain product gives.
 #include "linear_finish.cuh"
 #include "per_device.h"
 #include "sm100.cuh"
@@ -98,9 +98,6 @@ __device__ __forceinline__ void tmem_load_32x8(uint32_t taddr, uint32_t (&r)[8])
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
-
-// Whether the terms held what went into a sum.
-__device__ __forceinline__ bool held(float v) { return fabsf(v) <= 3.402823466e38f; }
 
 // A part's sum that the terms did not hold, by multiply-adds in runs of 256 products.
 __device__ __noinline__ float plain_sum(const float* __restrict__ a, const float* __restrict__ w, int k0, int k1) {

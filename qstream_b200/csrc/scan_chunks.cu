@@ -103,11 +103,11 @@ __device__ __noinline__ float plain_added(const Scan& p, int h, int i, int t0, i
     }
     return sum;
 }
-// The sums of a column that the terms gave no number for.
+// The sums of a column whose operands the terms did not hold.
 template <typename TI, int MODE>
 __device__ __noinline__ void mend_added(const Scan& p, float* to, int rows, int h, int i, int t0, int n, long long v_at, const float* s_w) {
     for (int x = 0; x < rows; ++x)
-        if (!is_number(to[(size_t)x * p.dvp])) to[(size_t)x * p.dvp] = plain_added<TI, MODE>(p, h, i + x, t0, n, v_at, s_w);
+        if (!held(to[(size_t)x * p.dvp])) to[(size_t)x * p.dvp] = plain_added<TI, MODE>(p, h, i + x, t0, n, v_at, s_w);
 }
 
 template <typename TI> constexpr int added_smem() { return 1024 + (3 + (sizeof(TI) == 2 ? 1 : 3)) * 2 * TILE; }
@@ -266,13 +266,13 @@ added_state_kernel(const __grid_constant__ Scan p) {
             float* to = added + (size_t)(base + at) * p.dvp + col0 + col;
             if (col < nv) {
                 const int rows = min(32, p.dk - base - at);
-                bool odd = false;
+                uint32_t odd = 0;
 #pragma unroll
                 for (int x = 0; x < 32; ++x) {
-                    odd |= !is_number(sum[x]);
+                    odd = max(odd, beyond(sum[x]));
                     if (x < rows) to[(size_t)x * p.dvp] = sum[x];
                 }
-                if (odd) mend_added<TI, MODE>(p, to, rows, h, base + at, t0, n, (long long)h * dvv + col0 + col, s_w);
+                if (odd > HELD) mend_added<TI, MODE>(p, to, rows, h, base + at, t0, n, (long long)h * dvv + col0 + col, s_w);
             }
         }
         tc_fence_before_sync();
@@ -565,15 +565,15 @@ channel_output_kernel(const __grid_constant__ Scan p) {
     const int in = quad * 32 + lane, rows = n - half * 32;
     if (in < nv) {
         float* const o = p.o + (size_t)t0 * p.ldo + (size_t)h * p.dv + col0 + in;
-        bool odd = false;
+        uint32_t odd = 0;
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
-            odd |= !is_number(out[x] + more[x]);
+            odd = max(odd, beyond(out[x] + more[x]));
             if (x < rows) o[(size_t)(half * 32 + x) * p.ldo] = out[x] + more[x];
         }
-        if (odd)                                        // by multiply-adds, where the terms gave no number: a later token's value meets no earlier one
+        if (odd > HELD)                                 // by multiply-adds, where the terms did not hold the operands: a later token's value meets no earlier one
             for (int t = half * 32; t < min(n, half * 32 + 32); ++t) {
-                if (is_number(o[(size_t)t * p.ldo])) continue;
+                if (held(o[(size_t)t * p.ldo])) continue;
                 float v = plain_from_state<TI, MODE>(p, S, h, t0, t, col0 + in);
                 for (int j = 0; j <= t && v == v; ++j)
                     v = fmaf(sp[j * PP + t], to_f32(((const TI*)p.v)[(size_t)(t0 + j) * p.ldv + (size_t)h * p.dv + col0 + in]), v);
@@ -594,7 +594,7 @@ template <typename TI, int NH> constexpr int tile_smem() {
     return 1024 + (slices > weights ? slices : weights);
 }
 
-// One output by multiply-adds, where the tensor unit gave no number.  The weights are taken from their terms at `tp` where they have some.
+// One output by multiply-adds, where the terms did not hold what went into it.  The weights are taken from their terms at `tp` where these held them.
 template <typename TI, int MODE>
 __device__ __noinline__ float plain_output(const Scan& p, const float* __restrict__ S, const float* __restrict__ a, const float* __restrict__ b, float cum,
                                            uint32_t tp, int h, int t0, int t, int col) {
@@ -611,7 +611,7 @@ __device__ __noinline__ float plain_output(const Scan& p, const float* __restric
             asm volatile("ld.shared.u16 %0, [%1];" : "=h"(term) : "r"(tp + i * TILE + place_in_tile(t, j)));
             w += __uint_as_float((uint32_t)term << 16);
         }
-        if (!is_number(w)) {
+        if (!held(w)) {
             const TI* k = (const TI*)p.k + (size_t)(t0 + j) * p.ldk + hq * p.dk;
             float raw = 0.f;
             for (int i = 0; i < p.dk; ++i) raw = fmaf(to_f32(q[i]) * p.q_scale, to_f32(k[i]), raw);
@@ -790,7 +790,7 @@ tile_output_kernel(const __grid_constant__ Scan p) {
     for (int x = 0; x < 32; ++x) out[x] *= s_cum[head][half * 32 + x] * p.q_scale;
     if (ONES && blockIdx.z == 0 && tid < n) {
         float sum = fmaf(s_cum[0][tid] * p.q_scale, ones_part, s_ones[0][tid] + s_ones[1][tid]);
-        if (!is_number(sum)) sum = plain_output<TI, MODE>(p, S, s_a[0], s_b[0], s_cum[0][tid], tp, h, t0, tid, dvv);
+        if (!held(sum)) sum = plain_output<TI, MODE>(p, S, s_a[0], s_b[0], s_cum[0][tid], tp, h, t0, tid, dvv);
         p.o[(size_t)(t0 + tid) * p.ldo + (size_t)h * p.dv + dvv] = sum;
     }
     if (ok) ok = wait_done(&done, slices & 1, p.status);
@@ -799,15 +799,15 @@ tile_output_kernel(const __grid_constant__ Scan p) {
     float* const o = p.o + (size_t)t0 * p.ldo + (size_t)(h + head) * p.dv + col;
     if (col < dvv) {
         const int rows = n - half * 32;
-        bool odd = false;
+        uint32_t odd = 0;
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
-            odd |= !is_number(out[x]);
+            odd = max(odd, beyond(out[x]));
             if (x < rows) o[(size_t)(half * 32 + x) * p.ldo] = out[x];
         }
-        if (odd)
+        if (odd > HELD)
             for (int t = half * 32; t < min(n, half * 32 + 32); ++t)
-                if (!is_number(o[(size_t)t * p.ldo])) o[(size_t)t * p.ldo] = plain_output<TI, MODE>(p, S, s_a[head], s_b[head], s_cum[head][t], tp + head * 3 * TILE, h + head, t0, t, col);
+                if (!held(o[(size_t)t * p.ldo])) o[(size_t)t * p.ldo] = plain_output<TI, MODE>(p, S, s_a[head], s_b[head], s_cum[head][t], tp + head * 3 * TILE, h + head, t0, t, col);
     }
     leave();
 }

@@ -9,8 +9,6 @@ using namespace sm100;
 
 namespace {
 
-__device__ __forceinline__ bool is_number(float x) { return fabsf(x) <= 3.402823466e38f; }
-
 // ---- tiles of terms in shared memory as tcgen05 operands: 64 elements to a row of 128 bytes, swizzled by 128 bytes.  A tile of
 // 64 rows is 8 KB; wider ones are several of them.  The same tile serves with its rows on the sum's side or on the other.
 constexpr int TILE = CT * 128;                          // bytes

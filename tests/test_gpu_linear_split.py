@@ -66,6 +66,26 @@ def test_numbers_without_terms_give_what_a_plain_product_gives():
         assert torch.equal(got[rows][:, cols], plain[rows][:, cols])      # nobody else's results change
 
 
+@pytest.mark.parametrize("low", [-100, -112, -120, -126])
+def test_very_small_operands_are_held_whole(low):
+    """Below 2^-109 a number's last bfloat16 term is cut: such sums are taken from the 32-bit numbers, and nobody else's results change."""
+    for M, N, K in ((40, 300, 2048), (300, 256, 512), (700, 600, 260)):
+        g = torch.Generator().manual_seed(K)
+        x, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+        plain = ops.linear_split(x, w)
+        small = x.clone()
+        small[M // 2:M // 2 + 3] *= 2.0 ** low
+        for a, b in ((small, w), (x, w * 2.0 ** low)):
+            got, ref, size = ops.linear_split(a, b), a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+            # runs of 256 products as a chain of rounded additions, then the runs; nothing below 2^-149
+            assert ((got.double() - ref).abs() <= (256 + -(-K // 64)) * EPS * size + K * 2.0 ** -149).all()
+            if a is small:
+                rows = torch.ones(M, dtype=torch.bool)
+                rows[M // 2:M // 2 + 3] = False
+                assert torch.equal(got[rows], plain[rows])
+    gemm_tc.check_status("cuda:0")
+
+
 @pytest.mark.parametrize("K", [258, 255])
 def test_rows_that_are_no_whole_pieces_are_refused(K):
     from qstream_b200 import QStreamError

@@ -142,3 +142,25 @@ def test_what_is_not_finite_reaches_no_earlier_token(mode):
                        chunks=cut([T]), **kw).cpu().numpy().reshape(T, H, n)
     assert np.isfinite(o[:90]).all() and np.isfinite(o[:100, 0]).all() and np.isfinite(o[90:, 1, :3]).all()
     assert not np.isfinite(o[90, 1, 3]) and not np.isfinite(o[100, 0]).any() and not np.isfinite(o[110, 0]).any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode", ["decay", "wkv", "gated", "gla", "ssd"])
+def test_very_small_values_are_held_whole(mode, dtype):
+    """Values and a state around 2^-120, where a number's last bfloat16 term is cut: outputs and state as near as for ordinary ones."""
+    T, H, dk, dv, low = 100, 2, 40, 36, 2.0 ** -120
+    q, k, v, a, b, u, kw = make(mode, T, H, H, dk, dv, 21)
+    q, k, v = (torch.from_numpy(x).to(dtype).double().numpy() for x in (q, k, v))
+    n = dv + (mode == "gated")
+    S0 = r32(np.random.default_rng(2).normal(0, 1, (1, H, n, dk)))
+    ones = np.ones((T, H, 1))
+    for small_v in (True, False):                       # all of it, or the state alone beside values of zero
+        vs = torch.from_numpy(v * low if small_v else 0 * v).to(dtype).double().numpy()
+        state = dev(S0 * low)
+        o = ops.state_scan(mode, dev(q.reshape(T, -1), dtype), dev(k.reshape(T, -1), dtype), dev(vs.reshape(T, -1), dtype), state, i32([0, T]), i32([0]), 1, H,
+                           dk, n, chunks=cut([T]), **kw).double().cpu().numpy().reshape(T, H, n)[:, :, :dv]
+        ref, S, _, _ = walk(mode, q, k, np.concatenate([vs, ones], 2) if mode == "gated" else vs, a, b, u, (S0[0] * low).transpose(0, 2, 1))
+        got = state.double().cpu().numpy()[0].transpose(0, 2, 1)[:, :, :dv]
+        for x, y in ((o, ref[:, :, :dv]), (got, S[:, :, :dv])):
+            x, y = x / low, y / low
+            assert np.linalg.norm(x - y) <= 4e-6 * np.linalg.norm(y) + 2.0 ** -149 / low * T * np.sqrt(y.size), np.linalg.norm(x - y) / np.linalg.norm(y)
