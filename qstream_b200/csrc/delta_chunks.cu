@@ -406,6 +406,7 @@ delta_walk_kernel(Delta p) {
                 sum.x += a.x; sum.y += a.y; sum.z += a.z; sum.w += a.w;
             }
             u.x -= sum.x; u.y -= sum.y; u.z -= sum.z; u.w -= sum.w;
+            if (row >= n) u = make_float4(0.f, 0.f, 0.f, 0.f);      // nobody's token writes nothing, whatever the state holds
             *reinterpret_cast<float4*>(sU + row * WC + quad) = u;
             if (quad < n_cols) *reinterpret_cast<float4*>(u_row) = u;
         }
@@ -467,7 +468,8 @@ delta_walk_kernel(Delta p) {
 //
 // A chain of 32 steps for 2,000 tokens of 16 heads of 128 x 128.  By multiply-adds a step took 4.2 us (shared memory's pipe: eight 16-byte reads per 32 paired
 // multiply-adds), 133 us in all; with each block splitting W and K for itself 119; now
-// 113.  With sixteen warps, each half of the columns: 119 (64 channels: 4 us less of 73).
+// 113; with the sums taken again where the terms did not hold their operands (three calls in the kernel, none on an ordinary path) 120. With sixteen
+// warps, each half of the columns: 119 instead of 113 (64 channels: 4 us less of 73).
 // MC channels, 64 or 128; pitches of W and K, of S and u: rows of 16 bytes meet all banks
 constexpr int SP = WC + 8;
 template <int MC> constexpr int mma_walk_smem() { return (2 * 3 * CT * (MC + 8) + 3 * MC * SP + 3 * CT * SP) * 2 + CT * WC * 4; }
@@ -484,6 +486,22 @@ __device__ __forceinline__ void put_two(__nv_bfloat16* at, int term, float x, fl
     terms_of(pack2(x, y), a[0], a[1], a[2]);
 #pragma unroll
     for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(at + i * term) = a[i];
+}
+
+// The sums of the walk whose operands the terms did not hold, by multiply-adds: token t's W S, and what the chunk's writes add to channel i.
+__device__ __noinline__ float plain_held(const Delta& p, size_t unit, int t, int col) {
+    const float *w = p.W + (unit * CT + t) * p.dkp, *S = p.start + unit * p.dk * p.dvp + col;
+    float sum = 0.f;
+    for (int i = 0; i < p.dk && sum == sum; ++i) sum = fmaf(w[i], S[(size_t)i * p.dvp], sum);        // NaN stays NaN
+    return sum;
+}
+__device__ __noinline__ float plain_written(const Delta& p, size_t unit, int t0, int n, int h, int i, int col) {
+    float sum = 0.f, run = 1.f;
+    for (int t = n - 1; t >= 0 && sum == sum; --t) {
+        sum = fmaf(p.k[(size_t)(t0 + t) * p.ldk + h / p.group * p.dk + i] * run, p.U[(unit * CT + t) * p.dvp + col], sum);
+        run *= p.g[(size_t)(t0 + t) * p.ldg + h * p.dk + i];
+    }
+    return sum;
 }
 
 template <int MC>
@@ -528,6 +546,17 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
         const int n = c < c1 ? p.chunk_start[c + 1] - p.chunk_start[c] : 0;
         return n > 0 && n <= CT;
     };
+    // The state after chunk c, where the terms did not hold what chunk c wrote.  Looked at where a chunk's u shows it (what is no number makes all u of its
+    // column none, what is small counts only where they are) and at the end.
+    auto mend_state = [&](int c) {
+        if (c < c0 || !whole(c)) return;
+        const size_t unit = (size_t)c * p.H + h;
+        const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0;
+        each([&](float& v, int i, int col) {
+            if (!held(v) && i < p.dk && col < n_cols)
+                v = fmaf(p.decay[unit * dkp + i], p.start[(unit * p.dk + i) * p.dvp + col0 + col], plain_written(p, unit, t0, n, h, i, col0 + col));
+        });
+    };
     const int w_at = tid / ROW, w_i = tid % ROW * 4;
     auto fetch_w = [&](int c) {
         const bool have = whole(c) && w_i < dkp;
@@ -566,6 +595,7 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
         const size_t unit = (size_t)c * p.H + h;
         const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0;
         if (n <= 0 || n > CT) {                         // token by token on the state in 32-bit, over u's and the state's terms: sixteen threads share a column
+            mend_state(c - 1);
             float* sS = reinterpret_cast<float*>(ts);   // [MC][17]
             each([&](float& v, int i, int col) { if (i < p.dk) sS[i * 17 + col] = v; });
             __syncthreads();
@@ -621,13 +651,16 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
             const int i = warp * 16 + 8 * x + g;
             d[x] = i < dkp ? p.decay[unit * dkp + i] : 0.f;
         }
+        auto put_start = [&]() {                        // the state this chunk starts from
 #pragma unroll
-        for (int x = 0; x < 2; ++x)                     // the state this chunk starts from
+            for (int x = 0; x < 2; ++x)
 #pragma unroll
-            for (int z = 0; z < 2; ++z) {
-                const int i = warp * 16 + 8 * x + g, col = 8 * z + q2;
-                if (i < p.dk && col < n_cols) *reinterpret_cast<float2*>(p.start + (unit * p.dk + i) * p.dvp + col0 + col) = make_float2(S[x][z][0], S[x][z][1]);
-            }
+                for (int z = 0; z < 2; ++z) {
+                    const int i = warp * 16 + 8 * x + g, col = 8 * z + q2;
+                    if (i < p.dk && col < n_cols) *reinterpret_cast<float2*>(p.start + (unit * p.dk + i) * p.dvp + col0 + col) = make_float2(S[x][z][0], S[x][z][1]);
+                }
+        };
+        put_start();
 #pragma unroll
         for (int i = part * 64; i < part * 64 + 64; i += 16) {
             uint32_t a[3][4], b[3][4];
@@ -645,21 +678,52 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
 #pragma unroll
                 for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(red + (tile * 16 + 8 * x + g) * WC + 8 * z + q2) = make_float2(y[z][2 * x], y[z][2 * x + 1]);
         __syncthreads();
-        if (part == 0)
+        uint32_t odd = 0;
+        const int tg = tile * 16 + g;
+        auto put_u = [&]() {
 #pragma unroll
             for (int x = 0; x < 2; ++x)
 #pragma unroll
                 for (int z = 0; z < 2; ++z) {
-                    const int t = tile * 16 + 8 * x + g, col = 8 * z + q2;
-                    const float2 more = PARTS > 1 ? *reinterpret_cast<const float2*>(red + t * WC + col) : make_float2(0.f, 0.f);
-                    const float2 v = make_float2(u[x][z][0] - (y[z][2 * x] + more.x), u[x][z][1] - (y[z][2 * x + 1] + more.y));
-                    put_two(tu + t * SP + col, CT * SP, v.x, v.y);
-                    if (col < n_cols) *reinterpret_cast<float2*>(p.U + (unit * CT + t) * p.dvp + col0 + col) = v;
+                    const int t = tg + 8 * x, col = 8 * z + q2;
+                    put_two(tu + t * SP + col, CT * SP, y[z][2 * x], y[z][2 * x + 1]);
+                    if (col < n_cols) *reinterpret_cast<float2*>(p.U + (unit * CT + t) * p.dvp + col0 + col) = make_float2(y[z][2 * x], y[z][2 * x + 1]);
                 }
+        };
+        if (part == 0) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {
+                    const float2 more = PARTS > 1 ? *reinterpret_cast<const float2*>(red + (tg + 8 * x) * WC + 8 * z + q2) : make_float2(0.f, 0.f);
+                    const bool have = tg + 8 * x < n;   // nobody's tokens write nothing, whatever the state holds
+                    y[z][2 * x] = have ? u[x][z][0] - (y[z][2 * x] + more.x) : 0.f;
+                    y[z][2 * x + 1] = have ? u[x][z][1] - (y[z][2 * x + 1] + more.y) : 0.f;
+                    if (have) odd = max(odd, max(beyond(y[z][2 * x]), beyond(y[z][2 * x + 1])));
+                }
+            put_u();
+        }
         put_w();                                        // behind the barrier: nobody reads W any more
         fetch_w(c + 2);
         copies_done();                                  // this chunk's K
-        __syncthreads();
+        if (__syncthreads_or(odd > HELD)) {             // u whose operands the terms did not hold
+            mend_state(c - 1);
+            put_start();
+            __syncthreads();
+            if (odd > HELD) {
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int z = 0; z < 2; ++z)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int t = tg + 8 * x, col = 8 * z + q2 + e;
+                            if (t < n && !held(y[z][2 * x + e]) && col < n_cols) y[z][2 * x + e] = u[x][z][e] - plain_held(p, unit, t, col0 + col);
+                        }
+                put_u();
+            }
+            __syncthreads();
+        }
         // 2
         float more[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
@@ -683,6 +747,7 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
         __syncthreads();
         copy_k(c + 1);
     }
+    mend_state(c1 - 1);
     each([&](float& v, int i, int col) { if (i < p.dk && col < n_cols) own[(size_t)col * p.dk + i] = v; });
 }
 

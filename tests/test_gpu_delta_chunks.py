@@ -98,3 +98,42 @@ def test_operands_in_bfloat16_and_absent_values():
             assert (a - c).norm() <= 4 * 2.0 ** -24 * (np.sqrt(64) + np.sqrt(dk)) * np.sqrt(T / 16) * c.norm()
         alone = scan(q, k, values, None, want_output=False)
         assert alone[0] is None and torch.equal(alone[1], walked[1])
+
+
+@pytest.mark.parametrize("dk", [40, 128, 130])
+def test_very_small_values_are_held_whole(dk):
+    """Values and a state around 2^-120, where a number's last bfloat16 term is cut."""
+    T, H, dv, low = 150, 2, 40, 2.0 ** -120
+    q, k, v, g, beta = make(T, H, H, dk, dv, 9, False)
+    S0 = r32(np.random.default_rng(2).normal(0, 1, (1, H, dv, dk)))
+    for vs in (v * low, 0 * v):
+        state = torch.from_numpy(S0 * low).float().cuda()
+        o = run(q, k, vs, g, beta, state, [0, T], [0], cut([T])).double().cpu().numpy().reshape(T, H, dv)
+        ref, S = walk(q, k, vs, g, beta, (S0[0] * low).transpose(0, 2, 1))
+        bound = 4 * 2.0 ** -24 * (np.sqrt(64) + np.sqrt(dk)) * np.sqrt(T / 16)
+        for x, y in ((o, ref), (state.double().cpu().numpy()[0].transpose(0, 2, 1), S)):
+            x, y = x / low, y / low
+            assert np.linalg.norm(x - y) <= bound * np.linalg.norm(y) + 2.0 ** -149 / low * T * np.sqrt(y.size), np.linalg.norm(x - y) / np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("T", [70, 128])
+@pytest.mark.parametrize("dk", [40, 128, 130])
+def test_numbers_above_the_largest_bfloat16_stay_in_the_state(dk, T):
+    """A channel that no token reads, writes or decays holds 3.4e38, which has no bfloat16 terms: it stays, and nothing else is touched."""
+    H, dv, big = 2, 40, np.float32(3.4e38)
+    q, k, v, g, beta = make(T, H, H, dk, dv, 13, False)
+    q[:, :, 5], k[:, :, 5], g[:, :, 5] = 0.0, 0.0, 1.0
+    S0 = r32(np.random.default_rng(4).normal(0, 1, (1, H, dv, dk)))
+    S0[:, :, :, 5] = 0.0
+    got = []
+    for held in (0.0, big):
+        S = S0.copy()
+        S[0, 1, 7, 5] = held
+        state = torch.from_numpy(S).float().cuda()
+        got.append((run(q, k, v, g, beta, state, [0, T], [0], cut([T])).cpu().numpy(), state.cpu().numpy()))
+    (o, state), (o_big, state_big) = got
+    assert state_big[0, 1, 7, 5] == big
+    state_big[0, 1, 7, 5] = 0.0
+    assert np.isfinite(o_big).all() and np.isfinite(state_big).all()
+    bound = 4 * 2.0 ** -24 * (np.sqrt(64) + np.sqrt(dk)) * np.sqrt(max(1, T / 16))        # as above: other sums of the same terms
+    assert np.linalg.norm(o_big - o) <= bound * np.linalg.norm(o) and np.linalg.norm(state_big - state) <= bound * np.linalg.norm(state)
