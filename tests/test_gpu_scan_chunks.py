@@ -164,3 +164,19 @@ def test_very_small_values_are_held_whole(mode, dtype):
         for x, y in ((o, ref[:, :, :dv]), (got, S[:, :, :dv])):
             x, y = x / low, y / low
             assert np.linalg.norm(x - y) <= 4e-6 * np.linalg.norm(y) + 2.0 ** -149 / low * T * np.sqrt(y.size), np.linalg.norm(x - y) / np.linalg.norm(y)
+
+
+def test_one_decay_per_head_over_many_chunks():
+    """Fifteen chunks under constant decays, operands above zero: the decays' roundings are the same in every chunk and must not add up."""
+    T, H, dk, dv = 900, 8, 64, 64
+    rng = np.random.default_rng(31)
+    q, k, v = (r32(rng.uniform(0, 1, (T, H, d))) for d in (dk, dk, dv))
+    d = r32(np.linspace(0.9, 0.9995, H))
+    state = torch.zeros(1, H, dv, dk, device="cuda")
+    o = ops.state_scan("decay", dev(q.reshape(T, -1)), dev(k.reshape(T, -1)), dev(v.reshape(T, -1)), state, i32([0, T]), i32([0]), 1, H, dk, dv,
+                       chunks=cut([T]), head_decay=dev(d)).double().cpu().numpy().reshape(T, H, dv)
+    ref, S, _, _ = walk("decay", q, k, v, np.broadcast_to(d[None, :, None], (T, H, dk)), np.ones((T, H)), None, np.zeros((H, dk, dv)))
+    # a term of the state passes two roundings per chunk, of the state and of the chunk's decay: the root of 30 times 0.29 of 2^-23 for the oldest, and
+    # what the unit cuts off, 2^-23; the outputs pass up to 63 more, of the decays within a chunk
+    assert np.linalg.norm(state.double().cpu().numpy()[0].transpose(0, 2, 1) - S) <= 3e-7 * np.linalg.norm(S)
+    assert np.linalg.norm(o - ref) <= 4e-7 * np.linalg.norm(ref)
