@@ -1,18 +1,19 @@
 // C = act(A W^T + bias) + res1 + res2 for bfloat16 A [M, K] and W [N, K] on the 5th-generation
 // tensor cores: TMA brings 128-byte-swizzled K-major tiles into a ring of shared-memory
 // stages, one elected thread issues tcgen05.mma (kind::f16, float32 accumulator in TMEM),
-// four warps read the accumulator back with tcgen05.ld and apply the epilogue in 32-bit.
+// the epilogue's warps read the accumulator back with tcgen05.ld and finish in 32-bit.
 //
-// Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner and MMA issuer,
-// warps 2..5 = epilogue (warp w reads TMEM lanes 32 * (w % 4) .. +31).
+// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner and MMA issuer, the others = epilogue
+// (warp w reads TMEM lanes 32 * (w % 4) .. +31): four of them, eight in the persistent kernel.
 //
-// Two kernels:
-//   many tokens (M > 128): rows of A on the MMA's M side, rows of W on its N side; a persistent CTA per SM
-//       walks over 128 x 256 output tiles with two TMEM accumulators, so the epilogue of one tile runs
-//       under the main loop of the next;
+// The kernels:
+//   many tokens (M > 128): rows of A on the MMA's M side, rows of W on its N side; above 128 features CTA
+//       pairs, else (and for grouped products) a persistent CTA per SM, over output tiles with two TMEM
+//       accumulators, so that the epilogue of one tile runs under the main loop of the next;
 //   few tokens (M <= 128): rows of W on the M side and the tokens on the N side (16, 32, 64 or 128), so no
 //       tensor-core row is spent on padding; one CTA per SM streams whole tiles of W, or - for a narrow
-//       N - an even share of all k-blocks (stream-K) with a deterministic reduction of partial tiles.
+//       N - an even share of all k-blocks (stream-K) with a deterministic reduction of partial tiles;
+//   few features: a kernel on mma.sync, blocks of 16 tokens by 16 features.
 // Each output element is accumulated over K in ascending k (in one TMEM cell, or in a fixed sequence of
 // partial sums), so a row's result does not depend on the other rows of the batch.
 //
@@ -70,7 +71,7 @@ template <int BN, bool WIDE> constexpr int p_stages() { return (SMEM_BUDGET_BIG 
 template <int BN, bool WIDE> constexpr int p_smem_bytes() { return p_stages<BN, WIDE>() * stage_bytes<BN>() + 1024 + 512 + (WIDE ? STAGING : 0); }
 
 // One CTA per SM walks over output tiles of 128 x BN (tile t = n_tile * m_tiles + m_tile, so CTAs that
-// run together share rows of W and all of A stays in L2).  Two accumulators in TMEM: while the four
+// run together share rows of W and all of A stays in L2).  Two accumulators in TMEM: while the
 // epilogue warps drain tile i, the MMA warp already accumulates tile i + 1 into the other one, and the
 // TMA producer runs ahead across tile borders through the same ring of stages.
 //
@@ -1023,22 +1024,22 @@ int launch_stream(const void* W, long long ldw, const CUtensorMap& ma, const Epi
 
 // ----------------------------------------------------------------------------- few features
 
-// N <= NARROW features (routers, step sizes, gates per head): a block takes 16 tokens, its sixteen warps (eight above 32 features) the k-range in turns of 32
+// N <= NARROW features (routers, step sizes, gates per head): a block takes 16 tokens and up to 16 features, its sixteen warps the k-range in turns of 32
 // elements each, on mma.sync straight from memory.  Within a turn a lane fetches 16 bytes of two rows of A and of one row of W per eight
-// features; the order of k inside the unit is that of the lanes, the same for both operands.  A warp's runs of a few turns are added with
+// features; the order of k inside the unit is that of the lanes, the same for both operands.  A warp's runs of four turns are added with
 // rounded additions, the warps' sums in the warps' order: nearer to float64 than a chain over all of K in the unit (K = 4,096: 2e-7 of the norm instead
 // of 5e-7 and, at over 128 tokens, 4e-6).
 //
 // Bound by latency: the whole chain is a fetch of rows, a few turns and one sum over the warps.  The tile kernels put such a product on one
-// column of tiles whose CTAs walk all of K one after the other: 8 x 16 x 4096 15.6 us, 3,000 x 16 x 2048 17, 2,048 x 64 x 2048 15.
-constexpr int NARROW = 64;
-template <int NT> constexpr int narrow_warps() { return NT == 8 ? 8 : 16; }
+// column of tiles whose CTAs walk all of K one after the other (figures of both at the rule).  More features per block than 16 made the chain as much longer: 16 x
+// 32 x 16384 76 us instead of 33, 16 x 64 x 4096 27 instead of 14.
+constexpr int NARROW = 64, NARROW_WARPS = 16;
 template <int NT>
-__global__ void __launch_bounds__(32 * narrow_warps<NT>())
+__global__ void __launch_bounds__(32 * NARROW_WARPS)
 gemm_narrow_kernel(const __nv_bfloat16* __restrict__ A, size_t lda, const __nv_bfloat16* __restrict__ W, size_t ldw, const Epilogue ep, int K) {
-    constexpr int COLS = 8 * NT, NARROW_WARPS = narrow_warps<NT>();
+    constexpr int COLS = 8 * NT;
     __shared__ float red[NARROW_WARPS][16][COLS + 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3, m0 = blockIdx.x * 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3, m0 = blockIdx.x * 16, n0 = blockIdx.y * COLS;
     grid_dep_launch();
     grid_dep_wait();
     const __nv_bfloat16* a0 = A + (size_t)(m0 + g) * lda;
@@ -1050,7 +1051,7 @@ gemm_narrow_kernel(const __nv_bfloat16* __restrict__ A, size_t lda, const __nv_b
 #pragma unroll
         for (int z = 0; z < 4; ++z) acc[n][z] = run[n][z] = 0.f;
     const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-    constexpr int TURNS = NT <= 2 ? 4 : 2;              // fetches under way together, and the unit's run: the unit cuts off where it adds
+    constexpr int TURNS = 4;              // fetches under way together, and the unit's run: the unit cuts off where it adds
     for (int k0 = warp * 32; k0 < K; k0 += TURNS * 32 * NARROW_WARPS) {
         uint4 x[TURNS], y[TURNS], w[TURNS][NT];
 #pragma unroll
@@ -1060,7 +1061,7 @@ gemm_narrow_kernel(const __nv_bfloat16* __restrict__ A, size_t lda, const __nv_b
             x[t] = in && has0 ? *reinterpret_cast<const uint4*>(a0 + k) : none;
             y[t] = in && has1 ? *reinterpret_cast<const uint4*>(a1 + k) : none;
 #pragma unroll
-            for (int n = 0; n < NT; ++n) w[t][n] = in && n * 8 + g < ep.N ? *reinterpret_cast<const uint4*>(W + (size_t)(n * 8 + g) * ldw + k) : none;
+            for (int n = 0; n < NT; ++n) w[t][n] = in && n0 + n * 8 + g < ep.N ? *reinterpret_cast<const uint4*>(W + (size_t)(n0 + n * 8 + g) * ldw + k) : none;
         }
 #pragma unroll
         for (int t = 0; t < TURNS; ++t)
@@ -1086,13 +1087,13 @@ gemm_narrow_kernel(const __nv_bfloat16* __restrict__ A, size_t lda, const __nv_b
         float v = 0.f;
 #pragma unroll
         for (int i = 0; i < NARROW_WARPS; ++i) v += red[i][r][n];
-        if (m0 + r < ep.M && n < ep.N) store_out(ep, m0 + r, n, v);
+        if (m0 + r < ep.M && n0 + n < ep.N) store_out(ep, m0 + r, n0 + n, v);
     }
 }
 
 template <int NT>
 int launch_narrow(const void* A, long long lda, const void* W, long long ldw, const Epilogue& ep, int K, cudaStream_t stream) {
-    const cudaError_t e = qs_launch_dependent(gemm_narrow_kernel<NT>, dim3((ep.M + 15) / 16), dim3(32 * narrow_warps<NT>()), 0, stream, (const __nv_bfloat16*)A, (size_t)lda,
+    const cudaError_t e = qs_launch_dependent(gemm_narrow_kernel<NT>, dim3((ep.M + 15) / 16, (ep.N + 8 * NT - 1) / (8 * NT)), dim3(32 * NARROW_WARPS), 0, stream, (const __nv_bfloat16*)A, (size_t)lda,
                                               (const __nv_bfloat16*)W, (size_t)ldw, ep, K);
     if (e != cudaSuccess) return qs_fail(QS_ERR_INTERNAL, "gemm_tc narrow: %s", cudaGetErrorString(e));
     return qs_check_launch("gemm_tc narrow");
@@ -1227,15 +1228,18 @@ QS_API int qs_gemm_tc(void* C, int c_dtype, const void* A, const void* W, const 
     Epilogue ep{C, c_dtype, ldc, bias, bias_dtype, act, (const __nv_bfloat16*)res1, (const __nv_bfloat16*)res2, ldr, M, N};
     CUtensorMap ma, mw;
     int rc;
-    // Few features, microseconds tiles | here (caches flushed): 8 x 16 x 4096 14.3 | 7.2, 128 x 16 x 2048 50 | 5.6, 3,000 x 16 x 2048 13.6 | 7.2, 16,000 x 16 x
-    // 2048 22.3 | 22.3, x 4096 32 | 46; 128 x 64 x 2048 51 | 9.2, 32 x 64 x 512 4.9 | 5.9, 300 x 64 x 512 7.4 | 5.1, x 2048 11.5 | 13.6,
-    // 8 x 64 x 4096 15 | 23.
-    if (M <= 4096 && (N <= 32 || (N <= NARROW && (M > 128 ? K <= 512 : M >= 64 && K <= 4096)))) {
-        if (N <= 8) return launch_narrow<1>(A, lda, W, ldw, ep, K, stream);
-        if (N <= 16) return launch_narrow<2>(A, lda, W, ldw, ep, K, stream);
-        if (N <= 32) return launch_narrow<4>(A, lda, W, ldw, ep, K, stream);
-        return launch_narrow<8>(A, lda, W, ldw, ep, K, stream);
-    }
+    // Few features, by N and K alone up to 128 rows (a row is the same bits in any batch of decoding sequences).  Microseconds, tiles | here (caches
+    // flushed, launches included), 16, 128, 1,000, 2,048 and 4,096 rows:
+    //   16 x 2048  16 | 10, 53 | 10, 18 | 10, 18 | 12, 20 | 16       16 x 16384  39 | 35, 227 | 33, 62 | 33, 66 | 39, 72 | 68
+    //   32 x 512   10 | 8, 12 | 8, 10 | 8, 10 | 10, 11 | 14          32 x 2048   16 | 10, 57 | 10, 14 | 10, 16 | 14, 16 | 20
+    //   32 x 4096  20 | 14, 86 | 12, 23 | 14, 22 | 20, 25 | 33       32 x 16384  35 | 33, 205 | 31, 60 | 35, 64 | 57, 70 | 113
+    //   64 x 512   10 | 8, 12 | 8, 12 | 10, 10 | 14, 12 | 20         64 x 2048   16 | 10, 59 | 10, 16 | 14, 16 | 20, 18 | 31
+    //   64 x 4096  20 | 14, 84 | 12, 22 | 20, 23 | 29, 25 | 47       64 x 16384  36 | 33, 205 | 31, 61 | 55, 66 | 88, 70 | 186
+    // So up to 256 blocks.  48 features lie between 32 and 64; longer K was not measured.  A K of up to 256 takes the tiles' single round whatever the rows
+    // (8,192 x 32 x 64 8): narrow up to 1,024 rows, where both take as long.
+    const long long narrow_blocks = (long long)((M + 15) / 16) * ((N + 15) / 16);
+    if (N <= NARROW && K <= 16384 && narrow_blocks <= 256 && (K > 256 || M <= 1024))
+        return N <= 8 ? launch_narrow<1>(A, lda, W, ldw, ep, K, stream) : launch_narrow<2>(A, lda, W, ldw, ep, K, stream);
     if (M > 128) {
         QS_REQUIRE((M + BM - 1) / BM <= 65535 * 1 && (N + 127) / 128 <= 65535, "gemm_tc: sizes exceed the grid");
         if ((rc = tensor_map(&ma, A, M, K, lda, BM)) != QS_OK) return rc;

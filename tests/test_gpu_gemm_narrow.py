@@ -31,3 +31,13 @@ def test_few_features(M, N, K):
     assert half.dtype == torch.bfloat16
     ref = torch.nn.functional.gelu(x.double() @ w.double().T + bias.double())
     assert ((half.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1.2 * (2 * (K / 16 + 1) + 40) * EPS * size + 1e-6).all()
+
+
+@pytest.mark.parametrize("N,K", [(16, 4096), (24, 8192), (33, 2048), (48, 512), (64, 4096)])
+def test_a_row_is_the_same_bits_in_any_batch_of_up_to_128(N, K):
+    """What the few-token kernels promise their callers holds for few features too."""
+    g = torch.Generator().manual_seed(N)
+    x, w = torch.randn(128, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+    whole = gemm_tc.linear(x, w, out_dtype=torch.float32)
+    for rows in (slice(0, 1), slice(5, 21), slice(0, 63), slice(64, 128), slice(1, 66)):
+        assert torch.equal(gemm_tc.linear(x[rows], w, out_dtype=torch.float32), whole[rows])
