@@ -296,8 +296,9 @@ inline size_t walk_smem(int dkp) {
     return (size_t)(walk_stage(dkp) + dkp * WC + CT * WC + (4 * CT * WC > dkp * WC ? 4 * CT * WC : dkp * WC)) * sizeof(float);
 }
 
-// The walk for more than 128 key channels, by multiply-adds.
-__global__ void __launch_bounds__(WALK)
+// The walk for more than 128 key channels, by multiply-adds.  Two blocks to an SM in the bounds, as many as shared memory holds: left to
+// itself the compiler took 80 registers and spilled, 4,000 tokens of 8 heads of 256 x 128 536 us instead of 466.
+__global__ void __launch_bounds__(WALK, 2)
 delta_walk_kernel(Delta p) {
     extern __shared__ __align__(16) float smem[];
     const int dkp = p.dkp, wp = dkp + 4;
