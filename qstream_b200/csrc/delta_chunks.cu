@@ -13,9 +13,9 @@
 //   delta_walk_kernel     per sequence, head and 16 value columns, the chunks in order: u and the next state, two small products each
 //   delta_output_kernel   per chunk and head, side by side: the outputs
 //
-// All 32-bit; decays only as products of factors up to one.  Three walks of every chunk token by token (what it does to an
+// 32-bit numbers and sums throughout, products on the tensor cores as exact products of bfloat16 terms (terms.cuh); decays only as products of factors up to one.  Three walks of every chunk token by token (what it does to an
 // identity, what it writes from nothing, its outputs) and a product of dk x dk matrices in the prefix stood here before: 2,000 tokens, 16
-// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 375 (the terms 108, the walk 113, the outputs 30).
+// heads of 128 x 128, with their projections, convolutions and norms 1,678 us, now 381 (the terms 108, the walk 118, the outputs 30).
 #include "scan.cuh"
 #include "scan_tiles.cuh"
 #include "term_tiles.cuh"
@@ -59,7 +59,7 @@ __device__ __forceinline__ int at_pass(int c, int t) { return c * CT + (t ^ (((c
 __device__ __forceinline__ void group_wait(int group) { asm volatile("bar.sync %0, 64;" :: "r"(1 + group) : "memory"); }
 
 // TERM_PLANES: K goes on as terms, split once instead of by every block of the walk (W as terms too: six 2-byte stores for two 4-byte ones in
-// the unrolled substitution, 130 us instead of 106).
+// the unrolled substitution, 130 us instead of 108).
 template <bool TERM_PLANES>
 __global__ void __launch_bounds__(TERMS, 2)
 delta_terms_kernel(Delta p) {
@@ -469,8 +469,8 @@ delta_walk_kernel(Delta p) {
 //
 // A chain of 32 steps for 2,000 tokens of 16 heads of 128 x 128.  By multiply-adds a step took 4.2 us (shared memory's pipe: eight 16-byte reads per 32 paired
 // multiply-adds), 133 us in all; with each block splitting W and K for itself 119; now
-// 113; with the sums taken again where the terms did not hold their operands (three calls in the kernel, none on an ordinary path) 120. With sixteen
-// warps, each half of the columns: 119 instead of 113 (64 channels: 4 us less of 73).
+// 113; with the way back for sums whose operands the terms do not hold (calls that no ordinary step makes) 118.  With sixteen warps, each half of
+// the columns: 119 instead of 113 (64 channels: 4 us less of 73).
 // MC channels, 64 or 128; pitches of W and K, of S and u: rows of 16 bytes meet all banks
 constexpr int SP = WC + 8;
 template <int MC> constexpr int mma_walk_smem() { return (2 * 3 * CT * (MC + 8) + 3 * MC * SP + 3 * CT * SP) * 2 + CT * WC * 4; }
@@ -489,20 +489,22 @@ __device__ __forceinline__ void put_two(__nv_bfloat16* at, int term, float x, fl
     for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(at + i * term) = a[i];
 }
 
-// The sums of the walk whose operands the terms did not hold, by multiply-adds: token t's W S, and what the chunk's writes add to channel i.
+// The sums of the walk whose operands the terms did not hold, by multiply-adds: token t's W S, and channel i of the state after chunk c.
 __device__ __noinline__ float plain_held(const Delta& p, size_t unit, int t, int col) {
     const float *w = p.W + (unit * CT + t) * p.dkp, *S = p.start + unit * p.dk * p.dvp + col;
     float sum = 0.f;
     for (int i = 0; i < p.dk && sum == sum; ++i) sum = fmaf(w[i], S[(size_t)i * p.dvp], sum);        // NaN stays NaN
     return sum;
 }
-__device__ __noinline__ float plain_written(const Delta& p, size_t unit, int t0, int n, int h, int i, int col) {
+__device__ __noinline__ float plain_state(const Delta& p, int c, int h, int i, int col) {
+    const size_t unit = (size_t)c * p.H + h;
+    const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0;
     float sum = 0.f, run = 1.f;
     for (int t = n - 1; t >= 0 && sum == sum; --t) {
         sum = fmaf(p.k[(size_t)(t0 + t) * p.ldk + h / p.group * p.dk + i] * run, p.U[(unit * CT + t) * p.dvp + col], sum);
         run *= p.g[(size_t)(t0 + t) * p.ldg + h * p.dk + i];
     }
-    return sum;
+    return fmaf(p.decay[unit * p.dkp + i], p.start[(unit * p.dk + i) * p.dvp + col], sum);
 }
 
 template <int MC>
@@ -551,12 +553,7 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
     // column none, what is small counts only where they are) and at the end.
     auto mend_state = [&](int c) {
         if (c < c0 || !whole(c)) return;
-        const size_t unit = (size_t)c * p.H + h;
-        const int t0 = p.chunk_start[c], n = p.chunk_start[c + 1] - t0;
-        each([&](float& v, int i, int col) {
-            if (!held(v) && i < p.dk && col < n_cols)
-                v = fmaf(p.decay[unit * dkp + i], p.start[(unit * p.dk + i) * p.dvp + col0 + col], plain_written(p, unit, t0, n, h, i, col0 + col));
-        });
+        each([&](float& v, int i, int col) { if (!held(v) && i < p.dk && col < n_cols) v = plain_state(p, c, h, i, col0 + col); });
     };
     const int w_at = tid / ROW, w_i = tid % ROW * 4;
     auto fetch_w = [&](int c) {
@@ -748,7 +745,9 @@ delta_walk_mma_kernel(const __grid_constant__ Delta p) {
         __syncthreads();
         copy_k(c + 1);
     }
-    mend_state(c1 - 1);
+    uint32_t odd_state = 0;
+    each([&](float& v, int, int) { odd_state = max(odd_state, beyond(v)); });
+    if (odd_state > HELD) mend_state(c1 - 1);
     each([&](float& v, int i, int col) { if (i < p.dk && col < n_cols) own[(size_t)col * p.dk + i] = v; });
 }
 
