@@ -17,8 +17,10 @@
 // with all of them behind the barrier; two k-blocks under way for few tokens: no gain, more registers.  Few rows (up to 64 or so) are bound by the latency of that
 // chain: 64 x 6144 x 2048 36 us (60).
 //
-// Error against float64, 2-norm, normal numbers, this | CUDA cores: K = 256 8.8e-8 | 2.9e-7, 2,048 1.1e-7 | 2.9e-7, 8,192 1.5e-7 |
-// 3.1e-7.
+// Error against float64, 2-norm, this | CUDA cores, K = 256, 2,048, 8,192: normal numbers 8.7e-8 | 2.9e-7, 1.1e-7 | 2.9e-7, 1.2e-7 | 3.1e-7;
+// activations of one sign (squared ReLU) against normal numbers 9.8e-8 | 2.0e-7, 1.2e-7 | 2.1e-7, 1.3e-7 | 2.3e-7.  The unit cuts off where it adds: operands
+// that are both of one sign, which a layer's are not, are 7.5e-8 to 8.5e-8 too small on average, 8.7e-8 | 2.2e-7, 9.2e-8 | 9.1e-8, 9.3e-8 | 8.7e-8
+// off in all (uniform), 9.6e-8 | 1.7e-7, 1.0e-7 | 7.5e-8, 1.0e-7 | 8.4e-8 (squared ReLU).
 //
 // The order of the sums depends on N and K alone: runs of 64 products in ascending k within a part of K, the parts' sums in ascending order
 // (`parts_of`).  A row's result is the same bits whatever else is in the batch, one row or thousands.  What the batch decides is who does the

@@ -29,6 +29,25 @@ def test_product_against_float64(M, N, K):
     assert torch.equal(got, ops.linear_split(x, w))
 
 
+@pytest.mark.parametrize("K", [256, 4096, 16384])
+def test_operands_of_one_sign(K):
+    """The unit cuts off where it adds: with operands that are both of one sign, which add up without cancelling, that is a bias.  A run's last four steps
+    are what counts: at a quarter, a half, three quarters and all of its sum each cuts off an ulp (2^-23) at most, half of one on average."""
+    g = torch.Generator().manual_seed(K)
+    for x, w in ((torch.rand(300, K, generator=g), torch.rand(512, K, generator=g)),
+                 (torch.relu(torch.randn(300, K, generator=g)) ** 2, torch.rand(512, K, generator=g)),
+                 (torch.sigmoid(torch.randn(300, K, generator=g)), torch.randn(512, K, generator=g).abs())):
+        x, w = x.cuda(), w.cuda()
+        ref = x.double() @ w.double().T
+        off = (ops.linear_split(x, w).double() - ref) / ref
+        runs = -(-K // 64)
+        assert off.abs().max() <= 2.5 * 2.0 ** -23 + (runs + 4) * EPS
+        # 2.5 halves of an ulp, an ulp being 0.72 of 2^-23 of a number on average, and the runs' roundings around it
+        assert -1.25 * 2.0 ** -23 <= off.mean() <= 0.1 * 2.0 ** -23
+        assert off.square().mean().sqrt() <= 1.25 * 2.0 ** -23
+    gemm_tc.check_status("cuda:0")
+
+
 def test_rows_apart_and_epilogue():
     g = torch.Generator().manual_seed(3)
     for M, N, K in ((40, 300, 2048), (200, 512, 260)):
