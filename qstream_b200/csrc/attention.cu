@@ -735,7 +735,8 @@ attention_tile_kernel(float* __restrict__ out, const float* __restrict__ q, size
 //   24         25 | 23   29 | 61   37 | 104  98 | 373   330 | 1,401         31 | 68    37 | 246   135 | 2,021  459 | 7,581
 //   32         18 | 29   27 | 63   37 | 109  88 | 377   287 | 1,401         22 | 100   37 | 317   121 | 2,409  383 | 9,252
 // (fewer than 32 rows behind no keys: measured with 64 rows to a block).  A prompt of 2,000 tokens beside 64 sequences that bring one token
-// behind 2,000 keys: 2.0 ms, 17.1 with a warp per query, 28.9 with tiles cut every 64 rows, whose blocks walk sequence after sequence.
+// behind 2,000 keys: 2.0 ms, 17.1 with a warp per query, 28.9 with tiles of 64 rows cut without a look at the sequences, which their blocks walk one after the
+// other.
 constexpr int TILE_ROWS = 16, TILE_ROWS_SHORT = 32, TILE_KEYS = 33;
 bool tiles_serve(long long rows, int n_seq, int longest) {
     return n_seq > 0 && rows >= (longest == 0 || longest >= TILE_KEYS ? TILE_ROWS : TILE_ROWS_SHORT) * (long long)n_seq;
@@ -758,7 +759,7 @@ int launch_attention(void* out, const void* q, long long ldo, long long ldq, con
         ((uintptr_t)k_cache % 16) == 0 && ((uintptr_t)v_cache % 16) == 0) {
         const int ng = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4);
         const size_t bytes = tile_smem_bytes(dh, ng);
-        if (n_seq == 1) seq_start = nullptr;            // cut every 64 rows all the same
+        if (n_seq == 1) seq_start = nullptr;            // cut every 32 rows all the same
         const int blocks = seq_start ? T_tokens / TQ + n_seq + 1 : (T_tokens + TQ - 1) / TQ;
         cudaError_t e = cudaSuccess;
         // the limit is set to what the widest heads need, whatever these need: another thread's launch may come between it and this one's

@@ -15,7 +15,8 @@
 // The products of 32-bit numbers run on tcgen05 as products of bfloat16 terms (terms.cuh), in runs of 64 whose sums are added outside; against
 // float64 they are nearer than the multiply-adds that stood here before (o, 2-norm: state-space form 1.4e-7 instead of 1.5e-7, gated memory
 // 1.4e-7 instead of 1.9e-7; decay per head, over 900 tokens, 1.4e-7 instead of 3.4e-7).  q, k and v that come as bfloat16 are one term: q k^T is then one product instead
-// of six.  Bound by each block's chain of fetch, split, barrier, MMAs and stores at two blocks per SM (leaving out the MMAs: 63 of 76 us
+// of six.  Bound by each block's chain of fetch, split, barrier, MMAs and stores at two blocks per SM, one for what chunks add under a decay per channel with float32 operands (117 KB of
+// tiles and decays; leaving out the MMAs: 63 of 76 us
 // for the outputs, 42 of 47 for what the chunks add, at 4,096 tokens of 16 heads of 128 x 128, float32 operands); the split needs half of
 // the issue slots.  On mma.sync the same products took 138 and 59 us, multiply-adds 139 and 66.
 //
@@ -97,9 +98,6 @@ constexpr int TILE_THREADS = 256;                       // eight warps: a quarte
 
 // ----------------------------------------------------------------------------- what a chunk adds
 
-// A block takes 64 NC value columns of one head's state, up to 128 key channels at a time: added[i][col] = sum_j kw_j[i] v_j[col], the
-// tokens on the sum's side, kw_j = b_j k_j times the decays behind token j.  kw in three terms, v in VT (one where it comes as bfloat16).
-// Columns on the TMEM lanes, so that a warp writes 32 neighbouring ones.
 // The sum of channel i over the chunk's tokens, from the last back, by multiply-adds; `v_at` < 0: of values that are all one.  `s_w`: the tokens' weights and
 // decays behind them, where there is one decay per head.
 template <typename TI, int MODE>
@@ -122,6 +120,10 @@ __device__ __noinline__ void mend_added(const Scan& p, float* to, int rows, int 
 
 template <typename TI> constexpr int added_smem() { return 1024 + (3 + (sizeof(TI) == 2 ? 1 : 3)) * 2 * TILE; }
 
+// A block takes 128 value columns of one head's state, up to 128 key channels at a time: added[i][col] = sum_j kw_j[i] v_j[col], the
+// tokens on the sum's side, kw_j = b_j k_j times the decays behind token j.  kw in three terms, v in VT (one where it comes as bfloat16).
+// Columns on the TMEM lanes, so that a warp writes 32 neighbouring ones.
+//
 // Three blocks per SM for the state-space form in bfloat16 (2,048 tokens of 64 heads of 128 x 64: 64 -> 56 us); in the other forms they were slower
 // (gated memory, 1,000 tokens: 79 -> 97 us for the scan; decay per head 38 -> 40).
 template <typename TI, int MODE>
@@ -297,7 +299,7 @@ added_state_kernel(const __grid_constant__ Scan p) {
 
 // ----------------------------------------------------------------------------- a chunk's outputs, a decay per key channel
 
-// The same with a decay per token and key channel: a block takes the 64 tokens of a chunk and 128 value columns of one head.  The weights P come from
+// A decay per token and key channel: a block takes the 64 tokens of a chunk and 128 value columns of one head.  The weights P come from
 // multiply-adds: pairs of tokens within a block of 16 with their decays as running products (a warp a block and half of the channels), a block's tokens
 // against all earlier ones as products of q times the decays since the block's start with k taken on to it (a warp eight channels).  The products with the
 // state and with the values run on tcgen05, in three terms per number (one for values that come as bfloat16).

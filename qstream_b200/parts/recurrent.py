@@ -42,15 +42,15 @@ from .linear import linear
 
 
 CHUNK_TOKENS = 64            # a long prompt is cut into chunks of this many tokens that run side by side
-# The longest sequence of a step from which the chunks serve: all forms gain there, with one sequence as with several.  Shorter prompts would
-# gain in some of them already.  Microseconds of the scan, walk | chunks (with their products on the CUDA cores; on the
-# tensor cores they take up to a third less), one sequence at 64, 128 and 256 tokens, then four sequences:
-#   decay per head, 16 heads of 128 x 128   59 | 44, 111 | 44, 213 | 70      53 | 83,  96 | 85,  182 | 95
-#   per channel (gla), 16 of 64 x 128       78 | 93, 147 | 97, 289 | 101     78 | 99,  147 | 101, 285 | 103
-#   per channel (wkv), 16 of 64 x 64        82 | 46, 156 | 46, 306 | 44      82 | 58,  156 | 56, 305 | 58
-#   state-space form, 64 of 128 x 64        70 | 48, 129 | 60, 254 | 67      74 | 79,  135 | 87, 260 | 142
-#   gated memory, 4 of 256 x 256            63 | 75, 117 | 81, 225 | 81      68 | 153, 127 | 151, 246 | 152
-#   delta rule, 16 of 128 x 128             72 | 79, 137 | 85, 264 | 103     72 | 101, 131 | 122, 254 | 179
+# The longest sequence of a step from which the chunks serve: all forms gain there by far, with one sequence as with several.  Shorter prompts would
+# gain too: from 128 tokens on in every form, from 64 in all but the two with the longest chains.  Microseconds of the scan (caches flushed, launches
+# included), walk | chunks, one sequence at 64, 128 and 256 tokens, then four sequences:
+#   decay per head, 16 heads of 128 x 128   59 | 29, 111 | 31, 213 | 33      53 | 39,  96 | 43, 182 | 45
+#   per channel (gla), 16 of 64 x 128       72 | 45, 133 | 47, 260 | 47      72 | 49, 133 | 53, 258 | 59
+#   per channel (wkv), 16 of 64 x 64        78 | 45, 148 | 45, 289 | 49      78 | 47, 150 | 49, 291 | 59
+#   state-space form, 64 of 128 x 64        70 | 33, 133 | 33, 256 | 39      74 | 47, 137 | 58, 260 | 86
+#   gated memory, 4 of 256 x 256            63 | 63, 117 | 66, 227 | 68      68 | 76, 127 | 74, 246 | 82
+#   delta rule, 16 of 128 x 128             74 | 64, 137 | 66, 266 | 74      72 | 80, 133 | 96, 256 | 141
 CHUNKED_FROM = 256
 
 
