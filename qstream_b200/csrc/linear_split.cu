@@ -11,11 +11,11 @@
 //
 // Bound by the tensor unit where there are many tiles (2048 x 16384 x 4096: 1,138 us, 240 TFLOP/s of products of 32-bit numbers, six times as
 // many in the unit: 0.89 of its measured peak; the CUDA-core product takes 5,155) and else by the chain of a
-// k-block: fetch, split, barrier of the pair, MMAs, sums (700 x 6144 x 2048: 96 us, 412 there; leaving out the loads gives 84, the sums'
-// way to registers 84, all but barriers, stores and MMAs 82).  Loads four rows of whole 128-byte lines at a time: eight rows of 32 bytes
+// k-block: fetch, split, barrier of the pair, MMAs, sums (700 x 6144 x 2048 with K in one part: 96 us, 412 there; leaving out the loads gives 84, the sums'
+// way to registers 84, all but barriers, stores and MMAs 82), and by a unit's two ends, where the pipeline fills and drains (9 us at 256 tokens).  Loads four rows of whole 128-byte lines at a time: eight rows of 32 bytes
 // per lane took 40 wavefronts instead of 4 each; loads set out as soon as their registers are free: 96 against 102 us
 // with all of them behind the barrier; two k-blocks under way for few tokens: no gain, more registers.  Few rows (up to 64 or so) are bound by the latency of that
-// chain: 64 x 6144 x 2048 36 us (60).
+// chain, W's lines in L2 three k-blocks ahead of the loads (16 x 14336 x 2048 62 -> 57 us; six ahead 59): 64 x 6144 x 2048 35 us (57).
 //
 // Error against float64, 2-norm, this | CUDA cores, K = 256, 2,048, 8,192: normal numbers 8.7e-8 | 2.9e-7, 1.1e-7 | 2.9e-7, 1.2e-7 | 3.1e-7;
 // activations of one sign (squared ReLU) against normal numbers 9.8e-8 | 2.0e-7, 1.2e-7 | 2.1e-7, 1.3e-7 | 2.3e-7.  The unit cuts off where it adds: operands
